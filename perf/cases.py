@@ -250,6 +250,97 @@ def work(case):
     return {"bytes": m * (9 * case["inter"] + 8) + 12 * case["inter"], "flops": 10.0 * m * case["inter"]}
 
 
+# ------------------------------------------------------------------------------------------ the same in 64 bits
+def _narrow64(v):
+    """fp32 -> fp16 -> int8 of the operators, ties to even both times, on values held in 64 bits."""
+    return v.to(torch.float16).double().round().clamp_(-128.0, 127.0)
+
+
+def _quant64(v):
+    amax = v.abs().amax(-1, keepdim=True).clamp_min(1e-12)
+    return _narrow64(v * (127.0 / amax)), (amax / 127.0).squeeze(-1)
+
+
+def _norm64(s):
+    """(int8 values, residual sum, per-row scale) of add_rms_norm_dynamic_quant."""
+    total = s["x"].double() + s["residual"].double()
+    z = total * s["gamma"].double()
+    rstd = (total.square().mean(-1, keepdim=True) + 1e-6).rsqrt()
+    q, scale = _quant64(z * rstd)
+    return q, total, scale
+
+
+def _matmul64(q, q_scale, w, w_scale, bias=None):
+    out = (q @ w.double()) * w_scale.double() * q_scale.unsqueeze(-1)
+    return out if bias is None else out + bias.double()
+
+
+def _swiglu64(gate, up):
+    return gate * torch.sigmoid(gate) * up
+
+
+def exact(case, seed):
+    """The floating results of `run` on the same inputs, worked out by torch in 64 bits; None beside int8 and index outputs."""
+    s = prepare(case, seed)
+    kind = s["kind"]
+    if kind == "linear":
+        q, qs = _quant64(s["x"].double())
+        return _matmul64(q, qs, s["w"], s["scale"], s["bias"])
+    if kind == "ffn":
+        q, total, qs = _norm64(s)
+        h = _matmul64(q, qs, s["w_up"], s["s_up"], s["b_up"]).to(s["x"].dtype).double()
+        gate, up = h.chunk(2, -1)
+        a, a_scale = _quant64(_swiglu64(gate, up))
+        return _matmul64(a, a_scale, s["w_down"], s["s_down"], s["b_down"]), total
+    if kind == "norm":
+        _, total, scale = _norm64(s)
+        return None, total, scale
+    if kind == "router":
+        return torch.softmax(s["x"].double(), -1).topk(s["topk"], -1).values, None, None
+    if kind == "up":
+        scale = torch.empty(case["rows"], dtype=torch.float64, device="cuda")
+        first = 0
+        for e, end in enumerate(s["ends"]):
+            h = _matmul64(s["x"][first:end].double(), s["x_scale"][first:end].double(), s["w"][e], s["s_up"][e])
+            gate, up = h.chunk(2, -1)
+            scale[first:end] = _quant64(_swiglu64(gate, up))[1]
+            first = end
+        return None, scale
+    if kind == "moe":
+        q, total, qs = _norm64(s)
+        shard, out = s["layer"].shard, torch.zeros_like(total)
+        for e in range(case["experts"]):
+            token, slot = torch.nonzero(s["idx"] == e, as_tuple=True)
+            if token.numel() == 0:
+                continue
+            gate, up = _matmul64(q[token], qs[token], shard.w_up[e], shard.s_up[e]).chunk(2, -1)
+            a, a_scale = _quant64(_swiglu64(gate, up))
+            y = _matmul64(a, a_scale, shard.w_down[e], shard.s_down[e])
+            out.index_add_(0, token, y * s["probs"][token, slot].double().unsqueeze(-1))
+        return out, total
+    if kind == "grouped":
+        out = torch.empty(case["rows"], case["n"], dtype=torch.float64, device="cuda")
+        first = 0
+        for e, end in enumerate(s["ends"]):
+            out[first:end] = s["x"][first:end].double() @ s["w"][e].double()
+            if s["bias"] is not None:
+                out[first:end] += s["bias"][e].double()
+            first = end
+        return [out]
+    if kind == "exchange":
+        cells = s["counts"].numel()
+        cell = torch.repeat_interleave(torch.arange(cells, device="cuda"), s["counts"].flatten())
+        order = torch.argsort(cell % case["experts"], stable=True)
+        tokens, k = s["probs"].shape
+        combined = s["skip"].double()
+        for j in range(k):
+            combined += s["rows"][s["pos"].view(k, tokens)[j].long()].double() * s["probs"][:, j:j + 1].double()
+        return (None, s["x_scale"][order].double(), None, None), combined
+    h = s["x"].double() * s["w_scale"].double() * s["x_scale"].double().unsqueeze(-1)
+    gate, up = h.chunk(2, -1)
+    return None, _quant64(_swiglu64(gate, up * s["smooth"].double()))[1]
+
+
 # About four times what the path's results differ by from the same operation sequence carried out in 64 bits (2-norm,
 # largest, and share of int8 values or indices that change), taken at reduced sizes of every kind.
 _FP32_RESULTS = {"rel": 4e-7, "max": 1.5e-6, "differ": 5e-6}  # fp32 scales / probabilities beside int8 values or indices
