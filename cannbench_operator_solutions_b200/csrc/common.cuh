@@ -140,6 +140,136 @@ __device__ __forceinline__ float canonical_silu(float l)
 }
 
 // ---------------------------------------------------------------------------
+// Pairs of fp32 values in one 64-bit register: sm_100 runs mul / add / fma on both halves in one issue slot, each
+// half rounded like the scalar instruction.  The exponential and the quotient below are issue bound wherever they
+// are used, so they are written on pairs.  Never feed mul2 to add2: the assembler contracts a pair multiplication
+// and the pair addition that uses it into one rounding, whatever the rounding modifiers say.
+// ---------------------------------------------------------------------------
+using f32x2 = unsigned long long;
+
+__device__ __forceinline__ f32x2 pair(float lo, float hi)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+
+__device__ __forceinline__ f32x2 pair(float both) { return pair(both, both); }
+
+__device__ __forceinline__ void unpair(f32x2 v, float& lo, float& hi)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// e = -canonical_expf(-g) of N pairs, bit for bit, for |g| <= EXP2_MAX_ABS (the result is then a normal number, so
+// the power of two is one integer add to the exponent field).  A NaN half gives an arbitrary value: callers
+// multiply something by g that carries the NaN.  Every step is canonical_expf's with the sign of the argument or of
+// the result folded into the constants, which round-to-nearest does not see.  The pairs go through each step
+// together: a pair instruction has no immediate operand, so a constant costs registers or moves, and N pairs share
+// them.
+constexpr float EXP2_MAX_ABS = 80.0f;
+
+template <int N>
+__device__ __forceinline__ void neg_exp_neg2(const f32x2 (&g)[N], f32x2 (&e)[N])
+{
+    f32x2 t[N], r[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        float g0, g1;
+        unpair(g[i], g0, g1);
+        // two scalar products: see above
+        t[i] = add2(pair(__fmul_rn(g0, 1.44269504088896341f), __fmul_rn(g1, 1.44269504088896341f)), pair(12582912.0f));
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        e[i] = add2(t[i], pair(-12582912.0f));
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        r[i] = fma2(e[i], pair(-0.693359375f), g[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        r[i] = fma2(e[i], pair(2.12194440e-4f), r[i]);  // minus the r of canonical_expf(-g)
+    }
+    constexpr float C[6] = {1.9875691500e-4f, -1.3981999507e-3f, 8.3334519073e-3f,
+                            -4.1665795894e-2f, 1.6666665459e-1f, -5.0000001201e-1f};
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        e[i] = pair(C[0]);
+    }
+#pragma unroll
+    for (int k = 1; k < 6; ++k) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            e[i] = fma2(e[i], r[i], pair(C[k]));
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        e[i] = add2(fma2(e[i], mul2(r[i], r[i]), r[i]), pair(-1.0f));
+        float e0, e1, t0, t1;
+        unpair(e[i], e0, e1);
+        unpair(t[i], t0, t1);
+        e[i] = pair(__int_as_float(__float_as_int(e0) - (__float_as_int(t0) << 23)),
+                    __int_as_float(__float_as_int(e1) - (__float_as_int(t1) << 23)));
+    }
+}
+
+__device__ __forceinline__ float approx_reciprocal(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// q = n / -nd of N pairs, correctly rounded, for -nd in [1, 2^116] and |n| in [2^-60, 2^100] (a zero numerator
+// gives a zero whose sign may differ): one Newton step on the approximate reciprocal, then one correction of the
+// quotient by its exactly computed remainder (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990).  Before the last rounding the quotient is within 2^-46 of n / d; the quotients
+// that lie so close to the middle of two floats are, for each d, a handful of numerators, and all of them over all
+// 2^23 significands d (5.6e8 divisions) agree with the IEEE division.
+template <int N>
+__device__ __forceinline__ void quotient2(const f32x2 (&n)[N], const f32x2 (&nd)[N], f32x2 (&q)[N])
+{
+    f32x2 y[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        float d0, d1;
+        unpair(nd[i], d0, d1);
+        y[i] = pair(approx_reciprocal(-d0), approx_reciprocal(-d1));
+        q[i] = fma2(nd[i], y[i], pair(1.0f));
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        y[i] = fma2(q[i], y[i], y[i]);
+        q[i] = mul2(n[i], y[i]);
+        q[i] = fma2(fma2(nd[i], q[i], n[i]), y[i], q[i]);
+    }
+}
+
+// ---------------------------------------------------------------------------
 // fp32 -> int8 narrowing.
 //
 // "As written" (the reference's two casts): fp32 -> fp16 RNE, then fp16 ->

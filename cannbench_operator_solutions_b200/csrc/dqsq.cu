@@ -17,9 +17,10 @@
 // can differ by one int8 step on the rare element where the two roundings disagree.  exp is the canonical fp32
 // sequence shared with the CPU oracle; a NaN activation quantises to 0.
 //
-// Mapping: one CTA of 256 threads per row (grid-stride).  Thread t owns 16-byte chunks t, t+256, ... of both
-// halves and keeps the fp32 results in registers between the row maximum and the quantisation, so x is read
-// once and y written once: 8H + H + 4 bytes per row for int32 input, 4H + H + 4 for 16-bit input.
+// Mapping: one CTA per row at a time (grid-stride, one wave), one or two 16-byte chunks of each half per thread and
+// as many threads as that takes.  The fp32 results stay in registers between the row maximum and the quantisation,
+// so x is read once and y written once: 8H + H + 4 bytes per row for int32 input, 4H + H + 4 for 16-bit input; the
+// next row's chunks are requested before the barrier of the present one.
 #include "common.cuh"
 
 namespace w8a8 {
@@ -27,7 +28,9 @@ namespace w8a8 {
 constexpr int DQSQ_X_I32 = 0;
 constexpr int DQSQ_X_F16 = 1;
 constexpr int DQSQ_X_BF16 = 2;
-constexpr int DQSQ_THREADS = 256;
+constexpr int DQSQ_THREADS = 256;       // any-length kernel
+constexpr int DQSQ_MAX_THREADS = 1024;  // register-resident rows
+constexpr int DQSQ_PAIR_THREADS = 576;  // up to here two CTAs share an SM's registers at 56 per thread
 
 template <int XT>
 struct DqsqChunk {
@@ -91,41 +94,71 @@ __device__ __forceinline__ float dqsq_element(float a, float b, float wa, float 
     return __fdiv_rn(__fmul_rn(a, b), den);
 }
 
-// The same element with the two halves named by role (g: the half the gate is formed from, o: the other one) and the
+// N elements with the two halves named by role (g: the half the gate is formed from, o: the other one) and the
 // smooth scale always applied (1 when the caller gave none; a multiplication by 1 is exact): a * b commutes, and
-// gate * -1 is a sign flip, so the bits are those of dqsq_element without its per-element case distinctions.
-template <int XT>
-__device__ __forceinline__ float dqsq_element_by_role(float g, float o, float wg, float wo, float qs, float as)
+// gate * -1 is a sign flip, so the bits are those of dqsq_element.  Two at a time by the pair forms where all of
+// them are in range, which only gates beyond +-80 or products beyond 2^100 are not.  (Products below 2^-60 may come
+// out one unit off there: at most 1e-18, they neither reach the scale, which is at least 1e-12, nor any value but 0.)
+template <int XT, int N>
+__device__ __forceinline__ void dqsq_elements(const float (&g)[N], const float (&o)[N], const float (&wg)[N],
+                                              const float (&wo)[N], const float (&qs)[N], float as, float (&out)[N])
 {
-    if constexpr (XT == DQSQ_X_I32) {
-        g = __fmul_rn(g, wg);
-        o = __fmul_rn(o, wo);
+    f32x2 gate[N / 2], num[N / 2], den[N / 2], res[N / 2];
+    float g_max = 0.0f, n_max = 0.0f;
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+        f32x2 op = pair(o[2 * i], o[2 * i + 1]);
+        gate[i] = pair(g[2 * i], g[2 * i + 1]);
+        if constexpr (XT == DQSQ_X_I32) {
+            gate[i] = mul2(mul2(gate[i], pair(wg[2 * i], wg[2 * i + 1])), pair(as));
+            op = mul2(op, pair(wo[2 * i], wo[2 * i + 1]));
+        }
+        op = mul2(op, pair(qs[2 * i], qs[2 * i + 1]));
+        if constexpr (XT == DQSQ_X_I32) {
+            op = mul2(op, pair(as));
+        }
+        num[i] = mul2(gate[i], op);
+        float a0, a1, n0, n1;
+        unpair(gate[i], a0, a1);
+        unpair(num[i], n0, n1);
+        g_max = fmaxf(g_max, fmaxf(fabsf(a0), fabsf(a1)));
+        n_max = fmaxf(n_max, fmaxf(fabsf(n0), fabsf(n1)));
     }
-    o = __fmul_rn(o, qs);
-    if constexpr (XT == DQSQ_X_I32) {
-        g = __fmul_rn(g, as);
-        o = __fmul_rn(o, as);
+    neg_exp_neg2<N / 2>(gate, den);
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+        den[i] = add2(den[i], pair(-1.0f));
     }
-    const float den = __fadd_rn(canonical_expf(-g), 1.0f);
-    return __fdiv_rn(__fmul_rn(g, o), den);
+    quotient2<N / 2>(num, den, res);
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+        unpair(res[i], out[2 * i], out[2 * i + 1]);
+    }
+    if (!(g_max <= EXP2_MAX_ABS && n_max <= 1.2676506e30f)) {
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) {
+            float a0, a1, n0, n1;
+            unpair(gate[i], a0, a1);
+            unpair(num[i], n0, n1);
+            out[2 * i] = __fdiv_rn(n0, __fadd_rn(canonical_expf(-a0), 1.0f));
+            out[2 * i + 1] = __fdiv_rn(n1, __fadd_rn(canonical_expf(-a1), 1.0f));
+        }
+    }
 }
 
-__device__ __forceinline__ float dqsq_block_max(float m, float* s_red, int parity)
+// `slots`: two sets of one float per warp of the CTA, used in turn
+__device__ __forceinline__ float dqsq_block_max(float m, float* slots, int parity)
 {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        m = fmaxf(m, __shfl_xor_sync(FULL_MASK, m, off));
-    }
-    float* slot = s_red + parity * (DQSQ_THREADS / 32);
-    if ((threadIdx.x & 31) == 0) {
-        slot[threadIdx.x >> 5] = m;
+    const int warps = static_cast<int>(blockDim.x >> 5);
+    const int lane = threadIdx.x & 31;
+    // non-negative floats order like their bit patterns
+    const int own = __reduce_max_sync(FULL_MASK, __float_as_int(m));
+    float* slot = slots + parity * 32;
+    if (lane == 0) {
+        slot[threadIdx.x >> 5] = __int_as_float(own);
     }
     __syncthreads();
-#pragma unroll
-    for (int w = 0; w < DQSQ_THREADS / 32; ++w) {
-        m = fmaxf(m, slot[w]);
-    }
-    return m;
+    return __int_as_float(__reduce_max_sync(FULL_MASK, lane < warps ? __float_as_int(slot[lane]) : 0));
 }
 
 // out / s, or out * (1 / s) with `s` already holding the reciprocal
@@ -135,7 +168,7 @@ __device__ __forceinline__ float dqsq_scaled(float o, float s, bool divide)
 }
 
 template <bool DIVIDE>
-__device__ __forceinline__ uint32_t dqsq_quant4(const float* o, float s, bool direct)
+__device__ __forceinline__ uint32_t dqsq_quant4_general(const float* o, float s, bool direct)
 {
     constexpr bool divide = DIVIDE;
     float v[4];
@@ -159,71 +192,133 @@ __device__ __forceinline__ uint32_t dqsq_quant4(const float* o, float s, bool di
     return packed;
 }
 
-// Register-resident rows: H a multiple of the chunk length, at most DQSQ_THREADS * EL * CPT long.
-template <int XT, int CPT, bool DIVIDE>
-__global__ void __launch_bounds__(DQSQ_THREADS, (CPT <= 2) ? 4 : 1) dqsq_rows_kernel(const void* __restrict__ x,
-                                                                 const float* __restrict__ weight_scale,
-                                                                 const float* __restrict__ activation_scale,
-                                                                 const float* __restrict__ quant_scale,
-                                                                 int8_t* __restrict__ y, float* __restrict__ scale,
-                                                                 int64_t M, int64_t H, int left, int direct, int)
+// Four results quantised the way narrow4_fp16_fast does, without the clamp: no |out| exceeds the row maximum, so
+// every quotient is at most 127 (1 + 2^-22) and rounds to at most 127 in fp16.  `inv` is RN(1 / s).  DIVIDE: out / s
+// by one remainder correction of out * inv (Markstein, as in quotient2; s is the same for the whole row, so the
+// reciprocal costs nothing here).  A NaN leaves a bit set in the fp16 sum that no value from 1408 to 1663 has.
+template <bool DIVIDE>
+__device__ __forceinline__ uint32_t dqsq_quant4(const float* o, float s, float inv, bool regular, bool direct)
+{
+    if (!regular) {
+        return dqsq_quant4_general<DIVIDE>(o, DIVIDE ? s : inv, direct);
+    }
+    __half2 h[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const f32x2 v = pair(o[2 * j], o[2 * j + 1]);
+        f32x2 q = mul2(v, pair(inv));
+        if constexpr (DIVIDE) {
+            q = fma2(fma2(q, pair(-s), v), pair(inv), q);
+        }
+        float q0, q1;
+        unpair(q, q0, q1);
+        h[j] = __hadd2(__floats2half2_rn(q0, q1), __floats2half2_rn(1536.0f, 1536.0f));
+    }
+    const uint32_t h01 = *reinterpret_cast<const uint32_t*>(&h[0]), h23 = *reinterpret_cast<const uint32_t*>(&h[1]);
+    if (((h01 | h23) & 0x10001000u) != 0) {
+        return dqsq_quant4_general<DIVIDE>(o, DIVIDE ? s : inv, direct);
+    }
+    return __byte_perm(h01, h23, 0x6420);
+}
+
+// Register-resident rows: H a multiple of the chunk length, at most blockDim.x * EL * CPT long.
+//
+// Bound: issue slots (44 warp instructions per 32 elements against 73 with a scalar exponential and the compiler's
+// division), then HBM.  int32 [16384, 4096] (302 MB): 64 us, was 83 - 85; fp16 [1531, 18432] (70 MB): 24 us, was 58
+// with a fixed 256 threads per row (eight chunks per thread, 44 % of them past the row's end).
+template <int XT, int CPT, bool DIVIDE, int MAX_THREADS>
+__global__ void __launch_bounds__(MAX_THREADS, MAX_THREADS <= DQSQ_PAIR_THREADS ? 2 : 1)
+    dqsq_rows_kernel(const void* __restrict__ x, const float* __restrict__ weight_scale,
+                     const float* __restrict__ activation_scale, const float* __restrict__ quant_scale,
+                     int8_t* __restrict__ y, float* __restrict__ scale, int64_t M, int64_t H, int left, int direct, int)
 {
     using C = DqsqChunk<XT>;
     constexpr int EL = C::EL;
-    __shared__ float s_red[2 * (DQSQ_THREADS / 32)];
+    constexpr int N = CPT * EL;
+    constexpr int GROUP = (EL == 4) ? CPT : 1;  // chunks that go through the arithmetic together: 8 elements
+    constexpr int GN = GROUP * EL;
+    constexpr size_t ELEM = (XT == DQSQ_X_I32) ? 4 : 2;
+    __shared__ float s_red[2 * 32];
     const int tid = threadIdx.x;
+    const int threads = static_cast<int>(blockDim.x);
     const int nchunks = static_cast<int>(H / EL);
-    const size_t elem = (XT == DQSQ_X_I32) ? 4 : 2;
     const bool has_q = (quant_scale != nullptr);
     // where the gate half and the other half start, in the row and in weight_scale
     const int64_t g_off = left ? 0 : H, o_off = left ? H : 0;
-    int parity = 0;
-    for (int64_t row = blockIdx.x; row < M; row += gridDim.x, parity ^= 1) {
-        const uint8_t* xr = static_cast<const uint8_t*>(x) + static_cast<size_t>(row) * 2 * H * elem;
-        const float as = (XT == DQSQ_X_I32) ? activation_scale[row] : 1.0f;
-        // every load of the row is issued before the first is used
-        uint4 ca[CPT], cb[CPT];
+    // a chunk past the end is all zeros: its results are zeros, and it is not stored
+    uint4 cg[CPT], co[CPT];
+#pragma unroll
+    for (int i = 0; i < CPT; ++i) {
+        cg[i] = co[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    float as = 1.0f;
+    const uint8_t* xg = static_cast<const uint8_t*>(x) + (static_cast<size_t>(blockIdx.x) * 2 * H + g_off) * ELEM + tid * 16;
+    const int64_t to_other = (o_off - g_off) * static_cast<int64_t>(ELEM);
+    const size_t row_step = static_cast<size_t>(gridDim.x) * 2 * H * ELEM;
+    auto load_row = [&](int64_t row) {
 #pragma unroll
         for (int i = 0; i < CPT; ++i) {
-            const int c = tid + i * DQSQ_THREADS;
-            if (c < nchunks) {
-                ca[i] = C::load_raw(xr, g_off + static_cast<int64_t>(c) * EL);
-                cb[i] = C::load_raw(xr, o_off + static_cast<int64_t>(c) * EL);
+            if (tid + i * threads < nchunks) {
+                cg[i] = C::load_raw(xg + i * threads * 16, 0);
+                co[i] = C::load_raw(xg + to_other + i * threads * 16, 0);
             }
         }
-        float out[CPT][EL];
-        float m = 0.0f;
+        if constexpr (XT == DQSQ_X_I32) {
+            as = activation_scale[row];
+        }
+        xg += row_step;
+    };
+    int parity = 0;
+    if (blockIdx.x < M) {
+        load_row(blockIdx.x);
+    }
+    for (int64_t row = blockIdx.x; row < M; row += gridDim.x, parity ^= 1) {
+        float out[N];
 #pragma unroll
-        for (int i = 0; i < CPT; ++i) {
-            const int c = tid + i * DQSQ_THREADS;
-            if (c < nchunks) {
-                const int64_t j0 = static_cast<int64_t>(c) * EL;
-                float a[EL], b[EL];
-                C::unpack(ca[i], a);
-                C::unpack(cb[i], b);
+        for (int i0 = 0; i0 < CPT; i0 += GROUP) {
+            float g[GN], o[GN], wg[GN], wo[GN], qs[GN];
+#pragma unroll
+            for (int i = 0; i < GROUP; ++i) {
+                float gi[EL], oi[EL];
+                C::unpack(cg[i0 + i], gi);
+                C::unpack(co[i0 + i], oi);
                 // per-channel vectors are re-read by every row: cached 128-bit loads (the launcher checks alignment)
-                float wa[EL], wb[EL], qs[EL];
+                const int64_t j0 = static_cast<int64_t>(min(tid + (i0 + i) * threads, nchunks - 1)) * EL;
 #pragma unroll
                 for (int q = 0; q < EL / 4; ++q) {
-                    float4 t = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+                    float4 a = make_float4(1.0f, 1.0f, 1.0f, 1.0f), b = a, c = a;
                     if constexpr (XT == DQSQ_X_I32) {
-                        t = __ldg(reinterpret_cast<const float4*>(weight_scale + g_off + j0) + q);
+                        a = __ldg(reinterpret_cast<const float4*>(weight_scale + g_off + j0) + q);
+                        b = __ldg(reinterpret_cast<const float4*>(weight_scale + o_off + j0) + q);
                     }
-                    wa[4 * q] = t.x, wa[4 * q + 1] = t.y, wa[4 * q + 2] = t.z, wa[4 * q + 3] = t.w;
-                    if constexpr (XT == DQSQ_X_I32) {
-                        t = __ldg(reinterpret_cast<const float4*>(weight_scale + o_off + j0) + q);
+                    if (has_q) {
+                        c = __ldg(reinterpret_cast<const float4*>(quant_scale + j0) + q);
                     }
-                    wb[4 * q] = t.x, wb[4 * q + 1] = t.y, wb[4 * q + 2] = t.z, wb[4 * q + 3] = t.w;
-                    t = has_q ? __ldg(reinterpret_cast<const float4*>(quant_scale + j0) + q)
-                              : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-                    qs[4 * q] = t.x, qs[4 * q + 1] = t.y, qs[4 * q + 2] = t.z, qs[4 * q + 3] = t.w;
+                    const int at = i * EL + 4 * q;
+                    wg[at] = a.x, wg[at + 1] = a.y, wg[at + 2] = a.z, wg[at + 3] = a.w;
+                    wo[at] = b.x, wo[at + 1] = b.y, wo[at + 2] = b.z, wo[at + 3] = b.w;
+                    qs[at] = c.x, qs[at + 1] = c.y, qs[at + 2] = c.z, qs[at + 3] = c.w;
                 }
 #pragma unroll
                 for (int j = 0; j < EL; ++j) {
-                    out[i][j] = dqsq_element_by_role<XT>(a[j], b[j], wa[j], wb[j], qs[j], as);
-                    m = fmaxf(m, fabsf(out[i][j]));
+                    g[i * EL + j] = gi[j];
+                    o[i * EL + j] = oi[j];
                 }
             }
+            float r[GN];
+            dqsq_elements<XT, GN>(g, o, wg, wo, qs, as, r);
+#pragma unroll
+            for (int j = 0; j < GN; ++j) {
+                out[i0 * EL + j] = r[j];
+            }
+        }
+        float m = 0.0f;
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            m = fmaxf(m, fabsf(out[j]));
+        }
+        if (row + gridDim.x < M) {
+            load_row(row + gridDim.x);
         }
         m = dqsq_block_max(m, s_red, parity);
         float s = __fmul_rn(m, INV127);
@@ -233,19 +328,21 @@ __global__ void __launch_bounds__(DQSQ_THREADS, (CPT <= 2) ? 4 : 1) dqsq_rows_ke
         if (tid == 0) {
             scale[row] = s;
         }
-        const float qf = DIVIDE ? s : __fdiv_rn(1.0f, s);
+        const float inv = __frcp_rn(s);
+        const bool regular = (direct == 0) && s < 1.0e18f;
         int8_t* yr = y + row * H;
 #pragma unroll
         for (int i = 0; i < CPT; ++i) {
-            const int c = tid + i * DQSQ_THREADS;
+            const int c = tid + i * threads;
             if (c < nchunks) {
                 const int64_t j0 = static_cast<int64_t>(c) * EL;
+                const float* oi = out + i * EL;
                 if constexpr (EL == 4) {
-                    *reinterpret_cast<uint32_t*>(yr + j0) = dqsq_quant4<DIVIDE>(out[i], qf, direct != 0);
+                    *reinterpret_cast<uint32_t*>(yr + j0) = dqsq_quant4<DIVIDE>(oi, s, inv, regular, direct != 0);
                 } else {
-                    const uint2 o = make_uint2(dqsq_quant4<DIVIDE>(out[i], qf, direct != 0),
-                                               dqsq_quant4<DIVIDE>(out[i] + 4, qf, direct != 0));
-                    *reinterpret_cast<uint2*>(yr + j0) = o;
+                    const uint2 w = make_uint2(dqsq_quant4<DIVIDE>(oi, s, inv, regular, direct != 0),
+                                               dqsq_quant4<DIVIDE>(oi + 4, s, inv, regular, direct != 0));
+                    *reinterpret_cast<uint2*>(yr + j0) = w;
                 }
             }
         }
@@ -262,7 +359,7 @@ __global__ void __launch_bounds__(DQSQ_THREADS) dqsq_long_rows_kernel(const void
                                                                       int64_t M, int64_t H, int left, int direct, int divide)
 {
     using C = DqsqChunk<XT>;
-    __shared__ float s_red[2 * (DQSQ_THREADS / 32)];
+    __shared__ float s_red[2 * 32];
     const size_t elem = (XT == DQSQ_X_I32) ? 4 : 2;
     const bool has_q = (quant_scale != nullptr);
     int parity = 0;
@@ -309,24 +406,35 @@ static cudaError_t dispatch_dqsq(const void* x, const float* ws, const float* as
     using Kern = void (*)(const void*, const float*, const float*, const float*, int8_t*, float*, int64_t, int64_t, int,
                           int, int);
     Kern kern = dqsq_long_rows_kernel<XT>;
-    if (vec && chunks <= DQSQ_THREADS) {
-        kern = divide ? dqsq_rows_kernel<XT, 1, true> : dqsq_rows_kernel<XT, 1, false>;
-    } else if (vec && chunks <= 2 * DQSQ_THREADS) {
-        kern = divide ? dqsq_rows_kernel<XT, 2, true> : dqsq_rows_kernel<XT, 2, false>;
-    } else if (vec && chunks <= 4 * DQSQ_THREADS) {
-        kern = dqsq_rows_kernel<XT, 4, false>;  // rows this long always take the reciprocal form
-    } else if (vec && chunks <= 8 * DQSQ_THREADS) {
-        kern = dqsq_rows_kernel<XT, 8, false>;
+    int threads = DQSQ_THREADS;
+    if (vec && chunks <= 2 * DQSQ_MAX_THREADS) {
+        // Two chunks of each half per thread (one where a row has at most a warp's worth), rounded up to whole warps:
+        // a thread count fitted to the row leaves few lanes idle on rows that are not a power of two long.  (Four
+        // int32 chunks per thread spill and take 79 us where two take 64 on [16384, 4096].)  16-bit rows take the
+        // 56-register form up to 576 threads: it puts two CTAs on an SM (24 against 27 us on fp16 [1531, 18432]).
+        const bool two = chunks > 32;
+        threads = static_cast<int>((((two ? (chunks + 1) / 2 : chunks) + 31) / 32) * 32);
+        if (!two) {
+            kern = dqsq_rows_kernel<XT, 1, true, DQSQ_PAIR_THREADS>;  // rows this short always divide
+        } else if (XT == DQSQ_X_I32) {
+            kern = divide ? dqsq_rows_kernel<XT, 2, true, DQSQ_MAX_THREADS> : dqsq_rows_kernel<XT, 2, false, DQSQ_MAX_THREADS>;
+        } else if (divide) {
+            kern = dqsq_rows_kernel<XT, 2, true, DQSQ_PAIR_THREADS>;
+        } else if (threads <= DQSQ_PAIR_THREADS) {
+            kern = dqsq_rows_kernel<XT, 2, false, DQSQ_PAIR_THREADS>;
+        } else {
+            kern = dqsq_rows_kernel<XT, 2, false, DQSQ_MAX_THREADS>;
+        }
     }
     // one wave: as many CTAs as are resident at once, each walking rows with a grid stride
     int per_sm = 1;
-    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, DQSQ_THREADS, 0);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, 0);
     if (e != cudaSuccess) {
         return e;
     }
     const int64_t cap = static_cast<int64_t>(sm_count()) * (per_sm < 1 ? 1 : per_sm);
     const unsigned grid = static_cast<unsigned>(M < cap ? M : cap);
-    kern<<<grid, DQSQ_THREADS, 0, st>>>(x, ws, as, qs, y, scale, M, H, left, direct, divide); w8a8::note_launch();
+    kern<<<grid, threads, 0, st>>>(x, ws, as, qs, y, scale, M, H, left, direct, divide); w8a8::note_launch();
     return cudaGetLastError();
 }
 
