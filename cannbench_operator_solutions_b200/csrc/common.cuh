@@ -237,6 +237,64 @@ __device__ __forceinline__ void neg_exp_neg2(const f32x2 (&g)[N], f32x2 (&e)[N])
     }
 }
 
+// e = canonical_expf(x) of N pairs, bit for bit, for x <= 0 (-inf included, NaN not): the power of two is applied as
+// an exact integer add that leaves a normal number, 2^64 too large, and one multiplication that rounds the
+// subnormal results.  (A pair addition that uses e may absorb that multiplication; it is exact unless the result is
+// subnormal, where a sum of at least 2^-126 does not see the difference.)
+template <int N>
+__device__ __forceinline__ void exp_nonpositive2(const f32x2 (&x)[N], f32x2 (&e)[N])
+{
+    f32x2 t[N], r[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        float x0, x1;
+        unpair(x[i], x0, x1);
+        x0 = fmaxf(x0, -104.0f);
+        x1 = fmaxf(x1, -104.0f);
+        r[i] = pair(x0, x1);
+        t[i] = add2(pair(__fmul_rn(x0, 1.44269504088896341f), __fmul_rn(x1, 1.44269504088896341f)), pair(12582912.0f));
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        e[i] = add2(t[i], pair(-12582912.0f));
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        r[i] = fma2(e[i], pair(-0.693359375f), r[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        r[i] = fma2(e[i], pair(2.12194440e-4f), r[i]);
+    }
+    constexpr float C[6] = {1.9875691500e-4f, 1.3981999507e-3f, 8.3334519073e-3f,
+                            4.1665795894e-2f, 1.6666665459e-1f, 5.0000001201e-1f};
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        e[i] = pair(C[0]);
+    }
+#pragma unroll
+    for (int k = 1; k < 6; ++k) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            e[i] = fma2(e[i], r[i], pair(C[k]));
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        e[i] = add2(fma2(e[i], mul2(r[i], r[i]), r[i]), pair(1.0f));
+        float e0, e1, t0, t1;
+        unpair(e[i], e0, e1);
+        unpair(t[i], t0, t1);
+        // the low bits of t are n, those above shift out
+        e[i] = pair(__int_as_float(__float_as_int(e0) + (__float_as_int(t0) << 23) + (64 << 23)),
+                    __int_as_float(__float_as_int(e1) + (__float_as_int(t1) << 23) + (64 << 23)));
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        e[i] = mul2(e[i], pair(5.42101086242752217e-20f));  // 2^-64
+    }
+}
+
 __device__ __forceinline__ float approx_reciprocal(float x)
 {
     float r;
