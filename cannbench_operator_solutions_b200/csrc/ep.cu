@@ -16,6 +16,197 @@
 
 namespace w8a8 {
 
+// ---------------------------------------------------------------------------
+// Route plan (stable counting sort by expert), E <= RP_MAX_EXPERTS: a CTA counts RP_PAIRS pairs in shared memory, the
+// scan turns the CTAs' counts into prefixes with a lane per expert and a warp per run of CTAs (coalesced, every load
+// independent), and the placing CTAs rank their pairs with warp matches.  With one CTA's worth of pairs all three
+// are one launch.  Bound: latency.  524288 pairs, 256 experts: 45 us beside the normalisation, was 465 (a thread per expert walked 2048
+// counts one load after the other); 512 pairs: 6 us, was 20 and a memset.
+// ---------------------------------------------------------------------------
+constexpr int RP_MAX_EXPERTS = 1024;
+constexpr int RP_PAIRS = 1024;
+constexpr int RP_THREADS = 256;
+constexpr int RP_WARPS = RP_THREADS / 32;
+
+__device__ __forceinline__ int rp_expert(const int32_t* expert_idx, int64_t p, int64_t P, int E)
+{
+    const int e = p < P ? expert_idx[p] : -1;
+    return (e >= 0 && e < E) ? e : -1;
+}
+
+__global__ void __launch_bounds__(RP_THREADS) rp_histogram_kernel(const int32_t* __restrict__ expert_idx, int64_t P,
+                                                                  int E, int32_t* __restrict__ block_count)
+{
+    __shared__ int32_t s_cnt[RP_MAX_EXPERTS];
+    for (int e = threadIdx.x; e < E; e += RP_THREADS) {
+        s_cnt[e] = 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < RP_PAIRS / RP_THREADS; ++it) {
+        const int e = rp_expert(expert_idx, static_cast<int64_t>(blockIdx.x) * RP_PAIRS + it * RP_THREADS + threadIdx.x, P, E);
+        if (e >= 0) {
+            atomicAdd(&s_cnt[e], 1);
+        }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += RP_THREADS) {
+        block_count[static_cast<int64_t>(blockIdx.x) * E + e] = s_cnt[e];
+    }
+}
+
+// block_count[B][E] becomes the exclusive prefix over blocks, count[E] the totals; a CTA takes 32 experts
+__global__ void __launch_bounds__(1024) rp_prefix_kernel(int32_t* __restrict__ block_count, int64_t B, int E,
+                                                         int64_t* __restrict__ count)
+{
+    __shared__ int32_t s_part[32][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int e = blockIdx.x * 32 + lane;
+    const int64_t per = (B + 31) / 32;
+    const int64_t first = warp * per, last = first + per < B ? first + per : B;
+    int32_t sum = 0;
+    if (e < E) {
+#pragma unroll 8
+        for (int64_t b = first; b < last; ++b) {
+            sum += block_count[b * E + e];
+        }
+    }
+    s_part[warp][lane] = sum;
+    __syncthreads();
+    int64_t run = 0;
+    for (int w = 0; w < warp; ++w) {
+        run += s_part[w][lane];
+    }
+    if (e < E) {
+        if (warp == 31) {
+            count[e] = run + sum;
+        }
+#pragma unroll 8
+        for (int64_t b = first; b < last; ++b) {
+            const int32_t c = block_count[b * E + e];
+            block_count[b * E + e] = static_cast<int32_t>(run);
+            run += c;
+        }
+    }
+}
+
+// ONE_CTA: counts its pairs itself and writes count; otherwise count and block_prefix come from rp_prefix_kernel.
+template <bool ONE_CTA>
+__global__ void __launch_bounds__(RP_THREADS) rp_rank_kernel(const int32_t* __restrict__ expert_idx, int64_t P, int E,
+                                                             const int32_t* __restrict__ block_prefix,
+                                                             int64_t* __restrict__ count, int64_t* __restrict__ cumsum,
+                                                             int64_t* __restrict__ expanded_pos)
+{
+    constexpr int ITS = RP_PAIRS / RP_THREADS;
+    constexpr int PER = RP_MAX_EXPERTS / RP_THREADS;  // experts per thread in the scan
+    __shared__ int64_t s_next[RP_MAX_EXPERTS];        // where the next pair of each expert goes
+    __shared__ uint32_t s_words[RP_WARPS * RP_MAX_EXPERTS / 4];
+    __shared__ int64_t s_sum[RP_WARPS];
+    uint8_t* s_warp = reinterpret_cast<uint8_t*>(s_words);  // [RP_WARPS][E]: pairs of each warp, one step at a time
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int mine[ITS];
+#pragma unroll
+    for (int it = 0; it < ITS; ++it) {
+        mine[it] = rp_expert(expert_idx, static_cast<int64_t>(blockIdx.x) * RP_PAIRS + it * RP_THREADS + tid, P, E);
+    }
+    if constexpr (ONE_CTA) {
+        int32_t* s_cnt = reinterpret_cast<int32_t*>(s_words);
+        for (int e = tid; e < E; e += RP_THREADS) {
+            s_cnt[e] = 0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int it = 0; it < ITS; ++it) {
+            if (mine[it] >= 0) {
+                atomicAdd(&s_cnt[mine[it]], 1);
+            }
+        }
+        __syncthreads();
+    }
+    int64_t c[PER], sum = 0;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int e = tid * PER + j;
+        c[j] = 0;
+        if (e < E) {
+            if constexpr (ONE_CTA) {
+                c[j] = reinterpret_cast<int32_t*>(s_words)[e];
+                count[e] = c[j];
+            } else {
+                c[j] = count[e];
+            }
+        }
+        sum += c[j];
+    }
+    int64_t incl = sum;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int64_t v = __shfl_up_sync(FULL_MASK, incl, off);
+        incl += lane >= off ? v : 0;
+    }
+    if (lane == 31) {
+        s_sum[warp] = incl;
+    }
+    __syncthreads();
+    int64_t run = incl - sum;
+    for (int w = 0; w < warp; ++w) {
+        run += s_sum[w];
+    }
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int e = tid * PER + j;
+        if (e < E) {
+            int64_t at = run;
+            if constexpr (!ONE_CTA) {
+                at += block_prefix[static_cast<int64_t>(blockIdx.x) * E + e];
+            }
+            s_next[e] = at;
+            run += c[j];
+            if (blockIdx.x == 0) {
+                cumsum[e] = run;
+            }
+        }
+    }
+    const int words = (RP_WARPS * E + 3) / 4;
+#pragma unroll 1
+    for (int it = 0; it < ITS; ++it) {
+        const int64_t p = static_cast<int64_t>(blockIdx.x) * RP_PAIRS + it * RP_THREADS + tid;
+        if (static_cast<int64_t>(blockIdx.x) * RP_PAIRS + it * RP_THREADS >= P) {
+            break;  // the same for the whole CTA
+        }
+        int e = mine[0];
+#pragma unroll
+        for (int j = 1; j < ITS; ++j) {
+            e = (it == j) ? mine[j] : e;
+        }
+        for (int i = tid; i < words; i += RP_THREADS) {
+            s_words[i] = 0;
+        }
+        __syncthreads();
+        const unsigned same = __match_any_sync(FULL_MASK, e);
+        const int rank = __popc(same & ((1u << lane) - 1u));
+        if (rank == 0 && e >= 0) {
+            s_warp[warp * E + e] = static_cast<uint8_t>(__popc(same));
+        }
+        __syncthreads();
+        if (p < P) {
+            int64_t at = -1;
+            if (e >= 0) {
+                at = s_next[e] + rank;
+                for (int w = 0; w < warp; ++w) {
+                    at += s_warp[w * E + e];
+                }
+            }
+            expanded_pos[p] = at;
+        }
+        __syncthreads();
+        if (rank == 0 && e >= 0) {
+            atomicAdd(reinterpret_cast<unsigned long long*>(&s_next[e]), static_cast<unsigned long long>(__popc(same)));
+        }
+    }
+}
+
+// More experts than that: counts in global memory.
 constexpr int RP_BLOCK = 256;  // pairs per counting block
 
 // workspace layout: int32 block_count[B][E] (becomes the exclusive prefix over
@@ -698,12 +889,47 @@ __global__ void __launch_bounds__(256) mfr_kernel(const void* __restrict__ rows,
 //   seg_first / seg_ptr       one segment per (local expert, source rank): first local row, and the address in
 //                             the source rank's return buffer where the segment's first output row goes
 //   status[0]                 1 when some rank would receive more rows than the buffers hold
-// One CTA; thread i < P walks rank i's counts, thread e < E a column.
+// One CTA of 1024 threads; the three prefixes (rank i's rows over experts, the experts' rows over all ranks, the
+// segments' rows) run as one block-wide scan of two cells per thread.  Bound: latency.  1 rank, 256 experts: 6 us,
+// was 48 - 63 with one thread per prefix.
 // ---------------------------------------------------------------------------
 constexpr int EP_MAX_RANKS = 64;
 constexpr int EP_MAX_CELLS = 2048;  // P * E, held in shared memory
+constexpr int EP_THREADS = 1024;
 
-__global__ void __launch_bounds__(1024) ep_tables_kernel(const int64_t* __restrict__ counts, int P, int E, int rank,
+// Inclusive prefix sums of three sequences of 2 * EP_THREADS elements at once; thread t holds elements 2 t and 2 t + 1.
+__device__ __forceinline__ void ep_scan3(int64_t (&v)[3][2], int64_t (*s_warp)[3])
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t incl[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        incl[a] = v[a][0] + v[a][1];
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int64_t t = __shfl_up_sync(FULL_MASK, incl[a], off);
+            incl[a] += lane >= off ? t : 0;
+        }
+        if (lane == 31) {
+            s_warp[warp][a] = incl[a];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        // the warps before this one, added by the lanes together
+        int64_t before = lane < warp ? s_warp[lane][a] : 0;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            before += __shfl_xor_sync(FULL_MASK, before, off);
+        }
+        const int64_t second = v[a][1];
+        v[a][1] = before + incl[a];
+        v[a][0] = v[a][1] - second;
+    }
+}
+
+__global__ void __launch_bounds__(EP_THREADS) ep_tables_kernel(const int64_t* __restrict__ counts, int P, int E, int rank,
                                                          const uint64_t* __restrict__ peer_base, uint64_t off_x,
                                                          uint64_t off_s, uint64_t off_back, int64_t row_bytes,
                                                          int64_t back_row_bytes, int64_t cap_rows,
@@ -714,25 +940,25 @@ __global__ void __launch_bounds__(1024) ep_tables_kernel(const int64_t* __restri
                                                          int64_t* __restrict__ seg_first,
                                                          uint64_t* __restrict__ seg_ptr, int32_t* __restrict__ status)
 {
-    // The whole matrix is staged in shared memory first (one coalesced pass), so that the sequential prefix loops
-    // below run on shared memory instead of waiting for a global load per step.  Row counts fit 32 bits (a rank's
-    // buffers hold fewer than 2^31 rows; larger counts set the overflow flag).
-    __shared__ int32_t s_cnt[EP_MAX_CELLS];   // [P][E]
-    __shared__ int32_t s_base[EP_MAX_CELLS];  // [P][E]: rank i's exclusive prefix over experts
-    __shared__ int32_t s_seg[EP_MAX_CELLS];   // [E/P][P]: first local row of each (local expert, source rank) segment
-    __shared__ int32_t s_col[1024];           // rows per expert over all ranks
-    __shared__ int32_t s_before[1024];        // rows of lower ranks inside each expert
-    __shared__ int32_t s_exbase[1024];        // expert's first row in its owner's buffer
+    // Row counts fit 32 bits (a rank's buffers hold fewer than 2^31 rows; larger counts set the overflow flag).
+    __shared__ int32_t s_cnt[EP_MAX_CELLS];       // [P][E]
+    __shared__ int64_t s_base[EP_MAX_CELLS + 1];  // exclusive prefix of s_cnt over all cells, rank-major
+    __shared__ int64_t s_ex[EP_MAX_CELLS / 2 + 1];   // exclusive prefix of the experts' rows (E <= 1024)
+    __shared__ int64_t s_seg[EP_MAX_CELLS / 2 + 1];  // exclusive prefix of this rank's segments
+    __shared__ int32_t s_before[EP_MAX_CELLS / 2];   // rows of lower ranks inside each expert
+    __shared__ int64_t s_warp[32][3];
     __shared__ int s_bad;
     const int tid = threadIdx.x;
     const int e_local = E / P;
     const int cells = P * E;
+    const int nseg = e_local * P;
     if (tid == 0) {
         s_bad = 0;
+        s_base[0] = s_ex[0] = s_seg[0] = 0;
     }
     __syncthreads();
     const int64_t limit = cap_rows < 0x7fffffffLL ? cap_rows : 0x7fffffffLL;
-    for (int c = tid; c < cells; c += blockDim.x) {
+    for (int c = tid; c < cells; c += EP_THREADS) {
         const int64_t v = counts[c];
         if (v < 0 || v > limit) {
             s_bad = 1;
@@ -740,94 +966,78 @@ __global__ void __launch_bounds__(1024) ep_tables_kernel(const int64_t* __restri
         s_cnt[c] = (v < 0 || v > limit) ? 0 : static_cast<int32_t>(v);
     }
     __syncthreads();
-    if (tid < P) {
-        int64_t run = 0;
-        for (int e = 0; e < E; ++e) {
-            s_base[tid * E + e] = static_cast<int32_t>(run);
-            run += s_cnt[tid * E + e];
+    int64_t v[3][2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int c = 2 * tid + h;
+        v[0][h] = c < cells ? s_cnt[c] : 0;
+        v[1][h] = v[2][h] = 0;
+        if (c < E) {
+            int64_t col = 0, before = 0;
+            for (int i = 0; i < P; ++i) {
+                const int32_t n = s_cnt[i * E + c];
+                before += i < rank ? n : 0;
+                col += n;
+            }
+            if (col > limit) {
+                s_bad = 1;
+                col = 0;
+                before = 0;
+            }
+            v[1][h] = col;
+            s_before[c] = static_cast<int32_t>(before);
         }
-        if (run > 0x7fffffffLL) {
-            s_bad = 1;
+        if (c < nseg) {  // segments in (local expert, source rank) order
+            const int j = c / P;
+            v[2][h] = s_cnt[(c - j * P) * E + rank * e_local + j];
         }
     }
-    for (int e = tid; e < E; e += blockDim.x) {
-        int64_t col = 0, before = 0;
-        for (int i = 0; i < P; ++i) {
-            const int32_t c = s_cnt[i * E + e];
-            if (i < rank) {
-                before += c;
-            }
-            col += c;
+    ep_scan3(v, s_warp);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int c = 2 * tid + h;
+        if (c < cells) {
+            s_base[c + 1] = v[0][h];
         }
-        if (col > limit) {
-            s_bad = 1;
-            col = 0;
-            before = 0;
+        if (c < E) {
+            s_ex[c + 1] = v[1][h];
         }
-        s_col[e] = static_cast<int32_t>(col);
-        s_before[e] = static_cast<int32_t>(before);
+        if (c < nseg) {
+            s_seg[c + 1] = v[2][h];
+        }
     }
     __syncthreads();
-    if (tid < P) {  // thread o: the experts of owner o
-        int64_t run = 0;
-        for (int j = 0; j < e_local; ++j) {
-            const int e = tid * e_local + j;
-            s_exbase[e] = static_cast<int32_t>(run < 0x7fffffffLL ? run : 0);
-            run += s_col[e];
-            if (tid == rank) {
-                group_list[j] = run;
-            }
-        }
-        if (run > cap_rows) {
+    if (tid < P) {  // thread o: source rank o's rows in all, and what owner o receives
+        if (s_base[(tid + 1) * E] - s_base[tid * E] > 0x7fffffffLL ||
+            s_ex[(tid + 1) * e_local] - s_ex[tid * e_local] > cap_rows) {
             s_bad = 1;
-        }
-    }
-    if (tid == 32) {  // segments in (local expert, source rank) order: exclusive prefix of their lengths
-        int64_t run = 0;
-        for (int j = 0; j < e_local; ++j) {
-            const int e = rank * e_local + j;
-            for (int i = 0; i < P; ++i) {
-                s_seg[j * P + i] = static_cast<int32_t>(run < 0x7fffffffLL ? run : 0);
-                run += s_cnt[i * E + e];
-            }
         }
     }
     __syncthreads();
     // Too many rows for some rank's buffers: nothing may be stored anywhere.  Every rank sees the same counts, so
     // every rank takes this branch together: zero destinations (dispatch skips them) and empty groups.
     const bool bad = (s_bad != 0);
-    const int nseg = e_local * P;
-    for (int e = tid; e < E; e += blockDim.x) {
+    const int64_t own_first = s_ex[rank * e_local];
+    for (int e = tid; e < E; e += EP_THREADS) {
         const int owner = e / e_local;
-        const uint64_t first = static_cast<uint64_t>(s_exbase[e]) + static_cast<uint64_t>(s_before[e]);
+        const uint64_t first = static_cast<uint64_t>(s_ex[e] - s_ex[owner * e_local]) + static_cast<uint64_t>(s_before[e]);
         row_dst[e] = bad ? 0 : peer_base[owner] + off_x + first * static_cast<uint64_t>(row_bytes);
         scale_dst[e] = bad ? 0 : peer_base[owner] + off_s + first * 4u;
-        my_base[e] = s_base[rank * E + e];
-    }
-    for (int sidx = tid; sidx < nseg; sidx += blockDim.x) {
-        const int j = sidx / P, i = sidx - j * P;
-        const int e = rank * e_local + j;
-        seg_first[sidx] = bad ? 0 : s_seg[sidx];
-        seg_ptr[sidx] = bad ? 0
-                            : peer_base[i] + off_back +
-                                  static_cast<uint64_t>(s_base[i * E + e]) * static_cast<uint64_t>(back_row_bytes);
-    }
-    if (bad) {
-        for (int j = tid; j < e_local; j += blockDim.x) {
-            group_list[j] = 0;
+        my_base[e] = s_base[rank * E + e] - s_base[rank * E];
+        if (owner == rank) {
+            group_list[e - rank * e_local] = bad ? 0 : s_ex[e + 1] - own_first;
         }
     }
-    if (tid == 0) {
-        // the last local expert's cumulative count is the number of rows this rank holds
-        int64_t total = 0;
-        for (int j = 0; j < e_local; ++j) {
-            total += s_col[rank * e_local + j];
+    for (int c = tid; c <= nseg; c += EP_THREADS) {
+        seg_first[c] = bad ? 0 : s_seg[c];
+        if (c < nseg) {
+            const int j = c / P, i = c - j * P;
+            const int64_t at = s_base[i * E + rank * e_local + j] - s_base[i * E];
+            seg_ptr[c] = bad ? 0 : peer_base[i] + off_back + static_cast<uint64_t>(at) * static_cast<uint64_t>(back_row_bytes);
         }
-        seg_first[nseg] = bad ? 0 : total;
-        // sticky: a later good step must not hide an overflowed one; the reader clears it
-        if (bad) {
-            status[0] = 1;
-        }
+    }
+    if (tid == 0 && bad) {
+        status[0] = 1;  // sticky: a later good step must not hide an overflowed one; the reader clears it
     }
 }
 
@@ -871,6 +1081,18 @@ extern "C" int w8a8_route_plan(const int32_t* expert_idx, int64_t T, int64_t top
     uint8_t* ws = static_cast<uint8_t*>(workspace);
     int32_t* bad = reinterpret_cast<int32_t*>(ws);
     int32_t* block_count = reinterpret_cast<int32_t*>(ws + 256);
+    if (E <= w8a8::RP_MAX_EXPERTS) {
+        const int experts = static_cast<int>(E);
+        const int64_t ctas = (P + w8a8::RP_PAIRS - 1) / w8a8::RP_PAIRS;
+        if (ctas <= 1) {
+            w8a8::rp_rank_kernel<true><<<1, w8a8::RP_THREADS, 0, st>>>(expert_idx, P, experts, nullptr, count, cumsum, expanded_pos); w8a8::note_launch();
+        } else {
+            w8a8::rp_histogram_kernel<<<static_cast<unsigned>(ctas), w8a8::RP_THREADS, 0, st>>>(expert_idx, P, experts, block_count); w8a8::note_launch();
+            w8a8::rp_prefix_kernel<<<static_cast<unsigned>((E + 31) / 32), 1024, 0, st>>>(block_count, ctas, experts, count); w8a8::note_launch();
+            w8a8::rp_rank_kernel<false><<<static_cast<unsigned>(ctas), w8a8::RP_THREADS, 0, st>>>(expert_idx, P, experts, block_count, count, cumsum, expanded_pos); w8a8::note_launch();
+        }
+        return (cudaGetLastError() == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    }
     const size_t bc_bytes = w8a8::align_up(static_cast<size_t>(B > 0 ? B : 1) * E * sizeof(int32_t), 256);
     int64_t* base = reinterpret_cast<int64_t*>(ws + 256 + bc_bytes);
     if (cudaMemsetAsync(ws, 0, 256 + bc_bytes, st) != cudaSuccess) {
@@ -1200,7 +1422,7 @@ extern "C" int w8a8_ep_tables(const int64_t* counts, int64_t P, int64_t E, int64
         status == nullptr) {
         return W8A8_ERR_INVALID;
     }
-    w8a8::ep_tables_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(
+    w8a8::ep_tables_kernel<<<1, w8a8::EP_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
         counts, static_cast<int>(P), static_cast<int>(E), static_cast<int>(rank), peer_base, off_x, off_s, off_back,
         row_bytes, back_row_bytes, cap_rows, row_dst, scale_dst, my_base, group_list, seg_first, seg_ptr, status); w8a8::note_launch();
     return (cudaGetLastError() == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;

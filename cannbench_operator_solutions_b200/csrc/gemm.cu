@@ -291,26 +291,34 @@ __device__ __forceinline__ void plan_groups_body(const int64_t* __restrict__ dev
     if (bad) {
         return;
     }
-    // one warp per group at a time fills that group's tile entries
-    for (int64_t g = wid; g < E; g += 8) {
-        int64_t start = (g == 0) ? 0 : end_of(g - 1);
-        int64_t rows = end_of(g) - start;
+    // a thread per tile looks up its group (the last one whose first tile is at or before it; groups without tiles
+    // share their first tile with the next one, and s_first[E] = total ends the search): 3.5 us for 512 rows of 256
+    // experts, 10 with a warp per group in turn, whose loads of the list waited for one another
+    for (int32_t i = tid; i < total; i += 256) {
+        int lo = 0, hi = static_cast<int>(E);
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (s_first[mid] <= i) {
+                lo = mid;
+            } else {
+                hi = mid;
+            }
+        }
+        int64_t start = (lo == 0) ? 0 : end_of(lo - 1);
+        int64_t rows = end_of(lo) - start;
         if (mode == PLAN_LEFTOVER) {
             const int64_t whole = rows / (2 * tile_m) * (2 * tile_m);
             start += whole;
             rows -= whole;
         }
-        const int32_t first = s_first[g];
-        const int32_t cnt = s_first[g + 1] - first;
-        for (int32_t t = lane; t < cnt; t += 32) {
-            TileEntry te;
-            te.group = static_cast<int32_t>(g);
-            te.m_start = static_cast<int32_t>(start + static_cast<int64_t>(t) * tile_m);
-            const int64_t left = rows - static_cast<int64_t>(t) * tile_m;
-            te.m_rows = static_cast<int32_t>(left < tile_m ? left : tile_m);
-            te.pad = 0;
-            tiles[first + t] = te;
-        }
+        const int32_t t = i - s_first[lo];
+        TileEntry te;
+        te.group = lo;
+        te.m_start = static_cast<int32_t>(start + static_cast<int64_t>(t) * tile_m);
+        const int64_t left = rows - static_cast<int64_t>(t) * tile_m;
+        te.m_rows = static_cast<int32_t>(left < tile_m ? left : tile_m);
+        te.pad = 0;
+        tiles[i] = te;
     }
 }
 

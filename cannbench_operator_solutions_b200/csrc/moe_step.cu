@@ -313,16 +313,11 @@ extern "C" int w8a8_moe_ffn_step(const W8A8MoeFfnStep* s, const void* x, const v
     if (rc != W8A8_OK) {
         return rc;
     }
-    // every rank learns every rank's per-expert counts; they stay on the device
-    if (P > 1) {
-        if (nccl().all_gather(b.count, b.gathered, static_cast<size_t>(E), NCCL_INT64, s->comm, st) != 0) {
-            return W8A8_ERR_CUDA;
-        }
-    } else if (cudaMemcpyAsync(b.gathered, b.count, static_cast<size_t>(E) * 8, cudaMemcpyDeviceToDevice, st) !=
-               cudaSuccess) {
+    // every rank learns every rank's per-expert counts; they stay on the device (one rank's are the whole matrix)
+    if (P > 1 && nccl().all_gather(b.count, b.gathered, static_cast<size_t>(E), NCCL_INT64, s->comm, st) != 0) {
         return W8A8_ERR_CUDA;
     }
-    rc = w8a8_ep_tables(b.gathered, P, E, s->rank, s->peer_base, s->off_x, s->off_s, s->off_back, hidden, hidden * elem,
+    rc = w8a8_ep_tables(P > 1 ? b.gathered : b.count, P, E, s->rank, s->peer_base, s->off_x, s->off_s, s->off_back, hidden, hidden * elem,
                         cap, b.row_dst, b.scale_dst, b.my_base, b.group_list, b.seg_first, b.seg_ptr, b.status, st);
     if (rc != W8A8_OK) {
         return rc;
