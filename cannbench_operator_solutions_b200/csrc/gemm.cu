@@ -101,27 +101,28 @@ static int64_t worker_count(int64_t max_tiles)
     return workers < 1 ? 1 : workers;
 }
 
-template <int CG, int BLOCK_N, int KIND, int EPI, bool B_MN, int EPI_WARPS = 8>
+template <int CG, int BLOCK_N, int KIND, int EPI, bool B_MN, int EPI_WARPS = 8, bool SPLITK = false>
 static cudaError_t launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int64_t max_tiles,
                                cudaStream_t st)
 {
-    auto kern = gemm_tc_kernel<CG, BLOCK_N, KIND, EPI, B_MN, EPI_WARPS>;
+    auto kern = gemm_tc_kernel<CG, BLOCK_N, KIND, EPI, B_MN, EPI_WARPS, SPLITK>;
     constexpr size_t smem = gemm_smem_bytes<CG, BLOCK_N>();
     // the attribute is per device; setting it on every call is cheap and covers multi-GPU processes
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) {
         return e;
     }
-    const int64_t workers = worker_count<CG>(max_tiles);
+    const unsigned cluster = SPLITK ? static_cast<unsigned>(p.split) : CG;
+    const int64_t workers = SPLITK ? max_tiles : worker_count<CG>(max_tiles);  // split K: one tile per cluster
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(workers * CG), 1, 1);
+    cfg.gridDim = dim3(static_cast<unsigned>(workers * cluster), 1, 1);
     cfg.blockDim = dim3(gemm_threads(EPI_WARPS), 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
-    if (CG == 2) {
+    if (cluster > 1) {
         attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
+        attr[0].val.clusterDim.x = cluster;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
@@ -160,6 +161,22 @@ static cudaError_t dispatch_gemm(int cta_group, int block_n, bool b_mn, const CU
     }
     return b_mn ? launch_gemm<1, 256, KIND, EPI, true>(ta, tb, p, max_tiles, st)
                 : launch_gemm<1, 256, KIND, EPI, false>(ta, tb, p, max_tiles, st);
+}
+
+// Dense problems with at most one 128 x 128 tile per SM run on single CTAs: a cluster launch costs about 3 us more
+// than a plain one (512 x 1024 x 1024: 7.4 us, 11 on pairs; 1024 x 2048 x 2048: 10.3, 13.8).  Where half of the SMs or
+// more would have no tile, clusters of two or four share a tile's K, if the K blocks saved (0.25 us each) pay for the
+// cluster and for the exchange of the accumulators, which a tile with few rows hardly has: 16 x 9216 x 7168 18 us
+// against 25, 16 x 7168 x 4096 11.8 (four) / 14.6 (two) against 20.5, 128 x 7168 x 2048 14.4 / 15.9 against 20.6,
+// but 1024 x 2048 x 512 12.5 / 10.4 and 128 x 1024 x 1024 9.9 / 9.0 against 7.1.  Clusters of eight do not find a
+// place for every tile (16 tiles take two waves); clusters of four count on 128 SMs.
+static int choose_split(int64_t tiles, int64_t k_blocks, int64_t rows)
+{
+    const bool few_rows = rows <= 64;
+    if (tiles * 4 <= 128 && tiles * 4 <= sm_count() && k_blocks >= (few_rows ? 16 : 48)) {
+        return 4;
+    }
+    return (tiles * 2 <= sm_count() && k_blocks >= (few_rows ? 12 : 24)) ? 2 : 1;
 }
 
 // Kernel shape: CTA pairs for dense problems with enough rows to fill 256-row tiles.  w8a8_set_gemm_shape()
@@ -746,7 +763,23 @@ static int quant_matmul_impl(const int8_t* x1, const int8_t* x2, const void* sca
     p.out_dtype = out_dtype;
     p.bias_batch_stride = bias_batch_stride;
     p.error = pipeline_error_word();  // null (no report) only if the symbol lookup failed
-    const int cg = choose_cta_group(M, false);
+    const int64_t tiles128 = batch * p.m_tiles_per_batch * ((N + 127) / 128);
+    const bool own_choice = g_shape_override.load(std::memory_order_relaxed) == 0;
+    const int split = own_choice ? choose_split(tiles128, p.num_k_blocks, M) : 1;
+    if (split > 1) {
+        p.split = split;
+        p.n_tiles = static_cast<int32_t>((N + 127) / 128);
+        cudaError_t e;
+        if (raw_i32) {
+            e = b_mn ? launch_gemm<1, 128, KIND_I8, EPI_RAW, true, 8, true>(ta, tb, p, tiles128, st)
+                     : launch_gemm<1, 128, KIND_I8, EPI_RAW, false, 8, true>(ta, tb, p, tiles128, st);
+        } else {
+            e = b_mn ? launch_gemm<1, 128, KIND_I8, EPI_QMM, true, 8, true>(ta, tb, p, tiles128, st)
+                     : launch_gemm<1, 128, KIND_I8, EPI_QMM, false, 8, true>(ta, tb, p, tiles128, st);
+        }
+        return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    }
+    const int cg = (own_choice && tiles128 <= sm_count()) ? 1 : choose_cta_group(M, false);
     const int tile_m = 128 * cg;
     p.m_tiles_per_batch = static_cast<int32_t>((M + tile_m - 1) / tile_m);
     // narrow tiles when wide ones would leave most SMs idle (single-CTA tiles only)

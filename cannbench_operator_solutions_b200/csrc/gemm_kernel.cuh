@@ -118,6 +118,7 @@ struct GemmParams {
     int32_t* tile_done;   // per (row tile, CTA of the tile): epilogue warps done with a column tile (zeroed by the caller)
     int8_t* y;            // [M, N/2]
     float* y_scale;       // [M]
+    int32_t split;  // SPLITK kernels: CTAs of a cluster that share a tile's K
     int32_t fuse_requant;
     int32_t round_direct;
 };
@@ -136,16 +137,17 @@ __device__ __forceinline__ float vec_elem_as_float(const void* p, int64_t i, int
     }
 }
 
-// 32 consecutive per-channel values starting at element `idx0` (16-byte aligned
+// NV (32 or 16) consecutive per-channel values starting at element `idx0` (16-byte aligned
 // for every kind because idx0 is a multiple of 16), widened to fp32; a vector
-// that is not per-channel broadcasts element 0.  `valid` is 32 or 16.
-__device__ __forceinline__ void load_vec32(const void* base, int64_t idx0, int kind, bool perchan, int valid,
-                                           float (&out)[32])
+// that is not per-channel broadcasts element 0.  `valid` is 32, 16 or 0.
+template <int NV>
+__device__ __forceinline__ void load_vec(const void* base, int64_t idx0, int kind, bool perchan, int valid,
+                                         float (&out)[NV])
 {
     if (!perchan) {
         const float s = vec_elem_as_float(base, 0, kind);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
+        for (int j = 0; j < NV; ++j) {
             out[j] = s;
         }
         return;
@@ -153,7 +155,7 @@ __device__ __forceinline__ void load_vec32(const void* base, int64_t idx0, int k
     if (kind == W8A8_QM_BIAS_F32 || kind == W8A8_QM_BIAS_I32) {
         const uint4* p4 = reinterpret_cast<const uint4*>(static_cast<const uint32_t*>(base) + idx0);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
+        for (int q = 0; q < NV / 4; ++q) {
             uint4 t = make_uint4(0, 0, 0, 0);
             if (q * 4 < valid) {
                 t = __ldg(p4 + q);
@@ -173,7 +175,7 @@ __device__ __forceinline__ void load_vec32(const void* base, int64_t idx0, int k
     } else {
         const uint4* p4 = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(base) + idx0);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < NV / 8; ++q) {
             uint4 t = make_uint4(0, 0, 0, 0);
             if (q * 8 < valid) {
                 t = __ldg(p4 + q);
@@ -191,6 +193,78 @@ __device__ __forceinline__ void load_vec32(const void* base, int64_t idx0, int k
     }
 }
 
+
+// What the dequant chain of quant_matmul needs besides the accumulator, the same for all columns of a row.
+struct QmmTerms {
+    float row_mul;
+    const void* bias;
+    int bias_kind;
+    bool has_pt, bias_perchan, scale_perchan, scale_bf16, has_offset, offset_perchan;
+};
+
+__device__ __forceinline__ QmmTerms qmm_terms(const GemmParams& p, int32_t group, int64_t row, bool row_ok)
+{
+    const int64_t f = p.flags;
+    QmmTerms t;
+    t.has_pt = (f & W8A8_QM_HAS_PT) != 0;
+    t.row_mul = 1.0f;
+    if (t.has_pt && row_ok) {
+        // the plugin's layouts make (row mod M) the token index in every case
+        t.row_mul = p.row_scale[(group == 0) ? row : (row - static_cast<int64_t>(group) * p.M)];
+    }
+    t.bias = p.bias;
+    t.bias_kind = static_cast<int>((f & W8A8_QM_BIAS_MASK) >> W8A8_QM_BIAS_SHIFT);
+    t.bias_perchan = (f & W8A8_QM_BIAS_PERCHAN) != 0;
+    t.scale_perchan = (f & W8A8_QM_SCALE_PERCHAN) != 0;
+    t.scale_bf16 = (f & W8A8_QM_SCALE_BF16) != 0;
+    t.has_offset = (f & W8A8_QM_HAS_OFFSET) != 0;
+    t.offset_perchan = (f & W8A8_QM_OFFSET_PERCHAN) != 0;
+    if (t.bias != nullptr && p.bias_batch_stride != 0) {
+        const int64_t esz = (t.bias_kind == W8A8_QM_BIAS_F16 || t.bias_kind == W8A8_QM_BIAS_BF16) ? 2 : 4;
+        t.bias = static_cast<const uint8_t*>(t.bias) + group * p.bias_batch_stride * esz;
+    }
+    return t;
+}
+
+// ((acc + i32 bias) * scale + offset) * pertoken + float bias of NV columns, each operation rounded
+template <int NV>
+__device__ __forceinline__ void qmm_dequant(const GemmParams& p, const QmmTerms& t, int64_t col0, int valid,
+                                            float (&v)[NV])
+{
+    float w[NV];
+    if (t.bias_kind == W8A8_QM_BIAS_I32) {
+        load_vec<NV>(t.bias, col0, t.bias_kind, t.bias_perchan, valid, w);
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            v[j] = __fadd_rn(v[j], w[j]);
+        }
+    }
+    load_vec<NV>(p.scale, col0, t.scale_bf16 ? W8A8_QM_BIAS_BF16 : W8A8_QM_BIAS_F32, t.scale_perchan, valid, w);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        v[j] = __fmul_rn(v[j], w[j]);
+    }
+    if (t.has_offset) {
+        load_vec<NV>(p.offset, col0, W8A8_QM_BIAS_F32, t.offset_perchan, valid, w);
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            v[j] = __fadd_rn(v[j], w[j]);
+        }
+    }
+    if (t.has_pt) {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            v[j] = __fmul_rn(v[j], t.row_mul);
+        }
+    }
+    if (t.bias_kind >= W8A8_QM_BIAS_F16) {
+        load_vec<NV>(t.bias, col0, t.bias_kind, t.bias_perchan, valid, w);
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            v[j] = __fadd_rn(v[j], w[j]);
+        }
+    }
+}
 
 // Requantisation of one finished row of SwiGLU activations, 16-byte pieces [c_lo, c_hi) of it, by one warp:
 // amax clamp at FLT_MIN, y_scale = amax * (1/127), inv = 127 / amax, clamp to [-128, 127], narrowing
@@ -330,30 +404,12 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, const TileInf
         }
     } else {
         // per-tile invariants of the dequant chain, hoisted out of the column loops
-        float row_mul = 1.0f;
-        bool has_pt = false;
-        int bias_kind = W8A8_QM_BIAS_NONE;
-        bool bias_perchan = false, scale_perchan = true, scale_bf16 = false, has_offset = false,
-             offset_perchan = false;
-        const void* bias = p.bias;
-        int64_t vec_base = 0;  // first element of the per-channel vectors for this tile's group
+        [[maybe_unused]] float row_mul = 1.0f;
+        [[maybe_unused]] int bias_kind = W8A8_QM_BIAS_NONE;
+        [[maybe_unused]] QmmTerms terms;
+        [[maybe_unused]] int64_t vec_base = 0;  // first element of the per-channel vectors for this tile's group
         if constexpr (EPI == EPI_QMM) {
-            const int64_t f = p.flags;
-            has_pt = (f & W8A8_QM_HAS_PT) != 0;
-            if (has_pt && row_ok) {
-                // the plugin's layouts make (row mod M) the token index in every case
-                row_mul = p.row_scale[(tl.group == 0) ? row : (row - static_cast<int64_t>(tl.group) * p.M)];
-            }
-            bias_kind = static_cast<int>((f & W8A8_QM_BIAS_MASK) >> W8A8_QM_BIAS_SHIFT);
-            bias_perchan = (f & W8A8_QM_BIAS_PERCHAN) != 0;
-            scale_perchan = (f & W8A8_QM_SCALE_PERCHAN) != 0;
-            scale_bf16 = (f & W8A8_QM_SCALE_BF16) != 0;
-            has_offset = (f & W8A8_QM_HAS_OFFSET) != 0;
-            offset_perchan = (f & W8A8_QM_OFFSET_PERCHAN) != 0;
-            if (bias != nullptr && p.bias_batch_stride != 0) {
-                const int64_t esz = (bias_kind == W8A8_QM_BIAS_F16 || bias_kind == W8A8_QM_BIAS_BF16) ? 2 : 4;
-                bias = static_cast<const uint8_t*>(bias) + tl.group * p.bias_batch_stride * esz;
-            }
+            terms = qmm_terms(p, tl.group, row, row_ok);
         } else if constexpr (EPI == EPI_GMM) {
             if constexpr (KIND == KIND_I8) {
                 row_mul = row_ok ? p.row_scale[row] : 0.0f;
@@ -363,7 +419,6 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, const TileInf
                 const int bdt = static_cast<int>(p.flags & 3);
                 bias_kind = (bdt == W8A8_DT_F16) ? W8A8_QM_BIAS_F16
                                                   : (bdt == W8A8_DT_BF16 ? W8A8_QM_BIAS_BF16 : W8A8_QM_BIAS_F32);
-                bias_perchan = true;
             }
         }
         constexpr int HALF_COLS = BLOCK_N / 2;
@@ -408,51 +463,19 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, const TileInf
                         v[j] = __uint_as_float(r[j]);
                     }
                 }
-                float w[32];
                 if constexpr (EPI == EPI_QMM) {
-                    if (bias_kind == W8A8_QM_BIAS_I32) {
-                        load_vec32(bias, col0, bias_kind, bias_perchan, valid, w);
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            v[j] = __fadd_rn(v[j], w[j]);
-                        }
-                    }
-                    load_vec32(p.scale, col0, scale_bf16 ? W8A8_QM_BIAS_BF16 : W8A8_QM_BIAS_F32, scale_perchan,
-                               valid, w);
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        v[j] = __fmul_rn(v[j], w[j]);
-                    }
-                    if (has_offset) {
-                        load_vec32(p.offset, col0, W8A8_QM_BIAS_F32, offset_perchan, valid, w);
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            v[j] = __fadd_rn(v[j], w[j]);
-                        }
-                    }
-                    if (has_pt) {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            v[j] = __fmul_rn(v[j], row_mul);
-                        }
-                    }
-                    if (bias_kind >= W8A8_QM_BIAS_F16) {
-                        load_vec32(bias, col0, bias_kind, bias_perchan, valid, w);
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            v[j] = __fadd_rn(v[j], w[j]);
-                        }
-                    }
+                    qmm_dequant<32>(p, terms, col0, valid, v);
                 } else {  // EPI_GMM
+                    float w[32];
                     if constexpr (KIND == KIND_I8) {
-                        load_vec32(p.scale, vec_base + col0, W8A8_QM_BIAS_F32, true, valid, w);
+                        load_vec<32>(p.scale, vec_base + col0, W8A8_QM_BIAS_F32, true, valid, w);
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
                             v[j] = __fmul_rn(__fmul_rn(v[j], w[j]), row_mul);
                         }
                     }
                     if (bias_kind != W8A8_QM_BIAS_NONE) {
-                        load_vec32(bias, vec_base + col0, bias_kind, true, valid, w);
+                        load_vec<32>(p.bias, vec_base + col0, bias_kind, true, valid, w);
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
                             v[j] = __fadd_rn(v[j], w[j]);
@@ -524,7 +547,114 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, const TileInf
     }
 }
 
-template <int CG, int BLOCK_N, int KIND, int EPI, bool B_MN, int EPI_WARPS>
+// Split K (SPLITK): the CTAs of a cluster each run the main loop over their share of a tile's K blocks, then deal the
+// tile's columns out in slices: every CTA sends the other CTAs their slices of its accumulator through distributed
+// shared memory (the stage memory, which nothing reads any more), adds what it received to its own slice - int32,
+// so the order does not matter - and runs the dequant chain on it.
+struct SplitSlices {
+    static constexpr int COLS = 16;            // columns exchanged as one piece, 64 bytes per row
+    static constexpr int PIECES = 128 / COLS;  // of a 128-column tile
+    // byte offset of row `row`'s 16-byte word `word` of piece `piece` from source slot `slot`; the words are permuted
+    // by the row so that eight lanes of a store hit eight different bank groups
+    static __device__ __forceinline__ uint32_t offset(int slot, int pieces_per_slice, int piece, int row, int word)
+    {
+        return static_cast<uint32_t>(((slot * pieces_per_slice + piece) * 128 + row) * 64 + ((word ^ ((row >> 1) & 3)) << 4));
+    }
+};
+
+template <int EPI>
+__device__ __forceinline__ void split_send(const GemmParams& p, int m_rows, uint32_t t_addr, int row, int half, int rank,
+                                           uint32_t smem_base)
+{
+    if ((row & ~31) >= m_rows) {
+        return;  // a whole warp
+    }
+    const int per = SplitSlices::PIECES / p.split;
+#pragma unroll 1
+    for (int piece = half; piece < SplitSlices::PIECES; piece += 2) {
+        const int owner = piece / per;
+        if (owner == rank) {
+            continue;
+        }
+        uint32_t r[16];
+        tc::tmem_ld_32x16(t_addr + piece * 16, r);
+        tc::tmem_ld_wait();
+        if (row < m_rows) {
+            const uint32_t to = tc::map_to_cta(smem_base, static_cast<uint32_t>(owner));
+            const int slot = rank < owner ? rank : rank - 1;
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                tc::st_cluster_v4(to + SplitSlices::offset(slot, per, piece - owner * per, row, w), r[4 * w], r[4 * w + 1],
+                                  r[4 * w + 2], r[4 * w + 3]);
+            }
+        }
+    }
+}
+
+template <int EPI>
+__device__ __forceinline__ void split_finish(const GemmParams& p, const TileInfo& tl, uint32_t t_addr, int row_in_tile,
+                                             int half, int rank, const uint8_t* smem)
+{
+    if ((row_in_tile & ~31) >= tl.m_rows) {
+        return;  // a whole warp
+    }
+    const int per = SplitSlices::PIECES / p.split;
+    const bool row_ok = row_in_tile < tl.m_rows;
+    const int64_t row = static_cast<int64_t>(tl.a_row0) + row_in_tile;
+    [[maybe_unused]] QmmTerms terms;
+    if constexpr (EPI == EPI_QMM) {
+        terms = qmm_terms(p, tl.group, row, row_ok);
+    }
+#pragma unroll 1
+    for (int piece = rank * per; piece < (rank + 1) * per; ++piece) {
+        if (per > 1 && (piece & 1) != half) {
+            continue;
+        }
+        if (per == 1 && half != 0) {
+            continue;
+        }
+        uint32_t r[16];
+        tc::tmem_ld_32x16(t_addr + piece * 16, r);
+        tc::tmem_ld_wait();
+        const int64_t col0 = static_cast<int64_t>(tl.nt) * 128 + piece * 16;
+        if (!row_ok || col0 >= p.N) {
+            continue;
+        }
+        for (int slot = 0; slot < p.split - 1; ++slot) {
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                const uint4 o = *reinterpret_cast<const uint4*>(
+                    smem + SplitSlices::offset(slot, per, piece - rank * per, row_in_tile, w));
+                r[4 * w] += o.x, r[4 * w + 1] += o.y, r[4 * w + 2] += o.z, r[4 * w + 3] += o.w;
+            }
+        }
+        if constexpr (EPI == EPI_RAW) {
+            uint4* dst = reinterpret_cast<uint4*>(static_cast<int32_t*>(p.out) + row * p.N + col0);
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                dst[w] = make_uint4(r[4 * w], r[4 * w + 1], r[4 * w + 2], r[4 * w + 3]);
+            }
+        } else {
+            float v[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                v[j] = static_cast<float>(static_cast<int32_t>(r[j]));
+            }
+            qmm_dequant<16>(p, terms, col0, 16, v);
+            uint32_t o[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                o[j] = (p.out_dtype == W8A8_DT_BF16) ? pack2<W8A8_DT_BF16>(v[2 * j], v[2 * j + 1])
+                                                     : pack2<W8A8_DT_F16>(v[2 * j], v[2 * j + 1]);
+            }
+            uint4* dst = reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.out) + row * p.N + col0);
+            dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+            dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+        }
+    }
+}
+
+template <int CG, int BLOCK_N, int KIND, int EPI, bool B_MN, int EPI_WARPS, bool SPLITK>
 __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                    const GemmParams p)
@@ -547,6 +677,8 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
     static_assert(BLOCK_N == 128 || BLOCK_N == 256, "BLOCK_N");
     static_assert(CG == 1 || BLOCK_N == 256, "CTA pairs use 256-column tiles");
     static_assert(EPI != EPI_GMSQ || BLOCK_N == 256, "the SwiGLU epilogue pairs 128 gate with 128 up columns");
+    static_assert(!SPLITK || (CG == 1 && BLOCK_N == 128 && KIND == KIND_I8 && (EPI == EPI_QMM || EPI == EPI_RAW)),
+                  "split K: dense int8 matmuls on single-CTA tiles of 128 columns");
     static_assert(EPI_WARPS == 8 || (EPI_WARPS == 16 && EPI == EPI_GMSQ), "16 epilogue warps: SwiGLU epilogue only");
 
     extern __shared__ uint8_t smem_raw[];
@@ -562,6 +694,15 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
     const int lane = threadIdx.x & 31;
     const uint32_t cta_rank = (CG == 2) ? tc::cluster_ctarank() : 0u;
     const bool leader = (cta_rank == 0);
+    // this CTA's share of the K blocks
+    int kb_first = 0, kb_last = p.num_k_blocks;
+    [[maybe_unused]] int split_rank = 0;
+    if constexpr (SPLITK) {
+        split_rank = static_cast<int>(tc::cluster_ctarank());
+        // the host splits no finer than one K block each: no share is empty
+        kb_first = static_cast<int>(static_cast<int64_t>(split_rank) * p.num_k_blocks / p.split);
+        kb_last = static_cast<int>(static_cast<int64_t>(split_rank + 1) * p.num_k_blocks / p.split);
+    }
     const uint32_t smem_base = tc::smem_u32(smem);
     const uint32_t bar_base = tc::smem_u32(bars);
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
@@ -610,8 +751,9 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
         total_tiles = static_cast<int64_t>(dense_m_tiles) * p.n_tiles;
     }
     const int64_t H = p.N / 2;  // GMSQ half width
-    const int64_t worker = blockIdx.x / CG;
-    const int64_t num_workers = gridDim.x / CG;
+    const int64_t ctas_per_tile = SPLITK ? p.split : CG;
+    const int64_t worker = blockIdx.x / ctas_per_tile;
+    const int64_t num_workers = gridDim.x / ctas_per_tile;
 
     auto decode = [&](int64_t t) {
         TileInfo tl;
@@ -666,12 +808,12 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
             const uint32_t full0 = (CG == 2) ? tc::map_to_cta(full_bar(0), 0) : full_bar(0);
             for (int64_t t = worker; ok && t < total_tiles; t += num_workers) {
                 const TileInfo tl = decode(t);
-                for (int kb0 = 0; kb0 < p.num_k_blocks; kb0 += KPS) {
+                for (int kb0 = kb_first; kb0 < kb_last; kb0 += KPS) {
                     if (!tc::mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) {
                         ok = false;
                         break;
                     }
-                    const int left = p.num_k_blocks - kb0;
+                    const int left = kb_last - kb0;
                     const int n_sub = left < KPS ? left : KPS;  // K blocks this stage carries (the tile's last may be short)
                     const uint32_t fb = full0 + 8u * stage;
                     // Only the leader announces the bytes (its own and its partner's).  The partner's copies may
@@ -761,7 +903,7 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
                 tc::tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BLOCK_N);
                 uint32_t accumulate = 0;
-                for (int kb0 = 0; kb0 < p.num_k_blocks; kb0 += KPS) {
+                for (int kb0 = kb_first; kb0 < kb_last; kb0 += KPS) {
                     // The copies are consumed by the tensor core (async proxy), not by this thread: the barrier's
                     // default acquire plus the tcgen05 fence is what orders them, also for the partner CTA's
                     // copies that complete on this barrier.
@@ -770,7 +912,7 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
                         break;
                     }
                     tc::tc_fence_after_sync();
-                    const int left = p.num_k_blocks - kb0;
+                    const int left = kb_last - kb0;
                     const int n_sub = left < KPS ? left : KPS;
 #pragma unroll
                     for (int sub = 0; sub < KPS; ++sub) {
@@ -875,6 +1017,9 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
                 break;
             }
             tc::tc_fence_after_sync();
+            if constexpr (SPLITK) {
+                break;  // one tile per cluster: its accumulators are exchanged below, by all warps together
+            }
             const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                                     static_cast<uint32_t>(acc * BLOCK_N);
             epilogue_tile<BLOCK_N, KIND, EPI, EPI_WARPS>(p, tl, t_addr, row_in_tile, col_half, H, no_epilogue, stage);
@@ -915,6 +1060,30 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
                 requant_share(late);
             }
         }
+    }
+
+    if constexpr (SPLITK) {
+        // Every CTA of the cluster has its accumulator: nothing reads the stage memory any more.
+        __syncwarp();
+        tc::tc_fence_before_sync();
+        tc::cluster_arrive();
+        tc::cluster_wait();
+        tc::tc_fence_after_sync();
+        const bool mine = warp >= 2 && worker < total_tiles && *abort_flag == 0;
+        const int row_in_tile = (warp & 3) * 32 + lane;
+        const uint32_t t_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+        TileInfo tl{};
+        if (mine) {
+            tl = decode(worker);
+            split_send<EPI>(p, tl.m_rows, t_addr, row_in_tile, (warp - 2) >> 2, split_rank, smem_base);
+        }
+        __syncwarp();
+        tc::cluster_arrive();
+        tc::cluster_wait();
+        if (mine) {
+            split_finish<EPI>(p, tl, t_addr, row_in_tile, (warp - 2) >> 2, split_rank, smem);
+        }
+        __syncwarp();
     }
 
     // ---- teardown ----

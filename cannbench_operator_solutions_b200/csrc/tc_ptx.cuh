@@ -259,6 +259,13 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank)
     return r;
 }
 
+// 16 bytes to the shared memory of a CTA of this cluster (address from map_to_cta)
+__device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d)
+{
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d)
+                 : "memory");
+}
+
 __device__ __forceinline__ void cluster_arrive()
 {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
