@@ -151,12 +151,10 @@ static cudaError_t launch(const void* x1, const void* x2, const void* gamma, int
 {
     auto kern = ardq_rows_kernel<DT, CPT, VEC, DIRECT>;
     int per_sm = 1;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ARDQ_THREADS, 0);
+    static KernelFacts facts;
+    const cudaError_t e = resident_ctas(facts, kern, ARDQ_THREADS, &per_sm);
     if (e != cudaSuccess) {
         return e;
-    }
-    if (per_sm < 1) {
-        per_sm = 1;
     }
     const int64_t cap = static_cast<int64_t>(sm_count()) * per_sm;
     const unsigned grid = static_cast<unsigned>(rows < cap ? rows : cap);

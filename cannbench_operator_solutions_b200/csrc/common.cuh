@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/w8a8ffn.h"
 
 namespace w8a8 {
@@ -478,6 +480,58 @@ __device__ __forceinline__ uint32_t chunk_absmax16(uint4 v, uint32_t m2)
 inline bool is_aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 
 int sm_count();  // cached multiprocessor count of the current device
+
+// Launch facts of one kernel that hold for the life of the process, asked for once per device (the queries cost 1 - 2 us
+// each, a good part of a small call).  Racing first calls store the same values.
+constexpr int MAX_CACHED_DEVICES = 64;
+struct KernelFacts {
+    std::atomic<int> value[MAX_CACHED_DEVICES];  // 0: not asked yet
+};
+
+// resident CTAs per SM, at least 1
+template <typename Kernel>
+cudaError_t resident_ctas(KernelFacts& facts, Kernel kern, int threads, int* ctas)
+{
+    int dev = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    const bool keep = dev >= 0 && dev < MAX_CACHED_DEVICES;
+    int n = keep ? facts.value[dev].load(std::memory_order_relaxed) : 0;
+    if (n == 0) {
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, 0);
+        if (e != cudaSuccess) {
+            return e;
+        }
+        n = n < 1 ? 1 : n;
+        if (keep) {
+            facts.value[dev].store(n, std::memory_order_relaxed);
+        }
+    }
+    *ctas = n;
+    return cudaSuccess;
+}
+
+// lets a kernel use `bytes` of dynamic shared memory on the current device
+template <typename Kernel>
+cudaError_t allow_dynamic_smem(KernelFacts& facts, Kernel kern, size_t bytes)
+{
+    int dev = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    const bool keep = dev >= 0 && dev < MAX_CACHED_DEVICES;
+    if (keep && facts.value[dev].load(std::memory_order_relaxed) != 0) {
+        return cudaSuccess;
+    }
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    if (e == cudaSuccess && keep) {
+        facts.value[dev].store(1, std::memory_order_relaxed);
+    }
+    return e;
+}
 void note_launch();  // counts one kernel launch of this library (w8a8_kernel_launch_count)
 
 }  // namespace w8a8

@@ -126,12 +126,10 @@ static cudaError_t launch_rows(const void* x, int8_t* y, float* scale, int64_t M
 {
     auto kern = dq_rows_kernel<DT, THREADS, CPT, VEC, DIRECT>;
     int per_sm = 1;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, 0);
+    static KernelFacts facts;
+    const cudaError_t e = resident_ctas(facts, kern, THREADS, &per_sm);
     if (e != cudaSuccess) {
         return e;
-    }
-    if (per_sm < 1) {
-        per_sm = 1;
     }
     const int64_t cap = static_cast<int64_t>(sm_count()) * per_sm;
     const unsigned grid = static_cast<unsigned>(M < cap ? M : cap);

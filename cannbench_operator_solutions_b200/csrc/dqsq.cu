@@ -21,6 +21,8 @@
 // as many threads as that takes.  The fp32 results stay in registers between the row maximum and the quantisation,
 // so x is read once and y written once: 8H + H + 4 bytes per row for int32 input, 4H + H + 4 for 16-bit input; the
 // next row's chunks are requested before the barrier of the present one.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace w8a8 {
@@ -407,6 +409,7 @@ static cudaError_t dispatch_dqsq(const void* x, const float* ws, const float* as
                           int, int);
     Kern kern = dqsq_long_rows_kernel<XT>;
     int threads = DQSQ_THREADS;
+    int regs = 40;
     if (vec && chunks <= 2 * DQSQ_MAX_THREADS) {
         // Two chunks of each half per thread (one where a row has at most a warp's worth), rounded up to whole warps:
         // a thread count fitted to the row leaves few lanes idle on rows that are not a power of two long.  (Four
@@ -414,6 +417,7 @@ static cudaError_t dispatch_dqsq(const void* x, const float* ws, const float* as
         // 56-register form up to 576 threads: it puts two CTAs on an SM (24 against 27 us on fp16 [1531, 18432]).
         const bool two = chunks > 32;
         threads = static_cast<int>((((two ? (chunks + 1) / 2 : chunks) + 31) / 32) * 32);
+        regs = (XT == DQSQ_X_I32 && two) || threads > DQSQ_PAIR_THREADS ? 64 : 56;
         if (!two) {
             kern = dqsq_rows_kernel<XT, 1, true, DQSQ_PAIR_THREADS>;  // rows this short always divide
         } else if (XT == DQSQ_X_I32) {
@@ -426,13 +430,9 @@ static cudaError_t dispatch_dqsq(const void* x, const float* ws, const float* as
             kern = dqsq_rows_kernel<XT, 2, false, DQSQ_MAX_THREADS>;
         }
     }
-    // one wave: as many CTAs as are resident at once, each walking rows with a grid stride
-    int per_sm = 1;
-    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, 0);
-    if (e != cudaSuccess) {
-        return e;
-    }
-    const int64_t cap = static_cast<int64_t>(sm_count()) * (per_sm < 1 ? 1 : per_sm);
+    // one wave: as many CTAs as the registers hold at once, each walking rows with a grid stride
+    const int64_t per_sm = std::max<int64_t>(1, (65536 / (regs * threads)));
+    const int64_t cap = static_cast<int64_t>(sm_count()) * std::min<int64_t>(per_sm, 32);
     const unsigned grid = static_cast<unsigned>(M < cap ? M : cap);
     kern<<<grid, threads, 0, st>>>(x, ws, as, qs, y, scale, M, H, left, direct, divide); w8a8::note_launch();
     return cudaGetLastError();

@@ -107,8 +107,8 @@ static cudaError_t launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, con
 {
     auto kern = gemm_tc_kernel<CG, BLOCK_N, KIND, EPI, B_MN, EPI_WARPS, SPLITK>;
     constexpr size_t smem = gemm_smem_bytes<CG, BLOCK_N>();
-    // the attribute is per device; setting it on every call is cheap and covers multi-GPU processes
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    static KernelFacts facts;
+    const cudaError_t e = allow_dynamic_smem(facts, kern, smem);
     if (e != cudaSuccess) {
         return e;
     }

@@ -10,6 +10,7 @@ device memory and the stream.
 """
 from __future__ import annotations
 
+from array import array
 from typing import List, Optional, Sequence, Tuple, Union
 
 import torch
@@ -22,8 +23,14 @@ def _check(cond: bool, msg: str) -> None:
         raise RuntimeError(msg)
 
 
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+def _call(device: torch.device, fn, *args) -> int:
+    """``fn(*args, stream)`` with ``device`` current, on its current stream.  (The device guard and the Stream object
+    of torch.cuda cost 6 us, more than the launch; they are only needed when another device is current.)"""
+    index = device.index
+    if index == torch._C._cuda_getDevice():
+        return fn(*args, torch._C._cuda_getCurrentRawStream(index))
+    with torch.cuda.device(device):
+        return fn(*args, torch._C._cuda_getCurrentRawStream(index))
 
 
 def _status(rc: int, op: str) -> None:
@@ -70,9 +77,8 @@ def dynamic_quant(x: torch.Tensor, *, round_direct: bool = False) -> Tuple[torch
     m = xc.numel() // n
     if m <= 0:
         return y, scale
-    with torch.cuda.device(xc.device):
-        rc = L.load().w8a8_dynamic_quant(xc.data_ptr(), y.data_ptr(), scale.data_ptr(), m, n, _dt(xc),
-                                         L.F_ROUND_DIRECT if round_direct else 0, _stream())
+    rc = _call(xc.device, L.load().w8a8_dynamic_quant, xc.data_ptr(), y.data_ptr(), scale.data_ptr(), m, n, _dt(xc),
+               L.F_ROUND_DIRECT if round_direct else 0)
     _status(rc, "dynamic_quant")
     return y, scale
 
@@ -98,10 +104,9 @@ def add_rms_norm_dynamic_quant(x1: torch.Tensor, x2: torch.Tensor, gamma: torch.
            "add_rms_norm_dynamic_quant: only float16/bfloat16 inputs are supported.")
     _check(n <= 16384, "add_rms_norm_dynamic_quant: row length must not exceed 16384.")
     rows = x1c.numel() // n
-    with torch.cuda.device(x1c.device):
-        rc = L.load().w8a8_add_rms_norm_dynamic_quant(x1c.data_ptr(), x2c.data_ptr(), gc.data_ptr(), y.data_ptr(),
-                                                      x_out.data_ptr(), scale.data_ptr(), rows, n, float(epsilon),
-                                                      _dt(x1c), L.F_ROUND_DIRECT if round_direct else 0, _stream())
+    rc = _call(x1c.device, L.load().w8a8_add_rms_norm_dynamic_quant, x1c.data_ptr(), x2c.data_ptr(), gc.data_ptr(),
+               y.data_ptr(), x_out.data_ptr(), scale.data_ptr(), rows, n, float(epsilon), _dt(x1c),
+               L.F_ROUND_DIRECT if round_direct else 0)
     _status(rc, "add_rms_norm_dynamic_quant")
     return y, x_out, scale
 
@@ -166,11 +171,9 @@ def quant_matmul(x1: torch.Tensor, x2: torch.Tensor, scale: torch.Tensor, *, off
             flags |= L.QM_BIAS_PERCHAN
     if batch > 1:
         flags |= L.QM_PT_MOD_M
-    with torch.cuda.device(x1.device):
-        rc = L.load().w8a8_quant_matmul(x1.data_ptr(), x2.data_ptr(), scale.data_ptr(), _ptr(offset),
-                                        _ptr(pertoken_scale), _ptr(bias), out.data_ptr(), batch, m, n, k, flags,
-                                        L.DT_BF16 if bf16out else L.DT_F16, L.W_NK if transpose_x2 else L.W_KN,
-                                        bias_batch_stride, _stream())
+    rc = _call(x1.device, L.load().w8a8_quant_matmul, x1.data_ptr(), x2.data_ptr(), scale.data_ptr(), _ptr(offset),
+               _ptr(pertoken_scale), _ptr(bias), out.data_ptr(), batch, m, n, k, flags,
+               L.DT_BF16 if bf16out else L.DT_F16, L.W_NK if transpose_x2 else L.W_KN, bias_batch_stride)
     _status(rc, "quant_matmul")
     return out
 
@@ -185,15 +188,23 @@ def _group_list(group_list: GroupList, e: int, m: int, op: str):
         _check(group_list.dtype == torch.int64 and group_list.is_contiguous() and group_list.numel() == e,
                f"{op}: a device group_list must be a contiguous int64 tensor of length E")
         return group_list.data_ptr(), 1, group_list
-    vals = [int(v) for v in (group_list.tolist() if isinstance(group_list, torch.Tensor) else group_list)]
-    _check(len(vals) == e, f"{op}: group_list length must equal the expert count")
-    prev = 0
-    for v in vals:
-        _check(prev <= v <= m, f"{op}: group_list must be a cumsum <= M")
-        prev = v
-    _check(prev == m, f"{op}: group_list[-1] must equal M")
-    host = torch.tensor(vals, dtype=torch.int64)
-    return host.data_ptr(), 0, host
+    vals = group_list.tolist() if isinstance(group_list, torch.Tensor) else list(group_list)
+    try:
+        host = array("q", vals)
+        vals = host.tolist()
+    except (TypeError, OverflowError):
+        vals, host = [int(v) for v in vals], None
+    # the whole list at once; one by one only to say what is wrong
+    if len(vals) != e or not vals or vals[0] < 0 or vals[-1] != m or sorted(vals) != vals:
+        _check(len(vals) == e, f"{op}: group_list length must equal the expert count")
+        prev = 0
+        for v in vals:
+            _check(prev <= v <= m, f"{op}: group_list must be a cumsum <= M")
+            prev = v
+        _check(prev == m, f"{op}: group_list[-1] must equal M")
+    if host is None:
+        host = array("q", vals)
+    return host.buffer_info()[0], 0, host
 
 
 def grouped_matmul_swiglu_quant(x: torch.Tensor, weight: torch.Tensor, weight_scale: torch.Tensor,
@@ -235,12 +246,10 @@ def grouped_matmul_swiglu_quant(x: torch.Tensor, weight: torch.Tensor, weight_sc
         workspace = torch.empty((need,), dtype=torch.uint8, device=xc.device)
     _check(workspace.is_cuda and workspace.numel() * workspace.element_size() >= need,
            "grouped_matmul_swiglu_quant: workspace too small")
-    with torch.cuda.device(xc.device):
-        rc = lib.w8a8_grouped_matmul_swiglu_quant(xc.data_ptr(), wc.data_ptr(), wsc.data_ptr(), xsc.data_ptr(),
-                                                  y.data_ptr(), y_scale.data_ptr(), m, k, n, e, gl_ptr, on_dev,
-                                                  L.W_NK if transpose_weight else L.W_KN,
-                                                  L.F_ROUND_DIRECT if round_direct else 0, workspace.data_ptr(),
-                                                  workspace.numel() * workspace.element_size(), _stream())
+    rc = _call(xc.device, lib.w8a8_grouped_matmul_swiglu_quant, xc.data_ptr(), wc.data_ptr(), wsc.data_ptr(),
+               xsc.data_ptr(), y.data_ptr(), y_scale.data_ptr(), m, k, n, e, gl_ptr, on_dev,
+               L.W_NK if transpose_weight else L.W_KN, L.F_ROUND_DIRECT if round_direct else 0, workspace.data_ptr(),
+               workspace.numel() * workspace.element_size())
     del keep
     _status(rc, "grouped_matmul_swiglu_quant")
     return y, y_scale
@@ -298,11 +307,10 @@ def grouped_matmul(x: torch.Tensor, weight: torch.Tensor, group_list: GroupList,
         _check(workspace.numel() * workspace.element_size() >= need, "grouped_matmul: workspace too small")
         xs = x_scale.contiguous() if x_scale is not None else None
         ws = weight_scale.contiguous() if weight_scale is not None else None
-        with torch.cuda.device(xc.device):
-            rc = lib.w8a8_grouped_matmul(xc.data_ptr(), wc.data_ptr(), _ptr(bc), y.data_ptr(), _ptr(xs), _ptr(ws), m,
-                                         n, k, e, gl_ptr, on_dev, dt, _dt(bc) if bc is not None else dt,
-                                         _dt(y), L.W_NK if transpose_weight else L.W_KN, workspace.data_ptr(),
-                                         workspace.numel() * workspace.element_size(), _stream())
+        rc = _call(xc.device, lib.w8a8_grouped_matmul, xc.data_ptr(), wc.data_ptr(), _ptr(bc), y.data_ptr(), _ptr(xs),
+                   _ptr(ws), m, n, k, e, gl_ptr, on_dev, dt, _dt(bc) if bc is not None else dt, _dt(y),
+                   L.W_NK if transpose_weight else L.W_KN, workspace.data_ptr(),
+                   workspace.numel() * workspace.element_size())
         _status(rc, "grouped_matmul")
     del keep
     if split_item in (0, 1):
@@ -359,11 +367,9 @@ def moe_re_routing(tokens: torch.Tensor, expert_token_num_per_rank: torch.Tensor
     if workspace is None:
         workspace = torch.empty((need,), dtype=torch.uint8, device=tok.device)
     _check(workspace.numel() * workspace.element_size() >= need, "moe_re_routing: workspace too small")
-    with torch.cuda.device(tok.device):
-        rc = lib.w8a8_moe_re_routing(tok.data_ptr(), cnt.data_ptr(), _ptr(scl), out_tok.data_ptr(),
-                                     out_scl.data_ptr(), out_idx.data_ptr(), out_num.data_ptr(), a,
-                                     h * tok.element_size(), n, e, cnt.element_size(), workspace.data_ptr(),
-                                     workspace.numel() * workspace.element_size(), _stream())
+    rc = _call(tok.device, lib.w8a8_moe_re_routing, tok.data_ptr(), cnt.data_ptr(), _ptr(scl), out_tok.data_ptr(),
+               out_scl.data_ptr(), out_idx.data_ptr(), out_num.data_ptr(), a, h * tok.element_size(), n, e,
+               cnt.element_size(), workspace.data_ptr(), workspace.numel() * workspace.element_size())
     _status(rc, "moe_re_routing")
     return out_tok, out_scl, out_idx, out_num
 
@@ -419,11 +425,10 @@ def moe_finalize_routing(expanded_permuted_rows: torch.Tensor, expanded_src_to_d
     bs = bias.contiguous() if has_bias else None
     sc = scales.contiguous() if scales is not None else None
     ex = expert_for_source_row.contiguous() if expert_for_source_row is not None else None
-    with torch.cuda.device(epr.device):
-        rc = L.load().w8a8_moe_finalize_routing(eprc.data_ptr(), esdr.data_ptr(), _ptr(s1), _ptr(s2), _ptr(bs), _ptr(sc),
-                                                _ptr(ex) if has_bias else None, out.data_ptr(), num_rows, h, k,
-                                                bs.size(0) if has_bias else 0, eprc.numel() // h, mode, _dt(eprc),
-                                                _dt(sc) if sc is not None else _dt(eprc), _stream())
+    rc = _call(epr.device, L.load().w8a8_moe_finalize_routing, eprc.data_ptr(), esdr.data_ptr(), _ptr(s1), _ptr(s2),
+               _ptr(bs), _ptr(sc), _ptr(ex) if has_bias else None, out.data_ptr(), num_rows, h, k,
+               bs.size(0) if has_bias else 0, eprc.numel() // h, mode, _dt(eprc),
+               _dt(sc) if sc is not None else _dt(eprc))
     _status(rc, "moe_finalize_routing")
     return out
 
@@ -456,9 +461,8 @@ def moe_gating_top_k_softmax(x: torch.Tensor, finished: Optional[torch.Tensor] =
     if finished is not None:
         fin = finished.contiguous()
         _check(fin.numel() == rows, "cann_bench.moe_gating_top_k_softmax: finished must have numel == rows.")
-    with torch.cuda.device(xc.device):
-        rc = L.load().w8a8_moe_gating_top_k_softmax(xc.data_ptr(), _ptr(fin), y.data_ptr(), ei.data_ptr(),
-                                                    ri.data_ptr(), rows, inner, k, _dt(xc), _stream())
+    rc = _call(xc.device, L.load().w8a8_moe_gating_top_k_softmax, xc.data_ptr(), _ptr(fin), y.data_ptr(),
+               ei.data_ptr(), ri.data_ptr(), rows, inner, k, _dt(xc))
     _status(rc, "moe_gating_top_k_softmax")
     return y, ei, ri
 
@@ -502,10 +506,8 @@ def dequant_swiglu_quant(x: torch.Tensor, weight_scale: Optional[torch.Tensor] =
         _check(quant_scale.dtype == torch.float32, "quant_scale must be float32.")
         _check(quant_scale.is_contiguous(), "quant_scale must be contiguous.")
         _check(quant_scale.numel() == h, "quant_scale must have H elements.")
-    with torch.cuda.device(x.device):
-        rc = L.load().w8a8_dequant_swiglu_quant(x.data_ptr(), _ptr(weight_scale), _ptr(activation_scale),
-                                                _ptr(quant_scale), y.data_ptr(), scale.data_ptr(), m, h, _dt(x),
-                                                1 if activate_left else 0, L.F_ROUND_DIRECT if round_direct else 0,
-                                                _stream())
+    rc = _call(x.device, L.load().w8a8_dequant_swiglu_quant, x.data_ptr(), _ptr(weight_scale), _ptr(activation_scale),
+               _ptr(quant_scale), y.data_ptr(), scale.data_ptr(), m, h, _dt(x), 1 if activate_left else 0,
+               L.F_ROUND_DIRECT if round_direct else 0)
     _status(rc, "dequant_swiglu_quant")
     return y, scale
