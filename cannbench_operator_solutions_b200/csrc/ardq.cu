@@ -32,6 +32,7 @@ __global__ void __launch_bounds__(ARDQ_THREADS)
     constexpr int WARPS = ARDQ_THREADS / 32;
     __shared__ float s_sum[2][WARPS];
     __shared__ uint32_t s_max[2][WARPS];
+    after_previous(x1, x2, gamma, y, x_out, scale_out);
     const int tid = threadIdx.x;
     const int nchunks = static_cast<int>((N + 7) / 8);
     int parity = 0;
@@ -159,10 +160,9 @@ static cudaError_t launch(const void* x1, const void* x2, const void* gamma, int
     const int64_t cap = static_cast<int64_t>(sm_count()) * per_sm;
     const unsigned grid = static_cast<unsigned>(rows < cap ? rows : cap);
     const float inv_n = 1.0f / static_cast<float>(N);
-    kern<<<grid, ARDQ_THREADS, 0, st>>>(static_cast<const uint16_t*>(x1), static_cast<const uint16_t*>(x2),
-                                        static_cast<const uint16_t*>(gamma), y, static_cast<uint16_t*>(x_out),
-                                        scale_out, rows, N, eps, inv_n); w8a8::note_launch();
-    return cudaGetLastError();
+    return launch_chained(kern, grid, ARDQ_THREADS, 0, st, static_cast<const uint16_t*>(x1),
+                          static_cast<const uint16_t*>(x2), static_cast<const uint16_t*>(gamma), y,
+                          static_cast<uint16_t*>(x_out), scale_out, rows, N, eps, inv_n);
 }
 
 template <int DT, bool VEC, bool DIRECT>

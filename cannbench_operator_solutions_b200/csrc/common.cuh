@@ -477,6 +477,44 @@ __device__ __forceinline__ uint32_t chunk_absmax16(uint4 v, uint32_t m2)
     return m2;
 }
 
+void note_launch();  // counts one kernel launch of this library (w8a8_kernel_launch_count)
+
+// ---------------------------------------------------------------------------
+// Programmatic dependent launch.  A kernel launched with launch_chained may start while the kernel before it on the
+// stream is still running: its launch, block setup and prologue then overlap that kernel's tail instead of following
+// it.  Every such kernel opens with after_previous(), which lets the next kernel do the same and then waits until the
+// kernel before it has completed and its writes are visible; no global memory is touched before that, neither read
+// nor written.  The pointers pass through the wait so that no load through them is moved above it.  Kernels that are
+// launched plainly (and memsets, copies, event waits) order themselves against these as against any other.
+// A dense layer of 16 rows 53.9 us (61.5 before), an expert layer of 2000 rows 160 (184) and of 64 rows 116 (129), a
+// grouped SwiGLU matmul of 512 rows 38 (42), regroup and combine of 8192 rows 56 (62).
+// ---------------------------------------------------------------------------
+template <typename... Pointers>
+__device__ __forceinline__ void after_previous(Pointers&... pointers)
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    (void(([&] { asm volatile("" : "+l"(pointers)); })()), ...);
+}
+
+template <typename... Params, typename... Args>
+cudaError_t launch_chained(void (*kern)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+                           Args&&... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(block, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    note_launch();
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+}
+
 inline bool is_aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 
 int sm_count();  // cached multiprocessor count of the current device
@@ -532,6 +570,5 @@ cudaError_t allow_dynamic_smem(KernelFacts& facts, Kernel kern, size_t bytes)
     }
     return e;
 }
-void note_launch();  // counts one kernel launch of this library (w8a8_kernel_launch_count)
 
 }  // namespace w8a8

@@ -22,6 +22,7 @@ __global__ void __launch_bounds__(THREADS) dq_rows_kernel(const uint16_t* __rest
 {
     constexpr int WARPS = THREADS / 32;
     __shared__ uint32_t s_max[2][WARPS];
+    after_previous(x, y, scale);
     const int tid = threadIdx.x;
     const int nchunks = static_cast<int>((N + 7) / 8);
     int parity = 0;
@@ -133,8 +134,7 @@ static cudaError_t launch_rows(const void* x, int8_t* y, float* scale, int64_t M
     }
     const int64_t cap = static_cast<int64_t>(sm_count()) * per_sm;
     const unsigned grid = static_cast<unsigned>(M < cap ? M : cap);
-    kern<<<grid, THREADS, 0, st>>>(static_cast<const uint16_t*>(x), y, scale, M, N); w8a8::note_launch();
-    return cudaGetLastError();
+    return launch_chained(kern, grid, THREADS, 0, st, static_cast<const uint16_t*>(x), y, scale, M, N);
 }
 
 template <int DT, bool VEC, bool DIRECT>

@@ -241,6 +241,7 @@ __global__ void __launch_bounds__(MAX_THREADS, MAX_THREADS <= DQSQ_PAIR_THREADS 
     constexpr int GN = GROUP * EL;
     constexpr size_t ELEM = (XT == DQSQ_X_I32) ? 4 : 2;
     __shared__ float s_red[2 * 32];
+    after_previous(x, weight_scale, activation_scale, quant_scale, y, scale);
     const int tid = threadIdx.x;
     const int threads = static_cast<int>(blockDim.x);
     const int nchunks = static_cast<int>(H / EL);
@@ -362,6 +363,7 @@ __global__ void __launch_bounds__(DQSQ_THREADS) dqsq_long_rows_kernel(const void
 {
     using C = DqsqChunk<XT>;
     __shared__ float s_red[2 * 32];
+    after_previous(x, weight_scale, activation_scale, quant_scale, y, scale);
     const size_t elem = (XT == DQSQ_X_I32) ? 4 : 2;
     const bool has_q = (quant_scale != nullptr);
     int parity = 0;
@@ -434,8 +436,8 @@ static cudaError_t dispatch_dqsq(const void* x, const float* ws, const float* as
     const int64_t per_sm = std::max<int64_t>(1, (65536 / (regs * threads)));
     const int64_t cap = static_cast<int64_t>(sm_count()) * std::min<int64_t>(per_sm, 32);
     const unsigned grid = static_cast<unsigned>(M < cap ? M : cap);
-    kern<<<grid, threads, 0, st>>>(x, ws, as, qs, y, scale, M, H, left, direct, divide); w8a8::note_launch();
-    return cudaGetLastError();
+    return launch_chained(kern, grid, static_cast<unsigned>(threads), 0, st, x, ws, as, qs, y, scale, M, H, left, direct,
+                          divide);
 }
 
 }  // namespace w8a8

@@ -37,6 +37,7 @@ __device__ __forceinline__ int rp_expert(const int32_t* expert_idx, int64_t p, i
 __global__ void __launch_bounds__(RP_THREADS) rp_histogram_kernel(const int32_t* __restrict__ expert_idx, int64_t P,
                                                                   int E, int32_t* __restrict__ block_count)
 {
+    after_previous(expert_idx, block_count);
     __shared__ int32_t s_cnt[RP_MAX_EXPERTS];
     for (int e = threadIdx.x; e < E; e += RP_THREADS) {
         s_cnt[e] = 0;
@@ -59,6 +60,7 @@ __global__ void __launch_bounds__(RP_THREADS) rp_histogram_kernel(const int32_t*
 __global__ void __launch_bounds__(1024) rp_prefix_kernel(int32_t* __restrict__ block_count, int64_t B, int E,
                                                          int64_t* __restrict__ count)
 {
+    after_previous(block_count, count);
     __shared__ int32_t s_part[32][33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int e = blockIdx.x * 32 + lane;
@@ -97,6 +99,7 @@ __global__ void __launch_bounds__(RP_THREADS) rp_rank_kernel(const int32_t* __re
                                                              int64_t* __restrict__ count, int64_t* __restrict__ cumsum,
                                                              int64_t* __restrict__ expanded_pos)
 {
+    after_previous(expert_idx, block_prefix, count, cumsum, expanded_pos);
     constexpr int ITS = RP_PAIRS / RP_THREADS;
     constexpr int PER = RP_MAX_EXPERTS / RP_THREADS;  // experts per thread in the scan
     __shared__ int64_t s_next[RP_MAX_EXPERTS];        // where the next pair of each expert goes
@@ -331,6 +334,7 @@ __global__ void __launch_bounds__(256) permute_rows_kernel(const uint8_t* __rest
                                                            const int64_t* __restrict__ index, int64_t rows,
                                                            int64_t row_bytes)
 {
+    after_previous(src, src_scale, dst, dst_scale, index);
     const int lane = threadIdx.x & 31;
     const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
     for (int64_t d = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); d < rows;
@@ -387,6 +391,7 @@ __global__ void __launch_bounds__(256) dispatch_rows_kernel(const uint8_t* __res
                                                             const int64_t* __restrict__ my_base, int64_t T, int topk,
                                                             int64_t row_bytes)
 {
+    after_previous(src, src_scale, expert_idx, pos, row_dst, scale_dst, my_base);
     __shared__ uint64_t s_dst[64];
     for (int64_t i = blockIdx.x; i < T; i += gridDim.x) {
         __syncthreads();
@@ -437,6 +442,7 @@ __global__ void __launch_bounds__(256) expand_row_pointers_kernel(const int64_t*
                                                                   int64_t rows, int64_t row_bytes,
                                                                   uint64_t* __restrict__ out)
 {
+    after_previous(seg_first, seg_ptr, out);
     const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (r >= rows) {
         return;
@@ -569,6 +575,7 @@ __global__ void __launch_bounds__(1024) rr_table_small_kernel(const CntT* __rest
                                                               int64_t* __restrict__ src_first,
                                                               CntT* __restrict__ expert_num)
 {
+    after_previous(cnt, hdr, dst_first, src_first, expert_num);
     __shared__ int64_t s_cnt[RR_SMALL_CELLS];
     // E + N <= cells + 1, so one array of cells + 2 entries holds both prefixes: columns first, rows after them
     __shared__ int64_t s_sums[RR_SMALL_CELLS + 2];
@@ -657,6 +664,7 @@ __global__ void __launch_bounds__(256) rr_index_kernel(const int32_t* __restrict
                                                        int64_t A, int64_t* __restrict__ index,
                                                        int32_t* __restrict__ out_idx)
 {
+    after_previous(hdr, dst_first, src_first, index, out_idx);
     const int64_t d = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (d >= A) {
         return;
@@ -778,6 +786,7 @@ __global__ void __launch_bounds__(256) mfr_kernel(const void* __restrict__ rows,
                                                   int64_t R, int64_t H, int K, int64_t E, int64_t num_dst,
                                                   int col_mode, int scale_dt)
 {
+    after_previous(rows, esdr, skip1, skip2, bias, scales, expert, out);
     using C = RowChunk<DT>;
     constexpr int EL = C::EL;
     __shared__ int64_t s_pos[MFR_MAX_STAGED_K];
@@ -940,6 +949,7 @@ __global__ void __launch_bounds__(EP_THREADS) ep_tables_kernel(const int64_t* __
                                                          int64_t* __restrict__ seg_first,
                                                          uint64_t* __restrict__ seg_ptr, int32_t* __restrict__ status)
 {
+    after_previous(counts, peer_base, row_dst, scale_dst, my_base, group_list, seg_first, seg_ptr, status);
     // Row counts fit 32 bits (a rank's buffers hold fewer than 2^31 rows; larger counts set the overflow flag).
     __shared__ int32_t s_cnt[EP_MAX_CELLS];       // [P][E]
     __shared__ int64_t s_base[EP_MAX_CELLS + 1];  // exclusive prefix of s_cnt over all cells, rank-major
@@ -1085,11 +1095,15 @@ extern "C" int w8a8_route_plan(const int32_t* expert_idx, int64_t T, int64_t top
         const int experts = static_cast<int>(E);
         const int64_t ctas = (P + w8a8::RP_PAIRS - 1) / w8a8::RP_PAIRS;
         if (ctas <= 1) {
-            w8a8::rp_rank_kernel<true><<<1, w8a8::RP_THREADS, 0, st>>>(expert_idx, P, experts, nullptr, count, cumsum, expanded_pos); w8a8::note_launch();
+            w8a8::launch_chained(w8a8::rp_rank_kernel<true>, 1, w8a8::RP_THREADS, 0, st, expert_idx, P, experts,
+                                 nullptr, count, cumsum, expanded_pos);
         } else {
-            w8a8::rp_histogram_kernel<<<static_cast<unsigned>(ctas), w8a8::RP_THREADS, 0, st>>>(expert_idx, P, experts, block_count); w8a8::note_launch();
-            w8a8::rp_prefix_kernel<<<static_cast<unsigned>((E + 31) / 32), 1024, 0, st>>>(block_count, ctas, experts, count); w8a8::note_launch();
-            w8a8::rp_rank_kernel<false><<<static_cast<unsigned>(ctas), w8a8::RP_THREADS, 0, st>>>(expert_idx, P, experts, block_count, count, cumsum, expanded_pos); w8a8::note_launch();
+            w8a8::launch_chained(w8a8::rp_histogram_kernel, static_cast<unsigned>(ctas), w8a8::RP_THREADS, 0, st,
+                                 expert_idx, P, experts, block_count);
+            w8a8::launch_chained(w8a8::rp_prefix_kernel, static_cast<unsigned>((E + 31) / 32), 1024, 0, st,
+                                 block_count, ctas, experts, count);
+            w8a8::launch_chained(w8a8::rp_rank_kernel<false>, static_cast<unsigned>(ctas), w8a8::RP_THREADS, 0, st,
+                                 expert_idx, P, experts, block_count, count, cumsum, expanded_pos);
         }
         return (cudaGetLastError() == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
     }
@@ -1156,13 +1170,11 @@ extern "C" int w8a8_permute_rows(const void* src, const float* src_scale, void* 
     const int64_t want = (rows + 7) / 8;                             // one warp per row
     const unsigned grid = static_cast<unsigned>(want < cap ? want : cap);
     if (vec) {
-        w8a8::permute_rows_kernel<true><<<grid, 256, 0, st>>>(static_cast<const uint8_t*>(src), src_scale,
-                                                             static_cast<uint8_t*>(dst), dst_scale, index, rows,
-                                                             row_bytes); w8a8::note_launch();
+        w8a8::launch_chained(w8a8::permute_rows_kernel<true>, grid, 256, 0, st, static_cast<const uint8_t*>(src),
+                             src_scale, static_cast<uint8_t*>(dst), dst_scale, index, rows, row_bytes);
     } else {
-        w8a8::permute_rows_kernel<false><<<grid, 256, 0, st>>>(static_cast<const uint8_t*>(src), src_scale,
-                                                              static_cast<uint8_t*>(dst), dst_scale, index, rows,
-                                                              row_bytes); w8a8::note_launch();
+        w8a8::launch_chained(w8a8::permute_rows_kernel<false>, grid, 256, 0, st, static_cast<const uint8_t*>(src),
+                             src_scale, static_cast<uint8_t*>(dst), dst_scale, index, rows, row_bytes);
     }
     return (cudaGetLastError() == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
 }
@@ -1187,13 +1199,13 @@ extern "C" int w8a8_dispatch_rows(const void* src, const float* src_scale, const
     const int64_t cap = static_cast<int64_t>(w8a8::sm_count()) * 8;
     const unsigned grid = static_cast<unsigned>(T < cap ? T : cap);
     if (vec) {
-        w8a8::dispatch_rows_kernel<true><<<grid, 256, 0, st>>>(static_cast<const uint8_t*>(src), src_scale, expert_idx,
-                                                              expanded_pos, row_dst, scale_dst, my_base, T,
-                                                              static_cast<int>(topk), row_bytes); w8a8::note_launch();
+        w8a8::launch_chained(w8a8::dispatch_rows_kernel<true>, grid, 256, 0, st, static_cast<const uint8_t*>(src),
+                             src_scale, expert_idx, expanded_pos, row_dst, scale_dst, my_base, T,
+                             static_cast<int>(topk), row_bytes);
     } else {
-        w8a8::dispatch_rows_kernel<false><<<grid, 256, 0, st>>>(static_cast<const uint8_t*>(src), src_scale,
-                                                               expert_idx, expanded_pos, row_dst, scale_dst, my_base,
-                                                               T, static_cast<int>(topk), row_bytes); w8a8::note_launch();
+        w8a8::launch_chained(w8a8::dispatch_rows_kernel<false>, grid, 256, 0, st, static_cast<const uint8_t*>(src),
+                             src_scale, expert_idx, expanded_pos, row_dst, scale_dst, my_base, T,
+                             static_cast<int>(topk), row_bytes);
     }
     return (cudaGetLastError() == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
 }
@@ -1212,8 +1224,8 @@ extern "C" int w8a8_expand_row_pointers(const int64_t* seg_first, const uint64_t
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const unsigned grid = static_cast<unsigned>((rows + 255) / 256);
-    w8a8::expand_row_pointers_kernel<<<grid, 256, 0, st>>>(seg_first, seg_ptr, static_cast<int>(nseg), rows, row_bytes,
-                                                           out); w8a8::note_launch();
+    w8a8::launch_chained(w8a8::expand_row_pointers_kernel, grid, 256, 0, st, seg_first, seg_ptr,
+                         static_cast<int>(nseg), rows, row_bytes, out);
     return (cudaGetLastError() == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
 }
 
@@ -1245,9 +1257,10 @@ extern "C" int w8a8_combine(const void* rows, const float* probs, const int64_t*
                            : w8a8::mfr_kernel<W8A8_DT_BF16, false, false, int64_t>)
                     : (vec ? w8a8::mfr_kernel<W8A8_DT_F16, true, false, int64_t>
                            : w8a8::mfr_kernel<W8A8_DT_F16, false, false, int64_t>);
-    kern<<<grid, 256, 0, st>>>(rows, expanded_pos, nullptr, nullptr, nullptr, probs, nullptr, out, T, H,
-                               static_cast<int>(topk), 0, INT64_MAX, 0, W8A8_DT_F32); w8a8::note_launch();
-    return (cudaGetLastError() == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    const cudaError_t e = w8a8::launch_chained(kern, grid, 256, 0, st, rows, expanded_pos, nullptr, nullptr, nullptr,
+                                               probs,
+                                               nullptr, out, T, H, static_cast<int>(topk), 0, INT64_MAX, 0, W8A8_DT_F32);
+    return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
 }
 
 // workspace: 256-byte header | dst_first[N*E+1] | src_first[N*E] | col_start[E+1] | row_start[N+1] | index[A]
@@ -1306,13 +1319,13 @@ extern "C" int w8a8_moe_re_routing(const void* tokens, const void* counts, const
 
     if (cells <= static_cast<size_t>(w8a8::RR_SMALL_CELLS)) {
         if (count_bytes == 4) {
-            w8a8::rr_table_small_kernel<int32_t><<<1, 1024, 0, st>>>(
-                static_cast<const int32_t*>(counts), static_cast<int>(N), static_cast<int>(E), A, hdr, dst_first,
-                src_first, static_cast<int32_t*>(expert_token_num)); w8a8::note_launch();
+            w8a8::launch_chained(w8a8::rr_table_small_kernel<int32_t>, 1, 1024, 0, st,
+                                 static_cast<const int32_t*>(counts), static_cast<int>(N), static_cast<int>(E), A, hdr,
+                                 dst_first, src_first, static_cast<int32_t*>(expert_token_num));
         } else {
-            w8a8::rr_table_small_kernel<int64_t><<<1, 1024, 0, st>>>(
-                static_cast<const int64_t*>(counts), static_cast<int>(N), static_cast<int>(E), A, hdr, dst_first,
-                src_first, static_cast<int64_t*>(expert_token_num)); w8a8::note_launch();
+            w8a8::launch_chained(w8a8::rr_table_small_kernel<int64_t>, 1, 1024, 0, st,
+                                 static_cast<const int64_t*>(counts), static_cast<int>(N), static_cast<int>(E), A, hdr,
+                                 dst_first, src_first, static_cast<int64_t*>(expert_token_num));
         }
     } else if (count_bytes == 4) {
         w8a8::rr_table_kernel<int32_t><<<1, 1024, 0, st>>>(static_cast<const int32_t*>(counts), N, E, A, hdr,
@@ -1330,8 +1343,8 @@ extern "C" int w8a8_moe_re_routing(const void* tokens, const void* counts, const
         return W8A8_OK;
     }
     const unsigned blocks = static_cast<unsigned>((A + 255) / 256);
-    w8a8::rr_index_kernel<<<blocks, 256, 0, st>>>(hdr, dst_first, src_first, static_cast<int64_t>(cells), A, index,
-                                                  out_idx); w8a8::note_launch();
+    w8a8::launch_chained(w8a8::rr_index_kernel, blocks, 256, 0, st, hdr, dst_first, src_first,
+                         static_cast<int64_t>(cells), A, index, out_idx);
     if (cudaGetLastError() != cudaSuccess) {
         return W8A8_ERR_CUDA;
     }
@@ -1350,9 +1363,10 @@ static int launch_mfr(const void* rows, const int32_t* esdr, const void* skip1, 
     auto kern = vec ? (has_bias ? w8a8::mfr_kernel<DT, true, true, int32_t> : w8a8::mfr_kernel<DT, true, false, int32_t>)
                     : (has_bias ? w8a8::mfr_kernel<DT, false, true, int32_t>
                                 : w8a8::mfr_kernel<DT, false, false, int32_t>);
-    kern<<<grid, 256, 0, st>>>(rows, esdr, skip1, skip2, bias, scales, expert, out, R, H, static_cast<int>(K), E,
-                               num_dst, col_mode, scale_dt); w8a8::note_launch();
-    return (cudaGetLastError() == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    const cudaError_t e = w8a8::launch_chained(kern, grid, 256, 0, st, rows, esdr, skip1, skip2, bias, scales, expert,
+                                               out, R,
+                                               H, static_cast<int>(K), E, num_dst, col_mode, scale_dt);
+    return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
 }
 
 extern "C" int w8a8_moe_finalize_routing(const void* rows, const int32_t* src_to_dst_row, const void* skip1,
@@ -1422,8 +1436,9 @@ extern "C" int w8a8_ep_tables(const int64_t* counts, int64_t P, int64_t E, int64
         status == nullptr) {
         return W8A8_ERR_INVALID;
     }
-    w8a8::ep_tables_kernel<<<1, w8a8::EP_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
-        counts, static_cast<int>(P), static_cast<int>(E), static_cast<int>(rank), peer_base, off_x, off_s, off_back,
-        row_bytes, back_row_bytes, cap_rows, row_dst, scale_dst, my_base, group_list, seg_first, seg_ptr, status); w8a8::note_launch();
+    w8a8::launch_chained(w8a8::ep_tables_kernel, 1, w8a8::EP_THREADS, 0, static_cast<cudaStream_t>(stream), counts,
+                         static_cast<int>(P), static_cast<int>(E), static_cast<int>(rank), peer_base, off_x, off_s,
+                         off_back, row_bytes, back_row_bytes, cap_rows, row_dst, scale_dst, my_base, group_list,
+                         seg_first, seg_ptr, status);
     return (cudaGetLastError() == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
 }

@@ -56,6 +56,7 @@ __global__ void __launch_bounds__(GATING_WARPS * 32) gating_kernel(const void* _
                                                                    int inner, int k)
 {
     __shared__ int2 lists[GATING_WARPS][(VPT + 1) * 32];
+    after_previous(x, finished, y, expert_idx, row_idx);
     const int lane = threadIdx.x & 31;
     int2* list = lists[threadIdx.x >> 5];
     const int64_t warps = static_cast<int64_t>(gridDim.x) * GATING_WARPS;
@@ -298,6 +299,7 @@ __global__ void __launch_bounds__(GATING_TOP_THREADS) gating_top8_kernel(const v
 {
     constexpr bool WIDE = (DT == W8A8_DT_F32);
     using Key = std::conditional_t<WIDE, unsigned long long, int>;
+    after_previous(x, finished, y, expert_idx, row_idx);
     const int lane = threadIdx.x & 31;
     const int q = lane & 3;
     const int64_t row0 = (static_cast<int64_t>(blockIdx.x) * GATING_TOP_THREADS + (threadIdx.x & ~31)) / 4;
@@ -458,13 +460,15 @@ static cudaError_t launch_gating_top8(const void* x, const uint8_t* finished, vo
 {
     constexpr int64_t ROWS = GATING_TOP_THREADS / 4;
     const unsigned grid = static_cast<unsigned>((rows + ROWS - 1) / ROWS);
+    cudaError_t e;
     if (inner % 8 == 0 && is_aligned(x, 16)) {
-        gating_top8_kernel<DT, true><<<grid, GATING_TOP_THREADS, 0, st>>>(x, finished, y, expert_idx, row_idx, rows, inner, k);
+        e = launch_chained(gating_top8_kernel<DT, true>, grid, GATING_TOP_THREADS, 0, st, x, finished, y, expert_idx, row_idx,
+                           rows, inner, k);
     } else {
-        gating_top8_kernel<DT, false><<<grid, GATING_TOP_THREADS, 0, st>>>(x, finished, y, expert_idx, row_idx, rows, inner, k);
+        e = launch_chained(gating_top8_kernel<DT, false>, grid, GATING_TOP_THREADS, 0, st, x, finished, y, expert_idx, row_idx,
+                           rows, inner, k);
     }
-    w8a8::note_launch();
-    return cudaGetLastError();
+    return e;
 }
 
 template <int DT, int VPT>
@@ -474,13 +478,15 @@ static cudaError_t launch_gating(const void* x, const uint8_t* finished, void* y
     const int64_t want = (rows + GATING_WARPS - 1) / GATING_WARPS;
     const int64_t cap = static_cast<int64_t>(sm_count()) * 16;
     const unsigned grid = static_cast<unsigned>(want < cap ? want : cap);
+    cudaError_t e;
     if (inner == 32 * VPT) {
-        gating_kernel<DT, VPT, true><<<grid, GATING_WARPS * 32, 0, st>>>(x, finished, y, expert_idx, row_idx, rows, inner, k);
+        e = launch_chained(gating_kernel<DT, VPT, true>, grid, GATING_WARPS * 32, 0, st, x, finished, y, expert_idx, row_idx,
+                           rows, inner, k);
     } else {
-        gating_kernel<DT, VPT, false><<<grid, GATING_WARPS * 32, 0, st>>>(x, finished, y, expert_idx, row_idx, rows, inner, k);
+        e = launch_chained(gating_kernel<DT, VPT, false>, grid, GATING_WARPS * 32, 0, st, x, finished, y, expert_idx, row_idx,
+                           rows, inner, k);
     }
-    w8a8::note_launch();
-    return cudaGetLastError();
+    return e;
 }
 
 template <int DT>

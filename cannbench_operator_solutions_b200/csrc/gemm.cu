@@ -119,15 +119,17 @@ static cudaError_t launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, con
     cfg.blockDim = dim3(gemm_threads(EPI_WARPS), 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
     if (cluster > 1) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = cluster;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = cluster;
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
     }
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     note_launch();
     return cudaLaunchKernelEx(&cfg, kern, ta, tb, p);
 }
@@ -345,6 +347,7 @@ __global__ void __launch_bounds__(256) plan_groups_kernel(const int64_t* __restr
                                                           TileEntry* tiles, int64_t max_tiles, int tile_m, int mode,
                                                           int32_t* shared_error, int allow_prefix)
 {
+    after_previous(dev_list, header, tiles, shared_error);
     plan_groups_body(dev_list, by_value, use_by_value, E, M, header, tiles, max_tiles, tile_m, mode, shared_error,
                      allow_prefix);
 }
@@ -363,6 +366,7 @@ __global__ void __launch_bounds__(256) plan_groups_both_kernel(const int64_t* __
                                                                int64_t tail_max_tiles, int allow_prefix,
                                                                uint4* __restrict__ clear, int64_t clear16)
 {
+    after_previous(dev_list, header, tiles, tail_header, tail_tiles, clear);
     if (blockIdx.x == 0) {
         plan_groups_body(dev_list, by_value, use_by_value, E, M, header, tiles, max_tiles, 256, PLAN_WHOLE, nullptr,
                          allow_prefix);
@@ -391,6 +395,7 @@ __global__ void __launch_bounds__(256) gmsq_requant_kernel(const float* __restri
                                                            int8_t* __restrict__ y, float* __restrict__ y_scale,
                                                            int64_t M, int64_t H, const GroupedHeader* header, int parts)
 {
+    after_previous(act, amax_bits, y, y_scale, header);
     if (header->error != 0) {
         return;
     }
@@ -578,19 +583,18 @@ static int plan_groups(const int64_t* group_list, int list_on_device, int64_t E,
     if (smem > 48 * 1024) {
         return W8A8_ERR_UNSUPPORTED;
     }
+    cudaError_t e;
     if (mode == PLAN_BOTH) {
         const int64_t clear16 = static_cast<int64_t>(clear_bytes / 16);
         const unsigned grid = 2 + (clear16 > 0 ? PLAN_CLEAR_CTAS : 0);
-        plan_groups_both_kernel<<<grid, 256, smem, st>>>(dev_list, bv, use_bv, E, M, g.header, g.tiles, g.max_tiles,
-                                                         g.tail_header, g.tail_tiles, g.tail_max_tiles,
-                                                         list_on_device == 2 ? 1 : 0, static_cast<uint4*>(clear),
-                                                         clear16);
+        e = launch_chained(plan_groups_both_kernel, grid, 256, smem, st, dev_list, bv, use_bv, E, M, g.header, g.tiles,
+                           g.max_tiles, g.tail_header, g.tail_tiles, g.tail_max_tiles, list_on_device == 2 ? 1 : 0,
+                           static_cast<uint4*>(clear), clear16);
     } else {
-        plan_groups_kernel<<<1, 256, smem, st>>>(dev_list, bv, use_bv, E, M, header, tiles, max_tiles, tile_m, mode,
-                                                 shared_error, list_on_device == 2 ? 1 : 0);
+        e = launch_chained(plan_groups_kernel, 1, 256, smem, st, dev_list, bv, use_bv, E, M, header, tiles, max_tiles,
+                           tile_m, mode, shared_error, list_on_device == 2 ? 1 : 0);
     }
-    w8a8::note_launch();
-    return (cudaGetLastError() == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
 }
 
 // Runs a grouped problem whose GemmParams are filled in except for the tile table: plans the groups and launches
@@ -889,14 +893,10 @@ extern "C" int w8a8_grouped_matmul_swiglu_quant(const int8_t* x, const int8_t* w
     if (blocks > cap) {
         blocks = cap;
     }
-    if (flags & W8A8_F_ROUND_DIRECT) {
-        gmsq_requant_kernel<true><<<static_cast<unsigned>(blocks), 256, 0, st>>>(g.act, g.amax, y, y_scale, M, H,
-                                                                                g.header, parts); w8a8::note_launch();
-    } else {
-        gmsq_requant_kernel<false><<<static_cast<unsigned>(blocks), 256, 0, st>>>(g.act, g.amax, y, y_scale, M, H,
-                                                                                 g.header, parts); w8a8::note_launch();
-    }
-    return (cudaGetLastError() == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    auto kern = (flags & W8A8_F_ROUND_DIRECT) ? gmsq_requant_kernel<true> : gmsq_requant_kernel<false>;
+    const cudaError_t e = launch_chained(kern, static_cast<unsigned>(blocks), 256, 0, st, g.act, g.amax, y, y_scale, M, H,
+                                         g.header, parts);
+    return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
 }
 
 // ===========================================================================

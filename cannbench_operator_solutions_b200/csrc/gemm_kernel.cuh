@@ -777,6 +777,8 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
     }
     tc::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    // everything above touches shared and tensor memory only and may run beside the kernel before
+    after_previous();
 
     // ---- tile enumeration (identical in every role and in both CTAs of a pair) ----
     constexpr int TILE_M = 128 * CG;
