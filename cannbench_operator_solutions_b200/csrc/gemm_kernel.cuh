@@ -840,7 +840,7 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
 
     if (warp == 0) {
         // ===================== TMA producer =====================
-        if (lane == 0) {
+        {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -849,62 +849,65 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
             for (int64_t t = worker; ok && t < total_tiles; t += num_workers) {
                 const TileInfo tl = decode(t);
                 for (int kb0 = kb_first; kb0 < kb_last; kb0 += KPS) {
-                    if (!tc::mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) {
+                    if (!__all_sync(FULL_MASK, tc::mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag))) {
                         ok = false;
                         break;
                     }
                     const int left = kb_last - kb0;
                     const int n_sub = left < KPS ? left : KPS;  // K blocks this stage carries (the tile's last may be short)
                     const uint32_t fb = full0 + 8u * stage;
-                    // Only the leader announces the bytes (its own and its partner's).  The partner's copies may
-                    // complete first: the barrier's phase cannot end before the leader's arrival, and a
-                    // transaction count may run ahead of its announcement.
-                    if (leader) {
-                        tc::mbar_arrive_expect_tx(full_bar(stage),
-                                                  CG * n_sub * (static_cast<uint32_t>(p.a_box_bytes) + B_BYTES));
-                    }
-#pragma unroll
-                    for (int sub = 0; sub < KPS; ++sub) {
-                        if (sub >= n_sub) {
-                            break;
+                    if (tc::elect_one()) {
+                        // Only the leader announces the bytes (its own and its partner's).  The partner's copies may
+                        // complete first: the barrier's phase cannot end before the leader's arrival, and a
+                        // transaction count may run ahead of its announcement.
+                        if (leader) {
+                            tc::mbar_arrive_expect_tx(full_bar(stage),
+                                                      CG * n_sub * (static_cast<uint32_t>(p.a_box_bytes) + B_BYTES));
                         }
-                        const int kb = kb0 + sub;
-                        const uint32_t a_dst = smem_base + stage * STAGE_BYTES + sub * KB_BYTES;
-                        const uint32_t b_dst = a_dst + GEMM_A_BYTES;
-                        if constexpr (CG == 2) {
-                            tc::tma_load_2d_pair(a_dst, &tm_a, fb, kb * BLOCK_K, tl.a_row0);
-                        } else {
-                            tc::tma_load_2d(a_dst, &tm_a, fb, kb * BLOCK_K, tl.a_row0);
-                        }
-                        if constexpr (B_MN) {
-                            // boxes of {128 bytes of N, BLOCK_K rows of K}
-                            constexpr int BOX_BYTES = BLOCK_K * 128;
-                            constexpr int BOX_COLS = 128 / ELEM;
 #pragma unroll
-                            for (int i = 0; i < NBOX; ++i) {
-                                const int32_t col = b_block_origin(tl.nt, i, BOX_COLS);
-                                if constexpr (CG == 2) {
-                                    tc::tma_load_3d_pair(b_dst + i * BOX_BYTES, &tm_b, fb, col, kb * BLOCK_K, tl.group);
-                                } else {
-                                    tc::tma_load_3d(b_dst + i * BOX_BYTES, &tm_b, fb, col, kb * BLOCK_K, tl.group);
+                        for (int sub = 0; sub < KPS; ++sub) {
+                            if (sub >= n_sub) {
+                                break;
+                            }
+                            const int kb = kb0 + sub;
+                            const uint32_t a_dst = smem_base + stage * STAGE_BYTES + sub * KB_BYTES;
+                            const uint32_t b_dst = a_dst + GEMM_A_BYTES;
+                            if constexpr (CG == 2) {
+                                tc::tma_load_2d_pair(a_dst, &tm_a, fb, kb * BLOCK_K, tl.a_row0);
+                            } else {
+                                tc::tma_load_2d(a_dst, &tm_a, fb, kb * BLOCK_K, tl.a_row0);
+                            }
+                            if constexpr (B_MN) {
+                                // boxes of {128 bytes of N, BLOCK_K rows of K}
+                                constexpr int BOX_BYTES = BLOCK_K * 128;
+                                constexpr int BOX_COLS = 128 / ELEM;
+#pragma unroll
+                                for (int i = 0; i < NBOX; ++i) {
+                                    const int32_t col = b_block_origin(tl.nt, i, BOX_COLS);
+                                    if constexpr (CG == 2) {
+                                        tc::tma_load_3d_pair(b_dst + i * BOX_BYTES, &tm_b, fb, col, kb * BLOCK_K, tl.group);
+                                    } else {
+                                        tc::tma_load_3d(b_dst + i * BOX_BYTES, &tm_b, fb, col, kb * BLOCK_K, tl.group);
+                                    }
+                                }
+                            } else {
+                                // boxes of {128 bytes of K, 128 rows of N}
+                                constexpr int BOXES = CTA_N / 128;
+#pragma unroll
+                                for (int i = 0; i < BOXES; ++i) {
+                                    const int32_t n_row = b_block_origin(tl.nt, i, 128);
+                                    if constexpr (CG == 2) {
+                                        tc::tma_load_3d_pair(b_dst + i * 128 * GEMM_KBYTES, &tm_b, fb, kb * BLOCK_K, n_row,
+                                                             tl.group);
+                                    } else {
+                                        tc::tma_load_3d(b_dst + i * 128 * GEMM_KBYTES, &tm_b, fb, kb * BLOCK_K, n_row,
+                                                        tl.group);
+                                    }
                                 }
                             }
-                        } else {
-                            // boxes of {128 bytes of K, 128 rows of N}
-                            constexpr int BOXES = CTA_N / 128;
-#pragma unroll
-                            for (int i = 0; i < BOXES; ++i) {
-                                const int32_t n_row = b_block_origin(tl.nt, i, 128);
-                                if constexpr (CG == 2) {
-                                    tc::tma_load_3d_pair(b_dst + i * 128 * GEMM_KBYTES, &tm_b, fb, kb * BLOCK_K, n_row,
-                                                         tl.group);
-                                } else {
-                                    tc::tma_load_3d(b_dst + i * 128 * GEMM_KBYTES, &tm_b, fb, kb * BLOCK_K, n_row,
-                                                    tl.group);
-                                }
-                            }
                         }
                     }
+                    __syncwarp();
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1u;
@@ -915,7 +918,10 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
         __syncwarp();
     } else if (warp == 1) {
         // ===================== MMA issuer (leader CTA only) =====================
-        if (lane == 0 && leader) {
+        // The whole warp walks the loop and waits; one elected lane issues.  (A loop run by lane 0 alone had every
+        // descriptor moved to a uniform register on its way into each instruction: 8192 x 7168 x 18432 with all-zero
+        // operands, which the power cap does not bound, 574 us, 590 then; 2048 x 7168 x 4096 47.2, 51.9.)
+        if (leader) {
             // Descriptors as {lo, hi}: hi is loop invariant; a byte offset adds (offset >> 4) to lo.
             const uint64_t a_desc0 = tc::smem_desc_sw128(smem_base, 16, 1024);
             const uint64_t b_desc0 = B_MN ? tc::smem_desc_sw128(smem_base + GEMM_A_BYTES, BLOCK_K * 128, 1024)
@@ -936,7 +942,7 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
             for (int64_t t = worker; ok && t < total_tiles; t += num_workers, ++it) {
                 const int acc = static_cast<int>(it & 1);
                 const uint32_t acc_phase = static_cast<uint32_t>((it >> 1) & 1);
-                if (!tc::mbar_wait_cluster(tempty_bar(acc), acc_phase ^ 1u, abort_flag)) {
+                if (!__all_sync(FULL_MASK, tc::mbar_wait_cluster(tempty_bar(acc), acc_phase ^ 1u, abort_flag))) {
                     ok = false;
                     break;
                 }
@@ -947,45 +953,49 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
                     // The copies are consumed by the tensor core (async proxy), not by this thread: the barrier's
                     // default acquire plus the tcgen05 fence is what orders them, also for the partner CTA's
                     // copies that complete on this barrier.
-                    if (!tc::mbar_wait(full_bar(stage), phase, abort_flag)) {
+                    if (!__all_sync(FULL_MASK, tc::mbar_wait(full_bar(stage), phase, abort_flag))) {
                         ok = false;
                         break;
                     }
                     tc::tc_fence_after_sync();
                     const int left = kb_last - kb0;
                     const int n_sub = left < KPS ? left : KPS;
+                    if (tc::elect_one()) {
 #pragma unroll
-                    for (int sub = 0; sub < KPS; ++sub) {
-                        if (sub >= n_sub) {
-                            break;
+                        for (int sub = 0; sub < KPS; ++sub) {
+                            if (sub >= n_sub) {
+                                break;
+                            }
+                            const uint32_t a_lo = a_lo0 + stage * STAGE_STEP + sub * KB_STEP;
+                            const uint32_t b_lo = b_lo0 + stage * STAGE_STEP + sub * KB_STEP;
+#pragma unroll
+                            for (int k = 0; k < KSTEPS; ++k) {
+                                tc::mma_lohi<CG, KIND == KIND_I8>(d_tmem, a_lo + k * A_KSTEP, a_hi, b_lo + k * B_KSTEP, b_hi,
+                                                                 IDESC, accumulate | static_cast<uint32_t>(sub | k));
+                            }
                         }
-                        const uint32_t a_lo = a_lo0 + stage * STAGE_STEP + sub * KB_STEP;
-                        const uint32_t b_lo = b_lo0 + stage * STAGE_STEP + sub * KB_STEP;
-#pragma unroll
-                        for (int k = 0; k < KSTEPS; ++k) {
-                            tc::mma_lohi<CG, KIND == KIND_I8>(d_tmem, a_lo + k * A_KSTEP, a_hi, b_lo + k * B_KSTEP, b_hi,
-                                                             IDESC, accumulate);
-                            accumulate = 1;
+                        // one commit hands the whole stage back to the producer
+                        if constexpr (CG == 2) {
+                            tc::tc_commit_pair(empty_bar(stage));
+                        } else {
+                            tc::tc_commit(empty_bar(stage));
                         }
                     }
-                    // one commit hands the whole stage back to the producer
-                    if constexpr (CG == 2) {
-                        tc::tc_commit_pair(empty_bar(stage));
-                    } else {
-                        tc::tc_commit(empty_bar(stage));
-                    }
+                    __syncwarp();
+                    accumulate = 1;
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1u;
                     }
                 }
-                if (ok) {
+                if (ok && tc::elect_one()) {
                     if constexpr (CG == 2) {
                         tc::tc_commit_pair(tfull_bar(acc));
                     } else {
                         tc::tc_commit(tfull_bar(acc));
                     }
                 }
+                __syncwarp();
             }
         }
         __syncwarp();

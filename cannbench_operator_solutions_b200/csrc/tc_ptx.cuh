@@ -29,6 +29,22 @@ __device__ __forceinline__ unsigned long long global_ns()
 }
 
 // ---------------------------------------------------------------- mbarrier
+// True in one lane of a converged warp.  Unlike a comparison with a lane number this keeps the branch it guards
+// warp-uniform for the compiler, so that descriptors, coordinates and barrier addresses stay in uniform registers,
+// which is where tcgen05 and TMA instructions take them from.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t one;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "elect.sync _|p, 0xffffffff;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(one));
+    return one != 0;
+}
+
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
