@@ -101,11 +101,11 @@ static int64_t worker_count(int64_t max_tiles)
     return workers < 1 ? 1 : workers;
 }
 
-template <int CG, int BLOCK_N, int KIND, int EPI, bool B_MN, int EPI_WARPS = 8, bool SPLITK = false>
+template <int CG, int BLOCK_N, int KIND, int EPI, bool B_MN, int EPI_WARPS = 8, bool SPLITK = false, bool ROW_BOXES = false>
 static cudaError_t launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int64_t max_tiles,
                                cudaStream_t st)
 {
-    auto kern = gemm_tc_kernel<CG, BLOCK_N, KIND, EPI, B_MN, EPI_WARPS, SPLITK>;
+    auto kern = gemm_tc_kernel<CG, BLOCK_N, KIND, EPI, B_MN, EPI_WARPS, SPLITK, ROW_BOXES>;
     constexpr size_t smem = gemm_smem_bytes<CG, BLOCK_N>();
     static KernelFacts facts;
     const cudaError_t e = allow_dynamic_smem(facts, kern, smem);
@@ -163,6 +163,21 @@ static cudaError_t dispatch_gemm(int cta_group, int block_n, bool b_mn, const CU
     }
     return b_mn ? launch_gemm<1, 256, KIND, EPI, true>(ta, tb, p, max_tiles, st)
                 : launch_gemm<1, 256, KIND, EPI, false>(ta, tb, p, max_tiles, st);
+}
+
+// Single-CTA tiles of a grouped problem that load their own rows only (see run_grouped).
+template <int KIND, int EPI>
+static cudaError_t dispatch_row_boxes(bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
+                                      int64_t max_tiles, cudaStream_t st)
+{
+    if constexpr (EPI == EPI_GMSQ) {
+        if (g_gmsq_epilogue_warps.load(std::memory_order_relaxed) == 16) {
+            return b_mn ? launch_gemm<1, 256, KIND, EPI, true, 16, false, true>(ta, tb, p, max_tiles, st)
+                        : launch_gemm<1, 256, KIND, EPI, false, 16, false, true>(ta, tb, p, max_tiles, st);
+        }
+    }
+    return b_mn ? launch_gemm<1, 256, KIND, EPI, true, 8, false, true>(ta, tb, p, max_tiles, st)
+                : launch_gemm<1, 256, KIND, EPI, false, 8, false, true>(ta, tb, p, max_tiles, st);
 }
 
 // Dense problems with at most one 128 x 128 tile per SM run on single CTAs: a cluster launch costs about 3 us more
@@ -610,7 +625,7 @@ static int plan_groups(const int64_t* group_list, int list_on_device, int64_t E,
 // the kernel shape(s) choose_cta_group picked.
 template <int KIND, int EPI>
 static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E, int64_t M, const GroupedWorkspace& g,
-                       bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, cudaStream_t st,
+                       bool b_mn, const void* a, const CUtensorMap& tb, GemmParams p, cudaStream_t st,
                        void* clear = nullptr, size_t clear_bytes = 0)
 {
     const int shape = choose_cta_group(M, true);
@@ -619,6 +634,24 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
     // 13.25 - 13.5 ms on two GPUs, 7.62 against 7.73 - 7.83 ms on four and 26.4 against 28.0 ms on one.)
     p.grouped = 1;
     p.error = &g.header->error;
+    // Rows per A load.  Pairs take whole tiles.  A single CTA's tile holds at most 128 rows of one group and often far
+    // fewer - what a group leaves over, or a whole group of a small batch.  Where there are 256 MB of weights to stream
+    // it loads its own rows in boxes of 32 or 16 instead of 128 rows that are mostly another group's, and multiplies
+    // zeros below them: 512 rows of 256 experts (7168 x 4096 and 2048 x 7168) 1.55 ms back to back, 1.80 before (the SM
+    // clock held near 0.8 GHz by the power cap), 1.44 and 1.53 from rest; 1500 rows of 32 experts of 2048 x 7168 bf16
+    // 161 us, 165.  Smaller problems do not pay for clearing the stages and the longer loop (512 rows of 32 experts of
+    // 2048 x 2048: 38.7 us, 37.6).
+    constexpr int64_t ELEM = (KIND == KIND_I8) ? 1 : 2;
+    int box_rows = (shape == GEMM_SHAPE_HYBRID) ? 32 : (M <= 12 * E ? 16 : (M <= 96 * E ? 32 : GEMM_BLOCK_M));
+    if (shape == 2 || E * p.N * p.K * ELEM < (int64_t(256) << 20)) {
+        box_rows = GEMM_BLOCK_M;
+    }
+    const bool row_boxes = box_rows < GEMM_BLOCK_M;
+    CUtensorMap ta;
+    p.a_box_rows = (shape == 1) ? box_rows : GEMM_BLOCK_M;
+    if (!make_map_a(&ta, a, M, p.K, KIND, p.a_box_rows)) {
+        return W8A8_ERR_CUDA;
+    }
     // `clear` (the SwiGLU form's row maxima and tile counters) must be zero before the first matmul launch: the
     // two-table planner does it in its own launch, the other shapes with a memset
     if (shape != GEMM_SHAPE_HYBRID) {
@@ -632,7 +665,9 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
         p.tiles = g.tiles;
         p.header = g.header;
         p.tile_done = g.tile_done;
-        const cudaError_t e = dispatch_gemm<KIND, EPI>(shape, 256, b_mn, ta, tb, p, g.max_tiles * p.n_tiles, st);
+        const int64_t most = g.max_tiles * p.n_tiles;
+        const cudaError_t e = row_boxes ? dispatch_row_boxes<KIND, EPI>(b_mn, ta, tb, p, most, st)
+                                        : dispatch_gemm<KIND, EPI>(shape, 256, b_mn, ta, tb, p, most, st);
         return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
     }
     const int rc = plan_groups(group_list, list_on_device, E, M, g, 256, st, PLAN_BOTH, clear, clear_bytes);
@@ -649,7 +684,16 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
     p.tiles = g.tail_tiles;
     p.header = g.tail_header;
     p.tile_done = g.tail_tile_done;
-    e = dispatch_gemm<KIND, EPI>(1, 256, b_mn, ta, tb, p, g.tail_max_tiles * p.n_tiles, st);
+    const int64_t most = g.tail_max_tiles * p.n_tiles;
+    if (row_boxes) {
+        p.a_box_rows = box_rows;
+        if (!make_map_a(&ta, a, M, p.K, KIND, box_rows)) {
+            return W8A8_ERR_CUDA;
+        }
+        e = dispatch_row_boxes<KIND, EPI>(b_mn, ta, tb, p, most, st);
+    } else {
+        e = dispatch_gemm<KIND, EPI>(1, 256, b_mn, ta, tb, p, most, st);
+    }
     return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
 }
 
@@ -732,7 +776,7 @@ static int quant_matmul_impl(const int8_t* x1, const int8_t* x2, const void* sca
         return W8A8_ERR_CUDA;
     }
     GemmParams p{};
-    p.a_box_bytes = a_box_rows * GEMM_KBYTES;
+    p.a_box_rows = a_box_rows;
     p.M = M;
     p.N = N;
     p.K = K;
@@ -860,12 +904,11 @@ extern "C" int w8a8_grouped_matmul_swiglu_quant(const int8_t* x, const int8_t* w
             return list_rc;
         }
         const bool b_mn = (w_layout == W8A8_W_KN);
-        CUtensorMap ta, tb;
-        if (!make_map_a(&ta, x, M, K, KIND_I8) || !make_map_b(&tb, w, E, N, K, KIND_I8, b_mn)) {
+        CUtensorMap tb;
+        if (!make_map_b(&tb, w, E, N, K, KIND_I8, b_mn)) {
             return W8A8_ERR_CUDA;
         }
         GemmParams p{};
-        p.a_box_bytes = GEMM_A_BYTES;
         p.M = M;
         p.N = N;
         p.K = K;
@@ -886,7 +929,7 @@ extern "C" int w8a8_grouped_matmul_swiglu_quant(const int8_t* x, const int8_t* w
         p.round_direct = (flags & W8A8_F_ROUND_DIRECT) ? 1 : 0;
         fused = p.fuse_requant != 0;
         // row maxima and finished-tile counters start at zero
-        const int rc = run_grouped<KIND_I8, EPI_GMSQ>(group_list, list_on_device, E, M, g, b_mn, ta, tb, p, st, g.amax,
+        const int rc = run_grouped<KIND_I8, EPI_GMSQ>(group_list, list_on_device, E, M, g, b_mn, x, tb, p, st, g.amax,
                                                       g.clear_bytes);
         if (rc != W8A8_OK) {
             return rc;
@@ -1024,12 +1067,11 @@ static int grouped_matmul_impl(const void* x, const void* w, const void* bias, v
         w = wsplit;
         K = SPLIT_TERMS * K;
     }
-    CUtensorMap ta, tb;
-    if (!make_map_a(&ta, x, M, K, kind) || !make_map_b(&tb, w, E, N, K, kind, b_mn)) {
+    CUtensorMap tb;
+    if (!make_map_b(&tb, w, E, N, K, kind, b_mn)) {
         return W8A8_ERR_CUDA;
     }
     GemmParams p{};
-    p.a_box_bytes = GEMM_A_BYTES;
     p.M = M;
     p.N = N;
     p.K = K;
@@ -1044,12 +1086,12 @@ static int grouped_matmul_impl(const void* x, const void* w, const void* bias, v
     p.out_dtype = out_dtype;
     p.n_tiles = static_cast<int32_t>((N + 255) / 256);
     if (kind == KIND_I8) {
-        return run_grouped<KIND_I8, EPI_GMM>(group_list, list_on_device, E, M, g, b_mn, ta, tb, p, st);
+        return run_grouped<KIND_I8, EPI_GMM>(group_list, list_on_device, E, M, g, b_mn, x, tb, p, st);
     }
     if (kind == KIND_F16) {
-        return run_grouped<KIND_F16, EPI_GMM>(group_list, list_on_device, E, M, g, b_mn, ta, tb, p, st);
+        return run_grouped<KIND_F16, EPI_GMM>(group_list, list_on_device, E, M, g, b_mn, x, tb, p, st);
     }
-    return run_grouped<KIND_BF16, EPI_GMM>(group_list, list_on_device, E, M, g, b_mn, ta, tb, p, st);
+    return run_grouped<KIND_BF16, EPI_GMM>(group_list, list_on_device, E, M, g, b_mn, x, tb, p, st);
 }
 
 extern "C" int w8a8_grouped_matmul(const void* x, const void* w, const void* bias, void* y, const float* x_scale,

@@ -111,7 +111,7 @@ struct GemmParams {
     int32_t out_dtype;
     int64_t bias_batch_stride;
     const uint64_t* out_row_ptrs;  // GMM: when set, row r is stored at this address instead of out + r*N
-    int32_t a_box_bytes;  // bytes one A load delivers: GEMM_A_BYTES, or less when the A map's box has fewer rows
+    int32_t a_box_rows;  // rows of one A load: 128, or fewer (a multiple of 8) on single CTAs
     float* act;       // GMSQ: fp32 activations [M, N/2]
     uint32_t* amax;   // GMSQ: per-row max|act| bit patterns
     // GMSQ with the requantisation fused in: the CTA that finishes the last column tile of its rows quantises them
@@ -692,7 +692,7 @@ __device__ __forceinline__ void split_finish(const GemmParams& p, const TileInfo
     }
 }
 
-template <int CG, int BLOCK_N, int KIND, int EPI, bool B_MN, int EPI_WARPS, bool SPLITK>
+template <int CG, int BLOCK_N, int KIND, int EPI, bool B_MN, int EPI_WARPS, bool SPLITK, bool ROW_BOXES>
 __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                    const GemmParams p)
@@ -715,6 +715,7 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
     static_assert(BLOCK_N == 128 || BLOCK_N == 256, "BLOCK_N");
     static_assert(CG == 1 || BLOCK_N == 256, "CTA pairs use 256-column tiles");
     static_assert(EPI != EPI_GMSQ || BLOCK_N == 256, "the SwiGLU epilogue pairs 128 gate with 128 up columns");
+    static_assert(!ROW_BOXES || (CG == 1 && BLOCK_N == 256), "row boxes: single CTAs of grouped problems");
     static_assert(!SPLITK || (CG == 1 && BLOCK_N == 128 && KIND == KIND_I8 && (EPI == EPI_QMM || EPI == EPI_RAW)),
                   "split K: dense int8 matmuls on single-CTA tiles of 128 columns");
     static_assert(EPI_WARPS == 8 || (EPI_WARPS == 16 && EPI == EPI_GMSQ), "16 epilogue warps: SwiGLU epilogue only");
@@ -767,6 +768,16 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
         // accumulator has the same column address in both, as the paired MMA requires
         tc::tmem_alloc(tc::smem_u32(tmem_slot), TMEM_COLS);
         tc::tmem_relinquish();
+    }
+    if constexpr (ROW_BOXES) {
+        // Rows that no load brings are zeros: their products are never stored, but multiplying what the shared memory
+        // happens to hold costs as much energy as multiplying operands, and the chip runs at its power limit.
+        for (int i = threadIdx.x; i < STAGES * KPS * (GEMM_A_BYTES / 16); i += gemm_threads(EPI_WARPS)) {
+            const int block = i / (GEMM_A_BYTES / 16), word = i % (GEMM_A_BYTES / 16);
+            reinterpret_cast<uint4*>(smem + (block / KPS) * STAGE_BYTES + (block % KPS) * KB_BYTES)[word] =
+                make_uint4(0u, 0u, 0u, 0u);
+        }
+        tc::fence_async_smem();
     }
     tc::tc_fence_before_sync();
     __syncthreads();
@@ -848,6 +859,10 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
             const uint32_t full0 = (CG == 2) ? tc::map_to_cta(full_bar(0), 0) : full_bar(0);
             for (int64_t t = worker; ok && t < total_tiles; t += num_workers) {
                 const TileInfo tl = decode(t);
+                // ROW_BOXES: the tile's rows only, in boxes of a_box_rows
+                const int a_loads = ROW_BOXES ? (tl.m_rows + p.a_box_rows - 1) / p.a_box_rows : 1;
+                const uint32_t a_box_bytes = static_cast<uint32_t>(p.a_box_rows) * GEMM_KBYTES;
+                const uint32_t stage_bytes = a_loads * a_box_bytes + B_BYTES;  // of one K block, per CTA
                 for (int kb0 = kb_first; kb0 < kb_last; kb0 += KPS) {
                     if (!__all_sync(FULL_MASK, tc::mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag))) {
                         ok = false;
@@ -862,7 +877,7 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
                         // transaction count may run ahead of its announcement.
                         if (leader) {
                             tc::mbar_arrive_expect_tx(full_bar(stage),
-                                                      CG * n_sub * (static_cast<uint32_t>(p.a_box_bytes) + B_BYTES));
+                                                      CG * n_sub * stage_bytes);
                         }
 #pragma unroll
                         for (int sub = 0; sub < KPS; ++sub) {
@@ -876,6 +891,13 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
                                 tc::tma_load_2d_pair(a_dst, &tm_a, fb, kb * BLOCK_K, tl.a_row0);
                             } else {
                                 tc::tma_load_2d(a_dst, &tm_a, fb, kb * BLOCK_K, tl.a_row0);
+                                if constexpr (ROW_BOXES) {
+#pragma unroll 1
+                                    for (int i = 1; i < a_loads; ++i) {
+                                        tc::tma_load_2d(a_dst + i * a_box_bytes, &tm_a, fb, kb * BLOCK_K,
+                                                        tl.a_row0 + i * p.a_box_rows);
+                                    }
+                                }
                             }
                             if constexpr (B_MN) {
                                 // boxes of {128 bytes of N, BLOCK_K rows of K}
