@@ -423,7 +423,7 @@ template <bool VEC>
 __device__ __forceinline__ uint4 load_chunk16_cached(const uint16_t* row, int c, int64_t N)
 {
     if constexpr (VEC) {
-        return __ldg(reinterpret_cast<const uint4*>(row) + c);
+        return __ldca(reinterpret_cast<const uint4*>(row) + c);
     } else {
         return load_chunk16<false>(row, c, N);
     }
@@ -484,8 +484,10 @@ void note_launch();  // counts one kernel launch of this library (w8a8_kernel_la
 // stream is still running: its launch, block setup and prologue then overlap that kernel's tail instead of following
 // it.  Every such kernel opens with after_previous(), which lets the next kernel do the same and then waits until the
 // kernel before it has completed and its writes are visible; no global memory is touched before that, neither read
-// nor written.  The pointers pass through the wait so that no load through them is moved above it.  Kernels that are
-// launched plainly (and memsets, copies, event waits) order themselves against these as against any other.
+// nor written.  The pointers pass through the wait so that no load through them is moved above it.  No load is a
+// non-coherent one (ld.global.nc, __ldg): those are for memory that nothing writes during the life of the kernel, and
+// the kernel before may write its outputs while this one already lives.  Kernels that are launched plainly (and
+// memsets, copies, event waits) order themselves against these as against any other.
 // A dense layer of 16 rows 53.9 us (61.5 before), an expert layer of 2000 rows 160 (184) and of 64 rows 116 (129), a
 // grouped SwiGLU matmul of 512 rows 38 (42), regroup and combine of 8192 rows 56 (62).
 // ---------------------------------------------------------------------------

@@ -291,11 +291,11 @@ __global__ void __launch_bounds__(MAX_THREADS, MAX_THREADS <= DQSQ_PAIR_THREADS 
                 for (int q = 0; q < EL / 4; ++q) {
                     float4 a = make_float4(1.0f, 1.0f, 1.0f, 1.0f), b = a, c = a;
                     if constexpr (XT == DQSQ_X_I32) {
-                        a = __ldg(reinterpret_cast<const float4*>(weight_scale + g_off + j0) + q);
-                        b = __ldg(reinterpret_cast<const float4*>(weight_scale + o_off + j0) + q);
+                        a = __ldca(reinterpret_cast<const float4*>(weight_scale + g_off + j0) + q);
+                        b = __ldca(reinterpret_cast<const float4*>(weight_scale + o_off + j0) + q);
                     }
                     if (has_q) {
-                        c = __ldg(reinterpret_cast<const float4*>(quant_scale + j0) + q);
+                        c = __ldca(reinterpret_cast<const float4*>(quant_scale + j0) + q);
                     }
                     const int at = i * EL + 4 * q;
                     wg[at] = a.x, wg[at + 1] = a.y, wg[at + 2] = a.z, wg[at + 3] = a.w;

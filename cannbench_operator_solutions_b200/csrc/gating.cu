@@ -218,10 +218,10 @@ __device__ __forceinline__ void gating_load8(const void* x, int64_t row, int inn
             }
         } else if constexpr (DT == W8A8_DT_F32) {
             const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(x) + row * inner) + 2 * c;
-            const float4 a = __ldg(p), b = __ldg(p + 1);
+            const float4 a = __ldca(p), b = __ldca(p + 1);
             v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
         } else {
-            const uint4 w = __ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(x) + row * inner) + c);
+            const uint4 w = __ldca(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(x) + row * inner) + c);
             unpack2<DT>(w.x, v[0], v[1]);
             unpack2<DT>(w.y, v[2], v[3]);
             unpack2<DT>(w.z, v[4], v[5]);

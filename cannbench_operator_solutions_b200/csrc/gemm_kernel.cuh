@@ -158,7 +158,7 @@ __device__ __forceinline__ void load_vec(const void* base, int64_t idx0, int kin
         for (int q = 0; q < NV / 4; ++q) {
             uint4 t = make_uint4(0, 0, 0, 0);
             if (q * 4 < valid) {
-                t = __ldg(p4 + q);
+                t = __ldca(p4 + q);
             }
             if (kind == W8A8_QM_BIAS_I32) {
                 out[q * 4 + 0] = static_cast<float>(static_cast<int32_t>(t.x));
@@ -178,7 +178,7 @@ __device__ __forceinline__ void load_vec(const void* base, int64_t idx0, int kin
         for (int q = 0; q < NV / 8; ++q) {
             uint4 t = make_uint4(0, 0, 0, 0);
             if (q * 8 < valid) {
-                t = __ldg(p4 + q);
+                t = __ldca(p4 + q);
             }
             const uint32_t w[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
@@ -340,7 +340,7 @@ __device__ __forceinline__ void swiglu8(const uint32_t* g, const uint32_t* u, fl
     float l_max = 0.0f;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-        const float4 p = __ldg(reinterpret_cast<const float4*>(wg) + i), o = __ldg(reinterpret_cast<const float4*>(wu) + i);
+        const float4 p = __ldca(reinterpret_cast<const float4*>(wg) + i), o = __ldca(reinterpret_cast<const float4*>(wu) + i);
         const f32x2 ws[4] = {pair(p.x, p.y), pair(p.z, p.w), pair(o.x, o.y), pair(o.z, o.w)};
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
