@@ -25,18 +25,18 @@ constexpr int ARDQ_THREADS = 256;
 
 template <int DT, int CPT, bool VEC, bool DIRECT>
 __global__ void __launch_bounds__(ARDQ_THREADS)
-    ardq_rows_kernel(const uint16_t* __restrict__ x1, const uint16_t* __restrict__ x2,
-                     const uint16_t* __restrict__ gamma, int8_t* __restrict__ y, uint16_t* __restrict__ x_out,
+    ardq_rows_kernel(const uint16_t* x1, const uint16_t* x2,
+                     const uint16_t* gamma, int8_t* __restrict__ y, uint16_t* __restrict__ x_out,
                      float* __restrict__ scale_out, int64_t rows, int64_t N, float eps, float inv_n)
 {
     constexpr int WARPS = ARDQ_THREADS / 32;
     __shared__ float s_sum[2][WARPS];
     __shared__ uint32_t s_max[2][WARPS];
-    after_previous(x1, x2, gamma, y, x_out, scale_out);
+    const int64_t zero = after_previous();
     const int tid = threadIdx.x;
     const int nchunks = static_cast<int>((N + 7) / 8);
     int parity = 0;
-    for (int64_t row = blockIdx.x; row < rows; row += gridDim.x, parity ^= 1) {
+    for (int64_t row = blockIdx.x + zero; row < rows; row += gridDim.x, parity ^= 1) {
         const uint16_t* r1 = x1 + row * N;
         const uint16_t* r2 = x2 + row * N;
         uint16_t* ro = x_out + row * N;

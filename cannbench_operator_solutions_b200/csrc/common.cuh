@@ -484,19 +484,27 @@ void note_launch();  // counts one kernel launch of this library (w8a8_kernel_la
 // stream is still running: its launch, block setup and prologue then overlap that kernel's tail instead of following
 // it.  Every such kernel opens with after_previous(), which lets the next kernel do the same and then waits until the
 // kernel before it has completed and its writes are visible; no global memory is touched before that, neither read
-// nor written.  The pointers pass through the wait so that no load through them is moved above it.  No load is a
-// non-coherent one (ld.global.nc, __ldg): those are for memory that nothing writes during the life of the kernel, and
-// the kernel before may write its outputs while this one already lives.  Kernels that are launched plainly (and
-// memsets, copies, event waits) order themselves against these as against any other.
+// nor written.  Two rules keep it so in the compiled code:
+//  - No load is a non-coherent one (ld.global.nc, __ldg): those are for memory that nothing writes during the life of
+//    the kernel, and the kernel before may write its outputs while this one already lives.  So the pointers that such a
+//    kernel only reads are not __restrict__ (the compiler makes those loads non-coherent, and free to move); the
+//    ones that it writes are, which is what lets loads be issued ahead of the stores.
+//  - after_previous() returns a zero that the compiler cannot see through.  It is part of the index that the kernel's
+//    first accesses are made with or guarded by, so that loads which the compiler takes for pure (__ldca, __ldcs,
+//    __ldcg) cannot move above the wait either.  (Passing the pointers through an asm instead did that too, but made
+//    every access a generic one and cost a register pair per pointer: the int32 form of the SwiGLU quantiser spilled,
+//    68.5 us on [16384, 4096] against 67.3, and 8192 sums of eight rows of 7164 took 744 us against 579.)
+// Kernels that are launched plainly (and memsets, copies, event waits) order themselves against these as against any
+// other.
 // A dense layer of 16 rows 53.9 us (61.5 before), an expert layer of 2000 rows 160 (184) and of 64 rows 116 (129), a
 // grouped SwiGLU matmul of 512 rows 38 (42), regroup and combine of 8192 rows 56 (62).
 // ---------------------------------------------------------------------------
-template <typename... Pointers>
-__device__ __forceinline__ void after_previous(Pointers&... pointers)
+__device__ __forceinline__ int64_t after_previous()
 {
+    int64_t zero;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    (void(([&] { asm volatile("" : "+l"(pointers)); })()), ...);
+    asm volatile("griddepcontrol.wait;\n\tmov.u64 %0, 0;" : "=l"(zero)::"memory");
+    return zero;
 }
 
 template <typename... Params, typename... Args>

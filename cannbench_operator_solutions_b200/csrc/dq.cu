@@ -17,16 +17,16 @@
 namespace w8a8 {
 
 template <int DT, int THREADS, int CPT, bool VEC, bool DIRECT>
-__global__ void __launch_bounds__(THREADS) dq_rows_kernel(const uint16_t* __restrict__ x, int8_t* __restrict__ y,
+__global__ void __launch_bounds__(THREADS) dq_rows_kernel(const uint16_t* x, int8_t* __restrict__ y,
                                                           float* __restrict__ scale, int64_t M, int64_t N)
 {
     constexpr int WARPS = THREADS / 32;
     __shared__ uint32_t s_max[2][WARPS];
-    after_previous(x, y, scale);
+    const int64_t zero = after_previous();
     const int tid = threadIdx.x;
     const int nchunks = static_cast<int>((N + 7) / 8);
     int parity = 0;
-    for (int64_t row = blockIdx.x; row < M; row += gridDim.x, parity ^= 1) {
+    for (int64_t row = blockIdx.x + zero; row < M; row += gridDim.x, parity ^= 1) {
         const uint16_t* xr = x + row * N;
         uint4 v[CPT];
         uint32_t m2 = 0;

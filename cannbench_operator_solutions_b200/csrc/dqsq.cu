@@ -230,8 +230,8 @@ __device__ __forceinline__ uint32_t dqsq_quant4(const float* o, float s, float i
 // with a fixed 256 threads per row (eight chunks per thread, 44 % of them past the row's end).
 template <int XT, int CPT, bool DIVIDE, int MAX_THREADS>
 __global__ void __launch_bounds__(MAX_THREADS, MAX_THREADS <= DQSQ_PAIR_THREADS ? 2 : 1)
-    dqsq_rows_kernel(const void* __restrict__ x, const float* __restrict__ weight_scale,
-                     const float* __restrict__ activation_scale, const float* __restrict__ quant_scale,
+    dqsq_rows_kernel(const void* x, const float* weight_scale,
+                     const float* activation_scale, const float* quant_scale,
                      int8_t* __restrict__ y, float* __restrict__ scale, int64_t M, int64_t H, int left, int direct, int)
 {
     using C = DqsqChunk<XT>;
@@ -241,7 +241,8 @@ __global__ void __launch_bounds__(MAX_THREADS, MAX_THREADS <= DQSQ_PAIR_THREADS 
     constexpr int GN = GROUP * EL;
     constexpr size_t ELEM = (XT == DQSQ_X_I32) ? 4 : 2;
     __shared__ float s_red[2 * 32];
-    after_previous(x, weight_scale, activation_scale, quant_scale, y, scale);
+    const int64_t zero = after_previous();
+    const int64_t first_row = blockIdx.x + zero;
     const int tid = threadIdx.x;
     const int threads = static_cast<int>(blockDim.x);
     const int nchunks = static_cast<int>(H / EL);
@@ -255,7 +256,7 @@ __global__ void __launch_bounds__(MAX_THREADS, MAX_THREADS <= DQSQ_PAIR_THREADS 
         cg[i] = co[i] = make_uint4(0u, 0u, 0u, 0u);
     }
     float as = 1.0f;
-    const uint8_t* xg = static_cast<const uint8_t*>(x) + (static_cast<size_t>(blockIdx.x) * 2 * H + g_off) * ELEM + tid * 16;
+    const uint8_t* xg = static_cast<const uint8_t*>(x) + (static_cast<size_t>(first_row) * 2 * H + g_off) * ELEM + tid * 16;
     const int64_t to_other = (o_off - g_off) * static_cast<int64_t>(ELEM);
     const size_t row_step = static_cast<size_t>(gridDim.x) * 2 * H * ELEM;
     auto load_row = [&](int64_t row) {
@@ -272,10 +273,10 @@ __global__ void __launch_bounds__(MAX_THREADS, MAX_THREADS <= DQSQ_PAIR_THREADS 
         xg += row_step;
     };
     int parity = 0;
-    if (blockIdx.x < M) {
-        load_row(blockIdx.x);
+    if (first_row < M) {
+        load_row(first_row);
     }
-    for (int64_t row = blockIdx.x; row < M; row += gridDim.x, parity ^= 1) {
+    for (int64_t row = first_row; row < M; row += gridDim.x, parity ^= 1) {
         float out[N];
 #pragma unroll
         for (int i0 = 0; i0 < CPT; i0 += GROUP) {
@@ -354,20 +355,20 @@ __global__ void __launch_bounds__(MAX_THREADS, MAX_THREADS <= DQSQ_PAIR_THREADS 
 
 // Any H and any alignment: two passes over the row, the second recomputes the activations (normally from L2).
 template <int XT>
-__global__ void __launch_bounds__(DQSQ_THREADS) dqsq_long_rows_kernel(const void* __restrict__ x,
-                                                                      const float* __restrict__ weight_scale,
-                                                                      const float* __restrict__ activation_scale,
-                                                                      const float* __restrict__ quant_scale,
+__global__ void __launch_bounds__(DQSQ_THREADS) dqsq_long_rows_kernel(const void* x,
+                                                                      const float* weight_scale,
+                                                                      const float* activation_scale,
+                                                                      const float* quant_scale,
                                                                       int8_t* __restrict__ y, float* __restrict__ scale,
                                                                       int64_t M, int64_t H, int left, int direct, int divide)
 {
     using C = DqsqChunk<XT>;
     __shared__ float s_red[2 * 32];
-    after_previous(x, weight_scale, activation_scale, quant_scale, y, scale);
+    const int64_t zero = after_previous();
     const size_t elem = (XT == DQSQ_X_I32) ? 4 : 2;
     const bool has_q = (quant_scale != nullptr);
     int parity = 0;
-    for (int64_t row = blockIdx.x; row < M; row += gridDim.x, parity ^= 1) {
+    for (int64_t row = blockIdx.x + zero; row < M; row += gridDim.x, parity ^= 1) {
         const uint8_t* xr = static_cast<const uint8_t*>(x) + static_cast<size_t>(row) * 2 * H * elem;
         const float as = (XT == DQSQ_X_I32) ? activation_scale[row] : 1.0f;
         auto element = [&](int64_t j) {

@@ -34,10 +34,10 @@ __device__ __forceinline__ int rp_expert(const int32_t* expert_idx, int64_t p, i
     return (e >= 0 && e < E) ? e : -1;
 }
 
-__global__ void __launch_bounds__(RP_THREADS) rp_histogram_kernel(const int32_t* __restrict__ expert_idx, int64_t P,
+__global__ void __launch_bounds__(RP_THREADS) rp_histogram_kernel(const int32_t* expert_idx, int64_t P,
                                                                   int E, int32_t* __restrict__ block_count)
 {
-    after_previous(expert_idx, block_count);
+    const int64_t zero = after_previous();
     __shared__ int32_t s_cnt[RP_MAX_EXPERTS];
     for (int e = threadIdx.x; e < E; e += RP_THREADS) {
         s_cnt[e] = 0;
@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(RP_THREADS) rp_histogram_kernel(const int32_t*
     __syncthreads();
 #pragma unroll
     for (int it = 0; it < RP_PAIRS / RP_THREADS; ++it) {
-        const int e = rp_expert(expert_idx, static_cast<int64_t>(blockIdx.x) * RP_PAIRS + it * RP_THREADS + threadIdx.x, P, E);
+        const int e = rp_expert(expert_idx, zero + static_cast<int64_t>(blockIdx.x) * RP_PAIRS + it * RP_THREADS + threadIdx.x, P, E);
         if (e >= 0) {
             atomicAdd(&s_cnt[e], 1);
         }
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(RP_THREADS) rp_histogram_kernel(const int32_t*
 __global__ void __launch_bounds__(1024) rp_prefix_kernel(int32_t* __restrict__ block_count, int64_t B, int E,
                                                          int64_t* __restrict__ count)
 {
-    after_previous(block_count, count);
+    after_previous();
     __shared__ int32_t s_part[32][33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int e = blockIdx.x * 32 + lane;
@@ -94,19 +94,19 @@ __global__ void __launch_bounds__(1024) rp_prefix_kernel(int32_t* __restrict__ b
 
 // ONE_CTA: counts its pairs itself and writes count; otherwise count and block_prefix come from rp_prefix_kernel.
 template <bool ONE_CTA>
-__global__ void __launch_bounds__(RP_THREADS) rp_rank_kernel(const int32_t* __restrict__ expert_idx, int64_t P, int E,
-                                                             const int32_t* __restrict__ block_prefix,
-                                                             int64_t* __restrict__ count, int64_t* __restrict__ cumsum,
+__global__ void __launch_bounds__(RP_THREADS) rp_rank_kernel(const int32_t* expert_idx, int64_t P, int E,
+                                                             const int32_t* block_prefix,
+                                                             int64_t* count, int64_t* __restrict__ cumsum,
                                                              int64_t* __restrict__ expanded_pos)
 {
-    after_previous(expert_idx, block_prefix, count, cumsum, expanded_pos);
+    const int64_t zero = after_previous();
     constexpr int ITS = RP_PAIRS / RP_THREADS;
     constexpr int PER = RP_MAX_EXPERTS / RP_THREADS;  // experts per thread in the scan
     __shared__ int64_t s_next[RP_MAX_EXPERTS];        // where the next pair of each expert goes
     __shared__ uint32_t s_words[RP_WARPS * RP_MAX_EXPERTS / 4];
     __shared__ int64_t s_sum[RP_WARPS];
     uint8_t* s_warp = reinterpret_cast<uint8_t*>(s_words);  // [RP_WARPS][E]: pairs of each warp, one step at a time
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = static_cast<int>(threadIdx.x + zero), lane = tid & 31, warp = tid >> 5;
     int mine[ITS];
 #pragma unroll
     for (int it = 0; it < ITS; ++it) {
@@ -328,16 +328,16 @@ __global__ void __launch_bounds__(256) scatter_rows_kernel(const uint8_t* __rest
 constexpr int PERMUTE_UNROLL = 8;
 
 template <bool VEC>
-__global__ void __launch_bounds__(256) permute_rows_kernel(const uint8_t* __restrict__ src,
-                                                           const float* __restrict__ src_scale,
+__global__ void __launch_bounds__(256) permute_rows_kernel(const uint8_t* src,
+                                                           const float* src_scale,
                                                            uint8_t* __restrict__ dst, float* __restrict__ dst_scale,
-                                                           const int64_t* __restrict__ index, int64_t rows,
+                                                           const int64_t* index, int64_t rows,
                                                            int64_t row_bytes)
 {
-    after_previous(src, src_scale, dst, dst_scale, index);
+    const int64_t zero = after_previous();
     const int lane = threadIdx.x & 31;
     const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-    for (int64_t d = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); d < rows;
+    for (int64_t d = zero + static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); d < rows;
          d += warps) {
         const int64_t s = index[d];
         if (s < 0) {
@@ -382,18 +382,18 @@ __global__ void __launch_bounds__(256) permute_rows_kernel(const uint8_t* __rest
 // order, pos[i, k] that pair's position: destination row = row_dst[e] + (pos - my_base[e]) rows.
 // This replaces pack + all-to-all + regroup with one pass; the row is read once and stored topk times.
 template <bool VEC>
-__global__ void __launch_bounds__(256) dispatch_rows_kernel(const uint8_t* __restrict__ src,
-                                                            const float* __restrict__ src_scale,
-                                                            const int32_t* __restrict__ expert_idx,
-                                                            const int64_t* __restrict__ pos,
-                                                            const uint64_t* __restrict__ row_dst,
-                                                            const uint64_t* __restrict__ scale_dst,
-                                                            const int64_t* __restrict__ my_base, int64_t T, int topk,
+__global__ void __launch_bounds__(256) dispatch_rows_kernel(const uint8_t* src,
+                                                            const float* src_scale,
+                                                            const int32_t* expert_idx,
+                                                            const int64_t* pos,
+                                                            const uint64_t* row_dst,
+                                                            const uint64_t* scale_dst,
+                                                            const int64_t* my_base, int64_t T, int topk,
                                                             int64_t row_bytes)
 {
-    after_previous(src, src_scale, expert_idx, pos, row_dst, scale_dst, my_base);
+    const int64_t zero = after_previous();
     __shared__ uint64_t s_dst[64];
-    for (int64_t i = blockIdx.x; i < T; i += gridDim.x) {
+    for (int64_t i = blockIdx.x + zero; i < T; i += gridDim.x) {
         __syncthreads();
         if (static_cast<int>(threadIdx.x) < topk) {
             const int64_t pr = i * topk + threadIdx.x;
@@ -437,13 +437,13 @@ __global__ void __launch_bounds__(256) dispatch_rows_kernel(const uint8_t* __res
 }
 
 // out[r] = seg_ptr[s] + (r - seg_first[s]) * row_bytes for the segment s with seg_first[s] <= r < seg_first[s+1]
-__global__ void __launch_bounds__(256) expand_row_pointers_kernel(const int64_t* __restrict__ seg_first,
-                                                                  const uint64_t* __restrict__ seg_ptr, int nseg,
+__global__ void __launch_bounds__(256) expand_row_pointers_kernel(const int64_t* seg_first,
+                                                                  const uint64_t* seg_ptr, int nseg,
                                                                   int64_t rows, int64_t row_bytes,
                                                                   uint64_t* __restrict__ out)
 {
-    after_previous(seg_first, seg_ptr, out);
-    const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t zero = after_previous();
+    const int64_t r = zero + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (r >= rows) {
         return;
     }
@@ -569,20 +569,20 @@ __global__ void __launch_bounds__(1024) rr_table_kernel(const CntT* __restrict__
 constexpr int RR_SMALL_CELLS = 2048;
 
 template <typename CntT>
-__global__ void __launch_bounds__(1024) rr_table_small_kernel(const CntT* __restrict__ cnt, int N, int E, int64_t A,
+__global__ void __launch_bounds__(1024) rr_table_small_kernel(const CntT* cnt, int N, int E, int64_t A,
                                                               int32_t* __restrict__ hdr,
                                                               int64_t* __restrict__ dst_first,
                                                               int64_t* __restrict__ src_first,
                                                               CntT* __restrict__ expert_num)
 {
-    after_previous(cnt, hdr, dst_first, src_first, expert_num);
+    const int64_t zero = after_previous();
     __shared__ int64_t s_cnt[RR_SMALL_CELLS];
     // E + N <= cells + 1, so one array of cells + 2 entries holds both prefixes: columns first, rows after them
     __shared__ int64_t s_sums[RR_SMALL_CELLS + 2];
     int64_t* s_col = s_sums;          // E + 1 entries: exclusive prefix of the column sums
     int64_t* s_row = s_sums + E + 1;  // N + 1 entries: exclusive prefix of the row sums
     __shared__ int s_bad;
-    const int tid = threadIdx.x;
+    const int tid = static_cast<int>(threadIdx.x + zero);
     const int cells = N * E;
     if (tid == 0) {
         s_bad = 0;
@@ -658,14 +658,14 @@ __global__ void __launch_bounds__(1024) rr_table_small_kernel(const CntT* __rest
 }
 
 // index[d] = source row of destination row d (-1 past the routed rows); out_idx[d] the same as int32.
-__global__ void __launch_bounds__(256) rr_index_kernel(const int32_t* __restrict__ hdr,
-                                                       const int64_t* __restrict__ dst_first,
-                                                       const int64_t* __restrict__ src_first, int64_t cells,
+__global__ void __launch_bounds__(256) rr_index_kernel(const int32_t* hdr,
+                                                       const int64_t* dst_first,
+                                                       const int64_t* src_first, int64_t cells,
                                                        int64_t A, int64_t* __restrict__ index,
                                                        int32_t* __restrict__ out_idx)
 {
-    after_previous(hdr, dst_first, src_first, index, out_idx);
-    const int64_t d = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t zero = after_previous();
+    const int64_t d = zero + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (d >= A) {
         return;
     }
@@ -779,14 +779,14 @@ constexpr int MFR_BATCH = 8;
 constexpr int MFR_MAX_STAGED_K = 128;
 
 template <int DT, bool VEC, bool HAS_BIAS, typename IdxT>
-__global__ void __launch_bounds__(256) mfr_kernel(const void* __restrict__ rows, const IdxT* __restrict__ esdr,
-                                                  const void* __restrict__ skip1, const void* __restrict__ skip2,
-                                                  const void* __restrict__ bias, const void* __restrict__ scales,
-                                                  const int32_t* __restrict__ expert, void* __restrict__ out,
+__global__ void __launch_bounds__(256) mfr_kernel(const void* rows, const IdxT* esdr,
+                                                  const void* skip1, const void* skip2,
+                                                  const void* bias, const void* scales,
+                                                  const int32_t* expert, void* __restrict__ out,
                                                   int64_t R, int64_t H, int K, int64_t E, int64_t num_dst,
                                                   int col_mode, int scale_dt)
 {
-    after_previous(rows, esdr, skip1, skip2, bias, scales, expert, out);
+    const int64_t zero = after_previous();
     using C = RowChunk<DT>;
     constexpr int EL = C::EL;
     __shared__ int64_t s_pos[2][MFR_MAX_STAGED_K];
@@ -816,8 +816,8 @@ __global__ void __launch_bounds__(256) mfr_kernel(const void* __restrict__ rows,
     // 65536 rows of 2048 regrouped, 32768 sums of two: 185 us, 191 when every row waited for its own look-up; 8192 sums of
     // eight rows of 7168 the same to 1 %.
     int buf = 0;
-    stage(blockIdx.x, 0, 0);
-    for (int64_t i = blockIdx.x; i < R; i += gridDim.x) {
+    stage(blockIdx.x + zero, 0, 0);
+    for (int64_t i = blockIdx.x + zero; i < R; i += gridDim.x) {
         for (int k0 = 0; k0 < K; k0 += MFR_MAX_STAGED_K, buf ^= 1) {
             const int kn = min(K - k0, MFR_MAX_STAGED_K);
             __syncthreads();
@@ -949,8 +949,8 @@ __device__ __forceinline__ void ep_scan3(int64_t (&v)[3][2], int64_t (*s_warp)[3
     }
 }
 
-__global__ void __launch_bounds__(EP_THREADS) ep_tables_kernel(const int64_t* __restrict__ counts, int P, int E, int rank,
-                                                         const uint64_t* __restrict__ peer_base, uint64_t off_x,
+__global__ void __launch_bounds__(EP_THREADS) ep_tables_kernel(const int64_t* counts, int P, int E, int rank,
+                                                         const uint64_t* peer_base, uint64_t off_x,
                                                          uint64_t off_s, uint64_t off_back, int64_t row_bytes,
                                                          int64_t back_row_bytes, int64_t cap_rows,
                                                          uint64_t* __restrict__ row_dst,
@@ -960,7 +960,7 @@ __global__ void __launch_bounds__(EP_THREADS) ep_tables_kernel(const int64_t* __
                                                          int64_t* __restrict__ seg_first,
                                                          uint64_t* __restrict__ seg_ptr, int32_t* __restrict__ status)
 {
-    after_previous(counts, peer_base, row_dst, scale_dst, my_base, group_list, seg_first, seg_ptr, status);
+    const int64_t zero = after_previous();
     // Row counts fit 32 bits (a rank's buffers hold fewer than 2^31 rows; larger counts set the overflow flag).
     __shared__ int32_t s_cnt[EP_MAX_CELLS];       // [P][E]
     __shared__ int64_t s_base[EP_MAX_CELLS + 1];  // exclusive prefix of s_cnt over all cells, rank-major
@@ -969,7 +969,7 @@ __global__ void __launch_bounds__(EP_THREADS) ep_tables_kernel(const int64_t* __
     __shared__ int32_t s_before[EP_MAX_CELLS / 2];   // rows of lower ranks inside each expert
     __shared__ int64_t s_warp[32][3];
     __shared__ int s_bad;
-    const int tid = threadIdx.x;
+    const int tid = static_cast<int>(threadIdx.x + zero);
     const int e_local = E / P;
     const int cells = P * E;
     const int nseg = e_local * P;

@@ -48,19 +48,19 @@ constexpr int GATING_WARPS = 4;
 
 // FULL: inner == 32 * VPT, so no element needs a bounds check.
 template <int DT, int VPT, bool FULL>
-__global__ void __launch_bounds__(GATING_WARPS * 32) gating_kernel(const void* __restrict__ x,
-                                                                   const uint8_t* __restrict__ finished,
+__global__ void __launch_bounds__(GATING_WARPS * 32) gating_kernel(const void* x,
+                                                                   const uint8_t* finished,
                                                                    void* __restrict__ y,
                                                                    int32_t* __restrict__ expert_idx,
                                                                    int32_t* __restrict__ row_idx, int64_t rows,
                                                                    int inner, int k)
 {
     __shared__ int2 lists[GATING_WARPS][(VPT + 1) * 32];
-    after_previous(x, finished, y, expert_idx, row_idx);
+    const int64_t zero = after_previous();
     const int lane = threadIdx.x & 31;
     int2* list = lists[threadIdx.x >> 5];
     const int64_t warps = static_cast<int64_t>(gridDim.x) * GATING_WARPS;
-    for (int64_t r = static_cast<int64_t>(blockIdx.x) * GATING_WARPS + (threadIdx.x >> 5); r < rows; r += warps) {
+    for (int64_t r = zero + static_cast<int64_t>(blockIdx.x) * GATING_WARPS + (threadIdx.x >> 5); r < rows; r += warps) {
         float v[VPT];
         float m = -INFINITY;
 #pragma unroll
@@ -290,8 +290,8 @@ __device__ __noinline__ void gating_row_by_warp(const void* x, int64_t row, int6
 }
 
 template <int DT, bool VEC>
-__global__ void __launch_bounds__(GATING_TOP_THREADS) gating_top8_kernel(const void* __restrict__ x,
-                                                                         const uint8_t* __restrict__ finished,
+__global__ void __launch_bounds__(GATING_TOP_THREADS) gating_top8_kernel(const void* x,
+                                                                         const uint8_t* finished,
                                                                          void* __restrict__ y,
                                                                          int32_t* __restrict__ expert_idx,
                                                                          int32_t* __restrict__ row_idx, int64_t rows,
@@ -299,10 +299,10 @@ __global__ void __launch_bounds__(GATING_TOP_THREADS) gating_top8_kernel(const v
 {
     constexpr bool WIDE = (DT == W8A8_DT_F32);
     using Key = std::conditional_t<WIDE, unsigned long long, int>;
-    after_previous(x, finished, y, expert_idx, row_idx);
+    const int64_t zero = after_previous();
     const int lane = threadIdx.x & 31;
     const int q = lane & 3;
-    const int64_t row0 = (static_cast<int64_t>(blockIdx.x) * GATING_TOP_THREADS + (threadIdx.x & ~31)) / 4;
+    const int64_t row0 = zero + (static_cast<int64_t>(blockIdx.x) * GATING_TOP_THREADS + (threadIdx.x & ~31)) / 4;
     if (row0 >= rows) {
         return;  // a whole warp
     }

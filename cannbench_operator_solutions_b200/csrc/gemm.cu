@@ -241,7 +241,7 @@ constexpr int PLAN_WHOLE = 1;
 constexpr int PLAN_LEFTOVER = 2;
 constexpr int PLAN_BOTH = 3;  // host side only: PLAN_WHOLE at 256 rows and PLAN_LEFTOVER at 128 rows in one launch
 
-__device__ __forceinline__ void plan_groups_body(const int64_t* __restrict__ dev_list,
+__device__ __forceinline__ void plan_groups_body(int64_t zero, const int64_t* dev_list,
                                                  const GroupEndsByValue& by_value, int use_by_value, int64_t E,
                                                  int64_t M, GroupedHeader* header, TileEntry* tiles,
                                                  int64_t max_tiles, int tile_m, int mode, int32_t* shared_error,
@@ -254,7 +254,7 @@ __device__ __forceinline__ void plan_groups_body(const int64_t* __restrict__ dev
     auto end_of = [&](int64_t g) -> int64_t {
         return use_by_value ? static_cast<int64_t>(by_value.ends[g]) : dev_list[g];
     };
-    const int tid = threadIdx.x;
+    const int tid = static_cast<int>(threadIdx.x + zero);
     const int lane = tid & 31;
     const int wid = tid >> 5;
     if (tid == 0) {
@@ -356,14 +356,14 @@ __device__ __forceinline__ void plan_groups_body(const int64_t* __restrict__ dev
     }
 }
 
-__global__ void __launch_bounds__(256) plan_groups_kernel(const int64_t* __restrict__ dev_list,
+__global__ void __launch_bounds__(256) plan_groups_kernel(const int64_t* dev_list,
                                                           const GroupEndsByValue by_value, int use_by_value,
                                                           int64_t E, int64_t M, GroupedHeader* header,
                                                           TileEntry* tiles, int64_t max_tiles, int tile_m, int mode,
                                                           int32_t* shared_error, int allow_prefix)
 {
-    after_previous(dev_list, header, tiles, shared_error);
-    plan_groups_body(dev_list, by_value, use_by_value, E, M, header, tiles, max_tiles, tile_m, mode, shared_error,
+    const int64_t zero = after_previous();
+    plan_groups_body(zero, dev_list, by_value, use_by_value, E, M, header, tiles, max_tiles, tile_m, mode, shared_error,
                      allow_prefix);
 }
 
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(256) plan_groups_kernel(const int64_t* __restr
 // SwiGLU form), which saves a second planner launch and a memset per call.
 constexpr int PLAN_CLEAR_CTAS = 30;
 
-__global__ void __launch_bounds__(256) plan_groups_both_kernel(const int64_t* __restrict__ dev_list,
+__global__ void __launch_bounds__(256) plan_groups_both_kernel(const int64_t* dev_list,
                                                                const GroupEndsByValue by_value, int use_by_value,
                                                                int64_t E, int64_t M, GroupedHeader* header,
                                                                TileEntry* tiles, int64_t max_tiles,
@@ -381,12 +381,12 @@ __global__ void __launch_bounds__(256) plan_groups_both_kernel(const int64_t* __
                                                                int64_t tail_max_tiles, int allow_prefix,
                                                                uint4* __restrict__ clear, int64_t clear16)
 {
-    after_previous(dev_list, header, tiles, tail_header, tail_tiles, clear);
+    const int64_t zero = after_previous();
     if (blockIdx.x == 0) {
-        plan_groups_body(dev_list, by_value, use_by_value, E, M, header, tiles, max_tiles, 256, PLAN_WHOLE, nullptr,
+        plan_groups_body(zero, dev_list, by_value, use_by_value, E, M, header, tiles, max_tiles, 256, PLAN_WHOLE, nullptr,
                          allow_prefix);
     } else if (blockIdx.x == 1) {
-        plan_groups_body(dev_list, by_value, use_by_value, E, M, tail_header, tail_tiles, tail_max_tiles, 128,
+        plan_groups_body(zero, dev_list, by_value, use_by_value, E, M, tail_header, tail_tiles, tail_max_tiles, 128,
                          PLAN_LEFTOVER, nullptr, allow_prefix);
     } else {
         const int64_t stride = static_cast<int64_t>(gridDim.x - 2) * blockDim.x;
@@ -405,17 +405,17 @@ __global__ void __launch_bounds__(256) plan_groups_both_kernel(const int64_t* __
 // 512 rows of a decode step: 5.5 us (12 with a warp per row).
 // ---------------------------------------------------------------------------
 template <bool DIRECT>
-__global__ void __launch_bounds__(256) gmsq_requant_kernel(const float* __restrict__ act,
-                                                           const uint32_t* __restrict__ amax_bits,
+__global__ void __launch_bounds__(256) gmsq_requant_kernel(const float* act,
+                                                           const uint32_t* amax_bits,
                                                            int8_t* __restrict__ y, float* __restrict__ y_scale,
                                                            int64_t M, int64_t H, const GroupedHeader* header, int parts)
 {
-    after_previous(act, amax_bits, y, y_scale, header);
+    const int64_t zero = after_previous();
     if (header->error != 0) {
         return;
     }
     const int lane = threadIdx.x & 31;
-    const int64_t warp_global = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int64_t warp_global = zero + ((static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
     const int64_t warps_total = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
     const int64_t n4 = H / 4;
     const int64_t per = (n4 + parts - 1) / parts;
@@ -477,13 +477,13 @@ __device__ __forceinline__ void split8(const float* src, uint4 (&word)[3])
 // multiple of 8 and both ends are 16-byte aligned (K of the operator is a multiple of 8).
 // Bound: HBM (16 bytes per value).  8 experts of 4096 x 4096 with 1000 rows, matmul included: 805 us, 944 with a value
 // and six 2-byte stores per thread.
-__global__ void __launch_bounds__(256) split_blocks_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst,
+__global__ void __launch_bounds__(256) split_blocks_kernel(const float* src, __nv_bfloat16* __restrict__ dst,
                                                            int64_t rows, int64_t len, int is_weight)
 {
-    after_previous(src, dst);
+    const int64_t zero = after_previous();
     const int64_t n8 = len / 8, total = rows * n8;
     const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += step) {
+    for (int64_t i = zero + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += step) {
         const int64_t r = i / n8, c = i - r * n8;
         uint4 w[3];
         split8(src + i * 8, w);

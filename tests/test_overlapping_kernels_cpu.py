@@ -5,6 +5,7 @@ writes during the life of the kernel, and may hit a line that was cached before 
 import glob
 import os
 import re
+import subprocess
 
 import pytest
 
@@ -22,3 +23,32 @@ def _code(path):
 @pytest.mark.parametrize("path", FILES, ids=os.path.basename)
 def test_no_non_coherent_loads(path):
     assert not re.findall(r"__ldg\s*\(|ld\.global\.nc\S*", _code(path))
+
+
+def _overlapping_kernels():
+    for path in FILES:
+        code = _code(path)
+        for m in re.finditer(r"__global__", code):
+            start = code.index("\n{", m.end())
+            if "after_previous(" in code[start:code.index("\n}", start)]:
+                signature = code[m.end():start]
+                yield re.search(r"(\w+_kernel)\s*\(", signature).group(1), signature
+
+
+def test_inputs_are_not_restrict():
+    """``const T* __restrict__`` lets the compiler make the loads non-coherent and move them above the wait."""
+    kernels = dict(_overlapping_kernels())
+    assert len(kernels) >= 15
+    assert [k for k, sig in kernels.items() if re.search(r"const\s+\w+\s*\*\s*__restrict__", sig)] == []
+
+
+def test_no_spills_in_the_swiglu_quantiser(tmp_path):
+    """The int32 form lives at the edge of its 64 registers: what the wait costs must not push it over."""
+    from cannbench_operator_solutions_b200 import build
+
+    cmd = [build._nvcc(), *build.NVCC_FLAGS, "-c", os.path.join(CSRC, "dqsq.cu"), "-o", str(tmp_path / "dqsq.o")]
+    log = subprocess.run(cmd, check=True, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True).stdout
+    spills = dict(re.findall(r"Compiling entry function '(\S*dqsq_rows_kernelILi0\S*)'.*?(\d+) bytes spill stores", log,
+                             flags=re.S))
+    assert len(spills) >= 3
+    assert {k: n for k, n in spills.items() if int(n) > 0} == {}
