@@ -482,9 +482,12 @@ void note_launch();  // counts one kernel launch of this library (w8a8_kernel_la
 // ---------------------------------------------------------------------------
 // Programmatic dependent launch.  A kernel launched with launch_chained may start while the kernel before it on the
 // stream is still running: its launch, block setup and prologue then overlap that kernel's tail instead of following
-// it.  Every such kernel opens with after_previous(), which lets the next kernel do the same and then waits until the
-// kernel before it has completed and its writes are visible; no global memory is touched before that, neither read
-// nor written.  Two rules keep it so in the compiled code:
+// it.  Every such kernel opens with after_previous(), which waits until the kernel before it has completed and its
+// writes are visible, and then lets the next kernel start; no global memory is touched before the wait, neither read nor
+// written.  The next kernel is let in after the wait, not ahead of it: with three kernels resident at once their blocks
+// share the SMs unevenly (back to back, the router on 16384 rows of 256 bf16 takes 9.0 us, 13.4 if it lets the next one
+// in ahead of the wait; the SwiGLU quantiser on 300 rows of 16384 int32 47 us, 67; kernels of 1.3 us take 0.1 us longer
+// this way).  Two rules keep the accesses behind the wait in the compiled code:
 //  - No load is a non-coherent one (ld.global.nc, __ldg): those are for memory that nothing writes during the life of
 //    the kernel, and the kernel before may write its outputs while this one already lives.  So the pointers that such a
 //    kernel only reads are not __restrict__ (the compiler makes those loads non-coherent, and free to move); the
@@ -493,7 +496,7 @@ void note_launch();  // counts one kernel launch of this library (w8a8_kernel_la
 //    first accesses are made with or guarded by, so that loads which the compiler takes for pure (__ldca, __ldcs,
 //    __ldcg) cannot move above the wait either.  (Passing the pointers through an asm instead did that too, but made
 //    every access a generic one and cost a register pair per pointer: the int32 form of the SwiGLU quantiser spilled,
-//    68.5 us on [16384, 4096] against 67.3, and 8192 sums of eight rows of 7164 took 744 us against 579.)
+//    68.5 us on [16384, 4096] against 67.3, and 8192 sums of eight rows of 7164 took 746 us against 590.)
 // Kernels that are launched plainly (and memsets, copies, event waits) order themselves against these as against any
 // other.
 // A dense layer of 16 rows 53.9 us (61.5 before), an expert layer of 2000 rows 160 (184) and of 64 rows 116 (129), a
@@ -502,8 +505,8 @@ void note_launch();  // counts one kernel launch of this library (w8a8_kernel_la
 __device__ __forceinline__ int64_t after_previous()
 {
     int64_t zero;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;\n\tmov.u64 %0, 0;" : "=l"(zero)::"memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     return zero;
 }
 

@@ -52,3 +52,10 @@ def test_no_spills_in_the_swiglu_quantiser(tmp_path):
                              flags=re.S))
     assert len(spills) >= 3
     assert {k: n for k, n in spills.items() if int(n) > 0} == {}
+
+
+def test_next_kernel_is_let_in_after_the_wait():
+    """Let in ahead of the wait, three kernels are resident at once and their blocks share the SMs unevenly."""
+    code = _code(os.path.join(CSRC, "common.cuh"))
+    order = re.findall(r"griddepcontrol\.(\w+)", code)
+    assert order == ["wait", "launch_dependents"]
