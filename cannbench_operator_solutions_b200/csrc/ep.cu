@@ -365,8 +365,24 @@ __global__ void __launch_bounds__(256) permute_rows_kernel(const uint8_t* src,
                 }
             }
         } else {
-            for (int64_t c = lane; c < row_bytes; c += 32) {
-                dst[d * row_bytes + c] = src[s * row_bytes + c];
+            // the loads of a step are all issued ahead of its stores: 65536 rows of 1000 bytes 49 us,
+            // 72 a byte at a time
+            for (int64_t base = 0; base < row_bytes; base += 32 * PERMUTE_UNROLL) {
+                uint8_t v[PERMUTE_UNROLL];
+#pragma unroll
+                for (int u = 0; u < PERMUTE_UNROLL; ++u) {
+                    const int64_t c = base + u * 32 + lane;
+                    if (c < row_bytes) {
+                        v[u] = src[s * row_bytes + c];
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < PERMUTE_UNROLL; ++u) {
+                    const int64_t c = base + u * 32 + lane;
+                    if (c < row_bytes) {
+                        dst[d * row_bytes + c] = v[u];
+                    }
+                }
             }
         }
         if (lane == 0 && src_scale != nullptr && dst_scale != nullptr) {

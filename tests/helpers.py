@@ -56,3 +56,24 @@ def zipf_group_list(rng, rows: int, experts: int, s: float = 1.1) -> np.ndarray:
     p /= p.sum()
     counts = rng.multinomial(rows, p)
     return np.cumsum(counts).astype(np.int64)
+
+
+def best_time(call, calls: int = 8, replays: int = 9) -> float:
+    """Shortest time of one call in ms, from a graph of several: for comparing two calls of one session, never for a
+    bound in absolute time."""
+    call()
+    stream = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        keep = [call() for _ in range(calls)]
+    start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    graph.replay()
+    best = float("inf")
+    for _ in range(replays):
+        start.record()
+        graph.replay()
+        stop.record()
+        stop.synchronize()
+        best = min(best, start.elapsed_time(stop) / calls)
+    del keep
+    return best
