@@ -412,7 +412,7 @@ static cudaError_t dispatch_dqsq(const void* x, const float* ws, const float* as
                           int, int);
     Kern kern = dqsq_long_rows_kernel<XT>;
     int threads = DQSQ_THREADS;
-    int regs = 40;
+    int64_t per_sm = 1;
     if (vec && chunks <= 2 * DQSQ_MAX_THREADS) {
         // Two chunks of each half per thread (one where a row has at most a warp's worth), rounded up to whole warps:
         // a thread count fitted to the row leaves few lanes idle on rows that are not a power of two long.  (Four
@@ -420,7 +420,7 @@ static cudaError_t dispatch_dqsq(const void* x, const float* ws, const float* as
         // 56-register form up to 576 threads: it puts two CTAs on an SM (24 against 27 us on fp16 [1531, 18432]).
         const bool two = chunks > 32;
         threads = static_cast<int>((((two ? (chunks + 1) / 2 : chunks) + 31) / 32) * 32);
-        regs = (XT == DQSQ_X_I32 && two) || threads > DQSQ_PAIR_THREADS ? 64 : 56;
+        const int regs = (XT == DQSQ_X_I32 && two) || threads > DQSQ_PAIR_THREADS ? 64 : 56;
         if (!two) {
             kern = dqsq_rows_kernel<XT, 1, true, DQSQ_PAIR_THREADS>;  // rows this short always divide
         } else if (XT == DQSQ_X_I32) {
@@ -432,10 +432,18 @@ static cudaError_t dispatch_dqsq(const void* x, const float* ws, const float* as
         } else {
             kern = dqsq_rows_kernel<XT, 2, false, DQSQ_MAX_THREADS>;
         }
+        per_sm = std::min(std::max(1, 65536 / (regs * threads)), 32);
+    } else {
+        static KernelFacts facts;
+        int ctas = 1;
+        const cudaError_t e = resident_ctas(facts, kern, threads, &ctas);
+        if (e != cudaSuccess) {
+            return e;
+        }
+        per_sm = ctas;
     }
     // one wave: as many CTAs as the registers hold at once, each walking rows with a grid stride
-    const int64_t per_sm = std::max<int64_t>(1, (65536 / (regs * threads)));
-    const int64_t cap = static_cast<int64_t>(sm_count()) * std::min<int64_t>(per_sm, 32);
+    const int64_t cap = static_cast<int64_t>(sm_count()) * per_sm;
     const unsigned grid = static_cast<unsigned>(M < cap ? M : cap);
     return launch_chained(kern, grid, static_cast<unsigned>(threads), 0, st, x, ws, as, qs, y, scale, M, H, left, direct,
                           divide);
