@@ -59,3 +59,16 @@ def test_next_kernel_is_let_in_after_the_wait():
     code = _code(os.path.join(CSRC, "common.cuh"))
     order = re.findall(r"griddepcontrol\.(\w+)", code)
     assert order == ["wait", "launch_dependents"]
+
+
+def test_registers_of_the_unvectorised_combine(tmp_path):
+    """Three blocks of 256 threads per SM need 80 registers or fewer, without spills: the look-up of the next row stays
+    with the vectorised form."""
+    from cannbench_operator_solutions_b200 import build
+
+    cmd = [build._nvcc(), *build.NVCC_FLAGS, "-c", os.path.join(CSRC, "ep.cu"), "-o", str(tmp_path / "ep.o")]
+    log = subprocess.run(cmd, check=True, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True).stdout
+    forms = re.findall(r"Compiling entry function '(\S*mfr_kernelILi[01]ELb0ELb0E\S*)'.*?(\d+) bytes spill stores"
+                       r".*?Used (\d+) registers", log, flags=re.S)
+    assert len(forms) == 4  # fp16 and bf16, 32- and 64-bit positions
+    assert [f for f in forms if int(f[1]) > 0 or int(f[2]) > 80] == []
