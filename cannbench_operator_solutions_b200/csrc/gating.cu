@@ -157,9 +157,10 @@ __global__ void __launch_bounds__(GATING_WARPS * 32) gating_kernel(const void* x
 // 16-bit rows are selected on one integer per element, the ordered bits of x above 8191 - column (the low 13 bits
 // of a bf16 or fp16 value widened to fp32 are zero).  That is the order of the exponentials too - the exponential
 // does not decrease, checked over all floats - except where two different x have the same exponential: such a row
-// (seen from the selected exponentials, and for the last one from the exponential of the next smaller x) is redone
-// by the whole warp on the exponentials, and so is a row whose maximum is not finite.  fp32 rows are selected on the
-// exponential above the column in 64 bits, where the question does not arise.
+// (seen from the selected exponentials, and for the last one from the exponential of the next smaller x) is selected
+// once more by gating_settle, which knows the two ways in which that happens to real rows.  What is left, and a
+// row whose maximum is not finite, goes to the whole warp.  fp32 rows are selected on the exponential above the column
+// in 64 bits, where the question does not arise.
 //
 // Bound: issue slots.  65536 x 256 bf16, k = 8: 26 us, was 55 with a warp per row (869 warp instructions per row); fp32: 50 us.
 // ---------------------------------------------------------------------------
@@ -289,6 +290,162 @@ __device__ __noinline__ void gating_row_by_warp(const void* x, int64_t row, int6
     }
 }
 
+// x in the order of its value as an integer with the low 13 bits clear, and back
+__device__ __forceinline__ int gating_ordered(float v)
+{
+    const int bits = __float_as_int(v);
+    return bits ^ ((bits >> 31) & (0x7fffffff & ~GATING_COL_MASK));
+}
+
+__device__ __forceinline__ float gating_value(int ordered)
+{
+    return __int_as_float(ordered ^ ((ordered >> 31) & (0x7fffffff & ~GATING_COL_MASK)));
+}
+
+// A lower bound of the 16-bit x next below one that is not zero, in the same order.  (Below +0 comes -0, 0x2000 away
+// for bf16 too: what is reached from +0 is a smaller x with the same exponential, which is what the caller asks for.)
+template <int DT>
+__device__ __forceinline__ int gating_next_below(int ordered)
+{
+    return ordered - ((DT == W8A8_DT_BF16) ? 0x10000 : 0x2000);
+}
+
+// lane q of a row stores the selections 2 q and 2 q + 1
+template <int DT>
+__device__ __forceinline__ void gating_store_two(int64_t row, int64_t rows, int inner, int k, const float (&e)[2],
+                                                 const int (&col)[2], float s, const uint8_t* finished, void* y,
+                                                 int32_t* expert_idx, int32_t* row_idx)
+{
+    const bool fin = (finished != nullptr) && (finished[row] != 0);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int j = 2 * (threadIdx.x & 3) + h;
+        if (j < k) {
+            const int64_t o = row * k + j;
+            gating_store<DT>(y, o, __fdiv_rn(e[h], s));
+            expert_idx[o] = fin ? inner : col[h];
+            row_idx[o] = static_cast<int32_t>(static_cast<int64_t>(j) * rows + row);
+        }
+    }
+}
+
+// entries 2 q and 2 q + 1 of a list that the lanes of a row hold alike
+template <typename Key>
+__device__ __forceinline__ void gating_own_two(const Key (&best)[8], Key (&own)[2])
+{
+    own[0] = best[0], own[1] = best[1];
+#pragma unroll
+    for (int h = 1; h < 4; ++h) {
+        if (static_cast<int>(threadIdx.x & 3) == h) {
+            own[0] = best[2 * h];
+            own[1] = best[2 * h + 1];
+        }
+    }
+}
+
+// Rows in which different x share an exponential, four lanes per row as in gating_top8_kernel (m: the maximum, s: the
+// sum of exponentials, which that kernel has).  Two sets of x share one in real rows: those so far below the maximum
+// that it is zero or nearly so (saturated or masked logits), and those around zero, whose difference from the maximum
+// rounds alike (all of a row of zeros: signed zeros and the smallest numbers).  The key of the first is the exponential
+// itself, below every ordered x, that of the second zero, so that the column decides among equal ones.
+// Returns whether the row is settled, and stored if `wanted`; an x shared otherwise leaves it unsettled.
+// 16384 rows of 256 zeros: 16.5 us, 78 by the whole warp (14.4 by the kernel with a warp per row).
+template <int DT, bool VEC>
+__device__ __forceinline__ bool gating_tied_rows(const void* x, int64_t row, int64_t rows, int inner, int k, float m,
+                                                 float s, bool wanted, const uint8_t* finished, void* y,
+                                                 int32_t* expert_idx, int32_t* row_idx)
+{
+    // exponentials with a bit pattern below 1024 fit between the smallest integer and the ordered bits of -inf
+    constexpr int LOW = INT32_MIN, LOW_END = LOW + (1023 << 13);
+    const int q = threadIdx.x & 3;
+    const int pieces = (inner + 31) / 32;
+    const float e_zero = m > 0.0f ? canonical_expf(-m) : 1.0f;  // of x = 0, or of the maximum where every x is negative
+    int best[8];
+    for (int i = 0; i < pieces; ++i) {
+        float v[8];
+        gating_load8<DT, VEC>(x, row, inner, 4 * i + q, v);
+        f32x2 d[4], e[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            d[j] = add2(pair(v[2 * j], v[2 * j + 1]), pair(-m));
+        }
+        exp_nonpositive2<4>(d, e);
+        int key[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            float e0, e1;
+            unpair(e[j / 2], e0, e1);
+            const float ej = (j & 1) ? e1 : e0;
+            const int bits = __float_as_int(ej);
+            const int value = bits < 1024 ? LOW + (bits << 13) : (ej == e_zero ? 0 : gating_ordered(v[j]));
+            key[j] = value + (GATING_COL_MASK - 32 * i - 8 * q - j);
+        }
+        sort8_desc(key);
+        if (i == 0) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                best[j] = key[j];
+            }
+        } else {
+            merge8_desc(best, key);
+        }
+    }
+#pragma unroll
+    for (int off = 2; off > 0; off >>= 1) {
+        int other[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            other[j] = __shfl_xor_sync(FULL_MASK, best[j], off);
+        }
+        merge8_desc(best, other);
+    }
+    int own[2], xo[2], col[2];
+    float e[2];
+    gating_own_two(best, own);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        col[h] = GATING_COL_MASK - (own[h] & GATING_COL_MASK);
+        xo[h] = own[h] & ~GATING_COL_MASK;
+        e[h] = xo[h] <= LOW_END ? __int_as_float((xo[h] - LOW) >> 13)
+                                : (xo[h] == 0 ? e_zero : canonical_expf(__fsub_rn(gating_value(xo[h]), m)));
+    }
+    const float next_e = __shfl_down_sync(FULL_MASK, e[0], 1);
+    const int next_x = __shfl_down_sync(FULL_MASK, xo[0], 1);
+    const int j = 2 * q;
+    bool shared = j + 1 < k && e[0] == e[1] && xo[0] != xo[1];
+    shared |= j + 2 < k && e[1] == next_e && xo[1] != next_x;
+    const bool last0 = j == k - 1;
+    const int last_x = last0 ? xo[0] : xo[1];
+    if ((last0 || j + 1 == k - 1) && last_x > LOW_END && last_x != 0) {
+        shared |= canonical_expf(__fsub_rn(gating_value(gating_next_below<DT>(last_x)), m)) == (last0 ? e[0] : e[1]);
+    }
+    const unsigned open = __ballot_sync(FULL_MASK, shared);
+    const bool settled = wanted && ((open >> (threadIdx.x & 28)) & 0xfu) == 0;
+    if (settled) {
+        gating_store_two<DT>(row, rows, inner, k, e, col, s, finished, y, expert_idx, row_idx);
+    }
+    return settled;
+}
+
+// What gating_top8_kernel leaves open: rows with `open` set in their four lanes (row0: the warp's first row)
+template <int DT, bool VEC>
+__device__ __noinline__ void gating_settle(const void* x, int64_t row0, int64_t row, int64_t rows, int inner, int k, float m,
+                                           float s, bool open, const uint8_t* finished, void* y, int32_t* expert_idx,
+                                           int32_t* row_idx)
+{
+    if constexpr (DT != W8A8_DT_F32) {
+        const bool finite = fabsf(m) < INFINITY;
+        open &= !gating_tied_rows<DT, VEC>(x, row, rows, inner, k, m, s, open && finite, finished, y, expert_idx, row_idx);
+    }
+    unsigned again = __ballot_sync(FULL_MASK, open);
+    while (again != 0) {
+        const int g = (__ffs(again) - 1) >> 2;
+        again &= ~(0xfu << (4 * g));
+        const bool fin = (finished != nullptr) && (finished[row0 + g] != 0);
+        gating_row_by_warp<DT>(x, row0 + g, rows, inner, k, fin, y, expert_idx, row_idx);
+    }
+}
+
 template <int DT, bool VEC>
 __global__ void __launch_bounds__(GATING_TOP_THREADS) gating_top8_kernel(const void* x,
                                                                          const uint8_t* finished,
@@ -354,8 +511,7 @@ __global__ void __launch_bounds__(GATING_TOP_THREADS) gating_top8_kernel(const v
         if constexpr (!WIDE) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const int bits = __float_as_int(v[j]);
-                key[j] = (bits ^ ((bits >> 31) & (0x7fffffff & ~GATING_COL_MASK))) + (GATING_COL_MASK - col - j);
+                key[j] = gating_ordered(v[j]) + (GATING_COL_MASK - col - j);
             }
         }
         sort8_desc(key);
@@ -393,15 +549,8 @@ __global__ void __launch_bounds__(GATING_TOP_THREADS) gating_top8_kernel(const v
     }
     const float s = part[0];
 
-    // lane q stores the selections 2 q and 2 q + 1
-    Key own[2] = {best[0], best[1]};
-#pragma unroll
-    for (int h = 1; h < 4; ++h) {
-        if (q == h) {
-            own[0] = best[2 * h];
-            own[1] = best[2 * h + 1];
-        }
-    }
+    Key own[2];
+    gating_own_two(best, own);
     float e[2];
     int col[2];
     if constexpr (WIDE) {
@@ -411,15 +560,12 @@ __global__ void __launch_bounds__(GATING_TOP_THREADS) gating_top8_kernel(const v
             col[h] = static_cast<int>(~static_cast<uint32_t>(own[h]));
         }
     } else {
-        constexpr int FLIP = 0x7fffffff & ~GATING_COL_MASK;
-        constexpr int STEP = (DT == W8A8_DT_BF16) ? 0x10000 : 0x2000;  // at most the distance to the next smaller x
-        auto value = [](int ordered) { return __int_as_float(ordered ^ ((ordered >> 31) & FLIP)); };
         int xo[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             col[h] = GATING_COL_MASK - (own[h] & GATING_COL_MASK);
             xo[h] = own[h] & ~GATING_COL_MASK;
-            e[h] = canonical_expf(__fsub_rn(value(xo[h]), m));
+            e[h] = canonical_expf(__fsub_rn(gating_value(xo[h]), m));
         }
         const float next_e = __shfl_down_sync(FULL_MASK, e[0], 1);
         const int next_x = __shfl_down_sync(FULL_MASK, xo[0], 1);
@@ -428,29 +574,17 @@ __global__ void __launch_bounds__(GATING_TOP_THREADS) gating_top8_kernel(const v
         redo |= j + 2 < k && e[1] == next_e && xo[1] != next_x;
         const bool last0 = j == k - 1;
         if (last0 || j + 1 == k - 1) {
-            redo |= canonical_expf(__fsub_rn(value((last0 ? xo[0] : xo[1]) - STEP), m)) == (last0 ? e[0] : e[1]);
+            redo |= canonical_expf(__fsub_rn(gating_value(gating_next_below<DT>(last0 ? xo[0] : xo[1])), m)) ==
+                    (last0 ? e[0] : e[1]);
         }
     }
-    unsigned again = __ballot_sync(FULL_MASK, redo && mine < rows);
-    const bool my_row_again = ((again >> (lane & ~3)) & 0xfu) != 0;
-    if (mine < rows && !my_row_again) {
-        const bool fin = (finished != nullptr) && (finished[row] != 0);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int j = 2 * q + h;
-            if (j < k) {
-                const int64_t o = row * k + j;
-                gating_store<DT>(y, o, __fdiv_rn(e[h], s));
-                expert_idx[o] = fin ? inner : col[h];
-                row_idx[o] = static_cast<int32_t>(static_cast<int64_t>(j) * rows + row);
-            }
-        }
+    const unsigned flagged = __ballot_sync(FULL_MASK, redo && mine < rows);
+    const bool open = ((flagged >> (lane & ~3)) & 0xfu) != 0;
+    if (mine < rows && !open) {
+        gating_store_two<DT>(row, rows, inner, k, e, col, s, finished, y, expert_idx, row_idx);
     }
-    while (again != 0) {
-        const int g = (__ffs(again) - 1) >> 2;
-        again &= ~(0xfu << (4 * g));
-        const bool fin = (finished != nullptr) && (finished[row0 + g] != 0);
-        gating_row_by_warp<DT>(x, row0 + g, rows, inner, k, fin, y, expert_idx, row_idx);
+    if (flagged != 0) {
+        gating_settle<DT, VEC>(x, row0, row, rows, inner, k, m, s, open, finished, y, expert_idx, row_idx);
     }
 }
 
