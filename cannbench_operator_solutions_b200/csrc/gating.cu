@@ -12,9 +12,9 @@
 // elements t, t+32, ... in ascending order, then a butterfly over lane distances 16, 8, 4, 2, 1).  Equal
 // exponentials are ordered by ascending expert index.
 //
-// Two kernels.  gating_top8_kernel (k <= 8, many rows) gives a row to four lanes, which is where the summation order puts whole
-// 8-element pieces of a row into one lane; see there.  gating_kernel (the rest) gives a row to a warp: lane t owns
-// elements t + 32 v, ranks its own once (larger exponential first, equal ones by ascending index) and parks them in
+// Two kernels.  gating_top8_kernel (k <= 8, many rows, see four_lanes_pay) gives a row to four lanes, which is where the
+// summation order puts whole 8-element pieces of a row into one lane; see there.  gating_kernel (the rest) gives a row
+// to a warp: lane t owns elements t + 32 v, ranks its own once (larger exponential first, equal ones by ascending index) and parks them in
 // that order in shared memory; the k selections are then k rounds of "largest head of the 32 lists" - two
 // `redux.sync`, one 8-byte shared-memory load and a counter per round.  The operator moves rows * inner input
 // elements and 10 k bytes of output per row; at router sizes (inner <= 1024) it is bound by issue slots, not by HBM.
@@ -625,13 +625,34 @@ static cudaError_t launch_gating(const void* x, const uint8_t* finished, void* y
     return e;
 }
 
+// Four lanes per row or a warp?  Both kernels' times in us are close to lines in the rows (r thousand of them), fitted to
+// 896 calls of 4096 - 65536 rows, 8 - 1024 columns, k = 1 - 8, bf16 and fp32, and the shorter one is taken.  A warp pays
+// for the columns rounded up to 32, 64, ... 1024 and for every selection; four lanes pay for the columns themselves, not
+// for k, more for fp32 (64-bit keys) and for rows that are read an element at a time, and start later.  Measured, warp
+// and four lanes: 65536 x 256 bf16, k = 8 53 and 24; 16384 x 256 fp32, k = 1 10.5 and 15.4; 4096 x 500 bf16, k = 1 8.0 and
+// 10.5; 4096 x 264 bf16, k = 1 7.3 and 5.4.  The choice lost 0.2 % on the average and 20 % at most (8192 x 500, k = 4).
+template <int DT>
+static bool four_lanes_pay(int64_t rows, int inner, int k, bool vec)
+{
+    constexpr double WARP_ROW[6] = {0.139, 0.174, 0.268, 0.500, 1.333, 5.393};
+    int v = 0;
+    while ((32 << v) < inner) {
+        ++v;
+    }
+    const double r = static_cast<double>(rows) * 1e-3;
+    const double warp = 1.76 + r * (WARP_ROW[v] + 0.033 * k);
+    const double four = (DT == W8A8_DT_F32) ? (vec ? 1.64 + 0.0079 * inner + r * (0.067 + 0.0026 * inner)
+                                                   : 1.77 + 0.0097 * inner + r * (0.056 + 0.0034 * inner))
+                                            : (vec ? 1.63 + 0.0068 * inner + r * (0.050 + 0.00118 * inner)
+                                                   : 1.66 + 0.0102 * inner + r * (0.048 + 0.00162 * inner));
+    return four < warp;
+}
+
 template <int DT>
 static cudaError_t dispatch_gating(const void* x, const uint8_t* finished, void* y, int32_t* expert_idx,
                                    int32_t* row_idx, int64_t rows, int inner, int k, cudaStream_t st)
 {
-    // Four lanes take 4.1 us for their first rows where a warp takes 2.5 (64 elements in turn against 8), and 0.36 us
-    // per 1024 rows of 256 against 0.82: they part at about 3700 rows.
-    if (k <= GATING_TOP && rows >= 4096) {
+    if (k <= GATING_TOP && rows >= 4096 && four_lanes_pay<DT>(rows, inner, k, inner % 8 == 0 && is_aligned(x, 16))) {
         return launch_gating_top8<DT>(x, finished, y, expert_idx, row_idx, rows, inner, k, st);
     }
     if (inner <= 32) {
