@@ -510,9 +510,10 @@ __device__ __forceinline__ int64_t after_previous()
     return zero;
 }
 
+// overlap = false: starts when the kernel before it has completed, like a plain launch.
 template <typename... Params, typename... Args>
-cudaError_t launch_chained(void (*kern)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
-                           Args&&... args)
+cudaError_t launch_chained_if(bool overlap, void (*kern)(Params...), unsigned grid, unsigned block, size_t smem,
+                              cudaStream_t st, Args&&... args)
 {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid, 1, 1);
@@ -521,11 +522,18 @@ cudaError_t launch_chained(void (*kern)(Params...), unsigned grid, unsigned bloc
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     note_launch();
     return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+}
+
+template <typename... Params, typename... Args>
+cudaError_t launch_chained(void (*kern)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+                           Args&&... args)
+{
+    return launch_chained_if(true, kern, grid, block, smem, st, static_cast<Args&&>(args)...);
 }
 
 inline bool is_aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }

@@ -28,3 +28,12 @@ def test_no_step_in_the_cost_where_four_lanes_become_possible(ops):
     t_few = best_time(lambda: ops.moe_gating_top_k_softmax(few, None, 1), calls=20)
     t_many = best_time(lambda: ops.moe_gating_top_k_softmax(many, None, 1), calls=20)
     assert t_many < 1.3 * t_few
+
+
+def test_calls_that_fill_most_of_the_chip_do_not_crowd_each_other(ops):
+    """32768 rows of 256 fill two thirds of the SMs' places: 1.5 times the time of 16384 rows in a row of calls, 1.9 when
+    each call starts beside the one before."""
+    half, whole = (torch.randn(n, 256, device="cuda").bfloat16() for n in (16384, 32768))
+    t_half = best_time(lambda: ops.moe_gating_top_k_softmax(half, None, 8), calls=20)
+    t_whole = best_time(lambda: ops.moe_gating_top_k_softmax(whole, None, 8), calls=20)
+    assert t_whole < 1.7 * t_half
