@@ -228,5 +228,5 @@ extern "C" int w8a8_add_rms_norm_dynamic_quant(const void* x1, const void* x2, c
         (dtype == W8A8_DT_BF16)
             ? w8a8::dispatch<W8A8_DT_BF16>(x1, x2, gamma, y, x_out, scale_out, rows, N, epsilon, vec, direct, st)
             : w8a8::dispatch<W8A8_DT_F16>(x1, x2, gamma, y, x_out, scale_out, rows, N, epsilon, vec, direct, st);
-    return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    return w8a8::launch_status(e);
 }

@@ -536,6 +536,17 @@ cudaError_t launch_chained(void (*kern)(Params...), unsigned grid, unsigned bloc
     return launch_chained_if(true, kern, grid, block, smem, st, static_cast<Args&&>(args)...);
 }
 
+// The status of an entry point's launches.  A failed one's error is also taken out of the thread's last-error slot, so
+// that whoever looks there next (torch does after each of its own launches) does not take it for its own.
+inline int launch_status(cudaError_t e)
+{
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        return W8A8_ERR_CUDA;
+    }
+    return W8A8_OK;
+}
+
 inline bool is_aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 
 int sm_count();  // cached multiprocessor count of the current device

@@ -203,5 +203,5 @@ extern "C" int w8a8_dynamic_quant(const void* x, int8_t* y, float* scale, int64_
     const cudaError_t e = (dtype == W8A8_DT_BF16)
                               ? w8a8::dispatch<W8A8_DT_BF16>(x, y, scale, M, N, vec, direct, st)
                               : w8a8::dispatch<W8A8_DT_F16>(x, y, scale, M, N, vec, direct, st);
-    return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    return w8a8::launch_status(e);
 }

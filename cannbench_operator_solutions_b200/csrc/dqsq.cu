@@ -493,5 +493,5 @@ extern "C" int w8a8_dequant_swiglu_quant(const void* x, const float* weight_scal
         e = w8a8::dispatch_dqsq<w8a8::DQSQ_X_BF16>(x, nullptr, nullptr, quant_scale, y, scale, M, H, left, direct, vec,
                                                    st);
     }
-    return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    return w8a8::launch_status(e);
 }

@@ -1294,7 +1294,7 @@ extern "C" int w8a8_combine(const void* rows, const float* probs, const int64_t*
     const cudaError_t e = w8a8::launch_chained(kern, grid, 256, 0, st, rows, expanded_pos, nullptr, nullptr, nullptr,
                                                probs,
                                                nullptr, out, T, H, static_cast<int>(topk), 0, INT64_MAX, 0, W8A8_DT_F32);
-    return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    return w8a8::launch_status(e);
 }
 
 // workspace: 256-byte header | dst_first[N*E+1] | src_first[N*E] | col_start[E+1] | row_start[N+1] | index[A]
@@ -1400,7 +1400,7 @@ static int launch_mfr(const void* rows, const int32_t* esdr, const void* skip1, 
     const cudaError_t e = w8a8::launch_chained(kern, grid, 256, 0, st, rows, esdr, skip1, skip2, bias, scales, expert,
                                                out, R,
                                                H, static_cast<int>(K), E, num_dst, col_mode, scale_dt);
-    return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    return w8a8::launch_status(e);
 }
 
 extern "C" int w8a8_moe_finalize_routing(const void* rows, const int32_t* src_to_dst_row, const void* skip1,

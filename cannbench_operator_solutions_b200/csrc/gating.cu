@@ -722,5 +722,5 @@ extern "C" int w8a8_moe_gating_top_k_softmax(const void* x, const uint8_t* finis
         e = w8a8::dispatch_gating<W8A8_DT_F32>(x, finished, y, expert_idx, row_idx, rows, in, kk, st);
         break;
     }
-    return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    return w8a8::launch_status(e);
 }

@@ -618,7 +618,7 @@ static int plan_groups(const int64_t* group_list, int list_on_device, int64_t E,
         e = launch_chained(plan_groups_kernel, 1, 256, smem, st, dev_list, bv, use_bv, E, M, header, tiles, max_tiles,
                            tile_m, mode, shared_error, list_on_device == 2 ? 1 : 0);
     }
-    return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    return launch_status(e);
 }
 
 // Runs a grouped problem whose GemmParams are filled in except for the tile table: plans the groups and launches
@@ -668,7 +668,7 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
         const int64_t most = g.max_tiles * p.n_tiles;
         const cudaError_t e = row_boxes ? dispatch_row_boxes<KIND, EPI>(b_mn, ta, tb, p, most, st)
                                         : dispatch_gemm<KIND, EPI>(shape, 256, b_mn, ta, tb, p, most, st);
-        return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+        return launch_status(e);
     }
     const int rc = plan_groups(group_list, list_on_device, E, M, g, 256, st, PLAN_BOTH, clear, clear_bytes);
     if (rc != W8A8_OK) {
@@ -679,7 +679,7 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
     p.tile_done = g.tile_done;
     cudaError_t e = dispatch_gemm<KIND, EPI>(2, 256, b_mn, ta, tb, p, (M / 256 + E + 1) * p.n_tiles, st);
     if (e != cudaSuccess) {
-        return W8A8_ERR_CUDA;
+        return launch_status(e);
     }
     p.tiles = g.tail_tiles;
     p.header = g.tail_header;
@@ -694,7 +694,7 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
     } else {
         e = dispatch_gemm<KIND, EPI>(1, 256, b_mn, ta, tb, p, most, st);
     }
-    return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    return launch_status(e);
 }
 
 // ---------------------------------------------------------------------------
@@ -807,7 +807,7 @@ static int quant_matmul_impl(const int8_t* x1, const int8_t* x2, const void* sca
             e = b_mn ? launch_gemm<1, 128, KIND_I8, EPI_QMM, true, 8, true>(ta, tb, p, tiles128, st)
                      : launch_gemm<1, 128, KIND_I8, EPI_QMM, false, 8, true>(ta, tb, p, tiles128, st);
         }
-        return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+        return launch_status(e);
     }
     const int cg = (own_choice && tiles128 <= sm_count()) ? 1 : choose_cta_group(M, false);
     const int tile_m = 128 * cg;
@@ -824,7 +824,7 @@ static int quant_matmul_impl(const int8_t* x1, const int8_t* x2, const void* sca
     } else {
         e = dispatch_gemm<KIND_I8, EPI_QMM>(cg, block_n, b_mn, ta, tb, p, total, st);
     }
-    return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    return launch_status(e);
 }
 
 extern "C" int w8a8_quant_matmul(const int8_t* x1, const int8_t* x2, const void* scale, const float* offset,
@@ -948,7 +948,7 @@ extern "C" int w8a8_grouped_matmul_swiglu_quant(const int8_t* x, const int8_t* w
     auto kern = (flags & W8A8_F_ROUND_DIRECT) ? gmsq_requant_kernel<true> : gmsq_requant_kernel<false>;
     const cudaError_t e = launch_chained(kern, static_cast<unsigned>(blocks), 256, 0, st, g.act, g.amax, y, y_scale, M, H,
                                          g.header, parts);
-    return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    return launch_status(e);
 }
 
 // ===========================================================================
@@ -1061,7 +1061,7 @@ static int grouped_matmul_impl(const void* x, const void* w, const void* bias, v
                                b_mn ? K * N : K, 1);
         }
         if (e != cudaSuccess) {
-            return W8A8_ERR_CUDA;
+            return launch_status(e);
         }
         x = xs;
         w = wsplit;

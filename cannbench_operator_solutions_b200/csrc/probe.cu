@@ -287,7 +287,7 @@ extern "C" int w8a8_mma_issue_probe(int cta_group, int umma_m, int umma_n, int a
                                accumulators, per_commit, depth, pattern, static_cast<long long>(batches), error_word);
     }
     note_launch();
-    return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+    return w8a8::launch_status(e);
 }
 
 extern "C" int64_t w8a8_mma_issue_probe_ops(int cta_group, int umma_m, int umma_n, int per_commit, int64_t batches)
