@@ -421,16 +421,16 @@ static cudaError_t dispatch_dqsq(const void* x, const float* ws, const float* as
         const bool two = chunks > 32;
         threads = static_cast<int>((((two ? (chunks + 1) / 2 : chunks) + 31) / 32) * 32);
         const int regs = (XT == DQSQ_X_I32 && two) || threads > DQSQ_PAIR_THREADS ? 64 : 56;
+        // (chosen where compiled, so that no form is built that no call reaches)
         if (!two) {
             kern = dqsq_rows_kernel<XT, 1, true, DQSQ_PAIR_THREADS>;  // rows this short always divide
-        } else if (XT == DQSQ_X_I32) {
+        } else if constexpr (XT == DQSQ_X_I32) {
             kern = divide ? dqsq_rows_kernel<XT, 2, true, DQSQ_MAX_THREADS> : dqsq_rows_kernel<XT, 2, false, DQSQ_MAX_THREADS>;
-        } else if (divide) {
-            kern = dqsq_rows_kernel<XT, 2, true, DQSQ_PAIR_THREADS>;
-        } else if (threads <= DQSQ_PAIR_THREADS) {
-            kern = dqsq_rows_kernel<XT, 2, false, DQSQ_PAIR_THREADS>;
         } else {
-            kern = dqsq_rows_kernel<XT, 2, false, DQSQ_MAX_THREADS>;
+            // rows that divide are at most 1984 long: 576 threads are enough
+            kern = divide ? dqsq_rows_kernel<XT, 2, true, DQSQ_PAIR_THREADS>
+                          : (threads <= DQSQ_PAIR_THREADS ? dqsq_rows_kernel<XT, 2, false, DQSQ_PAIR_THREADS>
+                                                          : dqsq_rows_kernel<XT, 2, false, DQSQ_MAX_THREADS>);
         }
         per_sm = std::min(std::max(1, 65536 / (regs * threads)), 32);
     } else {

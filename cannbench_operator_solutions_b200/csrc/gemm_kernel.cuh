@@ -600,7 +600,6 @@ struct SplitSlices {
     }
 };
 
-template <int EPI>
 __device__ __forceinline__ void split_send(const GemmParams& p, int m_rows, uint32_t t_addr, int row, int half, int rank,
                                            uint32_t smem_base)
 {
@@ -1147,7 +1146,7 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
         TileInfo tl{};
         if (mine) {
             tl = decode(worker);
-            split_send<EPI>(p, tl.m_rows, t_addr, row_in_tile, (warp - 2) >> 2, split_rank, smem_base);
+            split_send(p, tl.m_rows, t_addr, row_in_tile, (warp - 2) >> 2, split_rank, smem_base);
         }
         __syncwarp();
         tc::cluster_arrive();
