@@ -287,7 +287,7 @@ extern "C" int w8a8_mma_issue_probe(int cta_group, int umma_m, int umma_n, int a
                                accumulators, per_commit, depth, pattern, static_cast<long long>(batches), error_word);
     }
     note_launch();
-    return w8a8::launch_status(e);
+    return (e == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
 }
 
 extern "C" int64_t w8a8_mma_issue_probe_ops(int cta_group, int umma_m, int umma_n, int per_commit, int64_t batches)
@@ -319,6 +319,112 @@ __global__ void __launch_bounds__(256) exp_selftest_kernel(unsigned long long* o
     }
 }
 
+// The forms on pairs (see common.cuh) against the scalar ones, four pairs at a time as the kernels use them.
+// out[2 c] counts what differs in check c, out[2 c + 1] is the smallest pattern that does:
+//   0  neg_exp_neg2 against -canonical_expf(-g), every g in [-80, 80]
+//   1  exp_nonpositive2 against canonical_expf(x), every x <= 0
+//   2  canonical_expf of neighbouring floats: the one of the smaller must not be larger
+//   3  quotient2 against the IEEE division where the quotient lies nearest to the middle of two floats
+__device__ __forceinline__ void selftest_note(unsigned long long* out, int check, uint32_t pattern)
+{
+    atomicAdd(out + 2 * check, 1ull);
+    atomicMin(out + 2 * check + 1, static_cast<unsigned long long>(pattern));
+}
+
+__global__ void __launch_bounds__(256) pair_exp_selftest_kernel(unsigned long long* out)
+{
+    const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
+    for (unsigned long long i = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < (1ull << 29);
+         i += stride) {
+        const uint32_t first = static_cast<uint32_t>(i) * 8u;
+        float x[8], got[8];
+        f32x2 in[4], e[4];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            x[j] = __uint_as_float(first + j);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            in[j] = pair(x[2 * j], x[2 * j + 1]);
+        }
+        neg_exp_neg2<4>(in, e);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            unpair(e[j], got[2 * j], got[2 * j + 1]);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (fabsf(x[j]) <= EXP2_MAX_ABS && __float_as_uint(got[j]) != __float_as_uint(-canonical_expf(-x[j]))) {
+                selftest_note(out, 0, first + j);
+            }
+        }
+        exp_nonpositive2<4>(in, e);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            unpair(e[j], got[2 * j], got[2 * j + 1]);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (x[j] <= 0.0f && __float_as_uint(got[j]) != __float_as_uint(canonical_expf(x[j]))) {
+                selftest_note(out, 1, first + j);
+            }
+            // the next pattern is the neighbour away from zero
+            const float far = __uint_as_float(first + j + 1);
+            const float e_near = canonical_expf(x[j]), e_far = canonical_expf(far);
+            if (!isnan(x[j]) && !isnan(far) && (signbit(x[j]) ? e_far > e_near : e_near > e_far) &&
+                signbit(far) == signbit(x[j])) {
+                selftest_note(out, 2, first + j);
+            }
+        }
+    }
+}
+
+// Significands d of 24 bits, numerators n of 24 bits with n 2^k = (2 Q + 1) d + r: the quotient lies r / (d 2^k) from the
+// middle of two floats, where 2^k is 2^24 for n >= d and 2^25 below.  Every d, every n with |r| <= 15.
+__global__ void __launch_bounds__(256) pair_quotient_selftest_kernel(unsigned long long* out)
+{
+    const uint32_t d = (1u << 23) + blockIdx.x * blockDim.x + threadIdx.x;
+    const int even = __ffs(d) - 1;
+    if (even > 3 || d >= (1u << 24)) {
+        return;  // r is a multiple of the largest power of two in d
+    }
+    const uint32_t odd = d >> even;
+    unsigned long long tested = 0;
+#pragma unroll 1
+    for (int k = 24; k <= 25; ++k) {
+        uint64_t inverse = 1;  // of 2^(k - even), mod odd
+        for (int i = 0; i < k - even; ++i) {
+            inverse = (inverse & 1) ? (inverse + odd) >> 1 : inverse >> 1;
+        }
+        for (int r = -15; r <= 15; r += 2) {
+            if (r * (1 << even) > 15 || r * (1 << even) < -15) {
+                continue;
+            }
+            const uint32_t residue = static_cast<uint32_t>(r < 0 ? odd - static_cast<uint32_t>(-r) : static_cast<uint32_t>(r));
+            const uint32_t n0 = static_cast<uint32_t>(residue * inverse % odd);
+            // the first n0 + i odd of at least 2^23
+            const uint32_t steps = n0 >= (1u << 23) ? 0u : ((1u << 23) - n0 + odd - 1) / odd;
+            for (uint64_t n = n0 + static_cast<uint64_t>(steps) * odd; n < (1u << 24); n += odd) {
+                if ((n >= d) != (k == 24)) {
+                    continue;
+                }
+                const float fn = static_cast<float>(n), fd = static_cast<float>(d);
+                const f32x2 num[1] = {pair(fn, -fn)}, neg_den[1] = {pair(-fd)};
+                f32x2 q[1];
+                quotient2<1>(num, neg_den, q);
+                float q0, q1;
+                unpair(q[0], q0, q1);
+                const float want = __fdiv_rn(fn, fd);
+                tested += 2;
+                if (q0 != want || q1 != -want) {
+                    selftest_note(out, 3, d);
+                }
+            }
+        }
+    }
+    atomicAdd(out + 8, tested);
+}
+
 }  // namespace w8a8
 
 extern "C" int w8a8_selftest_exp(uint64_t* result, void* stream)
@@ -331,6 +437,28 @@ extern "C" int w8a8_selftest_exp(uint64_t* result, void* stream)
         return W8A8_ERR_CUDA;
     }
     w8a8::exp_selftest_kernel<<<w8a8::sm_count() * 8, 256, 0, st>>>(reinterpret_cast<unsigned long long*>(result));
+    w8a8::note_launch();
+    return (cudaGetLastError() == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+}
+
+extern "C" int w8a8_selftest_pairs(uint64_t* result, void* stream)
+{
+    if (result == nullptr) {
+        return W8A8_ERR_INVALID;
+    }
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    unsigned long long* out = reinterpret_cast<unsigned long long*>(result);
+    if (cudaMemsetAsync(result, 0, 9 * 8, st) != cudaSuccess) {
+        return W8A8_ERR_CUDA;
+    }
+    for (int c = 0; c < 4; ++c) {
+        if (cudaMemsetAsync(result + 2 * c + 1, 0xff, 8, st) != cudaSuccess) {
+            return W8A8_ERR_CUDA;
+        }
+    }
+    w8a8::pair_exp_selftest_kernel<<<w8a8::sm_count() * 8, 256, 0, st>>>(out);
+    w8a8::note_launch();
+    w8a8::pair_quotient_selftest_kernel<<<(1 << 23) / 256, 256, 0, st>>>(out);
     w8a8::note_launch();
     return (cudaGetLastError() == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
 }

@@ -538,6 +538,18 @@ int w8a8_selftest_bounded_wait(int64_t limit_cycles, int32_t* error_words, void*
  * such pattern (all ones when there is none).  One launch of a few milliseconds. */
 int w8a8_selftest_exp(uint64_t* result, void* stream);
 
+/* Self-test (no reference counterpart) of the arithmetic on pairs of fp32 values that the SwiGLU epilogues, the SwiGLU
+ * quantiser and the router use, and of what the router's selection rests on.  result: nine uint64 in device memory;
+ * for check c, [2c] = number of failures (0 expected), [2c + 1] = the smallest failing pattern (all ones when there
+ * is none):
+ *   0  the negated exponential of -g against the scalar one, every fp32 g in [-80, 80]
+ *   1  the exponential against the scalar one, every fp32 x <= 0
+ *   2  the exponential of neighbouring floats never decreases, every fp32 but NaN
+ *   3  the quotient against the IEEE division, every 24-bit significand of the divisor with the numerators that bring
+ *      the quotient nearest to the middle of two floats (within 15 2^-24 of the divisor's unit); [8] = how many
+ * Two launches of a few tens of milliseconds. */
+int w8a8_selftest_pairs(uint64_t* result, void* stream);
+
 /* Measurement aid (no reference counterpart): one launch that reads `bytes` (a multiple of 16, 16-byte aligned) of
  * device memory once with streaming loads and does nothing else - what pulling that many bytes out of HBM costs in
  * a single launch, the yardstick bench.py prints beside the weight-streaming quant_matmul shapes.  sink: 4 bytes of
