@@ -483,11 +483,13 @@ void note_launch();  // counts one kernel launch of this library (w8a8_kernel_la
 // Programmatic dependent launch.  A kernel launched with launch_chained may start while the kernel before it on the
 // stream is still running: its launch, block setup and prologue then overlap that kernel's tail instead of following
 // it.  Every such kernel opens with after_previous(), which waits until the kernel before it has completed and its
-// writes are visible, and then lets the next kernel start; no global memory is touched before the wait, neither read nor
-// written.  The next kernel is let in after the wait, not ahead of it: with three kernels resident at once their blocks
-// share the SMs unevenly (back to back, the router on 16384 rows of 256 bf16 takes 9.0 us, 13.4 if it lets the next one
-// in ahead of the wait; the SwiGLU quantiser on 300 rows of 16384 int32 47 us, 67; kernels of 1.3 us take 0.1 us longer
-// this way).  Two rules keep the accesses behind the wait in the compiled code:
+// writes are visible; no global memory is touched before that, neither read nor written.  It also lets the next kernel
+// start.  A grid of at most one block per SM does so before its own wait, which takes 0.2 - 0.3 us off a short kernel; a
+// larger one after it: with three kernels resident at once their blocks share the SMs unevenly (back to back, the router
+// on 16384 rows of 256 bf16 takes 9.0 us, 13.4 if it lets the next one in ahead of the wait; the SwiGLU quantiser on 300
+// rows of 16384 int32 47 us, 67).  BY_GRID = false: after it in any case, for the SwiGLU quantiser, whose registers are
+// used up (16384 rows of 2816 int32 90 us, 99 with the grid asked for).  Two rules keep the accesses behind the wait in
+// the compiled code:
 //  - No load is a non-coherent one (ld.global.nc, __ldg): those are for memory that nothing writes during the life of
 //    the kernel, and the kernel before may write its outputs while this one already lives.  So the pointers that such a
 //    kernel only reads are not __restrict__ (the compiler makes those loads non-coherent, and free to move); the
@@ -502,11 +504,18 @@ void note_launch();  // counts one kernel launch of this library (w8a8_kernel_la
 // A dense layer of 16 rows 53.9 us (61.5 before), an expert layer of 2000 rows 160 (184) and of 64 rows 116 (129), a
 // grouped SwiGLU matmul of 512 rows 38 (42), regroup and combine of 8192 rows 56 (62).
 // ---------------------------------------------------------------------------
+template <bool BY_GRID = true>
 __device__ __forceinline__ int64_t after_previous()
 {
+    constexpr unsigned SMS = 148;
     int64_t zero;
+    if (BY_GRID && gridDim.x <= SMS) {
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
     asm volatile("griddepcontrol.wait;\n\tmov.u64 %0, 0;" : "=l"(zero)::"memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (!BY_GRID || gridDim.x > SMS) {
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
     return zero;
 }
 

@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(MAX_THREADS, MAX_THREADS <= DQSQ_PAIR_THREADS 
     constexpr int GN = GROUP * EL;
     constexpr size_t ELEM = (XT == DQSQ_X_I32) ? 4 : 2;
     __shared__ float s_red[2 * 32];
-    const int64_t zero = after_previous();
+    const int64_t zero = after_previous<false>();
     const int64_t first_row = blockIdx.x + zero;
     const int tid = threadIdx.x;
     const int threads = static_cast<int>(blockDim.x);
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(DQSQ_THREADS) dqsq_long_rows_kernel(const void
 {
     using C = DqsqChunk<XT>;
     __shared__ float s_red[2 * 32];
-    const int64_t zero = after_previous();
+    const int64_t zero = after_previous<false>();
     const size_t elem = (XT == DQSQ_X_I32) ? 4 : 2;
     const bool has_q = (quant_scale != nullptr);
     int parity = 0;

@@ -30,7 +30,7 @@ def _overlapping_kernels():
         code = _code(path)
         for m in re.finditer(r"__global__", code):
             start = code.index("\n{", m.end())
-            if "after_previous(" in code[start:code.index("\n}", start)]:
+            if re.search(r"after_previous(<false>)?\(", code[start:code.index("\n}", start)]):
                 signature = code[m.end():start]
                 yield re.search(r"(\w+_kernel)\s*\(", signature).group(1), signature
 
@@ -55,11 +55,13 @@ def test_no_spills_in_the_swiglu_quantiser(tmp_path):
     assert len(spills) == 3 and log.count("Compiling entry function") == 3 + 4 + 4 + 3
 
 
-def test_next_kernel_is_let_in_after_the_wait():
-    """Let in ahead of the wait, three kernels are resident at once and their blocks share the SMs unevenly."""
+def test_next_kernel_is_let_in_after_the_wait_of_a_large_grid():
+    """Let in ahead of the wait of a grid with more blocks than SMs, three kernels are resident at once and their blocks
+    share the SMs unevenly."""
     code = _code(os.path.join(CSRC, "common.cuh"))
-    order = re.findall(r"griddepcontrol\.(\w+)", code)
-    assert order == ["wait", "launch_dependents"]
+    steps = re.findall(r"if \((.* SMS)\)|griddepcontrol\.(\w+)", code)
+    assert [a or b for a, b in steps] == ["BY_GRID && gridDim.x <= SMS", "launch_dependents", "wait",
+                                          "!BY_GRID || gridDim.x > SMS", "launch_dependents"]
 
 
 def test_registers_of_the_unvectorised_combine(tmp_path):
