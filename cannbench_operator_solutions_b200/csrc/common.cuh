@@ -184,7 +184,7 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
     return r;
 }
 
-// e = -canonical_expf(-g) of N pairs, bit for bit, for |g| <= EXP2_MAX_ABS (the result is then a normal number, so
+// e = -canonical_expf(-g) of N pairs, bit for bit (w8a8_selftest_pairs), for |g| <= EXP2_MAX_ABS (the result is then a normal number, so
 // the power of two is one integer add to the exponent field).  A NaN half gives an arbitrary value: callers
 // multiply something by g that carries the NaN.  Every step is canonical_expf's with the sign of the argument or of
 // the result folded into the constants, which round-to-nearest does not see.  The pairs go through each step
@@ -239,7 +239,7 @@ __device__ __forceinline__ void neg_exp_neg2(const f32x2 (&g)[N], f32x2 (&e)[N])
     }
 }
 
-// e = canonical_expf(x) of N pairs, bit for bit, for x <= 0 (-inf included, NaN not): the power of two is applied as
+// e = canonical_expf(x) of N pairs, bit for bit (w8a8_selftest_pairs), for x <= 0 (-inf included, NaN not): the power of two is applied as
 // an exact integer add that leaves a normal number, 2^64 too large, and one multiplication that rounds the
 // subnormal results.  (A pair addition that uses e may absorb that multiplication; it is exact unless the result is
 // subnormal, where a sum of at least 2^-126 does not see the difference.)
@@ -309,7 +309,7 @@ __device__ __forceinline__ float approx_reciprocal(float x)
 // quotient by its exactly computed remainder (P. Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", 1990).  Before the last rounding the quotient is within 2^-46 of n / d; the quotients
 // that lie so close to the middle of two floats are, for each d, a handful of numerators, and all of them over all
-// 2^23 significands d (5.6e8 divisions) agree with the IEEE division.
+// 2^23 significands d agree with the IEEE division (w8a8_selftest_pairs).
 template <int N>
 __device__ __forceinline__ void quotient2(const f32x2 (&n)[N], const f32x2 (&nd)[N], f32x2 (&q)[N])
 {

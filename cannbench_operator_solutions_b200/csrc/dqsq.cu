@@ -226,7 +226,7 @@ __device__ __forceinline__ uint32_t dqsq_quant4(const float* o, float s, float i
 // Register-resident rows: H a multiple of the chunk length, at most blockDim.x * EL * CPT long.
 //
 // Bound: issue slots (44 warp instructions per 32 elements against 73 with a scalar exponential and the compiler's
-// division), then HBM.  int32 [16384, 4096] (302 MB): 64 us, was 83 - 85; fp16 [1531, 18432] (70 MB): 24 us, was 58
+// division), then HBM.  int32 [16384, 4096] (302 MB): 66 us, was 86; fp16 [1531, 18432] (70 MB): 24 us, was 58
 // with a fixed 256 threads per row (eight chunks per thread, 44 % of them past the row's end).
 template <int XT, int CPT, bool DIVIDE, int MAX_THREADS>
 __global__ void __launch_bounds__(MAX_THREADS, MAX_THREADS <= DQSQ_PAIR_THREADS ? 2 : 1)

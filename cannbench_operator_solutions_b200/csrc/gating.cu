@@ -156,13 +156,13 @@ __global__ void __launch_bounds__(GATING_WARPS * 32) gating_kernel(const void* x
 //
 // 16-bit rows are selected on one integer per element, the ordered bits of x above 8191 - column (the low 13 bits
 // of a bf16 or fp16 value widened to fp32 are zero).  That is the order of the exponentials too - the exponential
-// does not decrease, checked over all floats - except where two different x have the same exponential: such a row
+// does not decrease (w8a8_selftest_pairs, over all floats) - except where two different x have the same exponential: such a row
 // (seen from the selected exponentials, and for the last one from the exponential of the next smaller x) is selected
 // once more by gating_settle, which knows the two ways in which that happens to real rows.  What is left, and a
 // row whose maximum is not finite, goes to the whole warp.  fp32 rows are selected on the exponential above the column
 // in 64 bits, where the question does not arise.
 //
-// Bound: issue slots.  65536 x 256 bf16, k = 8: 23 us, was 55 with a warp per row (869 warp instructions per row); fp32: 45 us.
+// Bound: issue slots.  65536 x 256 bf16, k = 8: 24 us, was 55 with a warp per row (869 warp instructions per row); fp32: 45 us.
 // ---------------------------------------------------------------------------
 constexpr int GATING_TOP = 8;
 constexpr int GATING_TOP_THREADS = 64;

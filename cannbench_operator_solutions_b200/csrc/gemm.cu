@@ -637,10 +637,13 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
     // Rows per A load.  Pairs take whole tiles.  A single CTA's tile holds at most 128 rows of one group and often far
     // fewer - what a group leaves over, or a whole group of a small batch.  Where there are 256 MB of weights to stream
     // it loads its own rows in boxes of 32 or 16 instead of 128 rows that are mostly another group's, and multiplies
-    // zeros below them: 512 rows of 256 experts (7168 x 4096 and 2048 x 7168) 1.55 ms back to back, 1.80 before (the SM
-    // clock held near 0.8 GHz by the power cap), 1.44 and 1.53 from rest; 1500 rows of 32 experts of 2048 x 7168 bf16
-    // 161 us, 165.  Smaller problems do not pay for clearing the stages and the longer loop (512 rows of 32 experts of
-    // 2048 x 2048: 38.7 us, 37.6).
+    // what the stages hold below them - zeros, as long as no taller tile of the CTA has used them: 512 rows of 256
+    // experts (7168 x 4096 and 2048 x 7168) 1.55 ms back to back, 1.80 before (the SM clock held near 0.8 GHz by the
+    // power cap), 1.44 and 1.53 from rest; 1500 rows of 32 experts of 2048 x 7168 bf16 161 us, 165.  Smaller problems do
+    // not pay for clearing the stages and the longer loop (512 rows of 32 experts of 2048 x 2048: 38.7 us, 37.6).
+    // Calls that the cap does not bound gain little - 64 experts of 4096 x 4096, 4 - 64 rows each: 152.8 - 182.8 us,
+    // 153.7 - 184 with whole tiles - the same with boxes of 16 and of 32, and nothing from 96 rows per expert on, which
+    // is where the rule ends; at 12 rows per expert most tiles still fit into one box of 16.
     constexpr int64_t ELEM = (KIND == KIND_I8) ? 1 : 2;
     int box_rows = (shape == GEMM_SHAPE_HYBRID) ? 32 : (M <= 12 * E ? 16 : (M <= 96 * E ? 32 : GEMM_BLOCK_M));
     if (shape == 2 || E * p.N * p.K * ELEM < (int64_t(256) << 20)) {

@@ -3,17 +3,19 @@
 // One CTA per SM, 320 threads (576 with the SwiGLU epilogue's sixteen epilogue warps):
 //   warp 0      TMA producer: fills a ring of shared-memory stages (128-byte
 //               swizzle) with A and B tiles, one mbarrier per stage.
-//   warp 1      MMA issuer: one thread issues tcgen05.mma into one of two TMEM
-//               accumulator stages; tcgen05.commit releases the shared-memory
-//               stage and finally publishes the accumulator.
+//   warp 1      MMA issuer: the warp walks the loop and waits together, an elected
+//               lane issues tcgen05.mma into one of two TMEM accumulator stages;
+//               tcgen05.commit releases the shared-memory stage and finally
+//               publishes the accumulator.
 //   warps 2-9   epilogue: tcgen05.ld the accumulator (a warp may read the 32 TMEM
 //               lanes its index modulo 4 selects; two warps share each lane
 //               quarter and split the columns), apply the operator's dequant
 //               chain, store.  Double-buffered TMEM lets the epilogue of tile i
 //               overlap the main loop of tile i+1.  The SwiGLU epilogue (an
-//               exponential and an IEEE division per element) runs on warps
-//               2-17, four per lane quarter: with eight warps it took as long
-//               per tile as the main loop.
+//               exponential and a correctly rounded quotient per element, two
+//               elements at a time) runs on warps 2-17, four per lane quarter:
+//               with eight warps and scalar arithmetic it took as long per tile
+//               as the main loop.
 //
 // Two shapes of the same kernel (template parameter CG):
 //   CG = 1  one CTA per tile of 128 rows x BLOCK_N columns, 4 stages of
@@ -45,8 +47,8 @@
 
 namespace w8a8 {
 
-// producer warp, MMA warp and the epilogue warps (8, or 16 for the SwiGLU epilogue, whose per-element arithmetic -
-// exp and an IEEE division - otherwise keeps eight warps busy for as long as the MMA warp needs for the tile)
+// producer warp, MMA warp and the epilogue warps (8, or 16 for the SwiGLU epilogue, whose exponential and quotient per
+// element kept eight warps busy for as long as the MMA warp needs for the tile)
 __host__ __device__ constexpr int gemm_threads(int epi_warps) { return 64 + 32 * epi_warps; }
 constexpr int GEMM_EPI_PATCH_BYTES = 8 * 4096;  // shared by the epilogue warps: 4 KB each for 8, 2 KB each for 16
 constexpr int GEMM_BLOCK_M = 128;
@@ -769,8 +771,10 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
         tc::tmem_relinquish();
     }
     if constexpr (ROW_BOXES) {
-        // Rows that no load brings are zeros: their products are never stored, but multiplying what the shared memory
-        // happens to hold costs as much energy as multiplying operands, and the chip runs at its power limit.
+        // Rows that no load has brought yet are zeros: their products are never stored, but multiplying what the shared
+        // memory happens to hold costs as much energy as multiplying operands, and the chip runs at its power limit.
+        // They stay zeros while a CTA's tiles do not shrink, which is so where every group has a few rows; a tile with
+        // fewer boxes than one before it multiplies what that one left in its stages.
         for (int i = threadIdx.x; i < STAGES * KPS * (GEMM_A_BYTES / 16); i += gemm_threads(EPI_WARPS)) {
             const int block = i / (GEMM_A_BYTES / 16), word = i % (GEMM_A_BYTES / 16);
             reinterpret_cast<uint4*>(smem + (block / KPS) * STAGE_BYTES + (block % KPS) * KB_BYTES)[word] =

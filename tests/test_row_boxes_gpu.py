@@ -1,5 +1,5 @@
-"""Grouped matmuls with enough weights that single-CTA tiles load their own rows only (boxes of 16 or 32 rows, zeros
-below): group sizes around the boxes and the tile, against the CTA-pair form of the same operator, which loads whole
+"""Grouped matmuls with enough weights that single-CTA tiles load their own rows only (boxes of 16 or 32 rows; what the
+stages hold below is multiplied and not stored): group sizes around the boxes and the tile, against the CTA-pair form of the same operator, which loads whole
 tiles."""
 import pytest
 import torch
