@@ -487,9 +487,10 @@ void note_launch();  // counts one kernel launch of this library (w8a8_kernel_la
 // start.  A grid of at most one block per SM does so before its own wait, which takes 0.2 - 0.3 us off a short kernel; a
 // larger one after it: with three kernels resident at once their blocks share the SMs unevenly (back to back, the router
 // on 16384 rows of 256 bf16 takes 9.0 us, 13.4 if it lets the next one in ahead of the wait; the SwiGLU quantiser on 300
-// rows of 16384 int32 47 us, 67).  BY_GRID = false: after it in any case, for the SwiGLU quantiser, whose registers are
-// used up (16384 rows of 2816 int32 90 us, 99 with the grid asked for).  Two rules keep the accesses behind the wait in
-// the compiled code:
+// rows of 16384 int32 47 us, 67).  BY_GRID = false: after it in any case - the SwiGLU quantiser, whose registers are used
+// up (16384 rows of 2816 int32 90 us, 99 with the grid asked for), and the sums of gathered rows, whose few blocks run
+// long (64 sums of eight fp32 rows of 4095 with bias 11.2 us, 13.8).
+// Two rules keep the accesses behind the wait in the compiled code:
 //  - No load is a non-coherent one (ld.global.nc, __ldg): those are for memory that nothing writes during the life of
 //    the kernel, and the kernel before may write its outputs while this one already lives.  So the pointers that such a
 //    kernel only reads are not __restrict__ (the compiler makes those loads non-coherent, and free to move); the

@@ -802,7 +802,7 @@ __global__ void __launch_bounds__(256) mfr_kernel(const void* rows, const IdxT* 
                                                   int64_t R, int64_t H, int K, int64_t E, int64_t num_dst,
                                                   int col_mode, int scale_dt)
 {
-    const int64_t zero = after_previous();
+    const int64_t zero = after_previous<false>();
     using C = RowChunk<DT>;
     constexpr int EL = C::EL;
     constexpr int BUFS = VEC ? 2 : 1;
