@@ -430,15 +430,9 @@ __global__ void __launch_bounds__(256) gmsq_requant_kernel(const float* act,
 static inline size_t align_up_sz(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // ---------------------------------------------------------------------------
-// fp32 operands on the bf16 tensor path: v = hi + mid + lo with three bf16 pieces (8 + 8 + 8 significand bits,
-// each remainder exact in fp32), and x.w is the sum of the six piece products whose orders add up to at most two
-// (hi.hi, hi.mid, mid.hi, hi.lo, mid.mid, lo.hi; what is dropped is below 2^-24 of |x||w|).  The pieces are laid
-// out along K, small terms first, so that ONE bf16 matmul over 6K accumulates all six in fp32:
-//   x' [M, 6K]  = [ lo | mid | mid | hi | hi  | hi ]
-//   w' [.., 6K] = [ hi | mid | hi  | lo | mid | hi ]   (K-blocks of the weight's K dimension, either layout)
+// fp32 operands on the bf16 tensor path (gemm_kernel.cuh): each operand is split once into SPLIT_PIECES arrays of bf16
+// pieces.
 // ---------------------------------------------------------------------------
-constexpr int SPLIT_TERMS = 6;
-
 __device__ __forceinline__ void split3(float v, __nv_bfloat16 (&piece)[3])
 {
     piece[0] = __float2bfloat16_rn(v);
@@ -472,29 +466,28 @@ __device__ __forceinline__ void split8(const float* src, uint4 (&word)[3])
     }
 }
 
-// src: `rows` blocks of `len` fp32 values (a row of K, or an expert's K x N weight) -> dst: the same blocks of
-// SPLIT_TERMS * len bf16 values, sub-block b holding piece pick[b] (0 hi, 1 mid, 2 lo) of all of them.  `len` is a
-// multiple of 8 and both ends are 16-byte aligned (K of the operator is a multiple of 8).
-// Bound: HBM (16 bytes per value).  8 experts of 4096 x 4096 with 1000 rows, matmul included: 805 us, 944 with a value
-// and six 2-byte stores per thread.
+// src: `blocks` blocks of `len` fp32 values (a row of x, or an expert's weight) -> dst: per block, its hi, its mid
+// and its lo pieces, `len` bf16 values each.  `len` is a multiple of 8 and both ends are 16-byte aligned (K of the
+// operator is a multiple of 8).
+// Bound: HBM (10 bytes per value).  With every piece stored once and found by the matmul's producer through its map,
+// instead of six copies laid out along K (16 bytes per value, twice the workspace): 8 experts of 4096 x 4096 with 1000
+// rows, matmul included, 629 us (769 before); 32 of 1024 x 2048 with 333 rows 241 (324); 32 of 4096 x 7168 with 2000
+// rows 3.47 ms (4.45); 16000 rows, bound by the six products, 2.62 (2.90).
 __global__ void __launch_bounds__(256) split_blocks_kernel(const float* src, __nv_bfloat16* __restrict__ dst,
-                                                           int64_t rows, int64_t len, int is_weight)
+                                                           int64_t blocks, int64_t len)
 {
     const int64_t zero = after_previous();
-    const int64_t n8 = len / 8, total = rows * n8;
+    const int64_t n8 = len / 8, total = blocks * n8;
     const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t i = zero + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += step) {
         const int64_t r = i / n8, c = i - r * n8;
-        uint4 w[3];
+        uint4 w[SPLIT_PIECES];
         split8(src + i * 8, w);
-        uint4* out = reinterpret_cast<uint4*>(dst + r * (SPLIT_TERMS * len)) + c;
-        // x: lo mid mid hi hi hi; w: hi mid hi lo mid hi
-        out[0 * n8] = is_weight ? w[0] : w[2];
-        out[1 * n8] = w[1];
-        out[2 * n8] = is_weight ? w[0] : w[1];
-        out[3 * n8] = is_weight ? w[2] : w[0];
-        out[4 * n8] = is_weight ? w[1] : w[0];
-        out[5 * n8] = w[0];
+        uint4* out = reinterpret_cast<uint4*>(dst + r * (SPLIT_PIECES * len)) + c;
+#pragma unroll
+        for (int t = 0; t < SPLIT_PIECES; ++t) {
+            out[t * n8] = w[t];
+        }
     }
 }
 
@@ -645,14 +638,17 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
     // 153.7 - 184 with whole tiles - the same with boxes of 16 and of 32, and nothing from 96 rows per expert on, which
     // is where the rule ends; at 12 rows per expert most tiles still fit into one box of 16.
     constexpr int64_t ELEM = (KIND == KIND_I8) ? 1 : 2;
+    const bool split = p.k_blocks_per_term != 0;
+    const int64_t a_cols = split ? SPLIT_PIECES * p.K : p.K;
+    const int64_t terms = split ? SPLIT_TERMS : 1;
     int box_rows = (shape == GEMM_SHAPE_HYBRID) ? 32 : (M <= 12 * E ? 16 : (M <= 96 * E ? 32 : GEMM_BLOCK_M));
-    if (shape == 2 || E * p.N * p.K * ELEM < (int64_t(256) << 20)) {
+    if (shape == 2 || E * p.N * p.K * terms * ELEM < (int64_t(256) << 20)) {
         box_rows = GEMM_BLOCK_M;
     }
     const bool row_boxes = box_rows < GEMM_BLOCK_M;
     CUtensorMap ta;
     p.a_box_rows = (shape == 1) ? box_rows : GEMM_BLOCK_M;
-    if (!make_map_a(&ta, a, M, p.K, KIND, p.a_box_rows)) {
+    if (!make_map_a(&ta, a, M, a_cols, KIND, p.a_box_rows)) {
         return W8A8_ERR_CUDA;
     }
     // `clear` (the SwiGLU form's row maxima and tile counters) must be zero before the first matmul launch: the
@@ -690,7 +686,7 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
     const int64_t most = g.tail_max_tiles * p.n_tiles;
     if (row_boxes) {
         p.a_box_rows = box_rows;
-        if (!make_map_a(&ta, a, M, p.K, KIND, box_rows)) {
+        if (!make_map_a(&ta, a, M, a_cols, KIND, box_rows)) {
             return W8A8_ERR_CUDA;
         }
         e = dispatch_row_boxes<KIND, EPI>(b_mn, ta, tb, p, most, st);
@@ -973,8 +969,8 @@ extern "C" size_t w8a8_grouped_matmul_f32_workspace_size(int64_t M, int64_t N, i
         return 0;
     }
     const size_t base = carve_workspace(nullptr, M, E, 0).total;
-    const size_t xs = align_up_sz(static_cast<size_t>(M) * SPLIT_TERMS * K * 2, 256);
-    const size_t ws = align_up_sz(static_cast<size_t>(E) * SPLIT_TERMS * K * N * 2, 256);
+    const size_t xs = align_up_sz(static_cast<size_t>(M) * SPLIT_PIECES * K * 2, 256);
+    const size_t ws = align_up_sz(static_cast<size_t>(E) * SPLIT_PIECES * K * N * 2, 256);
     return base + xs + ws;
 }
 
@@ -1048,30 +1044,26 @@ static int grouped_matmul_impl(const void* x, const void* w, const void* bias, v
     }
     const bool b_mn = (w_layout == W8A8_W_KN);
     if (f32) {
-        // split both operands into bf16 pieces laid out along K (6K in all), then run the bf16 path on them
         if (SPLIT_TERMS * K >= (int64_t(1) << 31)) {
             return W8A8_ERR_UNSUPPORTED;
         }
         uint8_t* base = static_cast<uint8_t*>(workspace) + g.total;
         __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(base);
         __nv_bfloat16* wsplit =
-            reinterpret_cast<__nv_bfloat16*>(base + align_up_sz(static_cast<size_t>(M) * SPLIT_TERMS * K * 2, 256));
+            reinterpret_cast<__nv_bfloat16*>(base + align_up_sz(static_cast<size_t>(M) * SPLIT_PIECES * K * 2, 256));
         const unsigned grid = static_cast<unsigned>(sm_count()) * 8;
-        // a weight [E, K, N] is E blocks of K * N values, one [E, N, K] is E * N of K
-        cudaError_t e = launch_chained(split_blocks_kernel, grid, 256, 0, st, static_cast<const float*>(x), xs, M, K, 0);
+        cudaError_t e = launch_chained(split_blocks_kernel, grid, 256, 0, st, static_cast<const float*>(x), xs, M, K);
         if (e == cudaSuccess) {
-            e = launch_chained(split_blocks_kernel, grid, 256, 0, st, static_cast<const float*>(w), wsplit, b_mn ? E : E * N,
-                               b_mn ? K * N : K, 1);
+            e = launch_chained(split_blocks_kernel, grid, 256, 0, st, static_cast<const float*>(w), wsplit, E, K * N);
         }
         if (e != cudaSuccess) {
             return launch_status(e);
         }
         x = xs;
         w = wsplit;
-        K = SPLIT_TERMS * K;
     }
     CUtensorMap tb;
-    if (!make_map_b(&tb, w, E, N, K, kind, b_mn)) {
+    if (!make_map_b(&tb, w, f32 ? E * SPLIT_PIECES : E, N, K, kind, b_mn)) {
         return W8A8_ERR_CUDA;
     }
     GemmParams p{};
@@ -1080,6 +1072,10 @@ static int grouped_matmul_impl(const void* x, const void* w, const void* bias, v
     p.K = K;
     const int block_k = GEMM_KBYTES / elem;
     p.num_k_blocks = static_cast<int32_t>((K + block_k - 1) / block_k);
+    if (f32) {
+        p.k_blocks_per_term = p.num_k_blocks;
+        p.num_k_blocks *= SPLIT_TERMS;
+    }
     p.scale = w_scale;
     p.row_scale = x_scale;
     p.bias = bias;

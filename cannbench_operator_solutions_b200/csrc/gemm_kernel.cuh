@@ -74,6 +74,17 @@ __host__ __device__ constexpr int gemm_kblocks_per_stage(int cg, int block_n)
 #endif
 }
 
+// fp32 operands on the bf16 tensor path: v = hi + mid + lo with three bf16 pieces (8 + 8 + 8 significand bits, each
+// remainder exact in fp32), and x.w is the sum of the six piece products whose orders add up to at most two (hi.hi,
+// hi.mid, mid.hi, hi.lo, mid.mid, lo.hi; what is dropped is below 2^-24 of |x||w|).  The products are accumulated one
+// after the other, hi.hi last, as one matmul of SPLIT_TERMS times the K blocks; two bits per term name the piece (0 hi,
+// 1 mid, 2 lo).  Neighbouring terms share a piece and every other one runs through K backwards, so that a term starts
+// on the K blocks that the one before it has left in L2.
+constexpr int SPLIT_PIECES = 3;
+constexpr int SPLIT_TERMS = 6;
+constexpr uint32_t SPLIT_PICK_A = 0x016;  // lo mid mid hi  hi  hi
+constexpr uint32_t SPLIT_PICK_B = 0x250;  // hi hi  mid mid lo  hi
+
 enum GemmKind { KIND_I8 = 0, KIND_F16 = 1, KIND_BF16 = 2 };
 enum GemmEpi { EPI_RAW = 0, EPI_QMM = 1, EPI_GMSQ = 2, EPI_GMM = 3 };
 
@@ -114,6 +125,9 @@ struct GemmParams {
     int64_t bias_batch_stride;
     const uint64_t* out_row_ptrs;  // GMM: when set, row r is stored at this address instead of out + r*N
     int32_t a_box_rows;  // rows of one A load: 128, or fewer (a multiple of 8) on single CTAs
+    // fp32 operands split into bf16 pieces (SPLIT_PIECES of each): K blocks of one piece product, num_k_blocks being
+    // SPLIT_TERMS times that; 0: operands as they are
+    int32_t k_blocks_per_term;
     float* act;       // GMSQ: fp32 activations [M, N/2]
     uint32_t* amax;   // GMSQ: per-row max|act| bit patterns
     // GMSQ with the requantisation fused in: the CTA that finishes the last column tile of its rows quantises them
@@ -701,6 +715,7 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
     constexpr int ELEM = (KIND == KIND_I8) ? 1 : 2;
     constexpr int BLOCK_K = GEMM_KBYTES / ELEM;    // elements of K per stage
     constexpr int UMMA_K = 32 / ELEM;              // elements of K per instruction
+    constexpr bool SPLIT_OPERANDS = (KIND == KIND_BF16 && EPI == EPI_GMM);  // may run on pieces of fp32 operands
     constexpr int CTA_N = BLOCK_N / CG;            // B columns this CTA loads
     constexpr int NBOX = CTA_N * ELEM / 128;       // MN-major: 128-byte-wide column blocks this CTA loads
     constexpr int B_BYTES = CTA_N * GEMM_KBYTES;
@@ -866,7 +881,23 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
                 const int a_loads = ROW_BOXES ? (tl.m_rows + p.a_box_rows - 1) / p.a_box_rows : 1;
                 const uint32_t a_box_bytes = static_cast<uint32_t>(p.a_box_rows) * GEMM_KBYTES;
                 const uint32_t stage_bytes = a_loads * a_box_bytes + B_BYTES;  // of one K block, per CTA
+                [[maybe_unused]] int term = 0, term_kb = 0;  // SPLIT_OPERANDS: the next K block's product, and place in it
                 for (int kb0 = kb_first; kb0 < kb_last; kb0 += KPS) {
+                    [[maybe_unused]] int piece_kb[KPS], a_piece[KPS], b_piece[KPS];
+                    if constexpr (SPLIT_OPERANDS) {
+                        // (counted along, and A on a 2D map: a division, or a third coordinate, per K block held the
+                        // producer up by 0.05 - 0.1 us)
+#pragma unroll
+                        for (int sub = 0; sub < KPS; ++sub) {
+                            piece_kb[sub] = (term & 1) ? p.k_blocks_per_term - 1 - term_kb : term_kb;
+                            a_piece[sub] = static_cast<int>((SPLIT_PICK_A >> (2 * term)) & 3u);
+                            b_piece[sub] = static_cast<int>((SPLIT_PICK_B >> (2 * term)) & 3u);
+                            if (++term_kb == p.k_blocks_per_term) {
+                                term_kb = 0;
+                                ++term;
+                            }
+                        }
+                    }
                     if (!__all_sync(FULL_MASK, tc::mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag))) {
                         ok = false;
                         break;
@@ -887,17 +918,26 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
                             if (sub >= n_sub) {
                                 break;
                             }
-                            const int kb = kb0 + sub;
+                            int kb = kb0 + sub;
+                            int b_group = tl.group;
                             const uint32_t a_dst = smem_base + stage * STAGE_BYTES + sub * KB_BYTES;
                             const uint32_t b_dst = a_dst + GEMM_A_BYTES;
+                            int a_x = kb * BLOCK_K;
+                            if (SPLIT_OPERANDS && p.k_blocks_per_term != 0) {
+                                kb = piece_kb[sub];
+                                // a piece's last K block may run into the next piece of the row: those columns meet
+                                // zeros, which is what B's map gives past K
+                                a_x = a_piece[sub] * static_cast<int>(p.K) + kb * BLOCK_K;
+                                b_group = b_group * SPLIT_PIECES + b_piece[sub];
+                            }
                             if constexpr (CG == 2) {
-                                tc::tma_load_2d_pair(a_dst, &tm_a, fb, kb * BLOCK_K, tl.a_row0);
+                                tc::tma_load_2d_pair(a_dst, &tm_a, fb, a_x, tl.a_row0);
                             } else {
-                                tc::tma_load_2d(a_dst, &tm_a, fb, kb * BLOCK_K, tl.a_row0);
+                                tc::tma_load_2d(a_dst, &tm_a, fb, a_x, tl.a_row0);
                                 if constexpr (ROW_BOXES) {
 #pragma unroll 1
                                     for (int i = 1; i < a_loads; ++i) {
-                                        tc::tma_load_2d(a_dst + i * a_box_bytes, &tm_a, fb, kb * BLOCK_K,
+                                        tc::tma_load_2d(a_dst + i * a_box_bytes, &tm_a, fb, a_x,
                                                         tl.a_row0 + i * p.a_box_rows);
                                     }
                                 }
@@ -910,9 +950,9 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
                                 for (int i = 0; i < NBOX; ++i) {
                                     const int32_t col = b_block_origin(tl.nt, i, BOX_COLS);
                                     if constexpr (CG == 2) {
-                                        tc::tma_load_3d_pair(b_dst + i * BOX_BYTES, &tm_b, fb, col, kb * BLOCK_K, tl.group);
+                                        tc::tma_load_3d_pair(b_dst + i * BOX_BYTES, &tm_b, fb, col, kb * BLOCK_K, b_group);
                                     } else {
-                                        tc::tma_load_3d(b_dst + i * BOX_BYTES, &tm_b, fb, col, kb * BLOCK_K, tl.group);
+                                        tc::tma_load_3d(b_dst + i * BOX_BYTES, &tm_b, fb, col, kb * BLOCK_K, b_group);
                                     }
                                 }
                             } else {
@@ -923,10 +963,10 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
                                     const int32_t n_row = b_block_origin(tl.nt, i, 128);
                                     if constexpr (CG == 2) {
                                         tc::tma_load_3d_pair(b_dst + i * 128 * GEMM_KBYTES, &tm_b, fb, kb * BLOCK_K, n_row,
-                                                             tl.group);
+                                                             b_group);
                                     } else {
                                         tc::tma_load_3d(b_dst + i * 128 * GEMM_KBYTES, &tm_b, fb, kb * BLOCK_K, n_row,
-                                                        tl.group);
+                                                        b_group);
                                     }
                                 }
                             }
