@@ -791,6 +791,7 @@ static int quant_matmul_impl(const int8_t* x1, const int8_t* x2, const void* sca
     p.flags = flags;
     p.out_dtype = out_dtype;
     p.bias_batch_stride = bias_batch_stride;
+    p.prefetch_k_blocks = GEMM_PREFETCH_K_BLOCKS;
     p.error = pipeline_error_word();  // null (no report) only if the symbol lookup failed
     const int64_t tiles128 = batch * p.m_tiles_per_batch * ((N + 127) / 128);
     const bool own_choice = g_shape_override.load(std::memory_order_relaxed) == 0;

@@ -53,6 +53,7 @@ __host__ __device__ constexpr int gemm_threads(int epi_warps) { return 64 + 32 *
 constexpr int GEMM_EPI_PATCH_BYTES = 8 * 4096;  // shared by the epilogue warps: 4 KB each for 8, 2 KB each for 16
 constexpr int GEMM_BLOCK_M = 128;
 constexpr int GEMM_KBYTES = 128;  // bytes of K per stage row (one swizzle atom)
+constexpr int GEMM_PREFETCH_K_BLOCKS = 4;  // of a dense problem's weights, asked into L2 ahead of the kernel's start
 constexpr int GEMM_A_BYTES = GEMM_BLOCK_M * GEMM_KBYTES;
 
 // pipeline depth: as many 1 KB-aligned stages as fit beside the barriers
@@ -128,6 +129,8 @@ struct GemmParams {
     // fp32 operands split into bf16 pieces (SPLIT_PIECES of each): K blocks of one piece product, num_k_blocks being
     // SPLIT_TERMS times that; 0: operands as they are
     int32_t k_blocks_per_term;
+    // dense: K blocks of a CTA's first tile of B that it asks L2 for while the kernel before it may still be running
+    int32_t prefetch_k_blocks;
     float* act;       // GMSQ: fp32 activations [M, N/2]
     uint32_t* amax;   // GMSQ: per-row max|act| bit patterns
     // GMSQ with the requantisation fused in: the CTA that finishes the last column tile of its rows quantises them
@@ -386,6 +389,63 @@ __device__ __forceinline__ void swiglu8(const uint32_t* g, const uint32_t* u, fl
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         unpair(mul2(q[j], r[j]), a[2 * j], a[2 * j + 1]);
+    }
+}
+
+// Brings what the epilogue of a tile reads besides the accumulator into L1 while the accumulator is being computed (with
+// the loads behind the wait for it, 128 x 1024 x 1024 with its quantisation takes 7.27 us, 7.13 so; 300 x 4096 x 4096
+// 15.49, 15.36).
+__device__ __forceinline__ void touch(const void* base, int64_t byte)
+{
+    uint32_t v;
+    asm volatile("ld.global.ca.b32 %0, [%1];" : "=r"(v) : "l"(static_cast<const uint8_t*>(base) + byte));
+}
+
+template <int BLOCK_N, int KIND, int EPI>
+__device__ __forceinline__ void touch_epilogue_operands(const GemmParams& p, const TileInfo& tl, int row_in_tile)
+{
+    const int lane = row_in_tile & 31;
+    const bool row_ok = row_in_tile < tl.m_rows;
+    const int64_t row = static_cast<int64_t>(tl.a_row0) + row_in_tile;
+    if constexpr (EPI == EPI_GMSQ) {
+        // lanes 0-15: 128 gate scales, 16-31: 128 up scales, a 32-byte sector each
+        const int64_t H = p.N / 2, col = static_cast<int64_t>(tl.nt) * 128 + (lane & 15) * 8;
+        if (col < H) {
+            touch(p.scale, ((static_cast<int64_t>(tl.group) * p.N) + (lane < 16 ? col : H + col)) * 4);
+        }
+        if (row_ok) {
+            touch(p.row_scale, row * 4);
+        }
+    } else if constexpr (EPI == EPI_QMM || EPI == EPI_GMM) {
+        const int64_t col = static_cast<int64_t>(tl.nt) * BLOCK_N + lane * (BLOCK_N / 32);
+        const int64_t at = (EPI == EPI_GMM ? static_cast<int64_t>(tl.group) * p.N : 0) + col;
+        const bool col_ok = col < p.N;
+        if constexpr (EPI == EPI_QMM) {
+            const int64_t f = p.flags;
+            if (col_ok && (f & W8A8_QM_SCALE_PERCHAN)) {
+                touch(p.scale, at * ((f & W8A8_QM_SCALE_BF16) ? 2 : 4) & ~int64_t(3));
+            }
+            if (row_ok && (f & W8A8_QM_HAS_PT)) {
+                touch(p.row_scale, (tl.group == 0 ? row : row - static_cast<int64_t>(tl.group) * p.M) * 4);
+            }
+            const int kind = static_cast<int>((f & W8A8_QM_BIAS_MASK) >> W8A8_QM_BIAS_SHIFT);
+            if (col_ok && kind != W8A8_QM_BIAS_NONE && (f & W8A8_QM_BIAS_PERCHAN)) {
+                const int size = (kind == W8A8_QM_BIAS_F16 || kind == W8A8_QM_BIAS_BF16) ? 2 : 4;
+                touch(p.bias, (tl.group * p.bias_batch_stride + col) * size & ~int64_t(3));
+            }
+        } else {
+            if constexpr (KIND == KIND_I8) {
+                if (col_ok) {
+                    touch(p.scale, at * 4);
+                }
+                if (row_ok) {
+                    touch(p.row_scale, row * 4);
+                }
+            }
+            if (col_ok && (p.flags & 4)) {
+                touch(p.bias, at * ((p.flags & 3) == W8A8_DT_F32 ? 4 : 2) & ~int64_t(3));
+            }
+        }
     }
 }
 
@@ -779,6 +839,36 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
         tc::prefetch_tensormap(&tm_a);
         tc::prefetch_tensormap(&tm_b);
     }
+    // Dense problems: the first K blocks of this CTA's first column tile are asked into L2 already here, beside the kernel
+    // before (usually a short one that leaves HBM idle).  Nothing is read: what that kernel still writes is what the loads
+    // behind the wait see.  An epilogue warp does it, the producer has its own start to prepare (with the producer, calls
+    // whose weights are in L2 anyway lose 0.15 us).  Dense layer of 100 rows of 4096 x 3008 30.0 us (30.7 without), of 40
+    // rows of 4096 x 8192 36.5 (37.7), of 16 rows of 7168 x 9216 49.2 (50.5); 30 rows x 4096 x 12288 15.2 (15.9); 2 rows x
+    // 4096 x 4096 out of L2 7.9 (7.8).  Two K blocks gain half of it, eight or more less than four.
+    if (warp == 2 && p.prefetch_k_blocks != 0 && tc::elect_one()) {
+        const int64_t first = blockIdx.x / (SPLITK ? p.split : CG);
+        const int32_t m_tiles = p.batch * p.m_tiles_per_batch;
+        const int32_t nt = static_cast<int32_t>(first / m_tiles);
+        const int32_t group = static_cast<int32_t>(first % m_tiles) / p.m_tiles_per_batch;
+        // (one CTA per column tile of a batch asks for it)
+        const bool mine = (first % m_tiles) % p.m_tiles_per_batch == 0;
+        const int last = mine ? min(kb_last, kb_first + p.prefetch_k_blocks) : kb_first;
+        for (int kb = kb_first; kb < last; ++kb) {
+            if constexpr (B_MN) {
+#pragma unroll
+                for (int i = 0; i < NBOX; ++i) {
+                    tc::tma_prefetch_l2_3d(&tm_b, nt * BLOCK_N + (static_cast<int>(cta_rank) * NBOX + i) * (128 / ELEM),
+                                           kb * BLOCK_K, group);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < CTA_N / 128; ++i) {
+                    tc::tma_prefetch_l2_3d(&tm_b, kb * BLOCK_K,
+                                           nt * BLOCK_N + (static_cast<int>(cta_rank) * (CTA_N / 128) + i) * 128, group);
+                }
+            }
+        }
+    }
     if (warp == 1) {
         // each CTA allocates its own tensor memory; a pair asks for all 512 columns in both CTAs, so the
         // accumulator has the same column address in both, as the paired MMA requires
@@ -1125,6 +1215,7 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
         };
         for (int64_t t = worker; ok && t < total_tiles; t += num_workers, ++it) {
             const TileInfo tl = decode(t);
+            touch_epilogue_operands<BLOCK_N, KIND, EPI>(p, tl, row_in_tile);
             const int acc = static_cast<int>(it & 1);
             const uint32_t acc_phase = static_cast<uint32_t>((it >> 1) & 1);
             if (!tc::mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) {
