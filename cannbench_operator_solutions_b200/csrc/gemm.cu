@@ -4,6 +4,7 @@
 // grouped_matmul_swiglu_quant and grouped_matmul.
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 
@@ -87,7 +88,8 @@ template <int CG, int BLOCK_N>
 constexpr size_t gemm_smem_bytes()
 {
     return static_cast<size_t>(gemm_stages(CG, BLOCK_N)) * (GEMM_A_BYTES + (BLOCK_N / CG) * GEMM_KBYTES) +
-           1024 /*alignment slack*/ + 512 /*barriers, tmem slot, abort flag*/ + GEMM_EPI_PATCH_BYTES /*store patches*/;
+           1024 /*alignment slack*/ + 512 /*barriers, tmem slot, abort flag*/ + GEMM_EPI_PATCH_BYTES /*store patches*/ +
+           (GROUPS_IN_CTA + 1) * sizeof(int32_t) /*first tiles of the groups*/;
 }
 
 // number of workers (CTAs, or CTA pairs) a persistent launch uses
@@ -103,7 +105,7 @@ static int64_t worker_count(int64_t max_tiles)
 
 template <int CG, int BLOCK_N, int KIND, int EPI, bool B_MN, int EPI_WARPS = 8, bool SPLITK = false, bool ROW_BOXES = false>
 static cudaError_t launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int64_t max_tiles,
-                               cudaStream_t st)
+                               cudaStream_t st, const GroupListOf<EPI>& groups = {})
 {
     auto kern = gemm_tc_kernel<CG, BLOCK_N, KIND, EPI, B_MN, EPI_WARPS, SPLITK, ROW_BOXES>;
     constexpr size_t smem = gemm_smem_bytes<CG, BLOCK_N>();
@@ -131,53 +133,54 @@ static cudaError_t launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, con
     cfg.attrs = attr;
     cfg.numAttrs = cluster > 1 ? 2 : 1;
     note_launch();
-    return cudaLaunchKernelEx(&cfg, kern, ta, tb, p);
+    return cudaLaunchKernelEx(&cfg, kern, ta, tb, p, groups);
 }
 
 static std::atomic<int> g_gmsq_epilogue_warps{16};
 
 template <int KIND, int EPI>
 static cudaError_t dispatch_gemm(int cta_group, int block_n, bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb,
-                                 const GemmParams& p, int64_t max_tiles, cudaStream_t st)
+                                 const GemmParams& p, int64_t max_tiles, cudaStream_t st,
+                                 const GroupListOf<EPI>& groups = {})
 {
     if constexpr (EPI == EPI_GMSQ) {
         // the SwiGLU epilogue with sixteen epilogue warps (see w8a8_set_gmsq_epilogue_warps)
         if (g_gmsq_epilogue_warps.load(std::memory_order_relaxed) == 16) {
             if (cta_group == 2) {
-                return b_mn ? launch_gemm<2, 256, KIND, EPI, true, 16>(ta, tb, p, max_tiles, st)
-                            : launch_gemm<2, 256, KIND, EPI, false, 16>(ta, tb, p, max_tiles, st);
+                return b_mn ? launch_gemm<2, 256, KIND, EPI, true, 16>(ta, tb, p, max_tiles, st, groups)
+                            : launch_gemm<2, 256, KIND, EPI, false, 16>(ta, tb, p, max_tiles, st, groups);
             }
-            return b_mn ? launch_gemm<1, 256, KIND, EPI, true, 16>(ta, tb, p, max_tiles, st)
-                        : launch_gemm<1, 256, KIND, EPI, false, 16>(ta, tb, p, max_tiles, st);
+            return b_mn ? launch_gemm<1, 256, KIND, EPI, true, 16>(ta, tb, p, max_tiles, st, groups)
+                        : launch_gemm<1, 256, KIND, EPI, false, 16>(ta, tb, p, max_tiles, st, groups);
         }
     }
     if (cta_group == 2) {
-        return b_mn ? launch_gemm<2, 256, KIND, EPI, true>(ta, tb, p, max_tiles, st)
-                    : launch_gemm<2, 256, KIND, EPI, false>(ta, tb, p, max_tiles, st);
+        return b_mn ? launch_gemm<2, 256, KIND, EPI, true>(ta, tb, p, max_tiles, st, groups)
+                    : launch_gemm<2, 256, KIND, EPI, false>(ta, tb, p, max_tiles, st, groups);
     }
     if constexpr (EPI != EPI_GMSQ) {
         if (block_n == 128) {
-            return b_mn ? launch_gemm<1, 128, KIND, EPI, true>(ta, tb, p, max_tiles, st)
-                        : launch_gemm<1, 128, KIND, EPI, false>(ta, tb, p, max_tiles, st);
+            return b_mn ? launch_gemm<1, 128, KIND, EPI, true>(ta, tb, p, max_tiles, st, groups)
+                        : launch_gemm<1, 128, KIND, EPI, false>(ta, tb, p, max_tiles, st, groups);
         }
     }
-    return b_mn ? launch_gemm<1, 256, KIND, EPI, true>(ta, tb, p, max_tiles, st)
-                : launch_gemm<1, 256, KIND, EPI, false>(ta, tb, p, max_tiles, st);
+    return b_mn ? launch_gemm<1, 256, KIND, EPI, true>(ta, tb, p, max_tiles, st, groups)
+                : launch_gemm<1, 256, KIND, EPI, false>(ta, tb, p, max_tiles, st, groups);
 }
 
 // Single-CTA tiles of a grouped problem that load their own rows only (see run_grouped).
 template <int KIND, int EPI>
 static cudaError_t dispatch_row_boxes(bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
-                                      int64_t max_tiles, cudaStream_t st)
+                                      int64_t max_tiles, cudaStream_t st, const GroupListOf<EPI>& groups)
 {
     if constexpr (EPI == EPI_GMSQ) {
         if (g_gmsq_epilogue_warps.load(std::memory_order_relaxed) == 16) {
-            return b_mn ? launch_gemm<1, 256, KIND, EPI, true, 16, false, true>(ta, tb, p, max_tiles, st)
-                        : launch_gemm<1, 256, KIND, EPI, false, 16, false, true>(ta, tb, p, max_tiles, st);
+            return b_mn ? launch_gemm<1, 256, KIND, EPI, true, 16, false, true>(ta, tb, p, max_tiles, st, groups)
+                        : launch_gemm<1, 256, KIND, EPI, false, 16, false, true>(ta, tb, p, max_tiles, st, groups);
         }
     }
-    return b_mn ? launch_gemm<1, 256, KIND, EPI, true, 8, false, true>(ta, tb, p, max_tiles, st)
-                : launch_gemm<1, 256, KIND, EPI, false, 8, false, true>(ta, tb, p, max_tiles, st);
+    return b_mn ? launch_gemm<1, 256, KIND, EPI, true, 8, false, true>(ta, tb, p, max_tiles, st, groups)
+                : launch_gemm<1, 256, KIND, EPI, false, 8, false, true>(ta, tb, p, max_tiles, st, groups);
 }
 
 // Dense problems with at most one 128 x 128 tile per SM run on single CTAs: a cluster launch costs about 3 us more
@@ -230,15 +233,6 @@ struct GroupEndsByValue {
     int32_t ends[PLAN_MAX_BY_VALUE];
 };
 
-// mode PLAN_ALL: every row of a group, in tiles of tile_m (the last one partial).
-// mode PLAN_WHOLE: the whole tile_m-row tiles of a group, plus its last partial tile when that holds more than
-//                  tile_m / 2 rows (as a pair tile it pads no more rows than two single tiles would).
-// mode PLAN_LEFTOVER: what a group leaves over after its (2 * tile_m)-row blocks when that is at most tile_m rows:
-//                  one tile of tile_m.
-// PLAN_WHOLE at 256 rows and PLAN_LEFTOVER at 128 rows together cover every row exactly once.
-constexpr int PLAN_ALL = 0;
-constexpr int PLAN_WHOLE = 1;
-constexpr int PLAN_LEFTOVER = 2;
 constexpr int PLAN_BOTH = 3;  // host side only: PLAN_WHOLE at 256 rows and PLAN_LEFTOVER at 128 rows in one launch
 
 __device__ __forceinline__ void plan_groups_body(int64_t zero, const int64_t* dev_list,
@@ -272,16 +266,7 @@ __device__ __forceinline__ void plan_groups_body(int64_t zero, const int64_t* de
             if (e < prev || e > M || (g == E - 1 && e != M && !allow_prefix)) {
                 s_bad = 1;
             } else {
-                const uint32_t rows = static_cast<uint32_t>(e - prev);
-                const uint32_t tm = static_cast<uint32_t>(tile_m);
-                if (mode == PLAN_WHOLE) {
-                    cnt = static_cast<int32_t>(rows / tm) + ((rows % tm > tm / 2) ? 1 : 0);
-                } else if (mode == PLAN_LEFTOVER) {
-                    const uint32_t rest = rows % (2 * tm);
-                    cnt = (rest >= 1 && rest <= tm) ? 1 : 0;
-                } else {
-                    cnt = static_cast<int32_t>((rows + tm - 1) / tm);
-                }
+                cnt = group_tiles(static_cast<uint32_t>(e - prev), static_cast<uint32_t>(tile_m), mode);
             }
         }
         int32_t incl = cnt;
@@ -338,21 +323,7 @@ __device__ __forceinline__ void plan_groups_body(int64_t zero, const int64_t* de
                 hi = mid;
             }
         }
-        int64_t start = (lo == 0) ? 0 : end_of(lo - 1);
-        int64_t rows = end_of(lo) - start;
-        if (mode == PLAN_LEFTOVER) {
-            const int64_t whole = rows / (2 * tile_m) * (2 * tile_m);
-            start += whole;
-            rows -= whole;
-        }
-        const int32_t t = i - s_first[lo];
-        TileEntry te;
-        te.group = lo;
-        te.m_start = static_cast<int32_t>(start + static_cast<int64_t>(t) * tile_m);
-        const int64_t left = rows - static_cast<int64_t>(t) * tile_m;
-        te.m_rows = static_cast<int32_t>(left < tile_m ? left : tile_m);
-        te.pad = 0;
-        tiles[i] = te;
+        tiles[i] = group_tile(lo, lo == 0 ? 0 : end_of(lo - 1), end_of(lo), i - s_first[lo], tile_m, mode);
     }
 }
 
@@ -365,6 +336,15 @@ __global__ void __launch_bounds__(256) plan_groups_kernel(const int64_t* dev_lis
     const int64_t zero = after_previous();
     plan_groups_body(zero, dev_list, by_value, use_by_value, E, M, header, tiles, max_tiles, tile_m, mode, shared_error,
                      allow_prefix);
+}
+
+__global__ void __launch_bounds__(256) zero_words_kernel(uint4* __restrict__ words, int64_t count)
+{
+    const int64_t zero = after_previous();
+    const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t i = zero + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += step) {
+        words[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
 }
 
 // Both tile tables of the two-launch form in one launch: CTA 0 plans the 256-row blocks, CTA 1 the leftovers of at
@@ -625,7 +605,6 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
     // (Rows stored one by one at caller-given addresses, possibly in peer memory, use the same shapes.  Single
     // tiles for them once measured faster on two GPUs; with the present kernels the chain steps are 13.26 against
     // 13.25 - 13.5 ms on two GPUs, 7.62 against 7.73 - 7.83 ms on four and 26.4 against 28.0 ms on one.)
-    p.grouped = 1;
     p.error = &g.header->error;
     // Rows per A load.  Pairs take whole tiles.  A single CTA's tile holds at most 128 rows of one group and often far
     // fewer - what a group leaves over, or a whole group of a small batch.  Where there are 256 MB of weights to stream
@@ -651,47 +630,60 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
     if (!make_map_a(&ta, a, M, a_cols, KIND, p.a_box_rows)) {
         return W8A8_ERR_CUDA;
     }
-    // `clear` (the SwiGLU form's row maxima and tile counters) must be zero before the first matmul launch: the
-    // two-table planner does it in its own launch, the other shapes with a memset
-    if (shape != GEMM_SHAPE_HYBRID) {
-        if (clear_bytes != 0 && cudaMemsetAsync(clear, 0, clear_bytes, st) != cudaSuccess) {
-            return W8A8_ERR_CUDA;
+    // Up to GROUPS_IN_CTA groups every CTA of the matmul plans its tiles itself; more take a table, planned by a kernel of
+    // its own.  `clear` (the SwiGLU form's row maxima and tile counters) must be zero before the first matmul launch: a
+    // kernel zeroes it, the planner's own launch where that builds two tables.
+    const bool hybrid = shape == GEMM_SHAPE_HYBRID;
+    GroupList groups{};
+    if (E <= GROUPS_IN_CTA) {
+        groups.E = static_cast<int32_t>(E);
+        groups.allow_prefix = list_on_device == 2 ? 1 : 0;
+        groups.mode = hybrid ? PLAN_WHOLE : PLAN_ALL;
+        groups.tile_m = hybrid ? 256 : 128 * shape;
+        if (list_on_device) {
+            groups.dev = group_list;
+        } else {
+            std::copy(group_list, group_list + E, groups.ends);  // checked by the caller
         }
-        const int rc = plan_groups(group_list, list_on_device, E, M, g, 128 * shape, st);
+    }
+    if (clear_bytes != 0 && (E <= GROUPS_IN_CTA || !hybrid)) {
+        const int64_t words = static_cast<int64_t>(clear_bytes / 16);
+        const unsigned ctas = static_cast<unsigned>(std::min<int64_t>((words + 255) / 256, sm_count()));
+        const cudaError_t e = launch_chained(zero_words_kernel, ctas, 256, 0, st, static_cast<uint4*>(clear), words);
+        if (e != cudaSuccess) {
+            return launch_status(e);
+        }
+    }
+    if (E > GROUPS_IN_CTA) {
+        const int rc = hybrid ? plan_groups(group_list, list_on_device, E, M, g, 256, st, PLAN_BOTH, clear, clear_bytes)
+                              : plan_groups(group_list, list_on_device, E, M, g, 128 * shape, st);
         if (rc != W8A8_OK) {
             return rc;
         }
-        p.tiles = g.tiles;
-        p.header = g.header;
-        p.tile_done = g.tile_done;
-        const int64_t most = g.max_tiles * p.n_tiles;
-        const cudaError_t e = row_boxes ? dispatch_row_boxes<KIND, EPI>(b_mn, ta, tb, p, most, st)
-                                        : dispatch_gemm<KIND, EPI>(shape, 256, b_mn, ta, tb, p, most, st);
-        return launch_status(e);
-    }
-    const int rc = plan_groups(group_list, list_on_device, E, M, g, 256, st, PLAN_BOTH, clear, clear_bytes);
-    if (rc != W8A8_OK) {
-        return rc;
     }
     p.tiles = g.tiles;
     p.header = g.header;
     p.tile_done = g.tile_done;
-    cudaError_t e = dispatch_gemm<KIND, EPI>(2, 256, b_mn, ta, tb, p, (M / 256 + E + 1) * p.n_tiles, st);
-    if (e != cudaSuccess) {
+    const int64_t most = (hybrid ? M / 256 + E + 1 : g.max_tiles) * p.n_tiles;
+    cudaError_t e = (!hybrid && row_boxes) ? dispatch_row_boxes<KIND, EPI>(b_mn, ta, tb, p, most, st, groups)
+                                           : dispatch_gemm<KIND, EPI>(hybrid ? 2 : shape, 256, b_mn, ta, tb, p, most, st, groups);
+    if (e != cudaSuccess || !hybrid) {
         return launch_status(e);
     }
     p.tiles = g.tail_tiles;
     p.header = g.tail_header;
     p.tile_done = g.tail_tile_done;
-    const int64_t most = g.tail_max_tiles * p.n_tiles;
+    groups.mode = PLAN_LEFTOVER;
+    groups.tile_m = 128;
+    const int64_t tail_most = g.tail_max_tiles * p.n_tiles;
     if (row_boxes) {
         p.a_box_rows = box_rows;
         if (!make_map_a(&ta, a, M, a_cols, KIND, box_rows)) {
             return W8A8_ERR_CUDA;
         }
-        e = dispatch_row_boxes<KIND, EPI>(b_mn, ta, tb, p, most, st);
+        e = dispatch_row_boxes<KIND, EPI>(b_mn, ta, tb, p, tail_most, st, groups);
     } else {
-        e = dispatch_gemm<KIND, EPI>(1, 256, b_mn, ta, tb, p, most, st);
+        e = dispatch_gemm<KIND, EPI>(1, 256, b_mn, ta, tb, p, tail_most, st, groups);
     }
     return launch_status(e);
 }
@@ -782,7 +774,6 @@ static int quant_matmul_impl(const int8_t* x1, const int8_t* x2, const void* sca
     p.num_k_blocks = static_cast<int32_t>((K + GEMM_KBYTES - 1) / GEMM_KBYTES);
     p.m_tiles_per_batch = static_cast<int32_t>((M + GEMM_BLOCK_M - 1) / GEMM_BLOCK_M);
     p.batch = static_cast<int32_t>(batch);
-    p.grouped = 0;
     p.scale = scale;
     p.offset = offset;
     p.row_scale = pertoken;

@@ -42,6 +42,8 @@
 // and the expert's weights stay L2-resident.
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "tc_ptx.cuh"
 
@@ -103,6 +105,131 @@ struct GroupedHeader {
     int32_t pad[61];
 };
 
+// How groups become row tiles:
+// PLAN_ALL: every row of a group, in tiles of tile_m (the last one partial).
+// PLAN_WHOLE: the whole tile_m-row tiles of a group, plus its last partial tile when that holds more than
+//             tile_m / 2 rows (as a pair tile it pads no more rows than two single tiles would).
+// PLAN_LEFTOVER: what a group leaves over after its (2 * tile_m)-row blocks when that is at most tile_m rows:
+//             one tile of tile_m.
+// PLAN_WHOLE at 256 rows and PLAN_LEFTOVER at 128 rows together cover every row exactly once.
+constexpr int PLAN_ALL = 0;
+constexpr int PLAN_WHOLE = 1;
+constexpr int PLAN_LEFTOVER = 2;
+
+__device__ __forceinline__ int32_t group_tiles(uint32_t rows, uint32_t tile_m, int mode)
+{
+    if (mode == PLAN_WHOLE) {
+        return static_cast<int32_t>(rows / tile_m) + ((rows % tile_m > tile_m / 2) ? 1 : 0);
+    }
+    if (mode == PLAN_LEFTOVER) {
+        const uint32_t rest = rows % (2 * tile_m);
+        return (rest >= 1 && rest <= tile_m) ? 1 : 0;
+    }
+    return static_cast<int32_t>((rows + tile_m - 1) / tile_m);
+}
+
+// tile `t` of group `group`, whose rows are [start, end)
+__device__ __forceinline__ TileEntry group_tile(int group, int64_t start, int64_t end, int32_t t, int tile_m, int mode)
+{
+    int64_t rows = end - start;
+    if (mode == PLAN_LEFTOVER) {
+        const int64_t whole = rows / (2 * tile_m) * (2 * tile_m);
+        start += whole;
+        rows -= whole;
+    }
+    TileEntry te;
+    te.group = group;
+    te.m_start = static_cast<int32_t>(start + static_cast<int64_t>(t) * tile_m);
+    const int64_t left = rows - static_cast<int64_t>(t) * tile_m;
+    te.m_rows = static_cast<int32_t>(left < tile_m ? left : tile_m);
+    te.pad = 0;
+    return te;
+}
+
+// The group list of a grouped problem with at most GROUPS_IN_CTA groups: every CTA plans the tiles for itself - one warp,
+// 0.5 us, and for a host list before the wait for the kernel before.  A planner kernel that wrote a table took 2 - 3 us of
+// every call (and, for the SwiGLU form of few rows, a memset that no launch overlaps): 64 rows of 4 experts of 512 x 512
+// bf16 6.7 us (8.7 with it), 200 of 8 of 1024 x 2048 14.1 (16.0); SwiGLU form, 64 rows of 32 experts of 1024 x 1024 16.1
+// (22.4), 100 of 8 of 4096 x 2048 23.5 (28.8).  The bound is the shared memory that is left beside the stages.
+constexpr int GROUPS_IN_CTA = 256;
+struct GroupList {
+    const int64_t* dev;  // device list, or null: `ends`
+    int32_t E;           // 0: the tiles come from the table of plan_groups_kernel
+    int32_t mode;
+    int32_t tile_m;
+    int32_t allow_prefix;
+    int32_t ends[GROUPS_IN_CTA];
+
+    __device__ __forceinline__ int64_t end_of(int g) const { return dev != nullptr ? dev[g] : ends[g]; }
+};
+struct NoGroupList {
+};
+template <int EPI>
+using GroupListOf = std::conditional_t<EPI == EPI_GMSQ || EPI == EPI_GMM, GroupList, NoGroupList>;
+
+// One warp: first[g] = the first tile of group g, first[E] = the number of tiles, and whether the list is in order.  An
+// invalid one has no tiles.
+__device__ __forceinline__ bool plan_in_cta(const GroupList& list, int64_t M, int32_t* first)
+{
+    constexpr int PER_LANE = GROUPS_IN_CTA / 32;
+    const int lane = threadIdx.x & 31;
+    int32_t count[PER_LANE], sum = 0;
+    bool bad = false;
+    int64_t prev = 0;
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) {
+        const int g = lane * PER_LANE + i;
+        count[i] = 0;
+        if (g < list.E) {
+            if (i == 0 && g > 0) {
+                prev = list.end_of(g - 1);
+            }
+            const int64_t end = list.end_of(g);
+            const bool ok = end >= prev && prev >= 0 && end <= M && (g != list.E - 1 || end == M || list.allow_prefix != 0);
+            bad |= !ok;
+            count[i] = ok ? group_tiles(static_cast<uint32_t>(end - prev), static_cast<uint32_t>(list.tile_m), list.mode) : 0;
+            prev = end;
+        }
+        sum += count[i];
+    }
+    bad = __any_sync(FULL_MASK, bad);
+    int32_t incl = sum;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int32_t v = __shfl_up_sync(FULL_MASK, incl, off);
+        incl += lane >= off ? v : 0;
+    }
+    int32_t at = incl - sum;
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) {
+        const int g = lane * PER_LANE + i;
+        if (g < list.E) {
+            first[g] = bad ? 0 : at;
+        }
+        at += count[i];
+        if (g == list.E - 1) {
+            first[list.E] = bad ? 0 : at;
+        }
+    }
+    return !bad;
+}
+
+// Tile `mt` by the first tiles: its group is the last one whose first tile is at or before it (groups without tiles
+// share their first tile with the next one, and first[E] ends the search).
+__device__ __forceinline__ TileEntry tile_in_cta(const GroupList& list, const int32_t* first, int32_t mt)
+{
+    int lo = 0, hi = list.E;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (first[mid] <= mt) {
+            lo = mid;
+        } else {
+            hi = mid;
+        }
+    }
+    return group_tile(lo, lo == 0 ? 0 : list.end_of(lo - 1), list.end_of(lo), mt - first[lo], list.tile_m, list.mode);
+}
+
 struct GemmParams {
     int64_t M;  // rows per batch (dense) or total rows (grouped)
     int64_t N;  // logical output columns of the matmul
@@ -111,7 +238,6 @@ struct GemmParams {
     int32_t n_tiles;
     int32_t m_tiles_per_batch;
     int32_t batch;
-    int32_t grouped;
     const TileEntry* tiles;
     GroupedHeader* header;  // grouped: tile count + error word; dense: may be null
     int32_t* error;         // device error word (may be null)
@@ -770,7 +896,7 @@ __device__ __forceinline__ void split_finish(const GemmParams& p, const TileInfo
 template <int CG, int BLOCK_N, int KIND, int EPI, bool B_MN, int EPI_WARPS, bool SPLITK, bool ROW_BOXES>
 __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
-                   const GemmParams p)
+                   const GemmParams p, const __grid_constant__ GroupListOf<EPI> groups)
 {
     constexpr int ELEM = (KIND == KIND_I8) ? 1 : 2;
     constexpr int BLOCK_K = GEMM_KBYTES / ELEM;    // elements of K per stage
@@ -804,6 +930,9 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
     // bars[0..S) full, [S..2S) empty, [2S..2S+2) tmem_full, [2S+2..2S+4) tmem_empty
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 6);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    // first tiles of the groups, behind the store patches
+    [[maybe_unused]] int32_t* first_tiles = reinterpret_cast<int32_t*>(smem + STAGES * STAGE_BYTES + 512 + GEMM_EPI_PATCH_BYTES);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -887,6 +1016,12 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
         }
         tc::fence_async_smem();
     }
+    constexpr bool GROUPED = (EPI == EPI_GMSQ || EPI == EPI_GMM);
+    if constexpr (GROUPED) {
+        if (warp == 3 && groups.E != 0 && groups.dev == nullptr) {
+            plan_in_cta(groups, p.M, first_tiles);
+        }
+    }
     tc::tc_fence_before_sync();
     __syncthreads();
     if constexpr (CG == 2) {
@@ -898,13 +1033,29 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
     const uint32_t tmem_base = *tmem_slot;
     // everything above touches shared and tensor memory only and may run beside the kernel before
     after_previous();
+    if constexpr (GROUPED) {
+        if (groups.E != 0) {
+            bool valid = true;
+            if (groups.dev != nullptr) {
+                if (warp == 3) {
+                    valid = plan_in_cta(groups, p.M, first_tiles);
+                }
+                __syncthreads();
+            }
+            if (blockIdx.x == 0 && threadIdx.x == 96) {  // warp 3: for the requantisation, and whoever asks for the error
+                p.header->num_m_tiles = first_tiles[groups.E];
+                p.header->error = valid ? 0 : 1;
+                p.header->rows_total = valid ? static_cast<int32_t>(groups.end_of(groups.E - 1)) : 0;
+            }
+        }
+    }
 
     // ---- tile enumeration (identical in every role and in both CTAs of a pair) ----
     constexpr int TILE_M = 128 * CG;
     int64_t total_tiles;
     int32_t dense_m_tiles = 0;
-    if (p.grouped) {
-        total_tiles = static_cast<int64_t>(p.header->num_m_tiles) * p.n_tiles;
+    if constexpr (GROUPED) {
+        total_tiles = static_cast<int64_t>(groups.E != 0 ? first_tiles[groups.E] : p.header->num_m_tiles) * p.n_tiles;
     } else {
         dense_m_tiles = p.batch * p.m_tiles_per_batch;
         total_tiles = static_cast<int64_t>(dense_m_tiles) * p.n_tiles;
@@ -918,11 +1069,11 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
         TileInfo tl;
         int64_t tile_row0;
         int32_t tile_rows;
-        if (p.grouped) {
+        if constexpr (GROUPED) {
             const int32_t mt = static_cast<int32_t>(t / p.n_tiles);
             tl.nt = static_cast<int32_t>(t % p.n_tiles);
             tl.mt = mt;
-            const TileEntry e = p.tiles[mt];
+            const TileEntry e = groups.E != 0 ? tile_in_cta(groups, first_tiles, mt) : p.tiles[mt];
             tile_row0 = e.m_start;
             tile_rows = e.m_rows;
             tl.group = e.group;
