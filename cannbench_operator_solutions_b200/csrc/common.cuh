@@ -483,8 +483,9 @@ void note_launch();  // counts one kernel launch of this library (w8a8_kernel_la
 // Programmatic dependent launch.  A kernel launched with launch_chained may start while the kernel before it on the
 // stream is still running: its launch, block setup and prologue then overlap that kernel's tail instead of following
 // it.  Every such kernel opens with after_previous(), which waits until the kernel before it has completed and its
-// writes are visible; no global memory is touched before that, neither read nor written.  It also lets the next kernel
-// start.  A grid of at most one block per SM does so before its own wait, which takes 0.2 - 0.3 us off a short kernel; a
+// writes are visible; no global memory is touched before that, neither read nor written (the dense matmuls ask for
+// weights into L2, which reads nothing; the second of a grouped matmul's two launches has an order of its own, see
+// gemm_kernel.cuh).  It also lets the next kernel start.  A grid of at most one block per SM does so before its own wait, which takes 0.2 - 0.3 us off a short kernel; a
 // larger one after it: with three kernels resident at once their blocks share the SMs unevenly (back to back, the router
 // on 16384 rows of 256 bf16 takes 9.0 us, 13.4 if it lets the next one in ahead of the wait; the SwiGLU quantiser on 300
 // rows of 16384 int32 47 us, 67).  BY_GRID = false: after it in any case - the SwiGLU quantiser, whose registers are used

@@ -664,6 +664,9 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
     p.tiles = g.tiles;
     p.header = g.header;
     p.tile_done = g.tile_done;
+    // (with a table of its own the second launch would read what the planner wrote: it waits)
+    const bool overlap = hybrid && E <= GROUPS_IN_CTA;
+    p.order = overlap ? ORDER_FIRST_OF_TWO : ORDER_ALONE;
     const int64_t most = (hybrid ? M / 256 + E + 1 : g.max_tiles) * p.n_tiles;
     cudaError_t e = (!hybrid && row_boxes) ? dispatch_row_boxes<KIND, EPI>(b_mn, ta, tb, p, most, st, groups)
                                            : dispatch_gemm<KIND, EPI>(hybrid ? 2 : shape, 256, b_mn, ta, tb, p, most, st, groups);
@@ -673,6 +676,7 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
     p.tiles = g.tail_tiles;
     p.header = g.tail_header;
     p.tile_done = g.tail_tile_done;
+    p.order = overlap ? ORDER_SECOND_OF_TWO : ORDER_ALONE;
     groups.mode = PLAN_LEFTOVER;
     groups.tile_m = 128;
     const int64_t tail_most = g.tail_max_tiles * p.n_tiles;

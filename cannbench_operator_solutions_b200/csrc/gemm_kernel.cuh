@@ -230,6 +230,17 @@ __device__ __forceinline__ TileEntry tile_in_cta(const GroupList& list, const in
     return group_tile(lo, lo == 0 ? 0 : list.end_of(lo - 1), list.end_of(lo), mt - first[lo], list.tile_m, list.mode);
 }
 
+// A grouped problem's two launches (pairs, then leftovers) share no output row and read nothing of one another, so the
+// second one's CTAs start as the first one's leave their SMs, whose last wave of tiles is rarely full.  What orders them:
+// the first one lets the second in only after its own wait, when all that came before is complete; the second one waits
+// for the first only before it ends, so that whoever waits for the second has waited for both.  2500 rows of 16 experts of
+// 1024 x 1024 bf16 21.1 us (28.1 one after the other), 4000 of 32 of 2048 x 7168 205 (214), 16000 of 4 of 4096 x 2048 223
+// (236); SwiGLU form, 2500 of 8 of 2048 x 2048 35.8 (39.3), 3000 of 32 of 7168 x 4096 206 (218); what the power cap bounds
+// (8000 of 32 of 2048 x 7168 317, the 131072-row Zipf load 4060) stays.
+constexpr int ORDER_ALONE = 0;
+constexpr int ORDER_FIRST_OF_TWO = 1;
+constexpr int ORDER_SECOND_OF_TWO = 2;
+
 struct GemmParams {
     int64_t M;  // rows per batch (dense) or total rows (grouped)
     int64_t N;  // logical output columns of the matmul
@@ -257,6 +268,7 @@ struct GemmParams {
     int32_t k_blocks_per_term;
     // dense: K blocks of a CTA's first tile of B that it asks L2 for while the kernel before it may still be running
     int32_t prefetch_k_blocks;
+    int32_t order;  // ORDER_*
     float* act;       // GMSQ: fp32 activations [M, N/2]
     uint32_t* amax;   // GMSQ: per-row max|act| bit patterns
     // GMSQ with the requantisation fused in: the CTA that finishes the last column tile of its rows quantises them
@@ -1032,7 +1044,15 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
     tc::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
     // everything above touches shared and tensor memory only and may run beside the kernel before
-    after_previous();
+    if (p.order == ORDER_FIRST_OF_TWO) {
+        after_previous<false>();  // the second one starts only when everything before this kernel is complete
+    } else if (p.order == ORDER_SECOND_OF_TWO) {
+        // reads nothing that the first one writes, and writes other rows: it waits for it only before it ends
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        __threadfence();  // no line that this SM's L1 holds from before
+    } else {
+        after_previous();
+    }
     if constexpr (GROUPED) {
         if (groups.E != 0) {
             bool valid = true;
@@ -1444,6 +1464,9 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
     }
 
     // ---- teardown ----
+    if (p.order == ORDER_SECOND_OF_TWO) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");  // whoever waits for this kernel waits for the first one too
+    }
     tc::tc_fence_before_sync();
     __syncthreads();
     if (*abort_flag != 0) {
