@@ -18,6 +18,7 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libw8a8ffn.so")
 PLUGIN_PATH = os.path.join(PKG_DIR, "libcann_bench_cuda.so")
+CALLS_PATH = os.path.join(PKG_DIR, "_calls.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -76,12 +77,11 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     return LIB_PATH
 
 
-def build_plugin(force: bool = False) -> str:
-    """Compile the torch plugin (host C++ only) against libw8a8ffn.so."""
-    src = os.path.join(CSRC, "plugin", "cann_bench_ops.cpp")
+def _build_torch_cpp(src: str, path: str, extra_libs, force: bool) -> str:
+    """Compile one host C++ source that uses torch, linked against libw8a8ffn.so."""
     deps = [src, os.path.join(PKG_DIR, "..", "include", "w8a8ffn.h")]
-    if not force and os.path.exists(PLUGIN_PATH) and os.path.getmtime(PLUGIN_PATH) >= _newest(deps):
-        return PLUGIN_PATH
+    if not force and os.path.exists(path) and os.path.getmtime(path) >= _newest(deps):
+        return path
     import torch
     from torch.utils import cpp_extension
 
@@ -95,21 +95,33 @@ def build_plugin(force: bool = False) -> str:
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
     cmd = [
         "/usr/bin/g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
-        "-DTORCH_API_INCLUDE_EXTENSION_H", *inc, src, "-o", PLUGIN_PATH,
-        f"-L{PKG_DIR}", "-l:libw8a8ffn.so", f"-L{tlib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda",
+        "-DTORCH_API_INCLUDE_EXTENSION_H", *inc, src, "-o", path,
+        f"-L{PKG_DIR}", "-l:libw8a8ffn.so", f"-L{tlib}", *extra_libs, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda",
         "-ltorch", "-L/usr/local/cuda/lib64", "-lcudart",
         "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{tlib}",
     ]
     subprocess.run(cmd, check=True)
-    return PLUGIN_PATH
+    return path
+
+
+def build_plugin(force: bool = False) -> str:
+    """The torch operator plugin."""
+    return _build_torch_cpp(os.path.join(CSRC, "plugin", "cann_bench_ops.cpp"), PLUGIN_PATH, [], force)
+
+
+def build_calls(force: bool = False) -> str:
+    """The native half of ops.py."""
+    return _build_torch_cpp(os.path.join(CSRC, "plugin", "py_calls.cpp"), CALLS_PATH, ["-ltorch_python"], force)
 
 
 def build_all(force: bool = False, verbose: bool = False) -> None:
     build_library(force=force, verbose=verbose)
     build_plugin(force=force)
+    build_calls(force=force)
 
 
 if __name__ == "__main__":
     build_all(force="--force" in sys.argv, verbose="-v" in sys.argv)
     print(LIB_PATH)
     print(PLUGIN_PATH)
+    print(CALLS_PATH)

@@ -17,6 +17,12 @@ import torch
 
 from . import _lib as L
 
+try:
+    # the same functions in native code for calls in their plain form; None comes back from any other call
+    from . import _calls
+except ImportError:  # not built yet, as while building
+    _calls = None
+
 
 def _check(cond: bool, msg: str) -> None:
     if not cond:
@@ -66,6 +72,10 @@ def _need_cuda(*ts: Optional[torch.Tensor]) -> None:
 def dynamic_quant(x: torch.Tensor, *, round_direct: bool = False) -> Tuple[torch.Tensor, torch.Tensor]:
     """``dynamic_quant(Tensor x) -> (Tensor y, Tensor scale)``
     (operators/dynamicquant/csrc/ops/dynamic_quant/op_plugin/dynamic_quant_plugin.cpp:30,33-87)."""
+    if _calls is not None:
+        done = _calls.dynamic_quant(x, round_direct)
+        if done is not None:
+            return done
     _check(x.dim() >= 2, "dynamic_quant requires a tensor with rank >= 2.")
     _check(x.dtype in (torch.float16, torch.bfloat16), "dynamic_quant only supports float16 / bfloat16 inputs.")
     _need_cuda(x)
@@ -87,6 +97,10 @@ def add_rms_norm_dynamic_quant(x1: torch.Tensor, x2: torch.Tensor, gamma: torch.
                                round_direct: bool = False) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """``add_rms_norm_dynamic_quant(Tensor x1, Tensor x2, Tensor gamma, float epsilon) -> (y, xOut, scaleOut)``
     (operators/addrmsnormdynamicquant/csrc/ops/add_rms_norm_dynamic_quant/op_plugin/add_rms_norm_dynamic_quant_plugin.cpp:32,36-112)."""
+    if _calls is not None:
+        done = _calls.add_rms_norm_dynamic_quant(x1, x2, gamma, epsilon, round_direct)
+        if done is not None:
+            return done
     _check(x1.dim() >= 1, "add_rms_norm_dynamic_quant: x1 must have at least one dimension.")
     _check(x1.shape == x2.shape, "add_rms_norm_dynamic_quant: x1 and x2 must have the same shape.")
     _check(gamma.dim() == 1 and gamma.size(0) == x1.size(-1),
@@ -118,6 +132,10 @@ def quant_matmul(x1: torch.Tensor, x2: torch.Tensor, scale: torch.Tensor, *, off
     str? output_dtype) -> Tensor`` (operators/quantmatmul/csrc/ops/quant_matmul/op_plugin/quant_matmul_plugin.cpp:48-49,77-267).
 
     ``transpose_x2=True`` (not in the reference) takes x2 as [..., N, K]."""
+    if _calls is not None:
+        done = _calls.quant_matmul(x1, x2, scale, offset, pertoken_scale, bias, output_dtype, transpose_x2)
+        if done is not None:
+            return done
     _check(x1.dtype == torch.int8 and x2.dtype == torch.int8, "quant_matmul requires int8 x1 and x2.")
     _check(x1.is_contiguous() and x2.is_contiguous() and scale.is_contiguous(),
            "quant_matmul requires contiguous x1/x2/scale.")
@@ -217,6 +235,11 @@ def grouped_matmul_swiglu_quant(x: torch.Tensor, weight: torch.Tensor, weight_sc
     Beyond the reference: any expert count (the reference stops at 64), ``group_list`` may be a CUDA int64
     tensor, ``transpose_weight=True`` takes weight as [E, N, K], and a caller-owned ``workspace`` avoids the
     per-call allocation."""
+    if _calls is not None and workspace is None:
+        done = _calls.grouped_matmul_swiglu_quant(x, weight, weight_scale, x_scale, group_list, transpose_weight,
+                                                  round_direct)
+        if done is not None:
+            return done
     _check(x.dim() == 2, "grouped_matmul_swiglu_quant: x must be 2D [M, K]")
     _check(weight.dim() == 3, "grouped_matmul_swiglu_quant: weight must be 3D [E, K, N]")
     _check(x.dtype == torch.int8, "grouped_matmul_swiglu_quant: x must be int8")
@@ -267,6 +290,10 @@ def grouped_matmul(x: torch.Tensor, weight: torch.Tensor, group_list: GroupList,
     (grouped_matmul_plugin.cpp:65-80).  Beyond the reference: int8 ``x``/``weight`` with ``x_scale`` [M] and
     ``weight_scale`` [E, N] (the quantised down projection; output ``output_dtype``, default bfloat16), any
     expert count, device group lists."""
+    if _calls is not None and workspace is None and output_dtype is None and split_item in (2, 3):
+        done = _calls.grouped_matmul(x, weight, group_list, bias, transpose_weight, x_scale, weight_scale)
+        if done is not None:
+            return [done]
     _check(x.dim() == 2, "grouped_matmul: x must be 2D [M, K]")
     _check(weight.dim() == 3, "grouped_matmul: weight must be 3D [E, K, N] or [E, N, K]")
     _need_cuda(x, weight, bias, x_scale, weight_scale)
@@ -339,6 +366,10 @@ def moe_re_routing(tokens: torch.Tensor, expert_token_num_per_rank: torch.Tensor
     reference ``expert_token_num_type`` is accepted and ignored (counts are always returned), ``idx_type`` must be
     0, and without ``per_token_scales`` the scale output is allocated but not written.  The whole path runs on the
     device: the count matrix is never read by the host."""
+    if _calls is not None and workspace is None and idx_type == 0:
+        done = _calls.moe_re_routing(tokens, expert_token_num_per_rank, per_token_scales)
+        if done is not None:
+            return done
     del expert_token_num_type
     _check(idx_type == 0, "moe_re_routing: only gather index mode (idx_type == 0) is supported.")
     _check(tokens.dim() == 2, "moe_re_routing: tokens must be 2D (A, H).")
@@ -388,6 +419,11 @@ def moe_finalize_routing(expanded_permuted_rows: torch.Tensor, expanded_src_to_d
     ``scales.size(1)`` (1 without scales), ``num_rows = expanded_src_to_dst_row.numel() / K``; ``drop_pad_mode`` is
     clamped to 0..3 (0/1: index arranged [K, num_rows], 2/3: [num_rows, K]); bias is only applied together with
     ``expert_for_source_row``."""
+    if _calls is not None:
+        done = _calls.moe_finalize_routing(expanded_permuted_rows, expanded_src_to_dst_row, skip1, skip2, bias, scales,
+                                           expert_for_source_row, drop_pad_mode)
+        if done is not None:
+            return done
     epr = expanded_permuted_rows
     _check(epr.dtype in (torch.float16, torch.float32, torch.bfloat16),
            "moe_finalize_routing: expanded_permuted_rows must be float16 / float32 / bfloat16.")
@@ -441,6 +477,10 @@ def moe_gating_top_k_softmax(x: torch.Tensor, finished: Optional[torch.Tensor] =
 
     Softmax over the last dimension in fp32, the ``k`` largest probabilities per row in ``x``'s dtype, their
     expert columns (int32; ``x.size(-1)`` for rows whose ``finished`` flag is set) and ``row_idx = j * rows + r``."""
+    if _calls is not None:
+        done = _calls.moe_gating_top_k_softmax(x, finished, k)
+        if done is not None:
+            return done
     _check(x.dtype in (torch.float32, torch.float16, torch.bfloat16),
            "cann_bench.moe_gating_top_k_softmax only supports float32, float16 and bfloat16 inputs.")
     _check(x.dim() >= 2, "cann_bench.moe_gating_top_k_softmax requires a tensor with rank >= 2.")
@@ -478,6 +518,10 @@ def dequant_swiglu_quant(x: torch.Tensor, weight_scale: Optional[torch.Tensor] =
 
     ``x`` [TokensNum, 2H] int32 (then both scales are required) or float16 / bfloat16 (then both must be None);
     returns int8 ``y`` [TokensNum, H] and float32 ``scale`` [TokensNum]."""
+    if _calls is not None:
+        done = _calls.dequant_swiglu_quant(x, weight_scale, activation_scale, quant_scale, activate_left, round_direct)
+        if done is not None:
+            return done
     _check(x.dim() == 2, "dequant_swiglu_quant requires a 2D input [TokensNum, 2H].")
     m, n2 = x.shape
     _check(n2 % 2 == 0, "dequant_swiglu_quant requires an even last dimension.")
