@@ -521,6 +521,20 @@ __device__ __forceinline__ int64_t after_previous()
     return zero;
 }
 
+// For a kernel that reads nothing of what the kernel before it writes and writes nothing that it reads, where that one
+// lets it in only after its own wait (after_previous<false>): all that came before the two is then complete, and this one
+// need not wait at its start.  It waits at its end instead (previous_complete), so that whoever waits for it has waited
+// for both.
+__device__ __forceinline__ int64_t beside_previous()
+{
+    int64_t zero;
+    // no line that this SM's L1 holds from before
+    asm volatile("griddepcontrol.launch_dependents;\n\tfence.acq_rel.gpu;\n\tmov.u64 %0, 0;" : "=l"(zero)::"memory");
+    return zero;
+}
+
+__device__ __forceinline__ void previous_complete() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // overlap = false: starts when the kernel before it has completed, like a plain launch.
 template <typename... Params, typename... Args>
 cudaError_t launch_chained_if(bool overlap, void (*kern)(Params...), unsigned grid, unsigned block, size_t smem,
@@ -557,6 +571,13 @@ inline int launch_status(cudaError_t e)
     }
     return W8A8_OK;
 }
+
+// w8a8_add_rms_norm_dynamic_quant launched beside the kernel before it (see beside_previous)
+int add_rms_norm_dynamic_quant_beside(const void* x1, const void* x2, const void* gamma, int8_t* y, void* x_out,
+                                      float* scale_out, int64_t rows, int64_t N, float epsilon, int dtype, void* stream);
+// w8a8_dispatch_rows where every pair's row goes to row `expanded_pos` of one buffer
+int dispatch_rows_local(const void* src, const float* src_scale, const int64_t* expanded_pos, void* dst, float* dst_scale,
+                        int64_t T, int64_t topk, int64_t row_bytes, void* stream);
 
 inline bool is_aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 

@@ -5,6 +5,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <cmath>
 #include <atomic>
 #include <mutex>
 
@@ -65,7 +66,10 @@ static bool make_map_a(CUtensorMap* m, const void* base, int64_t rows, int64_t K
 }
 
 // B: [G, K, N] (mn_major) or [G, N, K].  Box = 128 bytes of the contiguous
-// dimension x 128 bytes-worth of K rows (mn_major: BLOCK_K rows) or 128 N rows.
+// dimension x 128 bytes-worth of K rows (mn_major: BLOCK_K rows) or 128 N rows.  L2 promotion to 128 bytes: to 256, the
+// neighbouring column tile's half of each line pair came along, to be fetched again where that tile runs at another time
+// or on the other die (SwiGLU form, 512 rows of 256 experts of 7168 x 4096 927 us, 953 so; 7724 of 64 of 1712 x 3808 159,
+// 171).
 static bool make_map_b(CUtensorMap* m, const void* base, int64_t G, int64_t N, int64_t K, int kind, bool mn_major)
 {
     EncodeTiledFn fn = encode_tiled_fn();
@@ -80,7 +84,7 @@ static bool make_map_b(CUtensorMap* m, const void* base, int64_t G, int64_t N, i
     cuuint32_t box[3] = {static_cast<cuuint32_t>(128 / elem), static_cast<cuuint32_t>(mn_major ? 128 / elem : 128), 1};
     cuuint32_t estr[3] = {1, 1, 1};
     return fn(m, tm_dtype(kind), 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -123,7 +127,7 @@ static cudaError_t launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, con
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = p.order == ORDER_PLAIN ? 0 : 1;
     if (cluster > 1) {
         attr[1].id = cudaLaunchAttributeClusterDimension;
         attr[1].val.clusterDim.x = cluster;
@@ -199,27 +203,72 @@ static int choose_split(int64_t tiles, int64_t k_blocks, int64_t rows)
     return (tiles * 2 <= sm_count() && k_blocks >= (few_rows ? 12 : 24)) ? 2 : 1;
 }
 
-// Kernel shape: CTA pairs for dense problems with enough rows to fill 256-row tiles.  w8a8_set_gemm_shape()
-// (1, 2, or 3 = pairs plus singles for grouped problems; 0 = the library's choice) overrides it process-wide; the
-// tests use it to run every case on every shape.
+// w8a8_set_gemm_shape() (1, 2, or 3 = pairs plus singles for grouped problems; 0 = the library's choice) overrides the
+// kernel shape process-wide; the tests use it to run every case on every shape.
 constexpr int GEMM_SHAPE_HYBRID = 3;
 static std::atomic<int> g_shape_override{0};
 static std::atomic<int> g_fuse_requant{0};  // see w8a8_set_gmsq_fused_requant
 
-static int choose_cta_group(int64_t rows, bool grouped)
+// Dense problems: CTA pairs from 256 rows on (see also choose_split and quant_matmul_impl).
+static int choose_cta_group(int64_t rows)
 {
     const int v = g_shape_override.load(std::memory_order_relaxed);
-    if (v == 1 || v == 2 || (v == GEMM_SHAPE_HYBRID && grouped)) {
+    return (v == 1 || v == 2) ? v : (rows >= 256 ? 2 : 1);
+}
+
+// Grouped problems: single CTAs on 128-row tiles, CTA pairs on 256-row tiles, or both in two launches - pairs on every
+// group's 256-row blocks (the last one partial when it holds more than 128 rows) and singles on leftovers of at most 128
+// rows, which pads the least and takes the least energy, but starts and ends twice.  The shape is the one with the
+// smallest of three estimates, in us: waves of tiles over the SMs, a tile taking its K blocks (0.405 on a single CTA,
+// 0.326 on a pair) or its epilogue (2.7, 3.15) if that is longer; no less than the touched groups' weights at 7.7 TB/s; and
+// what the shape costs besides (2.5 for pairs, 20 for two launches, whose leftovers partly overlap the pairs: 0.55 of
+// their time counts).  Fitted to 290 problems of 200 - 65000 rows, 4 - 128 groups, int8 and 16-bit, both epilogues, each
+// timed under load in all three shapes: 0.2 % from the best shape of each on average and 6 % at worst.  Two launches from
+// 2048 rows on, as the rule was, are 6.4 % from it on average and 52 % at worst (3000 rows of 8 groups of 2048 x 4096 bf16
+// 74 us, 59 on single CTAs; SwiGLU form, 6000 of 8 of 4096 x 2048 69, 58).  Of a device list only the rows and the number of
+// groups are known here: even groups with remainders of all sizes are assumed (0.8 % and 31 % on the same problems).
+static int choose_grouped_shape(const int64_t* host_ends, int64_t E, int64_t M, int64_t n_tiles, int64_t k_blocks,
+                                double group_weight_bytes)
+{
+    const int v = g_shape_override.load(std::memory_order_relaxed);
+    if (v != 0) {
         return v;
     }
-    // Grouped problems with enough rows run in two launches: CTA pairs on every group's 256-row blocks (the last
-    // one partial when it holds more than 128 rows) and single CTAs on leftovers of at most 128 rows.  Pairs on everything would pad the end of every group to 256 rows,
-    // which with skewed group sizes costs more than pairing gains (measured on the 256-expert Zipf configuration:
-    // 4.94 ms against 4.66 ms with 128-row tiles only).
-    if (grouped) {
-        return rows >= 2048 ? GEMM_SHAPE_HYBRID : 1;
+    double singles = 0, pairs = 0, whole = 0, leftover = 0, touched = 0;  // row tiles of the three shapes
+    if (host_ends != nullptr) {
+        int64_t prev = 0;
+        for (int64_t g = 0; g < E; ++g) {
+            const int64_t rows = host_ends[g] - prev, rest = rows % 256;
+            prev = host_ends[g];
+            singles += static_cast<double>((rows + 127) / 128);
+            pairs += static_cast<double>((rows + 255) / 256);
+            whole += static_cast<double>(rows / 256 + (rest > 128 ? 1 : 0));
+            leftover += (rest > 0 && rest <= 128) ? 1 : 0;
+            touched += rows > 0 ? 1 : 0;
+        }
+    } else {
+        const double e = static_cast<double>(E), m = static_cast<double>(M);
+        touched = std::min(e, m);
+        if (M >= 256 * E) {
+            singles = m / 128 + e / 2;
+            pairs = m / 256 + e / 2;
+            whole = m / 256;
+            leftover = e / 2;
+        } else {
+            singles = M > 128 * E ? 2 * e : touched;
+            pairs = touched;
+            whole = M > 128 * E ? e : 0;
+            leftover = touched - whole;
+        }
     }
-    return rows >= 256 ? 2 : 1;
+    const double sms = sm_count(), nt = static_cast<double>(n_tiles), kb = static_cast<double>(k_blocks);
+    const double single_tile = std::max(0.405 * kb, 2.7), pair_tile = std::max(0.326 * kb, 3.15);
+    const double weights = touched * group_weight_bytes * 1e-6 / 7.7;
+    const double t1 = std::max(std::ceil(singles * nt / sms) * single_tile, weights);
+    const double t2 = std::max(std::ceil(pairs * nt / (sms / 2)) * pair_tile, weights) + 2.5;
+    const double t3 =
+        std::max(std::ceil(whole * nt / (sms / 2)) * pair_tile + leftover * nt / sms * single_tile * 0.55, weights) + 20.0;
+    return t1 <= t2 && t1 <= t3 ? 1 : (t2 <= t3 ? 2 : GEMM_SHAPE_HYBRID);
 }
 
 // ---------------------------------------------------------------------------
@@ -601,10 +650,12 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
                        bool b_mn, const void* a, const CUtensorMap& tb, GemmParams p, cudaStream_t st,
                        void* clear = nullptr, size_t clear_bytes = 0)
 {
-    const int shape = choose_cta_group(M, true);
-    // (Rows stored one by one at caller-given addresses, possibly in peer memory, use the same shapes.  Single
-    // tiles for them once measured faster on two GPUs; with the present kernels the chain steps are 13.26 against
-    // 13.25 - 13.5 ms on two GPUs, 7.62 against 7.73 - 7.83 ms on four and 26.4 against 28.0 ms on one.)
+    constexpr int64_t ELEM = (KIND == KIND_I8) ? 1 : 2;
+    const bool split = p.k_blocks_per_term != 0;
+    const int64_t a_cols = split ? SPLIT_PIECES * p.K : p.K;
+    const int64_t group_bytes = p.N * p.K * ELEM * (split ? SPLIT_TERMS : 1);  // of weights, as the kernel streams them
+    const int shape = choose_grouped_shape(list_on_device ? nullptr : group_list, E, M, p.n_tiles, p.num_k_blocks,
+                                           static_cast<double>(group_bytes));
     p.error = &g.header->error;
     // Rows per A load.  Pairs take whole tiles.  A single CTA's tile holds at most 128 rows of one group and often far
     // fewer - what a group leaves over, or a whole group of a small batch.  Where there are 256 MB of weights to stream
@@ -616,12 +667,8 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
     // Calls that the cap does not bound gain little - 64 experts of 4096 x 4096, 4 - 64 rows each: 152.8 - 182.8 us,
     // 153.7 - 184 with whole tiles - the same with boxes of 16 and of 32, and nothing from 96 rows per expert on, which
     // is where the rule ends; at 12 rows per expert most tiles still fit into one box of 16.
-    constexpr int64_t ELEM = (KIND == KIND_I8) ? 1 : 2;
-    const bool split = p.k_blocks_per_term != 0;
-    const int64_t a_cols = split ? SPLIT_PIECES * p.K : p.K;
-    const int64_t terms = split ? SPLIT_TERMS : 1;
     int box_rows = (shape == GEMM_SHAPE_HYBRID) ? 32 : (M <= 12 * E ? 16 : (M <= 96 * E ? 32 : GEMM_BLOCK_M));
-    if (shape == 2 || E * p.N * p.K * terms * ELEM < (int64_t(256) << 20)) {
+    if (shape == 2 || E * group_bytes < (int64_t(256) << 20)) {
         box_rows = GEMM_BLOCK_M;
     }
     const bool row_boxes = box_rows < GEMM_BLOCK_M;
@@ -666,7 +713,14 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
     p.tile_done = g.tile_done;
     // (with a table of its own the second launch would read what the planner wrote: it waits)
     const bool overlap = hybrid && E <= GROUPS_IN_CTA;
-    p.order = overlap ? ORDER_FIRST_OF_TWO : ORDER_ALONE;
+    // The SwiGLU form on single CTAs, with enough weights to be long, starts on an idle chip: launched beside the kernel
+    // before, its CTAs come to lie on the SMs as those fall free, and neighbouring column tiles no longer on the two SMs of a
+    // TPC, which share what they fetch.  9328 rows of 128 experts of 4784 x 2752 326 us (413 overlapped), 2296 of 128 of
+    // 2464 x 3360 196 (231), 20000 of 64 of 4096 x 2048 237 (244), 3000 of 32 of 7168 x 4096 201 (199); shorter calls lose
+    // the 2 us of the overlap (600 rows of 32 experts of 4096 x 2912, 381 MB: 80.7, 79.0).  The other epilogue, whose tiles
+    // are 256 contiguous columns, shows no difference.
+    const bool plain = EPI == EPI_GMSQ && shape == 1 && E * group_bytes >= int64_t(400000000);
+    p.order = overlap ? ORDER_FIRST_OF_TWO : (plain ? ORDER_PLAIN : ORDER_ALONE);
     const int64_t most = (hybrid ? M / 256 + E + 1 : g.max_tiles) * p.n_tiles;
     cudaError_t e = (!hybrid && row_boxes) ? dispatch_row_boxes<KIND, EPI>(b_mn, ta, tb, p, most, st, groups)
                                            : dispatch_gemm<KIND, EPI>(hybrid ? 2 : shape, 256, b_mn, ta, tb, p, most, st, groups);
@@ -804,7 +858,7 @@ static int quant_matmul_impl(const int8_t* x1, const int8_t* x2, const void* sca
         }
         return launch_status(e);
     }
-    const int cg = (own_choice && tiles128 <= sm_count()) ? 1 : choose_cta_group(M, false);
+    const int cg = (own_choice && tiles128 <= sm_count()) ? 1 : choose_cta_group(M);
     const int tile_m = 128 * cg;
     p.m_tiles_per_batch = static_cast<int32_t>((M + tile_m - 1) / tile_m);
     // narrow tiles when wide ones would leave most SMs idle (single-CTA tiles only)

@@ -240,6 +240,7 @@ __device__ __forceinline__ TileEntry tile_in_cta(const GroupList& list, const in
 constexpr int ORDER_ALONE = 0;
 constexpr int ORDER_FIRST_OF_TWO = 1;
 constexpr int ORDER_SECOND_OF_TWO = 2;
+constexpr int ORDER_PLAIN = 3;  // not launched beside the kernel before (see run_grouped)
 
 struct GemmParams {
     int64_t M;  // rows per batch (dense) or total rows (grouped)
@@ -1048,8 +1049,7 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
         after_previous<false>();  // the second one starts only when everything before this kernel is complete
     } else if (p.order == ORDER_SECOND_OF_TWO) {
         // reads nothing that the first one writes, and writes other rows: it waits for it only before it ends
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-        __threadfence();  // no line that this SM's L1 holds from before
+        beside_previous();
     } else {
         after_previous();
     }
@@ -1465,7 +1465,7 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
 
     // ---- teardown ----
     if (p.order == ORDER_SECOND_OF_TWO) {
-        asm volatile("griddepcontrol.wait;" ::: "memory");  // whoever waits for this kernel waits for the first one too
+        previous_complete();
     }
     tc::tc_fence_before_sync();
     __syncthreads();
