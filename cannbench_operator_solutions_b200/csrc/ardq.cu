@@ -27,12 +27,12 @@ template <int DT, int CPT, bool VEC, bool DIRECT>
 __global__ void __launch_bounds__(ARDQ_THREADS)
     ardq_rows_kernel(const uint16_t* x1, const uint16_t* x2,
                      const uint16_t* gamma, int8_t* __restrict__ y, uint16_t* __restrict__ x_out,
-                     float* __restrict__ scale_out, int64_t rows, int64_t N, float eps, float inv_n)
+                     float* __restrict__ scale_out, int64_t rows, int64_t N, float eps, float inv_n, bool beside)
 {
     constexpr int WARPS = ARDQ_THREADS / 32;
     __shared__ float s_sum[2][WARPS];
     __shared__ uint32_t s_max[2][WARPS];
-    const int64_t zero = after_previous();
+    const int64_t zero = beside ? beside_previous() : after_previous();
     const int tid = threadIdx.x;
     const int nchunks = static_cast<int>((N + 7) / 8);
     int parity = 0;
@@ -144,11 +144,14 @@ __global__ void __launch_bounds__(ARDQ_THREADS)
             }
         }
     }
+    if (beside) {
+        previous_complete();
+    }
 }
 
 template <int DT, int CPT, bool VEC, bool DIRECT>
 static cudaError_t launch(const void* x1, const void* x2, const void* gamma, int8_t* y, void* x_out, float* scale_out,
-                          int64_t rows, int64_t N, float eps, cudaStream_t st)
+                          int64_t rows, int64_t N, float eps, bool beside, cudaStream_t st)
 {
     auto kern = ardq_rows_kernel<DT, CPT, VEC, DIRECT>;
     int per_sm = 1;
@@ -162,44 +165,41 @@ static cudaError_t launch(const void* x1, const void* x2, const void* gamma, int
     const float inv_n = 1.0f / static_cast<float>(N);
     return launch_chained(kern, grid, ARDQ_THREADS, 0, st, static_cast<const uint16_t*>(x1),
                           static_cast<const uint16_t*>(x2), static_cast<const uint16_t*>(gamma), y,
-                          static_cast<uint16_t*>(x_out), scale_out, rows, N, eps, inv_n);
+                          static_cast<uint16_t*>(x_out), scale_out, rows, N, eps, inv_n, beside);
 }
 
 template <int DT, bool VEC, bool DIRECT>
 static cudaError_t dispatch_cpt(const void* x1, const void* x2, const void* gamma, int8_t* y, void* x_out,
-                                float* scale_out, int64_t rows, int64_t N, float eps, cudaStream_t st)
+                                float* scale_out, int64_t rows, int64_t N, float eps, bool beside, cudaStream_t st)
 {
     const int64_t chunks = (N + 7) / 8;
     if (chunks <= 256) {
-        return launch<DT, 1, VEC, DIRECT>(x1, x2, gamma, y, x_out, scale_out, rows, N, eps, st);
+        return launch<DT, 1, VEC, DIRECT>(x1, x2, gamma, y, x_out, scale_out, rows, N, eps, beside, st);
     }
     if (chunks <= 512) {
-        return launch<DT, 2, VEC, DIRECT>(x1, x2, gamma, y, x_out, scale_out, rows, N, eps, st);
+        return launch<DT, 2, VEC, DIRECT>(x1, x2, gamma, y, x_out, scale_out, rows, N, eps, beside, st);
     }
     if (chunks <= 1024) {
-        return launch<DT, 4, VEC, DIRECT>(x1, x2, gamma, y, x_out, scale_out, rows, N, eps, st);
+        return launch<DT, 4, VEC, DIRECT>(x1, x2, gamma, y, x_out, scale_out, rows, N, eps, beside, st);
     }
-    return launch<DT, 8, VEC, DIRECT>(x1, x2, gamma, y, x_out, scale_out, rows, N, eps, st);
+    return launch<DT, 8, VEC, DIRECT>(x1, x2, gamma, y, x_out, scale_out, rows, N, eps, beside, st);
 }
 
 template <int DT>
 static cudaError_t dispatch(const void* x1, const void* x2, const void* gamma, int8_t* y, void* x_out,
                             float* scale_out, int64_t rows, int64_t N, float eps, bool vec, bool direct,
-                            cudaStream_t st)
+                            bool beside, cudaStream_t st)
 {
     if (vec) {
-        return direct ? dispatch_cpt<DT, true, true>(x1, x2, gamma, y, x_out, scale_out, rows, N, eps, st)
-                      : dispatch_cpt<DT, true, false>(x1, x2, gamma, y, x_out, scale_out, rows, N, eps, st);
+        return direct ? dispatch_cpt<DT, true, true>(x1, x2, gamma, y, x_out, scale_out, rows, N, eps, beside, st)
+                      : dispatch_cpt<DT, true, false>(x1, x2, gamma, y, x_out, scale_out, rows, N, eps, beside, st);
     }
-    return direct ? dispatch_cpt<DT, false, true>(x1, x2, gamma, y, x_out, scale_out, rows, N, eps, st)
-                  : dispatch_cpt<DT, false, false>(x1, x2, gamma, y, x_out, scale_out, rows, N, eps, st);
+    return direct ? dispatch_cpt<DT, false, true>(x1, x2, gamma, y, x_out, scale_out, rows, N, eps, beside, st)
+                  : dispatch_cpt<DT, false, false>(x1, x2, gamma, y, x_out, scale_out, rows, N, eps, beside, st);
 }
 
-}  // namespace w8a8
-
-extern "C" int w8a8_add_rms_norm_dynamic_quant(const void* x1, const void* x2, const void* gamma, int8_t* y,
-                                               void* x_out, float* scale_out, int64_t rows, int64_t N, float epsilon,
-                                               int dtype, int flags, void* stream)
+static int ardq(const void* x1, const void* x2, const void* gamma, int8_t* y, void* x_out, float* scale_out, int64_t rows,
+                int64_t N, float epsilon, int dtype, int flags, bool beside, void* stream)
 {
     if (dtype != W8A8_DT_F16 && dtype != W8A8_DT_BF16) {
         return W8A8_ERR_INVALID;
@@ -216,17 +216,32 @@ extern "C" int w8a8_add_rms_norm_dynamic_quant(const void* x1, const void* x2, c
         scale_out == nullptr) {
         return W8A8_ERR_INVALID;
     }
-    if (!w8a8::is_aligned(x1, 2) || !w8a8::is_aligned(x2, 2) || !w8a8::is_aligned(gamma, 2) ||
-        !w8a8::is_aligned(x_out, 2) || !w8a8::is_aligned(scale_out, 4)) {
+    if (!is_aligned(x1, 2) || !is_aligned(x2, 2) || !is_aligned(gamma, 2) ||
+        !is_aligned(x_out, 2) || !is_aligned(scale_out, 4)) {
         return W8A8_ERR_ALIGN;
     }
-    const bool vec = (N % 8 == 0) && w8a8::is_aligned(x1, 16) && w8a8::is_aligned(x2, 16) &&
-                     w8a8::is_aligned(gamma, 16) && w8a8::is_aligned(x_out, 16) && w8a8::is_aligned(y, 8);
+    const bool vec = (N % 8 == 0) && is_aligned(x1, 16) && is_aligned(x2, 16) &&
+                     is_aligned(gamma, 16) && is_aligned(x_out, 16) && is_aligned(y, 8);
     const bool direct = (flags & W8A8_F_ROUND_DIRECT) != 0;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const cudaError_t e =
         (dtype == W8A8_DT_BF16)
-            ? w8a8::dispatch<W8A8_DT_BF16>(x1, x2, gamma, y, x_out, scale_out, rows, N, epsilon, vec, direct, st)
-            : w8a8::dispatch<W8A8_DT_F16>(x1, x2, gamma, y, x_out, scale_out, rows, N, epsilon, vec, direct, st);
-    return w8a8::launch_status(e);
+            ? dispatch<W8A8_DT_BF16>(x1, x2, gamma, y, x_out, scale_out, rows, N, epsilon, vec, direct, beside, st)
+            : dispatch<W8A8_DT_F16>(x1, x2, gamma, y, x_out, scale_out, rows, N, epsilon, vec, direct, beside, st);
+    return launch_status(e);
+}
+
+int add_rms_norm_dynamic_quant_beside(const void* x1, const void* x2, const void* gamma, int8_t* y, void* x_out,
+                                      float* scale_out, int64_t rows, int64_t N, float epsilon, int dtype, void* stream)
+{
+    return ardq(x1, x2, gamma, y, x_out, scale_out, rows, N, epsilon, dtype, 0, true, stream);
+}
+
+}  // namespace w8a8
+
+extern "C" int w8a8_add_rms_norm_dynamic_quant(const void* x1, const void* x2, const void* gamma, int8_t* y,
+                                               void* x_out, float* scale_out, int64_t rows, int64_t N, float epsilon,
+                                               int dtype, int flags, void* stream)
+{
+    return w8a8::ardq(x1, x2, gamma, y, x_out, scale_out, rows, N, epsilon, dtype, flags, false, stream);
 }

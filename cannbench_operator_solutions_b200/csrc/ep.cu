@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(RP_THREADS) rp_rank_kernel(const int32_t* expe
                                                              int64_t* count, int64_t* __restrict__ cumsum,
                                                              int64_t* __restrict__ expanded_pos)
 {
-    const int64_t zero = after_previous();
+    const int64_t zero = after_previous<false>();  // the next kernel may be one that does not wait for this one
     constexpr int ITS = RP_PAIRS / RP_THREADS;
     constexpr int PER = RP_MAX_EXPERTS / RP_THREADS;  // experts per thread in the scan
     __shared__ int64_t s_next[RP_MAX_EXPERTS];        // where the next pair of each expert goes
@@ -396,6 +396,7 @@ __global__ void __launch_bounds__(256) permute_rows_kernel(const uint8_t* src,
 // peer.  row_dst[e] / scale_dst[e] point at the first row / scale this rank may write for expert e in the
 // owner's buffer, my_base[e] is the position of this rank's first pair for expert e in its own expert-major
 // order, pos[i, k] that pair's position: destination row = row_dst[e] + (pos - my_base[e]) rows.
+// Without row_dst all of them are rows of one buffer, at their positions: destination row = base_row + pos rows.
 // This replaces pack + all-to-all + regroup with one pass; the row is read once and stored topk times.
 template <bool VEC>
 __global__ void __launch_bounds__(256) dispatch_rows_kernel(const uint8_t* src,
@@ -404,7 +405,8 @@ __global__ void __launch_bounds__(256) dispatch_rows_kernel(const uint8_t* src,
                                                             const int64_t* pos,
                                                             const uint64_t* row_dst,
                                                             const uint64_t* scale_dst,
-                                                            const int64_t* my_base, int64_t T, int topk,
+                                                            const int64_t* my_base, uint8_t* base_row,
+                                                            float* base_scale, int64_t T, int topk,
                                                             int64_t row_bytes)
 {
     const int64_t zero = after_previous();
@@ -413,10 +415,14 @@ __global__ void __launch_bounds__(256) dispatch_rows_kernel(const uint8_t* src,
         __syncthreads();
         if (static_cast<int>(threadIdx.x) < topk) {
             const int64_t pr = i * topk + threadIdx.x;
-            const int32_t e = expert_idx[pr];
             const int64_t p = pos[pr];
             uint64_t d = 0;
-            if (p >= 0 && row_dst[e] != 0) {  // a zero destination: the table builder found the buffers too small
+            if (row_dst == nullptr) {
+                if (p >= 0) {
+                    d = reinterpret_cast<uint64_t>(base_row + p * row_bytes);
+                    base_scale[p] = src_scale[i];
+                }
+            } else if (const int32_t e = expert_idx[pr]; p >= 0 && row_dst[e] != 0) {  // a zero destination: the table builder found the buffers too small
                 const int64_t off = p - my_base[e];
                 d = row_dst[e] + static_cast<uint64_t>(off) * static_cast<uint64_t>(row_bytes);
                 if (src_scale != nullptr) {
@@ -1234,14 +1240,29 @@ extern "C" int w8a8_dispatch_rows(const void* src, const float* src_scale, const
     const unsigned grid = static_cast<unsigned>(T < cap ? T : cap);
     if (vec) {
         w8a8::launch_chained(w8a8::dispatch_rows_kernel<true>, grid, 256, 0, st, static_cast<const uint8_t*>(src),
-                             src_scale, expert_idx, expanded_pos, row_dst, scale_dst, my_base, T,
+                             src_scale, expert_idx, expanded_pos, row_dst, scale_dst, my_base, nullptr, nullptr, T,
                              static_cast<int>(topk), row_bytes);
     } else {
         w8a8::launch_chained(w8a8::dispatch_rows_kernel<false>, grid, 256, 0, st, static_cast<const uint8_t*>(src),
-                             src_scale, expert_idx, expanded_pos, row_dst, scale_dst, my_base, T,
+                             src_scale, expert_idx, expanded_pos, row_dst, scale_dst, my_base, nullptr, nullptr, T,
                              static_cast<int>(topk), row_bytes);
     }
     return (cudaGetLastError() == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
+}
+
+int w8a8::dispatch_rows_local(const void* src, const float* src_scale, const int64_t* expanded_pos, void* dst,
+                              float* dst_scale, int64_t T, int64_t topk, int64_t row_bytes, void* stream)
+{
+    if (topk > 64) {
+        return W8A8_ERR_INVALID;
+    }
+    const bool vec = (row_bytes % 16 == 0) && is_aligned(src, 16) && is_aligned(dst, 16);
+    const int64_t cap = static_cast<int64_t>(sm_count()) * 8;
+    const unsigned grid = static_cast<unsigned>(T < cap ? T : cap);
+    return launch_status(launch_chained(vec ? dispatch_rows_kernel<true> : dispatch_rows_kernel<false>, grid, 256, 0,
+                                        static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(src), src_scale, nullptr,
+                                        expanded_pos, nullptr, nullptr, nullptr, static_cast<uint8_t*>(dst), dst_scale, T,
+                                        static_cast<int>(topk), row_bytes));
 }
 
 extern "C" int w8a8_expand_row_pointers(const int64_t* seg_first, const uint64_t* seg_ptr, int64_t nseg, int64_t rows,

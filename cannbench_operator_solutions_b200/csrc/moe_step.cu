@@ -253,6 +253,42 @@ static SideStream* side_stream()
     return &s;
 }
 
+// One rank, and room for all of its rows: expert-major positions are rows of its own buffers, so there are no address
+// tables, no overflow to find and no output addresses to expand, and the matmuls take the rows there are instead of the
+// buffers' capacity.  Everything is one chain of overlapping kernels on the caller's stream; the normalisation runs beside
+// the route plan, which it has nothing to do with, as the second stream had it.
+static int one_rank_step(const W8A8MoeFfnStep* s, const StepBuffers& b, const void* x, const void* residual, const void* gamma,
+                         float epsilon, const int32_t* expert_idx, const float* probs, void* out, void* x_out,
+                         cudaStream_t st)
+{
+    const int64_t T = s->tokens, topk = s->topk, hidden = s->hidden, inter = s->inter, E = s->num_experts;
+    const int64_t rows = T * topk;
+    uint8_t* local = static_cast<uint8_t*>(s->local_base);
+    int8_t* xe = reinterpret_cast<int8_t*>(local + s->off_x);
+    float* xe_scale = reinterpret_cast<float*>(local + s->off_s);
+    void* back = local + s->off_back;
+    int rc = w8a8_route_plan(expert_idx, T, topk, E, b.count, b.cumsum, b.pos, b.plan_ws, b.plan_ws_bytes, st);
+    if (rc == W8A8_OK) {
+        rc = add_rms_norm_dynamic_quant_beside(x, residual, gamma, b.xq, x_out, b.xs, T, hidden, epsilon, s->dtype, st);
+    }
+    if (rc == W8A8_OK) {
+        rc = dispatch_rows_local(b.xq, b.xs, b.pos, xe, xe_scale, T, topk, hidden, st);
+    }
+    // pairs without a valid expert have no row: the list may end before the rows do
+    if (rc == W8A8_OK) {
+        rc = w8a8_grouped_matmul_swiglu_quant(xe, s->w_up, s->s_up, xe_scale, b.h, b.hs, rows, hidden, 2 * inter, E, b.cumsum,
+                                              2, W8A8_W_KN, 0, b.mm_ws, b.mm_ws_bytes, st);
+    }
+    if (rc == W8A8_OK) {
+        rc = w8a8_grouped_matmul(b.h, s->w_down, nullptr, back, b.hs, s->s_down, rows, hidden, inter, E, b.cumsum, 2,
+                                 W8A8_DT_I8, W8A8_DT_F32, s->dtype, W8A8_W_KN, b.mm_ws, b.mm_ws_bytes, st);
+    }
+    if (rc == W8A8_OK) {
+        rc = w8a8_combine(back, probs, b.pos, out, T, topk, hidden, s->dtype, st);
+    }
+    return rc;
+}
+
 extern "C" int w8a8_moe_ffn_step(const W8A8MoeFfnStep* s, const void* x, const void* residual, const void* gamma,
                                  float epsilon, const int32_t* expert_idx, const float* probs, void* out, void* x_out,
                                  void* stream)
@@ -290,6 +326,10 @@ extern "C" int w8a8_moe_ffn_step(const W8A8MoeFfnStep* s, const void* x, const v
     int8_t* xe = reinterpret_cast<int8_t*>(local + s->off_x);
     float* xe_scale = reinterpret_cast<float*>(local + s->off_s);
     void* back = local + s->off_back;
+
+    if (P == 1 && T * topk <= cap) {
+        return one_rank_step(s, b, x, residual, gamma, epsilon, expert_idx, probs, out, x_out, st);
+    }
 
     SideStream* side = side_stream();
     if (side == nullptr) {
