@@ -158,18 +158,41 @@ static cudaError_t dispatch_gemm(int cta_group, int block_n, bool b_mn, const CU
                         : launch_gemm<1, 256, KIND, EPI, false, 16>(ta, tb, p, max_tiles, st, groups);
         }
     }
-    if (cta_group == 2) {
-        return b_mn ? launch_gemm<2, 256, KIND, EPI, true>(ta, tb, p, max_tiles, st, groups)
-                    : launch_gemm<2, 256, KIND, EPI, false>(ta, tb, p, max_tiles, st, groups);
-    }
-    if constexpr (EPI != EPI_GMSQ) {
-        if (block_n == 128) {
-            return b_mn ? launch_gemm<1, 128, KIND, EPI, true>(ta, tb, p, max_tiles, st, groups)
-                        : launch_gemm<1, 128, KIND, EPI, false>(ta, tb, p, max_tiles, st, groups);
+    // Sixteen warps for the int8 operators' 16-bit results: eight, at two per scheduler, take 6 us for a 128 x 256 tile, as
+    // long as the main loop of K = 2048 (8192 x 512 x 4096 with bias 43 us, 60 with eight; 4096 x 1024 x 8192 48.8, 50.4;
+    // 1000 x 2048 x 4096 16.1, 17.2; expert layer of 2000 x 8 rows over 64 experts of 2688 x 1008 295, 303).  16-bit operands,
+    // with nothing to convert or scale, are no faster (16000 rows of 8 experts of 512 x 4096 89.4, 88.3), and rows stored
+    // at addresses of their own, which may be another GPU's, leave eight warps in whole lines.
+    if constexpr (EPI == EPI_QMM || (EPI == EPI_GMM && KIND == KIND_I8)) {
+        if (EPI == EPI_QMM || p.out_row_ptrs == nullptr) {
+            if (cta_group == 2) {
+                return b_mn ? launch_gemm<2, 256, KIND, EPI, true, 16>(ta, tb, p, max_tiles, st, groups)
+                            : launch_gemm<2, 256, KIND, EPI, false, 16>(ta, tb, p, max_tiles, st, groups);
+            }
+            if constexpr (EPI == EPI_QMM) {
+                if (block_n == 128) {
+                    return b_mn ? launch_gemm<1, 128, KIND, EPI, true, 16>(ta, tb, p, max_tiles, st)
+                                : launch_gemm<1, 128, KIND, EPI, false, 16>(ta, tb, p, max_tiles, st);
+                }
+            }
+            return b_mn ? launch_gemm<1, 256, KIND, EPI, true, 16>(ta, tb, p, max_tiles, st, groups)
+                        : launch_gemm<1, 256, KIND, EPI, false, 16>(ta, tb, p, max_tiles, st, groups);
         }
     }
-    return b_mn ? launch_gemm<1, 256, KIND, EPI, true>(ta, tb, p, max_tiles, st, groups)
-                : launch_gemm<1, 256, KIND, EPI, false>(ta, tb, p, max_tiles, st, groups);
+    if constexpr (EPI != EPI_QMM) {
+        if (cta_group == 2) {
+            return b_mn ? launch_gemm<2, 256, KIND, EPI, true>(ta, tb, p, max_tiles, st, groups)
+                        : launch_gemm<2, 256, KIND, EPI, false>(ta, tb, p, max_tiles, st, groups);
+        }
+        if constexpr (EPI == EPI_RAW) {
+            if (block_n == 128) {
+                return b_mn ? launch_gemm<1, 128, KIND, EPI, true>(ta, tb, p, max_tiles, st)
+                            : launch_gemm<1, 128, KIND, EPI, false>(ta, tb, p, max_tiles, st);
+            }
+        }
+        return b_mn ? launch_gemm<1, 256, KIND, EPI, true>(ta, tb, p, max_tiles, st, groups)
+                    : launch_gemm<1, 256, KIND, EPI, false>(ta, tb, p, max_tiles, st, groups);
+    }
 }
 
 // Single-CTA tiles of a grouped problem that load their own rows only (see run_grouped).
@@ -179,6 +202,12 @@ static cudaError_t dispatch_row_boxes(bool b_mn, const CUtensorMap& ta, const CU
 {
     if constexpr (EPI == EPI_GMSQ) {
         if (g_gmsq_epilogue_warps.load(std::memory_order_relaxed) == 16) {
+            return b_mn ? launch_gemm<1, 256, KIND, EPI, true, 16, false, true>(ta, tb, p, max_tiles, st, groups)
+                        : launch_gemm<1, 256, KIND, EPI, false, 16, false, true>(ta, tb, p, max_tiles, st, groups);
+        }
+    }
+    if constexpr (EPI == EPI_GMM && KIND == KIND_I8) {
+        if (p.out_row_ptrs == nullptr) {
             return b_mn ? launch_gemm<1, 256, KIND, EPI, true, 16, false, true>(ta, tb, p, max_tiles, st, groups)
                         : launch_gemm<1, 256, KIND, EPI, false, 16, false, true>(ta, tb, p, max_tiles, st, groups);
         }

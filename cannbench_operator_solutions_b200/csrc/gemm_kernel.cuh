@@ -1,6 +1,6 @@
 // Persistent, warp-specialised tcgen05 GEMM for sm_100a with fused epilogues.
 //
-// One CTA per SM, 320 threads (576 with the SwiGLU epilogue's sixteen epilogue warps):
+// One CTA per SM, 320 threads (576 with sixteen epilogue warps):
 //   warp 0      TMA producer: fills a ring of shared-memory stages (128-byte
 //               swizzle) with A and B tiles, one mbarrier per stage.
 //   warp 1      MMA issuer: the warp walks the loop and waits together, an elected
@@ -11,11 +11,11 @@
 //               lanes its index modulo 4 selects; two warps share each lane
 //               quarter and split the columns), apply the operator's dequant
 //               chain, store.  Double-buffered TMEM lets the epilogue of tile i
-//               overlap the main loop of tile i+1.  The SwiGLU epilogue (an
-//               exponential and a correctly rounded quotient per element, two
-//               elements at a time) runs on warps 2-17, four per lane quarter:
-//               with eight warps and scalar arithmetic it took as long per tile
-//               as the main loop.
+//               overlap the main loop of tile i+1.  The epilogues that work on
+//               every element - SwiGLU with its exponential and correctly
+//               rounded quotient, the dequantisation of int8 products - run on
+//               warps 2-17, four per lane quarter: eight take as long per tile
+//               as the main loop, all of it where K is short.
 //
 // Two shapes of the same kernel (template parameter CG):
 //   CG = 1  one CTA per tile of 128 rows x BLOCK_N columns, 4 stages of
@@ -49,8 +49,7 @@
 
 namespace w8a8 {
 
-// producer warp, MMA warp and the epilogue warps (8, or 16 for the SwiGLU epilogue, whose exponential and quotient per
-// element kept eight warps busy for as long as the MMA warp needs for the tile)
+// producer warp, MMA warp and the epilogue warps (8 or 16)
 __host__ __device__ constexpr int gemm_threads(int epi_warps) { return 64 + 32 * epi_warps; }
 constexpr int GEMM_EPI_PATCH_BYTES = 8 * 4096;  // shared by the epilogue warps: 4 KB each for 8, 2 KB each for 16
 constexpr int GEMM_BLOCK_M = 128;
@@ -588,17 +587,230 @@ __device__ __forceinline__ void touch_epilogue_operands(const GemmParams& p, con
     }
 }
 
-// The work of one epilogue thread on one tile: row `row_in_tile` of this CTA's
-// accumulator, columns [col_half * BLOCK_N/2, (col_half+1) * BLOCK_N/2).
-template <int BLOCK_N, int KIND, int EPI, int EPI_WARPS>
-__device__ __forceinline__ void epilogue_tile(const GemmParams& p, const TileInfo& tl, uint32_t t_addr,
-                                              int row_in_tile, int col_half, int64_t H, bool no_epilogue,
-                                              uint4* stage)
+// Eight columns of a row in the form that most calls have - per-channel fp32 scales `w` (int8 operands), one factor per
+// row, a per-channel float bias or none - as four words of two 16-bit results.  The order and rounding of qmm_dequant; the
+// factors are multiplied two at a time, the bias is added one by one (see mul2).  `b16`: eight values of a 16-bit bias;
+// `b32`: where an fp32 one is.
+template <int KIND>
+__device__ __forceinline__ uint4 dequant8(const uint32_t* r, const f32x2* w, float row_mul, int bias_kind, uint4 b16,
+                                          const void* b32, bool bf16_out)
 {
-    const bool row_ok = (row_in_tile < tl.m_rows) && !no_epilogue;
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if constexpr (KIND == KIND_I8) {
+            const f32x2 a = pair(static_cast<float>(static_cast<int32_t>(r[2 * j])),
+                                 static_cast<float>(static_cast<int32_t>(r[2 * j + 1])));
+            unpair(mul2(mul2(a, w[j]), pair(row_mul)), v[2 * j], v[2 * j + 1]);
+        } else {
+            v[2 * j] = __uint_as_float(r[2 * j]);
+            v[2 * j + 1] = __uint_as_float(r[2 * j + 1]);
+        }
+    }
+    if (bias_kind != W8A8_QM_BIAS_NONE) {
+        float b[8];
+        if (bias_kind == W8A8_QM_BIAS_F32) {
+            load_vec<8>(b32, 0, W8A8_QM_BIAS_F32, true, 8, b);
+        } else {
+            const uint32_t word[4] = {b16.x, b16.y, b16.z, b16.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (bias_kind == W8A8_QM_BIAS_BF16) {
+                    unpack2<W8A8_DT_BF16>(word[j], b[2 * j], b[2 * j + 1]);
+                } else {
+                    unpack2<W8A8_DT_F16>(word[j], b[2 * j], b[2 * j + 1]);
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            v[j] = __fadd_rn(v[j], b[j]);
+        }
+    }
+    return bf16_out ? make_uint4(pack2<W8A8_DT_BF16>(v[0], v[1]), pack2<W8A8_DT_BF16>(v[2], v[3]),
+                                 pack2<W8A8_DT_BF16>(v[4], v[5]), pack2<W8A8_DT_BF16>(v[6], v[7]))
+                    : make_uint4(pack2<W8A8_DT_F16>(v[0], v[1]), pack2<W8A8_DT_F16>(v[2], v[3]),
+                                 pack2<W8A8_DT_F16>(v[4], v[5]), pack2<W8A8_DT_F16>(v[6], v[7]));
+}
+
+// The 16-bit epilogue of one thread on one tile: row `row_in_tile` of this CTA's accumulator, the `share`-th of
+// EPI_WARPS / 4 equal shares of its columns.
+// A chunk of results is 32 or 64 bytes of this thread's row.  They are not stored from here (every lane would write
+// 16-byte pieces of a different row): the warp parks two chunks, 64 or 128 bytes per row, in its private shared-memory
+// patch and then writes them as whole row segments, 4 or 8 lanes per row.  (Rows whose home is another GPU take eight
+// warps: NVLink carries full 128-byte lines, not fragments.)
+// Bound: its warps' latency, where K is short.  What a chunk is multiplied with is requested ahead of the wait for it, and
+// all that does not need the accumulator is done before the wait for that: 128 x 1024 x 1024 with its quantisation 6.8 us
+// (7.2 with eight warps and everything behind the waits; 5.1 without any epilogue), 8192 x 512 x 4096 40.8 (46.5; 18.5).
+template <int BLOCK_N, int KIND, int EPI, int EPI_WARPS, typename Wait>
+__device__ __forceinline__ bool epilogue_16bit(const GemmParams& p, const TileInfo& tl, uint32_t t_addr, int row_in_tile,
+                                               int share, uint4* stage, Wait accumulator_ready)
+{
+    constexpr int COLS = BLOCK_N / (EPI_WARPS / 4);  // of this warp
+    constexpr int CH = (EPI_WARPS == 16) ? 16 : 32;  // columns of a chunk
+    constexpr int PIECES = CH / 4;                   // 16-byte pieces of a row in the patch (two chunks)
+    constexpr int COPY_ROWS = 32 / PIECES;           // rows per instruction of the copy out
+    static_assert(COLS % (2 * CH) == 0, "whole patches");
+    const int lane = row_in_tile & 31, first_row = row_in_tile & ~31;
+    const bool row_ok = row_in_tile < tl.m_rows;
+    const int64_t row = static_cast<int64_t>(tl.a_row0) + row_in_tile;
+    const int64_t col_first = static_cast<int64_t>(tl.nt) * BLOCK_N + share * COLS;
+    if (first_row >= tl.m_rows || col_first >= p.N) {
+        return accumulator_ready();  // a whole warp without results
+    }
+    [[maybe_unused]] QmmTerms terms;
+    const float* scale = static_cast<const float*>(p.scale);
+    const uint8_t* bias = static_cast<const uint8_t*>(p.bias);
+    float row_mul = 1.0f;
+    int bias_kind = W8A8_QM_BIAS_NONE;
+    bool plain = true;
+    if constexpr (EPI == EPI_QMM) {
+        terms = qmm_terms(p, tl.group, row, row_ok);
+        row_mul = terms.row_mul;
+        bias = static_cast<const uint8_t*>(terms.bias);
+        bias_kind = terms.bias_kind;
+        plain = terms.scale_perchan && !terms.scale_bf16 && !terms.has_offset && bias_kind != W8A8_QM_BIAS_I32 &&
+                (bias_kind == W8A8_QM_BIAS_NONE || terms.bias_perchan);
+    } else {
+        scale += static_cast<int64_t>(tl.group) * p.N;
+        if constexpr (KIND == KIND_I8) {
+            row_mul = row_ok ? p.row_scale[row] : 0.0f;
+        }
+        if (p.flags & 4) {
+            const int bdt = static_cast<int>(p.flags & 3);
+            bias_kind = (bdt == W8A8_DT_F16) ? W8A8_QM_BIAS_F16 : (bdt == W8A8_DT_BF16 ? W8A8_QM_BIAS_BF16 : W8A8_QM_BIAS_F32);
+            bias += static_cast<int64_t>(tl.group) * p.N * (bias_kind == W8A8_QM_BIAS_F32 ? 4 : 2);
+        }
+    }
+    const bool bias16 = bias_kind == W8A8_QM_BIAS_F16 || bias_kind == W8A8_QM_BIAS_BF16;
+    const bool bf16_out = p.out_dtype == W8A8_DT_BF16;
+    // where this lane's pieces of the copy out go: row first_row + COPY_ROWS * it + lane / PIECES, piece lane % PIECES
+    const int piece = lane % PIECES, copy_row = lane / PIECES;
+    const bool addressed = EPI == EPI_GMM && EPI_WARPS == 8 && p.out_row_ptrs != nullptr;
+    uint64_t row_ptr = 0;  // addressed: of this thread's own row, else of the first row that it copies
+    if (addressed) {
+        // the row's home may be another GPU's memory: plain peer stores over NVLink
+        row_ptr = row_ok ? p.out_row_ptrs[row] : 0;
+    } else {
+        row_ptr = reinterpret_cast<uint64_t>(p.out) +
+                  static_cast<uint64_t>(static_cast<int64_t>(tl.a_row0) + first_row + copy_row) * p.N * 2;
+    }
+    // the place of row `r`'s piece `q` in the patch: permuted by the row so that the eight lanes of a store or load phase
+    // hit eight different bank groups
+    auto patch = [&](int r, int q) -> uint4& { return stage[r * PIECES + (PIECES == 8 ? q ^ (r & 7) : q ^ ((r >> 1) & 3))]; };
+    f32x2 w[CH / 2];
+    uint4 b16[CH / 8];
+    // (N is a multiple of 16: a chunk has 32, 16 or no valid columns)
+    auto request = [&](int cc) {
+#pragma unroll
+        for (int q = 0; q < CH / 8; ++q) {
+            const int64_t col = col_first + cc + 8 * q;
+            if (col < p.N) {
+                if (KIND == KIND_I8 && plain) {
+                    const ulonglong2* s2 = reinterpret_cast<const ulonglong2*>(scale + col);
+                    const ulonglong2 lo = __ldca(s2), hi = __ldca(s2 + 1);
+                    w[4 * q] = lo.x, w[4 * q + 1] = lo.y, w[4 * q + 2] = hi.x, w[4 * q + 3] = hi.y;
+                }
+                if (bias16 && plain) {
+                    b16[q] = __ldca(reinterpret_cast<const uint4*>(bias + col * 2));
+                }
+            }
+        }
+    };
+    auto chunk = [&](const uint32_t (&r)[CH], int cc, int sub) {
+#pragma unroll
+        for (int h = 0; h < CH / 16; ++h) {
+            const int64_t col = col_first + cc + 16 * h;
+            if (col >= p.N) {
+                break;  // what the patch holds there is not copied out
+            }
+            uint4 o[2];
+            if (EPI != EPI_QMM || plain) {
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    o[q] = dequant8<KIND>(r + 16 * h + 8 * q, w + 8 * h + 4 * q, row_mul, bias_kind, b16[2 * h + q],
+                                          bias + (col + 8 * q) * 4, bf16_out);
+                }
+            } else {
+                float v[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    v[j] = static_cast<float>(static_cast<int32_t>(r[16 * h + j]));
+                }
+                qmm_dequant<16>(p, terms, col, 16, v);
+                uint32_t x[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    x[j] = bf16_out ? pack2<W8A8_DT_BF16>(v[2 * j], v[2 * j + 1]) : pack2<W8A8_DT_F16>(v[2 * j], v[2 * j + 1]);
+                }
+                o[0] = make_uint4(x[0], x[1], x[2], x[3]);
+                o[1] = make_uint4(x[4], x[5], x[6], x[7]);
+            }
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                patch(lane, sub * (PIECES / 2) + 2 * h + q) = o[q];
+            }
+        }
+    };
+    auto load = [&](int cc, uint32_t (&r)[CH]) {
+        if constexpr (CH == 16) {
+            tc::tmem_ld_32x16(t_addr + share * COLS + cc, r);
+        } else {
+            tc::tmem_ld_32x32(t_addr + share * COLS + cc, r);
+        }
+    };
+    // all of the above, and what the first chunk is multiplied with, while the accumulator is being computed
+    request(0);
+    if (!accumulator_ready()) {
+        return false;
+    }
+#pragma unroll 1
+    for (int cc = 0; cc < COLS; cc += 2 * CH) {
+#pragma unroll
+        for (int sub = 0; sub < 2; ++sub) {
+            uint32_t r[CH];
+            load(cc + sub * CH, r);
+            if (cc + sub * CH != 0) {
+                request(cc + sub * CH);
+            }
+            tc::tmem_ld_wait(r);
+            chunk(r, cc + sub * CH, sub);
+        }
+        __syncwarp();
+        const int64_t pc = col_first + cc + piece * 8;
+#pragma unroll
+        for (int it = 0; it < PIECES; ++it) {
+            const int rr = it * COPY_ROWS + copy_row;  // row within the warp's 32
+            uint64_t rp = row_ptr + static_cast<uint64_t>(it) * (COPY_ROWS * 2) * p.N;
+            if (addressed) {
+                rp = __shfl_sync(FULL_MASK, row_ptr, rr);
+            }
+            const uint4 val = patch(rr, piece);
+            if (first_row + rr < tl.m_rows && pc < p.N) {
+                *reinterpret_cast<uint4*>(rp + static_cast<uint64_t>(pc) * 2) = val;
+            }
+        }
+        __syncwarp();
+    }
+    return true;
+}
+
+// The work of one epilogue thread on one tile: row `row_in_tile` of this CTA's accumulator, the `col_half`-th of
+// EPI_WARPS / 4 equal shares of its columns.  accumulator_ready() waits for the accumulator; false: it never came.
+template <int BLOCK_N, int KIND, int EPI, int EPI_WARPS, typename Wait>
+__device__ __forceinline__ bool epilogue_tile(const GemmParams& p, const TileInfo& tl, uint32_t t_addr,
+                                              int row_in_tile, int col_half, int64_t H, uint4* stage, Wait accumulator_ready)
+{
+    const bool row_ok = row_in_tile < tl.m_rows;
     const int64_t row = static_cast<int64_t>(tl.a_row0) + row_in_tile;  // global row (A and output)
     if constexpr (EPI == EPI_GMSQ) {
         const float xs = row_ok ? p.row_scale[row] : 0.0f;
+        if (!accumulator_ready()) {
+            return false;
+        }
+        if ((row_in_tile & ~31) >= tl.m_rows) {
+            return true;  // a whole warp without rows
+        }
         const float* wsg = static_cast<const float*>(p.scale) + static_cast<int64_t>(tl.group) * p.N;
         float local_max = 0.0f;
         // `col_half` counts this warp among the EPI_WARPS / 4 warps that share a TMEM lane quarter: each takes
@@ -643,7 +855,7 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, const TileInf
 #pragma unroll
                 for (int it = 0; it < 4; ++it) {
                     const int rr = it * 8 + (lane >> 2);
-                    if (first_row + rr < tl.m_rows && !no_epilogue && col < H) {
+                    if (first_row + rr < tl.m_rows && col < H) {
                         const uint4 val = stage[rr * 4 + (piece ^ ((rr ^ (rr >> 2)) & 3))];
                         *reinterpret_cast<uint4*>(p.act + (static_cast<int64_t>(tl.a_row0) + first_row + rr) * H + col) =
                             val;
@@ -655,149 +867,48 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, const TileInf
         if (row_ok) {
             atomicMax(reinterpret_cast<int*>(p.amax + row), __float_as_int(local_max));
         }
-    } else {
-        // per-tile invariants of the dequant chain, hoisted out of the column loops
-        [[maybe_unused]] float row_mul = 1.0f;
-        [[maybe_unused]] int bias_kind = W8A8_QM_BIAS_NONE;
-        [[maybe_unused]] QmmTerms terms;
-        [[maybe_unused]] int64_t vec_base = 0;  // first element of the per-channel vectors for this tile's group
-        if constexpr (EPI == EPI_QMM) {
-            terms = qmm_terms(p, tl.group, row, row_ok);
-        } else if constexpr (EPI == EPI_GMM) {
-            if constexpr (KIND == KIND_I8) {
-                row_mul = row_ok ? p.row_scale[row] : 0.0f;
-            }
-            vec_base = static_cast<int64_t>(tl.group) * p.N;
-            if (p.flags & 4) {
-                const int bdt = static_cast<int>(p.flags & 3);
-                bias_kind = (bdt == W8A8_DT_F16) ? W8A8_QM_BIAS_F16
-                                                  : (bdt == W8A8_DT_BF16 ? W8A8_QM_BIAS_BF16 : W8A8_QM_BIAS_F32);
-            }
+    } else if (EPI == EPI_RAW || (KIND == KIND_BF16 && p.out_dtype == W8A8_DT_F32)) {
+        // 32-bit results - accumulators, or fp32 of the split operands: 32 of them are one whole 128-byte line of the row
+        if (!accumulator_ready()) {
+            return false;
         }
-        constexpr int HALF_COLS = BLOCK_N / 2;
-        // byte address of this thread's output row (16-bit outputs; fp32 outputs are addressed where they are stored)
-        uint64_t row_ptr = reinterpret_cast<uint64_t>(p.out) + static_cast<uint64_t>(row) * p.N * 2;
-        if constexpr (EPI == EPI_GMM) {
-            if (p.out_row_ptrs != nullptr) {
-                // the row's home may be another GPU's memory: plain peer stores over NVLink
-                row_ptr = (row_in_tile < tl.m_rows) ? p.out_row_ptrs[row] : 0;
-            }
-        }
+        constexpr int COLS = BLOCK_N / (EPI_WARPS / 4);
 #pragma unroll 1
-        for (int cc = 0; cc < HALF_COLS; cc += 32) {
-            const int c = col_half * HALF_COLS + cc;
+        for (int cc = 0; cc < COLS; cc += 32) {
+            const int c = col_half * COLS + cc;
             uint32_t r[32];
             tc::tmem_ld_32x32(t_addr + c, r);
             tc::tmem_ld_wait();
             const int64_t col0 = static_cast<int64_t>(tl.nt) * BLOCK_N + c;
-            if constexpr (EPI == EPI_RAW) {
-                if (!row_ok || col0 >= p.N) {
-                    continue;
+            if (!row_ok || col0 >= p.N) {
+                continue;
+            }
+            const int valid = (col0 + 32 <= p.N) ? 32 : 16;  // N is a multiple of 16
+            if constexpr (EPI == EPI_GMM) {
+                if (p.flags & 4) {
+                    const int bdt = static_cast<int>(p.flags & 3);
+                    float b[32];
+                    load_vec<32>(p.bias, static_cast<int64_t>(tl.group) * p.N + col0,
+                                 bdt == W8A8_DT_F16 ? W8A8_QM_BIAS_F16 : (bdt == W8A8_DT_BF16 ? W8A8_QM_BIAS_BF16 : W8A8_QM_BIAS_F32),
+                                 true, valid, b);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        r[j] = __float_as_uint(__fadd_rn(__uint_as_float(r[j]), b[j]));
+                    }
                 }
             }
-            // N is a multiple of 16: a chunk holds 32, 16 or no valid columns
-            const int valid = (col0 >= p.N) ? 0 : ((col0 + 32 <= p.N) ? 32 : 16);
-            if constexpr (EPI == EPI_RAW) {
-                int32_t* dst = static_cast<int32_t*>(p.out) + row * p.N + col0;
+            uint4* dst = reinterpret_cast<uint4*>(static_cast<uint32_t*>(p.out) + row * p.N + col0);
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    if (q * 4 < valid) {
-                        *reinterpret_cast<uint4*>(dst + q * 4) =
-                            make_uint4(r[q * 4], r[q * 4 + 1], r[q * 4 + 2], r[q * 4 + 3]);
-                    }
-                }
-            } else {
-                float v[32];
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    if constexpr (KIND == KIND_I8) {
-                        v[j] = static_cast<float>(static_cast<int32_t>(r[j]));
-                    } else {
-                        v[j] = __uint_as_float(r[j]);
-                    }
-                }
-                if constexpr (EPI == EPI_QMM) {
-                    qmm_dequant<32>(p, terms, col0, valid, v);
-                } else {  // EPI_GMM
-                    float w[32];
-                    if constexpr (KIND == KIND_I8) {
-                        load_vec<32>(p.scale, vec_base + col0, W8A8_QM_BIAS_F32, true, valid, w);
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            v[j] = __fmul_rn(__fmul_rn(v[j], w[j]), row_mul);
-                        }
-                    }
-                    if (bias_kind != W8A8_QM_BIAS_NONE) {
-                        load_vec<32>(p.bias, vec_base + col0, bias_kind, true, valid, w);
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            v[j] = __fadd_rn(v[j], w[j]);
-                        }
-                    }
-                }
-                if constexpr (EPI == EPI_GMM && KIND == KIND_BF16) {
-                    if (p.out_dtype == W8A8_DT_F32) {
-                        // fp32 output (the split-operand path): 32 values are one whole 128-byte line of the row
-                        if (row_ok) {
-                            float* dst = static_cast<float*>(p.out) + row * p.N + col0;
-#pragma unroll
-                            for (int q = 0; q < 8; ++q) {
-                                if (q * 4 < valid) {
-                                    *reinterpret_cast<float4*>(dst + q * 4) =
-                                        make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
-                                }
-                            }
-                        }
-                        continue;
-                    }
-                }
-                // 32 outputs = 64 bytes of this thread's row.  They are not stored from here (every lane would
-                // write 16-byte pieces of a different row): the warp parks two such chunks, 128 bytes per row, in
-                // its private shared-memory patch and then writes whole 128-byte row segments, 8 lanes per row.
-                // That matters most when the row's home is another GPU: NVLink carries full lines, not fragments.
-                uint4 o[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    if (p.out_dtype == W8A8_DT_BF16) {
-                        o[q] = make_uint4(pack2<W8A8_DT_BF16>(v[q * 8], v[q * 8 + 1]),
-                                          pack2<W8A8_DT_BF16>(v[q * 8 + 2], v[q * 8 + 3]),
-                                          pack2<W8A8_DT_BF16>(v[q * 8 + 4], v[q * 8 + 5]),
-                                          pack2<W8A8_DT_BF16>(v[q * 8 + 6], v[q * 8 + 7]));
-                    } else {
-                        o[q] = make_uint4(pack2<W8A8_DT_F16>(v[q * 8], v[q * 8 + 1]),
-                                          pack2<W8A8_DT_F16>(v[q * 8 + 2], v[q * 8 + 3]),
-                                          pack2<W8A8_DT_F16>(v[q * 8 + 4], v[q * 8 + 5]),
-                                          pack2<W8A8_DT_F16>(v[q * 8 + 6], v[q * 8 + 7]));
-                    }
-                }
-                const int lane = row_in_tile & 31;
-                const int sub = (cc >> 5) & 1;  // which half of the 64-column patch
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    // row `lane`, 16-byte piece (sub*4 + q), pieces xor-swizzled by the row so that the eight
-                    // lanes of a quarter-warp hit eight different bank groups
-                    stage[lane * 8 + ((sub * 4 + q) ^ (lane & 7))] = o[q];
-                }
-                if (sub == 1) {
-                    __syncwarp();
-                    const int64_t patch_col0 = col0 - 32;  // first column of the 64-column patch
-                    const int piece = lane & 7;
-                    const int64_t pc = patch_col0 + piece * 8;
-                    const int first_row = row_in_tile & ~31;
-#pragma unroll
-                    for (int it = 0; it < 8; ++it) {
-                        const int rr = it * 4 + (lane >> 3);  // row within the warp's 32
-                        const uint64_t rp = __shfl_sync(FULL_MASK, row_ptr, rr);
-                        const uint4 val = stage[rr * 8 + (piece ^ (rr & 7))];
-                        if (first_row + rr < tl.m_rows && !no_epilogue && pc < p.N) {
-                            *reinterpret_cast<uint4*>(rp + static_cast<uint64_t>(pc) * 2) = val;
-                        }
-                    }
-                    __syncwarp();
+            for (int q = 0; q < 8; ++q) {
+                if (q * 4 < valid) {
+                    dst[q] = make_uint4(r[q * 4], r[q * 4 + 1], r[q * 4 + 2], r[q * 4 + 3]);
                 }
             }
         }
+    } else if constexpr (EPI == EPI_QMM || EPI == EPI_GMM) {
+        return epilogue_16bit<BLOCK_N, KIND, EPI, EPI_WARPS>(p, tl, t_addr, row_in_tile, col_half, stage, accumulator_ready);
     }
+    return true;
 }
 
 // Split K (SPLITK): the CTAs of a cluster each run the main loop over their share of a tile's K blocks, then deal the
@@ -933,7 +1044,7 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
     static_assert(!ROW_BOXES || (CG == 1 && BLOCK_N == 256), "row boxes: single CTAs of grouped problems");
     static_assert(!SPLITK || (CG == 1 && BLOCK_N == 128 && KIND == KIND_I8 && (EPI == EPI_QMM || EPI == EPI_RAW)),
                   "split K: dense int8 matmuls on single-CTA tiles of 128 columns");
-    static_assert(EPI_WARPS == 8 || (EPI_WARPS == 16 && EPI == EPI_GMSQ), "16 epilogue warps: SwiGLU epilogue only");
+    static_assert(EPI_WARPS == 8 || EPI_WARPS == 16, "epilogue warps");
 
     extern __shared__ uint8_t smem_raw[];
     // 1024-byte alignment: required by the 128-byte swizzle atoms.  The dynamic shared memory window starts at
@@ -1331,7 +1442,6 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
         const int quarter = warp & 3;          // TMEM lanes [32*quarter, 32*quarter+32)
         const int col_half = (warp - 2) >> 2;  // which share of the columns
         const int row_in_tile = quarter * 32 + lane;
-        const bool no_epilogue = false;
         // this warp's patch (4 KB, or 2 KB with 16 warps) for turning per-thread rows into whole-segment stores
         uint4* stage = reinterpret_cast<uint4*>(smem + STAGES * STAGE_BYTES + 512) +
                        (warp - 2) * (GEMM_EPI_PATCH_BYTES / 16 / EPI_WARPS);
@@ -1389,17 +1499,22 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
             touch_epilogue_operands<BLOCK_N, KIND, EPI>(p, tl, row_in_tile);
             const int acc = static_cast<int>(it & 1);
             const uint32_t acc_phase = static_cast<uint32_t>((it >> 1) & 1);
-            if (!tc::mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) {
-                ok = false;
-                break;
-            }
-            tc::tc_fence_after_sync();
+            auto accumulator_ready = [&]() {
+                const bool ready = tc::mbar_wait(tfull_bar(acc), acc_phase, abort_flag);
+                tc::tc_fence_after_sync();
+                return ready;
+            };
             if constexpr (SPLITK) {
+                ok = accumulator_ready();
                 break;  // one tile per cluster: its accumulators are exchanged below, by all warps together
             }
             const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                                     static_cast<uint32_t>(acc * BLOCK_N);
-            epilogue_tile<BLOCK_N, KIND, EPI, EPI_WARPS>(p, tl, t_addr, row_in_tile, col_half, H, no_epilogue, stage);
+            if (!epilogue_tile<BLOCK_N, KIND, EPI, EPI_WARPS>(p, tl, t_addr, row_in_tile, col_half, H, stage,
+                                                              accumulator_ready)) {
+                ok = false;
+                break;
+            }
             // accumulator stage drained: hand it back to the MMA issuer (one arrival per warp)
             tc::tc_fence_before_sync();
             __syncwarp();
