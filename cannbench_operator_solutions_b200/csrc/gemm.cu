@@ -216,33 +216,58 @@ static cudaError_t dispatch_row_boxes(bool b_mn, const CUtensorMap& ta, const CU
                 : launch_gemm<1, 256, KIND, EPI, false, 8, false, true>(ta, tb, p, max_tiles, st, groups);
 }
 
-// Dense problems with at most one 128 x 128 tile per SM run on single CTAs: a cluster launch costs about 3 us more
-// than a plain one (512 x 1024 x 1024: 7.4 us, 11 on pairs; 1024 x 2048 x 2048: 10.3, 13.8).  Where half of the SMs or
-// more would have no tile, clusters of two or four share a tile's K, if the K blocks saved (0.25 us each) pay for the
-// cluster and for the exchange of the accumulators, which a tile with few rows hardly has: 16 x 9216 x 7168 18 us
-// against 25, 16 x 7168 x 4096 11.8 (four) / 14.6 (two) against 20.5, 128 x 7168 x 2048 14.4 / 15.9 against 20.6,
-// but 1024 x 2048 x 512 12.5 / 10.4 and 128 x 1024 x 1024 9.9 / 9.0 against 7.1.  Clusters of eight do not find a
-// place for every tile (16 tiles take two waves); clusters of four count on 128 SMs.
-static int choose_split(int64_t tiles, int64_t k_blocks, int64_t rows)
-{
-    const bool few_rows = rows <= 64;
-    if (tiles * 4 <= 128 && tiles * 4 <= sm_count() && k_blocks >= (few_rows ? 16 : 48)) {
-        return 4;
-    }
-    return (tiles * 2 <= sm_count() && k_blocks >= (few_rows ? 12 : 24)) ? 2 : 1;
-}
-
 // w8a8_set_gemm_shape() (1, 2, or 3 = pairs plus singles for grouped problems; 0 = the library's choice) overrides the
 // kernel shape process-wide; the tests use it to run every case on every shape.
 constexpr int GEMM_SHAPE_HYBRID = 3;
 static std::atomic<int> g_shape_override{0};
 static std::atomic<int> g_fuse_requant{0};  // see w8a8_set_gmsq_fused_requant
 
-// Dense problems: CTA pairs from 256 rows on (see also choose_split and quant_matmul_impl).
-static int choose_cta_group(int64_t rows)
+struct DenseShape {
+    int cta_group, block_n, split;
+};
+
+// Dense problems: single CTAs on 128 x 128 or 128 x 256 tiles, CTA pairs on 256 x 256, or, where most SMs would have no
+// tile, clusters of two or four CTAs that share a 128 x 128 tile's K (clusters of eight do not find a place for every tile,
+// clusters of four count on 128 SMs).  The shape is the one with the smallest estimate, in us: waves of tiles over the SMs,
+// a tile taking its K blocks (0.244, 0.356, 0.245) or its epilogue (1.8, 3.1, 3.3) if that is longer; no less than the
+// weights at 5.5 TB/s; and what the shape costs besides - wide tiles 0.5, a pair's cluster 3, a split 0.8 and the exchange of
+// the accumulators, by the 32-row quarters of a tile that hold rows (0.55 for two CTAs, 0.83 for four).  Fitted to 220
+// problems of 1 - 8192 rows, 512 - 9216 x 512 - 18432, each timed in all shapes: 0.2 % from the best of each on average and
+// 8 % at worst, where the rule before it - singles up to one tile per SM, pairs from 256 rows on, splits by thresholds - is
+// 2.3 % and 41 % from it (1112 x 1760 x 4032 15.8 us, 11.2 on wide singles; 178 x 4384 x 11920 26.2, 20.5 on pairs; 85 x 5776 x
+// 816 14.9, 11.3 split over four).
+static DenseShape choose_dense_shape(int64_t batch, int64_t M, int64_t N, int64_t k_blocks, double weight_bytes)
 {
     const int v = g_shape_override.load(std::memory_order_relaxed);
-    return (v == 1 || v == 2) ? v : (rows >= 256 ? 2 : 1);
+    const int64_t sms = sm_count();
+    const auto tiles = [&](int64_t rows, int64_t cols) { return batch * ((M + rows - 1) / rows) * ((N + cols - 1) / cols); };
+    if (v == 1 || v == 2) {
+        return {v, v == 1 && tiles(128, 256) < sms ? 128 : 256, 1};
+    }
+    const double kb = static_cast<double>(k_blocks), weights = weight_bytes * 1e-6 / 5.5;
+    const auto estimate = [&](int64_t count, int64_t workers, double tile, double besides) {
+        return std::max(static_cast<double>((count + workers - 1) / workers) * tile, weights) + besides;
+    };
+    const int64_t narrow = tiles(128, 128);
+    const double quarters = static_cast<double>(std::min<int64_t>(4, (M + 31) / 32));
+    DenseShape best{1, 128, 1};
+    double least = estimate(narrow, sms, std::max(0.244 * kb, 1.8), 0.0);
+    const auto offer = [&](const DenseShape& shape, double us) {
+        if (us < least) {
+            least = us;
+            best = shape;
+        }
+    };
+    offer({1, 256, 1}, estimate(tiles(128, 256), sms, std::max(0.356 * kb, 3.1), 0.5));
+    offer({2, 256, 1}, estimate(tiles(256, 256), sms / 2, std::max(0.245 * kb, 3.3), 3.0));
+    for (int split : {2, 4}) {
+        // no share of a tile's K blocks may be empty
+        if (narrow * split <= std::min<int64_t>(sms, split == 4 ? 128 : sms) && k_blocks >= split) {
+            const double share = static_cast<double>((k_blocks + split - 1) / split);
+            offer({1, 128, split}, std::max(share * 0.244, weights) + 0.8 + quarters * (split == 2 ? 0.55 : 0.83));
+        }
+    }
+    return best;
 }
 
 // Grouped problems: single CTAs on 128-row tiles, CTA pairs on 256-row tiles, or both in two launches - pairs on every
@@ -673,7 +698,7 @@ static int plan_groups(const int64_t* group_list, int list_on_device, int64_t E,
 }
 
 // Runs a grouped problem whose GemmParams are filled in except for the tile table: plans the groups and launches
-// the kernel shape(s) choose_cta_group picked.
+// the kernel shape(s) choose_grouped_shape picked.
 template <int KIND, int EPI>
 static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E, int64_t M, const GroupedWorkspace& g,
                        bool b_mn, const void* a, const CUtensorMap& tb, GemmParams p, cudaStream_t st,
@@ -871,29 +896,25 @@ static int quant_matmul_impl(const int8_t* x1, const int8_t* x2, const void* sca
     p.bias_batch_stride = bias_batch_stride;
     p.prefetch_k_blocks = GEMM_PREFETCH_K_BLOCKS;
     p.error = pipeline_error_word();  // null (no report) only if the symbol lookup failed
-    const int64_t tiles128 = batch * p.m_tiles_per_batch * ((N + 127) / 128);
-    const bool own_choice = g_shape_override.load(std::memory_order_relaxed) == 0;
-    const int split = own_choice ? choose_split(tiles128, p.num_k_blocks, M) : 1;
-    if (split > 1) {
-        p.split = split;
+    const DenseShape shape = choose_dense_shape(batch, M, N, p.num_k_blocks, static_cast<double>(batch * N * K));
+    if (shape.split > 1) {
+        p.split = shape.split;
         p.n_tiles = static_cast<int32_t>((N + 127) / 128);
+        const int64_t tiles = batch * p.m_tiles_per_batch * p.n_tiles;
         cudaError_t e;
         if (raw_i32) {
-            e = b_mn ? launch_gemm<1, 128, KIND_I8, EPI_RAW, true, 8, true>(ta, tb, p, tiles128, st)
-                     : launch_gemm<1, 128, KIND_I8, EPI_RAW, false, 8, true>(ta, tb, p, tiles128, st);
+            e = b_mn ? launch_gemm<1, 128, KIND_I8, EPI_RAW, true, 8, true>(ta, tb, p, tiles, st)
+                     : launch_gemm<1, 128, KIND_I8, EPI_RAW, false, 8, true>(ta, tb, p, tiles, st);
         } else {
-            e = b_mn ? launch_gemm<1, 128, KIND_I8, EPI_QMM, true, 8, true>(ta, tb, p, tiles128, st)
-                     : launch_gemm<1, 128, KIND_I8, EPI_QMM, false, 8, true>(ta, tb, p, tiles128, st);
+            e = b_mn ? launch_gemm<1, 128, KIND_I8, EPI_QMM, true, 8, true>(ta, tb, p, tiles, st)
+                     : launch_gemm<1, 128, KIND_I8, EPI_QMM, false, 8, true>(ta, tb, p, tiles, st);
         }
         return launch_status(e);
     }
-    const int cg = (own_choice && tiles128 <= sm_count()) ? 1 : choose_cta_group(M);
+    const int cg = shape.cta_group, block_n = shape.block_n;
     const int tile_m = 128 * cg;
     p.m_tiles_per_batch = static_cast<int32_t>((M + tile_m - 1) / tile_m);
-    // narrow tiles when wide ones would leave most SMs idle (single-CTA tiles only)
     const int64_t m_tiles = batch * p.m_tiles_per_batch;
-    const int64_t tiles256 = m_tiles * ((N + 255) / 256);
-    const int block_n = (cg == 1 && tiles256 < sm_count()) ? 128 : 256;
     p.n_tiles = static_cast<int32_t>((N + block_n - 1) / block_n);
     const int64_t total = m_tiles * p.n_tiles;
     cudaError_t e;
