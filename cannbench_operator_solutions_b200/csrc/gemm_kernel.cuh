@@ -115,31 +115,27 @@ constexpr int PLAN_ALL = 0;
 constexpr int PLAN_WHOLE = 1;
 constexpr int PLAN_LEFTOVER = 2;
 
+// (tile_m is a power of two)
 __device__ __forceinline__ int32_t group_tiles(uint32_t rows, uint32_t tile_m, int mode)
 {
-    if (mode == PLAN_WHOLE) {
-        return static_cast<int32_t>(rows / tile_m) + ((rows % tile_m > tile_m / 2) ? 1 : 0);
-    }
     if (mode == PLAN_LEFTOVER) {
-        const uint32_t rest = rows % (2 * tile_m);
+        const uint32_t rest = rows & (2 * tile_m - 1);
         return (rest >= 1 && rest <= tile_m) ? 1 : 0;
     }
-    return static_cast<int32_t>((rows + tile_m - 1) / tile_m);
+    const uint32_t whole = rows >> (31 - __clz(tile_m)), rest = rows & (tile_m - 1);
+    return static_cast<int32_t>(whole + (rest > (mode == PLAN_WHOLE ? tile_m / 2 : 0) ? 1 : 0));
 }
 
 // tile `t` of group `group`, whose rows are [start, end)
 __device__ __forceinline__ TileEntry group_tile(int group, int64_t start, int64_t end, int32_t t, int tile_m, int mode)
 {
-    int64_t rows = end - start;
     if (mode == PLAN_LEFTOVER) {
-        const int64_t whole = rows / (2 * tile_m) * (2 * tile_m);
-        start += whole;
-        rows -= whole;
+        start += (end - start) & ~static_cast<int64_t>(2 * tile_m - 1);
     }
     TileEntry te;
     te.group = group;
     te.m_start = static_cast<int32_t>(start + static_cast<int64_t>(t) * tile_m);
-    const int64_t left = rows - static_cast<int64_t>(t) * tile_m;
+    const int64_t left = end - te.m_start;
     te.m_rows = static_cast<int32_t>(left < tile_m ? left : tile_m);
     te.pad = 0;
     return te;
@@ -163,11 +159,14 @@ struct GroupList {
 };
 struct NoGroupList {
 };
+// how many groups a CTA has planned for itself (0: none)
+__device__ __forceinline__ int32_t groups_planned(const GroupList& list) { return list.E; }
+__device__ __forceinline__ int32_t groups_planned(const NoGroupList&) { return 0; }
 template <int EPI>
 using GroupListOf = std::conditional_t<EPI == EPI_GMSQ || EPI == EPI_GMM, GroupList, NoGroupList>;
 
 // One warp: first[g] = the first tile of group g, first[E] = the number of tiles, and whether the list is in order.  An
-// invalid one has no tiles.
+// invalid one has no tiles.  Behind first[E] come numbers that no tile has.
 __device__ __forceinline__ bool plan_in_cta(const GroupList& list, int64_t M, int32_t* first)
 {
     constexpr int PER_LANE = GROUPS_IN_CTA / 32;
@@ -202,8 +201,8 @@ __device__ __forceinline__ bool plan_in_cta(const GroupList& list, int64_t M, in
 #pragma unroll
     for (int i = 0; i < PER_LANE; ++i) {
         const int g = lane * PER_LANE + i;
-        if (g < list.E) {
-            first[g] = bad ? 0 : at;
+        if (g != list.E) {
+            first[g] = g < list.E ? (bad ? 0 : at) : INT32_MAX;
         }
         at += count[i];
         if (g == list.E - 1) {
@@ -214,19 +213,19 @@ __device__ __forceinline__ bool plan_in_cta(const GroupList& list, int64_t M, in
 }
 
 // Tile `mt` by the first tiles: its group is the last one whose first tile is at or before it (groups without tiles
-// share their first tile with the next one, and first[E] ends the search).
+// share their first tile with the next one), found by a whole warp at once.  (Between two tiles an epilogue warp has
+// nothing else to do: with a search by halves and the tile number divided, SwiGLU tiles of K = 1280 took 4 % longer.)
 __device__ __forceinline__ TileEntry tile_in_cta(const GroupList& list, const int32_t* first, int32_t mt)
 {
-    int lo = 0, hi = list.E;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (first[mid] <= mt) {
-            lo = mid;
-        } else {
-            hi = mid;
-        }
+    const int4* mine = reinterpret_cast<const int4*>(first) + (threadIdx.x & 31) * (GROUPS_IN_CTA / 32 / 4);
+    int at_or_before = 0;
+#pragma unroll
+    for (int i = 0; i < GROUPS_IN_CTA / 32 / 4; ++i) {
+        const int4 f = mine[i];
+        at_or_before += (f.x <= mt) + (f.y <= mt) + (f.z <= mt) + (f.w <= mt);
     }
-    return group_tile(lo, lo == 0 ? 0 : list.end_of(lo - 1), list.end_of(lo), mt - first[lo], list.tile_m, list.mode);
+    const int g = __reduce_add_sync(FULL_MASK, at_or_before) - 1;
+    return group_tile(g, g == 0 ? 0 : list.end_of(g - 1), list.end_of(g), mt - first[g], list.tile_m, list.mode);
 }
 
 // A grouped problem's two launches (pairs, then leftovers) share no output row and read nothing of one another, so the
@@ -1183,38 +1182,46 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
 
     // ---- tile enumeration (identical in every role and in both CTAs of a pair) ----
     constexpr int TILE_M = 128 * CG;
-    int64_t total_tiles;
-    int32_t dense_m_tiles = 0;
-    if constexpr (GROUPED) {
-        total_tiles = static_cast<int64_t>(groups.E != 0 ? first_tiles[groups.E] : p.header->num_m_tiles) * p.n_tiles;
-    } else {
-        dense_m_tiles = p.batch * p.m_tiles_per_batch;
-        total_tiles = static_cast<int64_t>(dense_m_tiles) * p.n_tiles;
-    }
+    // Tiles are numbered with the column tile (grouped) or the row tile (dense) fastest; a worker's are num_workers apart.
+    const int32_t fast_count = GROUPED ? p.n_tiles : p.batch * p.m_tiles_per_batch;
+    const int32_t slow_count =
+        GROUPED ? (groups_planned(groups) ? first_tiles[groups_planned(groups)] : p.header->num_m_tiles) : p.n_tiles;
+    const int64_t total_tiles = static_cast<int64_t>(slow_count) * fast_count;
     const int64_t H = p.N / 2;  // GMSQ half width
-    const int64_t ctas_per_tile = SPLITK ? p.split : CG;
-    const int64_t worker = blockIdx.x / ctas_per_tile;
-    const int64_t num_workers = gridDim.x / ctas_per_tile;
+    const int32_t ctas_per_tile = SPLITK ? p.split : CG;
+    const int32_t worker = static_cast<int32_t>(blockIdx.x) / ctas_per_tile;
+    const int32_t num_workers = static_cast<int32_t>(gridDim.x) / ctas_per_tile;
+    struct Walk {
+        int32_t fast, slow;
+    };
+    auto first_step = [&] { return Walk{worker % fast_count, worker / fast_count}; };
+    const Walk stride{num_workers % fast_count, num_workers / fast_count};
+    auto next_step = [&](Walk& w) {
+        w.fast += stride.fast;
+        w.slow += stride.slow;
+        if (w.fast >= fast_count) {
+            w.fast -= fast_count;
+            ++w.slow;
+        }
+    };
 
-    auto decode = [&](int64_t t) {
+    // by a whole warp
+    auto decode = [&](const Walk& w) {
         TileInfo tl;
         int64_t tile_row0;
         int32_t tile_rows;
         if constexpr (GROUPED) {
-            const int32_t mt = static_cast<int32_t>(t / p.n_tiles);
-            tl.nt = static_cast<int32_t>(t % p.n_tiles);
-            tl.mt = mt;
-            const TileEntry e = groups.E != 0 ? tile_in_cta(groups, first_tiles, mt) : p.tiles[mt];
+            tl.nt = w.fast;
+            tl.mt = w.slow;
+            const TileEntry e = groups.E != 0 ? tile_in_cta(groups, first_tiles, w.slow) : p.tiles[w.slow];
             tile_row0 = e.m_start;
             tile_rows = e.m_rows;
             tl.group = e.group;
         } else {
-            const int32_t mg = static_cast<int32_t>(t % dense_m_tiles);
-            tl.nt = static_cast<int32_t>(t / dense_m_tiles);
-            tl.mt = mg;
-            const int32_t b = mg / p.m_tiles_per_batch;
-            const int32_t mt = mg % p.m_tiles_per_batch;
-            const int64_t m0 = static_cast<int64_t>(mt) * TILE_M;
+            tl.nt = w.slow;
+            tl.mt = w.fast;
+            const int32_t b = p.batch == 1 ? 0 : w.fast / p.m_tiles_per_batch;
+            const int64_t m0 = static_cast<int64_t>(w.fast - b * p.m_tiles_per_batch) * TILE_M;
             tile_row0 = b * p.M + m0;
             const int64_t left = p.M - m0;
             tile_rows = static_cast<int32_t>(left < TILE_M ? left : TILE_M);
@@ -1247,8 +1254,9 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
             bool ok = true;
             // a pair credits both CTAs' bytes to the leader's barrier
             const uint32_t full0 = (CG == 2) ? tc::map_to_cta(full_bar(0), 0) : full_bar(0);
-            for (int64_t t = worker; ok && t < total_tiles; t += num_workers) {
-                const TileInfo tl = decode(t);
+            Walk at = first_step();
+            for (int64_t t = worker; ok && t < total_tiles; t += num_workers, next_step(at)) {
+                const TileInfo tl = decode(at);
                 // ROW_BOXES: the tile's rows only, in boxes of a_box_rows
                 const int a_loads = ROW_BOXES ? (tl.m_rows + p.a_box_rows - 1) / p.a_box_rows : 1;
                 const uint32_t a_box_bytes = static_cast<uint32_t>(p.a_box_rows) * GEMM_KBYTES;
@@ -1494,8 +1502,9 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
             }
             return true;
         };
-        for (int64_t t = worker; ok && t < total_tiles; t += num_workers, ++it) {
-            const TileInfo tl = decode(t);
+        Walk at = first_step();
+        for (int64_t t = worker; ok && t < total_tiles; t += num_workers, ++it, next_step(at)) {
+            const TileInfo tl = decode(at);
             touch_epilogue_operands<BLOCK_N, KIND, EPI>(p, tl, row_in_tile);
             const int acc = static_cast<int>(it & 1);
             const uint32_t acc_phase = static_cast<uint32_t>((it >> 1) & 1);
@@ -1566,7 +1575,7 @@ __global__ void __launch_bounds__(gemm_threads(EPI_WARPS), 1)
         const uint32_t t_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
         TileInfo tl{};
         if (mine) {
-            tl = decode(worker);
+            tl = decode(first_step());
             split_send(p, tl.m_rows, t_addr, row_in_tile, (warp - 2) >> 2, split_rank, smem_base);
         }
         __syncwarp();
