@@ -169,11 +169,9 @@ static cudaError_t dispatch_gemm(int cta_group, int block_n, bool b_mn, const CU
                 return b_mn ? launch_gemm<2, 256, KIND, EPI, true, 16>(ta, tb, p, max_tiles, st, groups)
                             : launch_gemm<2, 256, KIND, EPI, false, 16>(ta, tb, p, max_tiles, st, groups);
             }
-            if constexpr (EPI == EPI_QMM) {
-                if (block_n == 128) {
-                    return b_mn ? launch_gemm<1, 128, KIND, EPI, true, 16>(ta, tb, p, max_tiles, st)
-                                : launch_gemm<1, 128, KIND, EPI, false, 16>(ta, tb, p, max_tiles, st);
-                }
+            if (block_n == 128) {
+                return b_mn ? launch_gemm<1, 128, KIND, EPI, true, 16>(ta, tb, p, max_tiles, st, groups)
+                            : launch_gemm<1, 128, KIND, EPI, false, 16>(ta, tb, p, max_tiles, st, groups);
             }
             return b_mn ? launch_gemm<1, 256, KIND, EPI, true, 16>(ta, tb, p, max_tiles, st, groups)
                         : launch_gemm<1, 256, KIND, EPI, false, 16>(ta, tb, p, max_tiles, st, groups);
@@ -184,10 +182,10 @@ static cudaError_t dispatch_gemm(int cta_group, int block_n, bool b_mn, const CU
             return b_mn ? launch_gemm<2, 256, KIND, EPI, true>(ta, tb, p, max_tiles, st, groups)
                         : launch_gemm<2, 256, KIND, EPI, false>(ta, tb, p, max_tiles, st, groups);
         }
-        if constexpr (EPI == EPI_RAW) {
+        if constexpr (EPI == EPI_RAW || (EPI == EPI_GMM && KIND != KIND_I8)) {
             if (block_n == 128) {
-                return b_mn ? launch_gemm<1, 128, KIND, EPI, true>(ta, tb, p, max_tiles, st)
-                            : launch_gemm<1, 128, KIND, EPI, false>(ta, tb, p, max_tiles, st);
+                return b_mn ? launch_gemm<1, 128, KIND, EPI, true>(ta, tb, p, max_tiles, st, groups)
+                            : launch_gemm<1, 128, KIND, EPI, false>(ta, tb, p, max_tiles, st, groups);
             }
         }
         return b_mn ? launch_gemm<1, 256, KIND, EPI, true>(ta, tb, p, max_tiles, st, groups)
@@ -219,6 +217,7 @@ static cudaError_t dispatch_row_boxes(bool b_mn, const CUtensorMap& ta, const CU
 // w8a8_set_gemm_shape() (1, 2, or 3 = pairs plus singles for grouped problems; 0 = the library's choice) overrides the
 // kernel shape process-wide; the tests use it to run every case on every shape.
 constexpr int GEMM_SHAPE_HYBRID = 3;
+constexpr int GEMM_SHAPE_NARROW = 4;  // single CTAs on 128 x 128 tiles: never forced
 static std::atomic<int> g_shape_override{0};
 static std::atomic<int> g_fuse_requant{0};  // see w8a8_set_gmsq_fused_requant
 
@@ -281,8 +280,12 @@ static DenseShape choose_dense_shape(int64_t batch, int64_t M, int64_t N, int64_
 // 2048 rows on, as the rule was, are 6.4 % from it on average and 52 % at worst (3000 rows of 8 groups of 2048 x 4096 bf16
 // 74 us, 59 on single CTAs; SwiGLU form, 6000 of 8 of 4096 x 2048 69, 58).  Of a device list only the rows and the number of
 // groups are known here: even groups with remainders of all sizes are assumed (0.8 % and 31 % on the same problems).
-static int choose_grouped_shape(const int64_t* host_ends, int64_t E, int64_t M, int64_t n_tiles, int64_t k_blocks,
-                                double group_weight_bytes)
+// Where one wave of narrow tiles holds the whole problem (`n_narrow` > 0 of them side by side: not for the SwiGLU epilogue,
+// whose tile is 128 gate and 128 up columns), they are one more candidate, 0.244 a K block and 1.8 an epilogue as in the
+// dense estimate: 64 rows of 4 groups of 512 x 512 bf16 5.2 us (6.6 on wide tiles), 200 of 8 of 1024 x 2048 10.3 (12.4), 500 of
+// 8 of 2048 x 1024 12.8 (17.1), 200 of 8 of 4000 x 2048 29.4 (35.9).
+static int choose_grouped_shape(const int64_t* host_ends, int64_t E, int64_t M, int64_t n_tiles, int64_t n_narrow,
+                                int64_t k_blocks, double group_weight_bytes)
 {
     const int v = g_shape_override.load(std::memory_order_relaxed);
     if (v != 0) {
@@ -322,6 +325,10 @@ static int choose_grouped_shape(const int64_t* host_ends, int64_t E, int64_t M, 
     const double t2 = std::max(std::ceil(pairs * nt / (sms / 2)) * pair_tile, weights) + 2.5;
     const double t3 =
         std::max(std::ceil(whole * nt / (sms / 2)) * pair_tile + leftover * nt / sms * single_tile * 0.55, weights) + 20.0;
+    const double t4 = std::max(std::max(0.244 * kb, 1.8), weights);
+    if (n_narrow > 0 && singles * static_cast<double>(n_narrow) <= sms && t4 < std::min({t1, t2, t3})) {
+        return GEMM_SHAPE_NARROW;
+    }
     return t1 <= t2 && t1 <= t3 ? 1 : (t2 <= t3 ? 2 : GEMM_SHAPE_HYBRID);
 }
 
@@ -708,8 +715,14 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
     const bool split = p.k_blocks_per_term != 0;
     const int64_t a_cols = split ? SPLIT_PIECES * p.K : p.K;
     const int64_t group_bytes = p.N * p.K * ELEM * (split ? SPLIT_TERMS : 1);  // of weights, as the kernel streams them
-    const int shape = choose_grouped_shape(list_on_device ? nullptr : group_list, E, M, p.n_tiles, p.num_k_blocks,
-                                           static_cast<double>(group_bytes));
+    const int64_t n_narrow = (EPI == EPI_GMM && p.out_row_ptrs == nullptr) ? (p.N + 127) / 128 : 0;
+    const int chosen = choose_grouped_shape(list_on_device ? nullptr : group_list, E, M, p.n_tiles, n_narrow, p.num_k_blocks,
+                                            static_cast<double>(group_bytes));
+    const bool narrow = chosen == GEMM_SHAPE_NARROW;
+    const int shape = narrow ? 1 : chosen;
+    if (narrow) {
+        p.n_tiles = static_cast<int32_t>(n_narrow);
+    }
     p.error = &g.header->error;
     // Rows per A load.  Pairs take whole tiles.  A single CTA's tile holds at most 128 rows of one group and often far
     // fewer - what a group leaves over, or a whole group of a small batch.  Where there are 256 MB of weights to stream
@@ -722,7 +735,7 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
     // 153.7 - 184 with whole tiles - the same with boxes of 16 and of 32, and nothing from 96 rows per expert on, which
     // is where the rule ends; at 12 rows per expert most tiles still fit into one box of 16.
     int box_rows = (shape == GEMM_SHAPE_HYBRID) ? 32 : (M <= 12 * E ? 16 : (M <= 96 * E ? 32 : GEMM_BLOCK_M));
-    if (shape == 2 || E * group_bytes < (int64_t(256) << 20)) {
+    if (shape == 2 || narrow || E * group_bytes < (int64_t(256) << 20)) {
         box_rows = GEMM_BLOCK_M;
     }
     const bool row_boxes = box_rows < GEMM_BLOCK_M;
@@ -777,7 +790,7 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
     p.order = overlap ? ORDER_FIRST_OF_TWO : (plain ? ORDER_PLAIN : ORDER_ALONE);
     const int64_t most = (hybrid ? M / 256 + E + 1 : g.max_tiles) * p.n_tiles;
     cudaError_t e = (!hybrid && row_boxes) ? dispatch_row_boxes<KIND, EPI>(b_mn, ta, tb, p, most, st, groups)
-                                           : dispatch_gemm<KIND, EPI>(hybrid ? 2 : shape, 256, b_mn, ta, tb, p, most, st, groups);
+                                           : dispatch_gemm<KIND, EPI>(hybrid ? 2 : shape, narrow ? 128 : 256, b_mn, ta, tb, p, most, st, groups);
     if (e != cudaSuccess || !hybrid) {
         return launch_status(e);
     }
