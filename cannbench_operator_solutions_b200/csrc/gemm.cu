@@ -487,34 +487,89 @@ __global__ void __launch_bounds__(256) plan_groups_both_kernel(const int64_t* de
 }
 
 // ---------------------------------------------------------------------------
-// Requantisation of the SwiGLU activations (second, bandwidth-bound half of
-// grouped_matmul_swiglu_quant): amax clamp at FLT_MIN, y_scale = amax*(1/127),
-// inv = 127/amax, clamp to [-128,127], two-step narrowing
-// (gmsq_vec_kernel.cpp:233-257).  A warp takes one of `parts` pieces of a row, eight 16-byte loads in flight per lane.
-// Bound: HBM (5 H bytes per row).  131072 x 2048: 207 us = 6.5 TB/s (237 with the loads of one loop step in flight);
-// 512 rows of a decode step: 5.5 us (12 with a warp per row).
+// Requantisation of the SwiGLU activations (second, bandwidth-bound half of grouped_matmul_swiglu_quant): a CTA holds a row
+// in registers between its maximum and its quantisation, so the matmul keeps no maxima and nothing has to be zeroed for them.
+// Bound: HBM (5 H bytes per row).  131072 x 2048 198 us, 40000 x 1792 56, 8000 x 512 5.5, 64 x 2048 1.8; with two pieces per
+// thread 248, 71, 7.9, 1.8, with eight 209, 56, 6.5, 2.0.  The operator: 64 rows of 8 experts of 1024 x 1024 10.7 us (12.1 with a
+// zeroing kernel ahead, a maximum per row and column tile kept by the matmul, and warps that read it), 100 of 8 of 4096 x 2048
+// 22.4 (24.2), 40000 of 32 of 1280 x 3584 312 (320).
+// CPT: 16-byte pieces of the row per thread; 0: rows of any length, read twice (the second time from L2).
 // ---------------------------------------------------------------------------
-template <bool DIRECT>
-__global__ void __launch_bounds__(256) gmsq_requant_kernel(const float* act,
-                                                           const uint32_t* amax_bits,
-                                                           int8_t* __restrict__ y, float* __restrict__ y_scale,
-                                                           int64_t M, int64_t H, const GroupedHeader* header, int parts)
+template <bool DIRECT, int CPT>
+__global__ void __launch_bounds__(1024) gmsq_requant_kernel(const float* act, int8_t* __restrict__ y,
+                                                            float* __restrict__ y_scale, int64_t M, int64_t H,
+                                                            const GroupedHeader* header)
 {
+    __shared__ int s_max[2][32];
     const int64_t zero = after_previous();
     if (header->error != 0) {
         return;
     }
-    const int lane = threadIdx.x & 31;
-    const int64_t warp_global = zero + ((static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
-    const int64_t warps_total = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+    const int64_t rows = min(M, static_cast<int64_t>(header->rows_total));  // a device list may end before M
+    const int tid = threadIdx.x, threads = blockDim.x, lane = tid & 31, warps = threads >> 5;
     const int64_t n4 = H / 4;
-    const int64_t per = (n4 + parts - 1) / parts;
-    const int64_t units = min(M, static_cast<int64_t>(header->rows_total)) * parts;  // a device list may end before M
-    for (int64_t u = warp_global; u < units; u += warps_total) {
-        const int64_t row = u / parts;
-        const int64_t lo = (u - row * parts) * per;
-        requant_row_part<DIRECT>(act, amax_bits, y, y_scale, row, H, lo, min(lo + per, n4), lo == 0, lane);
+    int parity = 0;
+    for (int64_t row = blockIdx.x + zero; row < rows; row += gridDim.x, parity ^= 1) {
+        const float4* src = reinterpret_cast<const float4*>(act + row * H);
+        uint32_t* dst = reinterpret_cast<uint32_t*>(y + row * H);
+        constexpr int HELD = CPT > 0 ? CPT : 1;
+        float4 a[HELD];
+        float m = 0.0f;
+        if constexpr (CPT > 0) {
+#pragma unroll
+            for (int i = 0; i < CPT; ++i) {
+                const int c = tid + i * threads;
+                a[i] = c < n4 ? __ldcs(src + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+#pragma unroll
+            for (int i = 0; i < CPT; ++i) {
+                m = requant_max4(m, a[i]);
+            }
+        } else {
+            for (int64_t c = tid; c < n4; c += threads) {
+                m = requant_max4(m, src[c]);
+            }
+        }
+        // magnitudes order like their bit patterns
+        const int own = __reduce_max_sync(FULL_MASK, __float_as_int(m));
+        if (lane == 0) {
+            s_max[parity][tid >> 5] = own;
+        }
+        __syncthreads();
+        const int top = __reduce_max_sync(FULL_MASK, lane < warps ? s_max[parity][lane] : 0);
+        const float amax = requant_amax(__int_as_float(top));
+        if (tid == 0) {
+            y_scale[row] = __fmul_rn(amax, INV127);
+        }
+        const float inv = __fdiv_rn(127.0f, amax);
+        if constexpr (CPT > 0) {
+#pragma unroll
+            for (int i = 0; i < CPT; ++i) {
+                const int c = tid + i * threads;
+                if (c < n4) {
+                    __stcs(dst + c, requant4<DIRECT>(a[i], inv));
+                }
+            }
+        } else {
+            for (int64_t c = tid; c < n4; c += threads) {
+                __stcs(dst + c, requant4<DIRECT>(src[c], inv));
+            }
+        }
     }
+}
+
+template <bool DIRECT>
+static cudaError_t requant(const float* act, int8_t* y, float* y_scale, int64_t M, int64_t H, const GroupedHeader* header,
+                           cudaStream_t st)
+{
+    constexpr int CPT = 4;
+    const int64_t n4 = H / 4;
+    const bool held = n4 <= 1024 * CPT;
+    const int threads = held ? static_cast<int>((n4 + 32 * CPT - 1) / (32 * CPT)) * 32 : 1024;
+    auto kern = held ? gmsq_requant_kernel<DIRECT, CPT> : gmsq_requant_kernel<DIRECT, 0>;
+    const int64_t cap = static_cast<int64_t>(sm_count()) * std::min(32, std::max(1, 65536 / (40 * threads)));  // 37 registers
+    return launch_chained(kern, static_cast<unsigned>(std::min(M, cap)), static_cast<unsigned>(threads), 0, st, act, y, y_scale,
+                          M, H, header);
 }
 
 static inline size_t align_up_sz(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -1040,9 +1095,9 @@ extern "C" int w8a8_grouped_matmul_swiglu_quant(const int8_t* x, const int8_t* w
         p.y_scale = y_scale;
         p.round_direct = (flags & W8A8_F_ROUND_DIRECT) ? 1 : 0;
         fused = p.fuse_requant != 0;
-        // row maxima and finished-tile counters start at zero
-        const int rc = run_grouped<KIND_I8, EPI_GMSQ>(group_list, list_on_device, E, M, g, b_mn, x, tb, p, st, g.amax,
-                                                      g.clear_bytes);
+        // row maxima and finished-tile counters, where the matmul kernels requantise, start at zero
+        const int rc = run_grouped<KIND_I8, EPI_GMSQ>(group_list, list_on_device, E, M, g, b_mn, x, tb, p, st,
+                                                      fused ? g.amax : nullptr, fused ? g.clear_bytes : 0);
         if (rc != W8A8_OK) {
             return rc;
         }
@@ -1050,16 +1105,8 @@ extern "C" int w8a8_grouped_matmul_swiglu_quant(const int8_t* x, const int8_t* w
     if (!run_requant || fused) {
         return W8A8_OK;
     }
-    // few rows: up to four warps share one, so that its loads do not wait for one another
-    const int64_t cap = static_cast<int64_t>(sm_count()) * 8;
-    const int parts = (M * 4 <= cap * 8) ? 4 : 1;
-    int64_t blocks = (M * parts + 7) / 8;
-    if (blocks > cap) {
-        blocks = cap;
-    }
-    auto kern = (flags & W8A8_F_ROUND_DIRECT) ? gmsq_requant_kernel<true> : gmsq_requant_kernel<false>;
-    const cudaError_t e = launch_chained(kern, static_cast<unsigned>(blocks), 256, 0, st, g.act, g.amax, y, y_scale, M, H,
-                                         g.header, parts);
+    const cudaError_t e = (flags & W8A8_F_ROUND_DIRECT) ? requant<true>(g.act, y, y_scale, M, H, g.header, st)
+                                                        : requant<false>(g.act, y, y_scale, M, H, g.header, st);
     return launch_status(e);
 }
 

@@ -269,7 +269,7 @@ struct GemmParams {
     int32_t prefetch_k_blocks;
     int32_t order;  // ORDER_*
     float* act;       // GMSQ: fp32 activations [M, N/2]
-    uint32_t* amax;   // GMSQ: per-row max|act| bit patterns
+    uint32_t* amax;   // GMSQ with fuse_requant: per-row max|act| bit patterns
     // GMSQ with the requantisation fused in: the CTA that finishes the last column tile of its rows quantises them
     int32_t* tile_done;   // per (row tile, CTA of the tile): epilogue warps done with a column tile (zeroed by the caller)
     int8_t* y;            // [M, N/2]
@@ -422,19 +422,43 @@ __device__ __forceinline__ void qmm_dequant(const GemmParams& p, const QmmTerms&
     }
 }
 
-// Requantisation of one finished row of SwiGLU activations, 16-byte pieces [c_lo, c_hi) of it, by one warp:
-// amax clamp at FLT_MIN, y_scale = amax * (1/127), inv = 127 / amax, clamp to [-128, 127], narrowing
-// (gmsq_vec_kernel.cpp:233-257).  The activations and row maxima were written by other SMs: they are read through
-// L2 (ld.global.cg), never through this SM's L1.
+// Requantisation of a row of SwiGLU activations by its largest magnitude: amax clamp at FLT_MIN, y_scale = amax * (1/127),
+// inv = 127 / amax, clamp to [-128, 127], narrowing (gmsq_vec_kernel.cpp:233-257).
+__device__ __forceinline__ float requant_amax(float amax) { return amax > 1.1754944e-38f ? amax : 1.1754944e-38f; }
+
+// largest magnitude of four activations and `m`, NaN left out
+__device__ __forceinline__ float requant_max4(float m, const float4& a)
+{
+    return fmaxf(fmaxf(fmaxf(m, fabsf(a.x)), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w)));
+}
+
+template <bool DIRECT>
+__device__ __forceinline__ uint32_t requant4(const float4& a, float inv)
+{
+    const float w[4] = {__fmul_rn(a.x, inv), __fmul_rn(a.y, inv), __fmul_rn(a.z, inv), __fmul_rn(a.w, inv)};
+    float v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        v[q] = fminf(fmaxf(w[q], -128.0f), 127.0f);
+    }
+    uint32_t packed = narrow4_fast<DIRECT>(v[0], v[1], v[2], v[3]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (w[q] != w[q]) {  // a NaN activation narrows to 0 (fmaxf / fminf turned it into a bound)
+            packed &= ~(0xffu << (8 * q));
+        }
+    }
+    return packed;
+}
+
+// 16-byte pieces [c_lo, c_hi) of one finished row by one warp, inside the matmul kernel.  The activations and row maxima
+// were written by other SMs: they are read through L2 (ld.global.cg), never through this SM's L1.
 template <bool DIRECT>
 __device__ __forceinline__ void requant_row_part(const float* act, const uint32_t* amax_bits, int8_t* y, float* y_scale,
                                                  int64_t row, int64_t H, int64_t c_lo, int64_t c_hi, bool write_scale,
                                                  int lane)
 {
-    float amax = __uint_as_float(__ldcg(amax_bits + row));
-    if (!(amax > 1.1754944e-38f)) {
-        amax = 1.1754944e-38f;
-    }
+    const float amax = requant_amax(__uint_as_float(__ldcg(amax_bits + row)));
     if (write_scale && lane == 0) {
         y_scale[row] = __fmul_rn(amax, INV127);
     }
@@ -454,24 +478,9 @@ __device__ __forceinline__ void requant_row_part(const float* act, const uint32_
 #pragma unroll
         for (int j = 0; j < DEPTH; ++j) {
             const int64_t c = c0 + lane + 32 * j;
-            if (c >= c_hi) {
-                continue;
+            if (c < c_hi) {
+                __stcs(dst + c, requant4<DIRECT>(a[j], inv));
             }
-            const float w[4] = {__fmul_rn(a[j].x, inv), __fmul_rn(a[j].y, inv), __fmul_rn(a[j].z, inv),
-                                __fmul_rn(a[j].w, inv)};
-            float v[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                v[q] = fminf(fmaxf(w[q], -128.0f), 127.0f);
-            }
-            uint32_t packed = narrow4_fast<DIRECT>(v[0], v[1], v[2], v[3]);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                if (w[q] != w[q]) {  // a NaN activation narrows to 0 (fmaxf / fminf turned it into a bound)
-                    packed &= ~(0xffu << (8 * q));
-                }
-            }
-            __stcs(dst + c, packed);
         }
     }
 }
@@ -830,7 +839,7 @@ __device__ __forceinline__ bool epilogue_tile(const GemmParams& p, const TileInf
                     float a[8];
                     swiglu8(g + 8 * h, u + 8 * h, xs, wsg + col0 + 8 * h, wsg + H + col0 + 8 * h, a);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
+                    for (int j = 0; j < 8 && p.fuse_requant; ++j) {
                         local_max = fmaxf(local_max, fabsf(a[j]));
                     }
 #pragma unroll
@@ -863,7 +872,7 @@ __device__ __forceinline__ bool epilogue_tile(const GemmParams& p, const TileInf
             }
             __syncwarp();
         }
-        if (row_ok) {
+        if (p.fuse_requant && row_ok) {  // (the kernel that requantises otherwise has whole rows in hand)
             atomicMax(reinterpret_cast<int*>(p.amax + row), __float_as_int(local_max));
         }
     } else if (EPI == EPI_RAW || (KIND == KIND_BF16 && p.out_dtype == W8A8_DT_F32)) {
