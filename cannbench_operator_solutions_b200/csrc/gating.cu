@@ -162,7 +162,8 @@ __global__ void __launch_bounds__(GATING_WARPS * 32) gating_kernel(const void* x
 // row whose maximum is not finite, goes to the whole warp.  fp32 rows are selected on the exponential above the column
 // in 64 bits, where the question does not arise.
 //
-// Bound: issue slots.  65536 x 256 bf16, k = 8: 24 us, was 55 with a warp per row (869 warp instructions per row); fp32: 45 us.
+// Bound: issue slots.  65536 x 256 bf16, k = 8: 24 us (18 where rows are held, see below), was 55 with a warp per row (869
+// warp instructions per row); fp32: 45 us.
 // ---------------------------------------------------------------------------
 constexpr int GATING_TOP = 8;
 constexpr int GATING_TOP_THREADS = 64;
@@ -446,7 +447,143 @@ __device__ __noinline__ void gating_settle(const void* x, int64_t row0, int64_t 
     }
 }
 
-template <int DT, bool VEC>
+// ---------------------------------------------------------------------------
+// Rows of 129 to 256 aligned 16-bit elements: the four lanes hold their row, up to eight pieces of eight elements each, and
+// sort only what can be selected.  The eighth largest of the row's 32 piece maxima is no larger than its eighth largest
+// element, so only elements at or above it count: about eleven of 256, found with packed comparisons and picked out one by
+// one.  A lane that has more than eight of them (rows of ties) sends its warp back to sorting every piece.
+// Bound: issue slots, the integer pipe above all, of which sorting every piece takes half.  65536 x 256 bf16, k = 8 18.3 us
+// (24.3 sorting every piece), x 160 14.7 (16.1), 16384 x 256 7.3 (8.3); rows that come back - few different values, or in
+// order - 25.5 (22.9).  A grid that does not fill the chip twice waits for the longer chain: 8192 x 256 5.7 (5.5).
+// ---------------------------------------------------------------------------
+constexpr int GATING_HELD_PIECES = 8;
+constexpr int64_t GATING_HELD_ROWS = 12288;
+
+template <int DT>
+struct Half2 {
+    using type = std::conditional_t<DT == W8A8_DT_BF16, __nv_bfloat162, __half2>;
+    static constexpr uint32_t NEG_INF = (DT == W8A8_DT_BF16) ? 0xff80ff80u : 0xfc00fc00u;
+    static __device__ __forceinline__ type of(uint32_t w) { return *reinterpret_cast<const type*>(&w); }
+    static __device__ __forceinline__ uint32_t bits(type v) { return *reinterpret_cast<const uint32_t*>(&v); }
+    static __device__ __forceinline__ uint32_t max_nan(uint32_t a, uint32_t b) { return bits(__hmax2_nan(of(a), of(b))); }
+    // all ones in the halves in which a >= b
+    static __device__ __forceinline__ uint32_t at_least(uint32_t a, uint32_t b) { return __hge2_mask(of(a), of(b)); }
+};
+
+// The row's pieces of this lane, the row's maximum, and whether the row is not a regular one
+template <int DT>
+__device__ __forceinline__ void gating_hold(const void* x, int64_t row, int inner, int q, uint4 (&raw)[GATING_HELD_PIECES],
+                                            float (&top)[GATING_HELD_PIECES])
+{
+    using H = Half2<DT>;
+    const uint4* p = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(x) + row * inner) + q;
+#pragma unroll
+    for (int i = 0; i < GATING_HELD_PIECES; ++i) {
+        raw[i] = make_uint4(H::NEG_INF, H::NEG_INF, H::NEG_INF, H::NEG_INF);
+        if (8 * (4 * i + q) < inner) {
+            raw[i] = __ldca(p + 4 * i);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < GATING_HELD_PIECES; ++i) {
+        float lo, hi;
+        unpack2<DT>(H::max_nan(H::max_nan(raw[i].x, raw[i].y), H::max_nan(raw[i].z, raw[i].w)), lo, hi);
+        top[i] = max_nan(lo, hi);
+    }
+}
+
+// best = the lane's eight largest keys (fewer, and INT32_MIN, where it has fewer elements that can be selected)
+template <int DT>
+__device__ __forceinline__ void gating_held_best(const void* x, int64_t row, int inner, int q,
+                                                 const uint4 (&raw)[GATING_HELD_PIECES],
+                                                 const float (&top)[GATING_HELD_PIECES], int (&best)[8])
+{
+    using H = Half2<DT>;
+    int t[8], other[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        t[i] = gating_ordered(top[i]);
+    }
+    sort8_desc(t);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        other[i] = __shfl_xor_sync(FULL_MASK, t[i], 2);
+    }
+    merge8_desc(t, other);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        other[i] = __shfl_xor_sync(FULL_MASK, t[i], 1);
+    }
+    int eighth = max(t[0], other[7]);
+#pragma unroll
+    for (int i = 1; i < 8; ++i) {
+        eighth = min(eighth, max(t[i], other[7 - i]));
+    }
+    const float least = gating_value(eighth);
+    const uint32_t least2 = pack2<DT>(least, least);
+    // bit 4 (i % 4) + w of half h: element 2 w + h of piece i
+    uint32_t found[2] = {0u, 0u};
+#pragma unroll
+    for (int i = 0; i < GATING_HELD_PIECES; ++i) {
+        const uint32_t word[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            found[i >> 2] |= H::at_least(word[w], least2) & (0x00010001u << (4 * (i & 3) + w));
+        }
+    }
+    const int count = __popc(found[0]) + __popc(found[1]);
+    const int most = __reduce_max_sync(FULL_MASK, count);
+    if (most > 8) {
+        const int pieces = (inner + 31) / 32;
+#pragma unroll 1
+        for (int i = 0; i < pieces; ++i) {
+            float v[8];
+            gating_load8<DT, true>(x, row, inner, 4 * i + q, v);
+            int key[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                key[j] = gating_ordered(v[j]) + (GATING_COL_MASK - 32 * i - 8 * q - j);
+            }
+            sort8_desc(key);
+            if (i == 0) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    best[j] = key[j];
+                }
+            } else {
+                merge8_desc(best, key);
+            }
+        }
+        return;
+    }
+    const uint16_t* xr = static_cast<const uint16_t*>(x) + row * inner;
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+        best[n] = INT32_MIN;
+    }
+#pragma unroll
+    for (int n0 = 0; n0 < 8; n0 += 4) {
+        if (n0 < most) {
+#pragma unroll
+            for (int n = n0; n < n0 + 4; ++n) {
+                const bool low = found[0] != 0u;
+                const uint32_t from = low ? found[0] : found[1];
+                const int bit = __ffs(from) - 1;
+                found[0] &= found[0] - 1u;
+                found[1] = low ? found[1] : (found[1] & (found[1] - 1u));
+                const int at = bit & 15;
+                const int col = 32 * ((at >> 2) + (low ? 0 : 4)) + 8 * q + 2 * (at & 3) + (bit >> 4);
+                if (n < count) {
+                    best[n] = gating_ordered(bits16_to_float<DT>(xr[col])) + (GATING_COL_MASK - col);
+                }
+            }
+        }
+    }
+    sort8_desc(best);
+}
+
+// HELD: rows of 129 to 256 aligned 16-bit elements
+template <int DT, bool VEC, bool HELD>
 __global__ void __launch_bounds__(GATING_TOP_THREADS) gating_top8_kernel(const void* x,
                                                                          const uint8_t* finished,
                                                                          void* __restrict__ y,
@@ -467,65 +604,95 @@ __global__ void __launch_bounds__(GATING_TOP_THREADS) gating_top8_kernel(const v
     const int64_t row = mine < rows ? mine : rows - 1;  // lanes past the last row work on it and store nothing
     const int pieces = (inner + 31) / 32;
 
-    float m = -INFINITY;
-#pragma unroll 4
-    for (int i = 0; i < pieces; ++i) {
-        float v[8];
-        gating_load8<DT, VEC>(x, row, inner, 4 * i + q, v);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            m = max_nan(m, v[j]);
-        }
-    }
-    m = max_nan(m, __shfl_xor_sync(FULL_MASK, m, 1));
-    m = max_nan(m, __shfl_xor_sync(FULL_MASK, m, 2));
-    bool redo = !(fabsf(m) < INFINITY);
-
     Key best[8];
     f32x2 sum[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         sum[i] = pair(0.0f);
     }
-    // two pieces per step: 4096 x 256 bf16 4.5 us, 4.9 one at a time; 4096 x 1024 12.4, 13.2; 65536 x 256 22.8, 23.8
+    float m = -INFINITY;
+    if constexpr (HELD) {
+        uint4 raw[GATING_HELD_PIECES];
+        float top[GATING_HELD_PIECES];
+        gating_hold<DT>(x, row, inner, q, raw, top);
+#pragma unroll
+        for (int i = 0; i < GATING_HELD_PIECES; ++i) {
+            m = max_nan(m, top[i]);
+        }
+        m = max_nan(m, __shfl_xor_sync(FULL_MASK, m, 1));
+        m = max_nan(m, __shfl_xor_sync(FULL_MASK, m, 2));
+        gating_held_best<DT>(x, row, inner, q, raw, top, best);
+#pragma unroll
+        for (int i = 0; i < GATING_HELD_PIECES; ++i) {
+            if (i < pieces) {
+                const uint32_t word[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+                f32x2 d[4], e[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    float lo, hi;
+                    unpack2<DT>(word[j], lo, hi);
+                    d[j] = add2(pair(lo, hi), pair(-m));
+                }
+                exp_nonpositive2<4>(d, e);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    sum[j] = add2(sum[j], e[j]);
+                }
+            }
+        }
+    } else {
+#pragma unroll 4
+        for (int i = 0; i < pieces; ++i) {
+            float v[8];
+            gating_load8<DT, VEC>(x, row, inner, 4 * i + q, v);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                m = max_nan(m, v[j]);
+            }
+        }
+        m = max_nan(m, __shfl_xor_sync(FULL_MASK, m, 1));
+        m = max_nan(m, __shfl_xor_sync(FULL_MASK, m, 2));
+        // two pieces per step: 4096 x 256 bf16 4.5 us, 4.9 one at a time; 4096 x 1024 12.4, 13.2; 65536 x 256 22.8, 23.8
 #pragma unroll 2
-    for (int i = 0; i < pieces; ++i) {
-        float v[8];
-        gating_load8<DT, VEC>(x, row, inner, 4 * i + q, v);
-        const int col = 32 * i + 8 * q;
-        f32x2 d[4], e[4];
+        for (int i = 0; i < pieces; ++i) {
+            float v[8];
+            gating_load8<DT, VEC>(x, row, inner, 4 * i + q, v);
+            const int col = 32 * i + 8 * q;
+            f32x2 d[4], e[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            d[j] = add2(pair(v[2 * j], v[2 * j + 1]), pair(-m));
-        }
-        exp_nonpositive2<4>(d, e);
-        Key key[8];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            sum[j] = add2(sum[j], e[j]);
-            if constexpr (WIDE) {
-                float e0, e1;
-                unpair(e[j], e0, e1);
-                key[2 * j] = (static_cast<Key>(__float_as_uint(e0)) << 32) | static_cast<uint32_t>(~(col + 2 * j));
-                key[2 * j + 1] = (static_cast<Key>(__float_as_uint(e1)) << 32) | static_cast<uint32_t>(~(col + 2 * j + 1));
+            for (int j = 0; j < 4; ++j) {
+                d[j] = add2(pair(v[2 * j], v[2 * j + 1]), pair(-m));
             }
-        }
-        if constexpr (!WIDE) {
+            exp_nonpositive2<4>(d, e);
+            Key key[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                key[j] = gating_ordered(v[j]) + (GATING_COL_MASK - col - j);
+            for (int j = 0; j < 4; ++j) {
+                sum[j] = add2(sum[j], e[j]);
+                if constexpr (WIDE) {
+                    float e0, e1;
+                    unpair(e[j], e0, e1);
+                    key[2 * j] = (static_cast<Key>(__float_as_uint(e0)) << 32) | static_cast<uint32_t>(~(col + 2 * j));
+                    key[2 * j + 1] = (static_cast<Key>(__float_as_uint(e1)) << 32) | static_cast<uint32_t>(~(col + 2 * j + 1));
+                }
             }
-        }
-        sort8_desc(key);
-        if (i == 0) {
+            if constexpr (!WIDE) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                best[j] = key[j];
+                for (int j = 0; j < 8; ++j) {
+                    key[j] = gating_ordered(v[j]) + (GATING_COL_MASK - col - j);
+                }
             }
-        } else {
-            merge8_desc(best, key);
+            sort8_desc(key);
+            if (i == 0) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    best[j] = key[j];
+                }
+            } else {
+                merge8_desc(best, key);
+            }
         }
     }
+    bool redo = !(fabsf(m) < INFINITY);
     float part[8];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -613,10 +780,16 @@ static cudaError_t launch_gating_top8(const void* x, const uint8_t* finished, vo
     constexpr int64_t ROWS = GATING_TOP_THREADS / 4;
     const unsigned grid = static_cast<unsigned>((rows + ROWS - 1) / ROWS);
     if (inner % 8 == 0 && is_aligned(x, 16)) {
-        return launch_router<gating_top8_kernel<DT, true>>(grid, GATING_TOP_THREADS, st, x, finished, y, expert_idx, row_idx,
+        if constexpr (DT != W8A8_DT_F32) {
+            if (inner > 128 && inner <= 32 * GATING_HELD_PIECES && rows >= GATING_HELD_ROWS) {
+                return launch_router<gating_top8_kernel<DT, true, true>>(grid, GATING_TOP_THREADS, st, x, finished, y,
+                                                                         expert_idx, row_idx, rows, inner, k);
+            }
+        }
+        return launch_router<gating_top8_kernel<DT, true, false>>(grid, GATING_TOP_THREADS, st, x, finished, y, expert_idx, row_idx,
                                                            rows, inner, k);
     }
-    return launch_router<gating_top8_kernel<DT, false>>(grid, GATING_TOP_THREADS, st, x, finished, y, expert_idx, row_idx,
+    return launch_router<gating_top8_kernel<DT, false, false>>(grid, GATING_TOP_THREADS, st, x, finished, y, expert_idx, row_idx,
                                                         rows, inner, k);
 }
 
