@@ -17,6 +17,7 @@
 //
 // Mapping: one 256-thread CTA per row at a time; the row's z values stay in
 // registers between the reductions and the quantisation.
+#include "beside.cuh"
 #include "common.cuh"
 
 namespace w8a8 {

@@ -484,9 +484,9 @@ void note_launch();  // counts one kernel launch of this library (w8a8_kernel_la
 // stream is still running: its launch, block setup and prologue then overlap that kernel's tail instead of following
 // it.  Every such kernel opens with after_previous(), which waits until the kernel before it has completed and its
 // writes are visible; no global memory is touched before that, neither read nor written (the dense matmuls ask for
-// weights into L2, which reads nothing; the second of a grouped matmul's two launches has an order of its own, see
-// gemm_kernel.cuh).  It also lets the next kernel start.  A grid of at most one block per SM does so before its own wait, which takes 0.2 - 0.3 us off a short kernel; a
-// larger one after it: with three kernels resident at once their blocks share the SMs unevenly (back to back, the router
+// weights into L2, which reads nothing; kernels beside the one before them have an order of their own, see
+// beside.cuh).  It also lets the next kernel start.  A grid of at most one block per SM does so before its own wait,
+// which takes 0.2 - 0.3 us off a short kernel; a larger one after it: with three kernels resident at once their blocks share the SMs unevenly (back to back, the router
 // on 16384 rows of 256 bf16 takes 9.0 us, 13.4 if it lets the next one in ahead of the wait; the SwiGLU quantiser on 300
 // rows of 16384 int32 47 us, 67).  BY_GRID = false: after it in any case - the SwiGLU quantiser, whose registers are used
 // up (16384 rows of 2816 int32 90 us, 99 with the grid asked for), and the sums of gathered rows, whose few blocks run
@@ -520,20 +520,6 @@ __device__ __forceinline__ int64_t after_previous()
     }
     return zero;
 }
-
-// For a kernel that reads nothing of what the kernel before it writes and writes nothing that it reads, where that one
-// lets it in only after its own wait (after_previous<false>): all that came before the two is then complete, and this one
-// need not wait at its start.  It waits at its end instead (previous_complete), so that whoever waits for it has waited
-// for both.
-__device__ __forceinline__ int64_t beside_previous()
-{
-    int64_t zero;
-    // no line that this SM's L1 holds from before
-    asm volatile("griddepcontrol.launch_dependents;\n\tfence.acq_rel.gpu;\n\tmov.u64 %0, 0;" : "=l"(zero)::"memory");
-    return zero;
-}
-
-__device__ __forceinline__ void previous_complete() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // overlap = false: starts when the kernel before it has completed, like a plain launch.
 template <typename... Params, typename... Args>
@@ -572,7 +558,7 @@ inline int launch_status(cudaError_t e)
     return W8A8_OK;
 }
 
-// w8a8_add_rms_norm_dynamic_quant launched beside the kernel before it (see beside_previous)
+// w8a8_add_rms_norm_dynamic_quant launched beside the kernel before it (see beside.cuh)
 int add_rms_norm_dynamic_quant_beside(const void* x1, const void* x2, const void* gamma, int8_t* y, void* x_out,
                                       float* scale_out, int64_t rows, int64_t N, float epsilon, int dtype, void* stream);
 // w8a8_dispatch_rows where every pair's row goes to row `expanded_pos` of one buffer

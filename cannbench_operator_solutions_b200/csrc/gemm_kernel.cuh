@@ -36,14 +36,16 @@
 //
 // Dense problems enumerate (row tile, column tile) with the row index fastest
 // so that concurrently running CTAs share a B column block in L2.  Grouped
-// problems read a tile table built on the device from the cumulative group
-// list (tiles never straddle groups; rows past a group's end inside a tile
-// are computed and discarded) with the column index fastest, so the A tile
-// and the expert's weights stay L2-resident.
+// problems cut the cumulative group list into tiles - every CTA for itself, or
+// a kernel ahead of this one where there are many groups - that never straddle
+// groups (rows past a group's end inside a tile are computed and discarded),
+// with the column index fastest, so the A tile and the expert's weights stay
+// L2-resident.
 #pragma once
 
 #include <type_traits>
 
+#include "beside.cuh"
 #include "common.cuh"
 #include "tc_ptx.cuh"
 
