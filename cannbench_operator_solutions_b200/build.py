@@ -2,9 +2,9 @@
 
 ``python -m cannbench_operator_solutions_b200.build`` compiles
 ``libw8a8ffn.so`` (the C-ABI library, plain CUDA runtime, no torch) for
-sm_100a next to this file, then the torch plugin that registers the
-``cann_bench::*`` operator schemas on top of it.  nvcc cross-compiles without
-a GPU.
+sm_100a next to this file, then, on top of it, the torch plugin that registers
+the ``cann_bench::*`` operator schemas and the native half of ``ops.py``.  nvcc
+cross-compiles without a GPU.
 """
 from __future__ import annotations
 

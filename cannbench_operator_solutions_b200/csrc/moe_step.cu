@@ -7,6 +7,8 @@
 //   barrier -> grouped_matmul_swiglu_quant -> int8 down projection whose
 //   epilogue stores every row where its home rank's combine reads it ->
 //   barrier -> combine (MoeFinalizeRouting's weighted sum).
+// With one rank and room for all its rows the exchange, its tables and the
+// second stream fall away (one_rank_step).
 // The only collectives are the all-gather of the per-expert counts and two
 // one-word all-reduces used as stream-ordered barriers; they run on an NCCL
 // communicator this file creates.  NCCL is not a link-time dependency: its

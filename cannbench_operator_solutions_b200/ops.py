@@ -6,7 +6,8 @@ ai-jiaqian/cannbench-operator-solutions (schemas cited per function; paths
 relative to that project).  Validation mirrors the reference plugins'
 ``TORCH_CHECK``s and raises ``RuntimeError`` like they do.  The work itself is
 one call through the C-ABI on the current CUDA stream; PyTorch only provides
-device memory and the stream.
+device memory and the stream.  Calls in their plain form take the same steps in
+native code (``csrc/plugin/py_calls.cpp``).
 """
 from __future__ import annotations
 

@@ -57,10 +57,10 @@ extern "C" {
 
 /* grouped_matmul_swiglu_quant only: run one of its two stages, which the
  * reference exposes as two launchers (launch_gmsq_cube, launch_gmsq_vec).
- * Neither bit set = both stages.  The workspace carries the activations and
- * row maxima from the first stage to the second. */
-#define W8A8_F_STAGE_MATMUL 2  /* plan + tensor-core matmul + fused dequant/SwiGLU/row-max */
-#define W8A8_F_STAGE_REQUANT 4 /* per-row requantisation of the stored activations        */
+ * Neither bit set = both stages.  The workspace carries the activations from
+ * the first stage to the second. */
+#define W8A8_F_STAGE_MATMUL 2  /* plan + tensor-core matmul + fused dequant/SwiGLU        */
+#define W8A8_F_STAGE_REQUANT 4 /* per-row maximum and requantisation of the activations  */
 
 /* weight layout of the matmuls */
 #define W8A8_W_KN 0 /* [.., K, N], N contiguous: the reference's layout       */
@@ -458,8 +458,8 @@ int w8a8_gmsq_host_pipe_destroy(W8A8HostPipe* pipe);
  * A step that routes more than cap_rows rows to some rank stores nothing out of bounds: that step's tables are
  * zeroed, its output is meaningless, and a sticky flag is raised that w8a8_moe_ffn_step_status reads and clears
  * (returns 1; it synchronises the stream).  Every rank must make the same sequence of step calls.
- * The step runs two of its pieces (the normalisation + quantisation of the tokens, the row-pointer expansion) on a
- * second stream that the library keeps per device, forked from and joined to `stream` by events: for the caller
+ * With one rank and cap_rows for all of its rows the step is one chain of kernels on `stream`.  Otherwise it runs two of
+ * its pieces (the normalisation + quantisation of the tokens, the row-pointer expansion) on a second stream that the library keeps per device, forked from and joined to `stream` by events: for the caller
  * the step is ordered on `stream` like any other call, a stream capture follows both streams, and one step at a
  * time may be in the making per device (two host threads must not call it for the same device at once).
  */
