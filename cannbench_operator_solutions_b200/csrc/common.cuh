@@ -558,7 +558,7 @@ inline int launch_status(cudaError_t e)
     return W8A8_OK;
 }
 
-// w8a8_add_rms_norm_dynamic_quant launched beside the kernel before it (see beside.cuh)
+// w8a8_add_rms_norm_dynamic_quant beside the kernel before it (see beside.cuh); unvectorised rows wait for it as ever
 int add_rms_norm_dynamic_quant_beside(const void* x1, const void* x2, const void* gamma, int8_t* y, void* x_out,
                                       float* scale_out, int64_t rows, int64_t N, float epsilon, int dtype, void* stream);
 // w8a8_dispatch_rows where every pair's row goes to row `expanded_pos` of one buffer

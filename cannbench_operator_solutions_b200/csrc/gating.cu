@@ -611,6 +611,7 @@ __global__ void __launch_bounds__(GATING_TOP_THREADS) gating_top8_kernel(const v
         sum[i] = pair(0.0f);
     }
     float m = -INFINITY;
+    bool redo;
     if constexpr (HELD) {
         uint4 raw[GATING_HELD_PIECES];
         float top[GATING_HELD_PIECES];
@@ -621,6 +622,7 @@ __global__ void __launch_bounds__(GATING_TOP_THREADS) gating_top8_kernel(const v
         }
         m = max_nan(m, __shfl_xor_sync(FULL_MASK, m, 1));
         m = max_nan(m, __shfl_xor_sync(FULL_MASK, m, 2));
+        redo = !(fabsf(m) < INFINITY);
         gating_held_best<DT>(x, row, inner, q, raw, top, best);
 #pragma unroll
         for (int i = 0; i < GATING_HELD_PIECES; ++i) {
@@ -652,6 +654,7 @@ __global__ void __launch_bounds__(GATING_TOP_THREADS) gating_top8_kernel(const v
         }
         m = max_nan(m, __shfl_xor_sync(FULL_MASK, m, 1));
         m = max_nan(m, __shfl_xor_sync(FULL_MASK, m, 2));
+        redo = !(fabsf(m) < INFINITY);
         // two pieces per step: 4096 x 256 bf16 4.5 us, 4.9 one at a time; 4096 x 1024 12.4, 13.2; 65536 x 256 22.8, 23.8
 #pragma unroll 2
         for (int i = 0; i < pieces; ++i) {
@@ -692,7 +695,6 @@ __global__ void __launch_bounds__(GATING_TOP_THREADS) gating_top8_kernel(const v
             }
         }
     }
-    bool redo = !(fabsf(m) < INFINITY);
     float part[8];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
