@@ -523,11 +523,11 @@ __device__ __forceinline__ int64_t after_previous()
 
 // overlap = false: starts when the kernel before it has completed, like a plain launch.
 template <typename... Params, typename... Args>
-cudaError_t launch_chained_if(bool overlap, void (*kern)(Params...), unsigned grid, unsigned block, size_t smem,
+cudaError_t launch_chained_if(bool overlap, void (*kern)(Params...), dim3 grid, unsigned block, size_t smem,
                               cudaStream_t st, Args&&... args)
 {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(block, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -541,7 +541,7 @@ cudaError_t launch_chained_if(bool overlap, void (*kern)(Params...), unsigned gr
 }
 
 template <typename... Params, typename... Args>
-cudaError_t launch_chained(void (*kern)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+cudaError_t launch_chained(void (*kern)(Params...), dim3 grid, unsigned block, size_t smem, cudaStream_t st,
                            Args&&... args)
 {
     return launch_chained_if(true, kern, grid, block, smem, st, static_cast<Args&&>(args)...);

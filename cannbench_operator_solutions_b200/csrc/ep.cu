@@ -12,6 +12,8 @@
 //
 // All three are HBM-bound byte movers: 128-bit accesses, a row read once and
 // written topk times (scatter) or topk rows read and one written (combine).
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace w8a8 {
@@ -792,15 +794,16 @@ __device__ __forceinline__ float load_scalar_as_f32(const void* p, int64_t i, in
     return (dt == W8A8_DT_BF16) ? bits16_to_float<W8A8_DT_BF16>(b) : bits16_to_float<W8A8_DT_F16>(b);
 }
 
-// One CTA per output row.  The K (position, scale, expert) triples of the row are staged in shared memory once;
-// every thread then owns 16-byte chunks of the hidden dimension and, for MFR_BATCH values of k at a time, issues
-// all its row (and bias) loads before it touches the accumulator, so up to MFR_BATCH gathers are in flight per
+// One CTA per output row, or several (grid.y; see mfr_shape).  The K (position, scale, expert) triples of the row are
+// staged in shared memory once; every thread then owns 16-byte chunks of the hidden dimension and, for MFR_BATCH values
+// of k at a time, issues all its row (and bias) loads before it touches the accumulator, so up to MFR_BATCH gathers are in flight per
 // thread.  Arithmetic order per element: acc = fp32(skip1); acc += fp32(skip2); for ascending k:
 // term = fp32(row) [+ fp32(bias)]; term *= scale; acc += term (no fused multiply-add); RNE store.
 constexpr int MFR_BATCH = 8;
 constexpr int MFR_MAX_STAGED_K = 128;
 
-template <int DT, bool VEC, bool HAS_BIAS, typename IdxT>
+// SPLIT: grid.y CTAs share a row.
+template <int DT, bool VEC, bool HAS_BIAS, typename IdxT, bool SPLIT = false>
 __global__ void __launch_bounds__(256) mfr_kernel(const void* rows, const IdxT* esdr,
                                                   const void* skip1, const void* skip2,
                                                   const void* bias, const void* scales,
@@ -855,7 +858,8 @@ __global__ void __launch_bounds__(256) mfr_kernel(const void* rows, const IdxT* 
             } else {
                 stage(i + gridDim.x, 0, buf ^ 1);
             }
-            for (int c = threadIdx.x; c < nchunks; c += blockDim.x) {
+            for (int c = (SPLIT ? blockIdx.y * blockDim.x : 0) + threadIdx.x; c < nchunks;
+                 c += SPLIT ? gridDim.y * blockDim.x : blockDim.x) {
                 float acc[EL];
                 if (k0 == 0) {
                     if (skip1 != nullptr) {
@@ -1284,6 +1288,58 @@ extern "C" int w8a8_expand_row_pointers(const int64_t* seg_first, const uint64_t
     return (cudaGetLastError() == cudaSuccess) ? W8A8_OK : W8A8_ERR_CUDA;
 }
 
+namespace w8a8 {
+
+struct MfrShape {
+    dim3 grid;
+    unsigned threads;
+};
+
+// The combine's CTAs, for rows of `chunks` 16-byte chunks.  VEC: few rows take one pass over a row - on one CTA of as
+// many threads as that needs (256 if no SM has two: 41 sums of eight of 1120 after their regrouping 8.6 us, 8.9 on
+// 160), or, where 256 are not enough and `may_split`, on several (one sum of eight rows of 6256 16-bit elements 6.6 ->
+// 2.7 us, 64 of eight of 4096 4.25 -> 2.97, 653 of four of 1072 4.55 -> 3.47, in a row of calls).  Others run on 96,
+// 128 or 160 threads - the fewest that leave no more than 6 % more of their passes over a row empty than the best of
+// the three - and 3072 threads per SM in all: 256 left most of a last pass empty (a row of 2176 elements is 272 chunks)
+// and let all of them wait for a row's look-up at once (16000 sums of four of 2176 122.7 -> 91.7 us, 23000 of two of
+// 1184 90.4 -> 68.4, 3761 of eight of 4432 64.8 -> 56.1, 8192 of eight of 7168 193 -> 189).  256 threads and 8 CTAs per
+// SM, as it was for all rows, stay where their passes are as full (50000 rows of 6144 regrouped, then summed by eights:
+// 232 us, 237 on 96), where the rows are too few to fill half of the smaller CTAs' places (470 sums of eight of 4432
+// after their regrouping 22.7 us, 31 on 96), and for rows that are read an element at a time.  The split is a form of
+// its own: in every kernel it cost 8 % (59463 rows of 2176 regrouped, summed by fours: 119 us, 129).
+static MfrShape mfr_shape(int64_t rows, int64_t chunks, int64_t K, bool vec, bool may_split)
+{
+    const int64_t sms = sm_count();
+    const unsigned few = static_cast<unsigned>(std::min<int64_t>(rows, sms * 8));
+    if (!vec) {
+        return {dim3(few), 256};
+    }
+    // (a CTA looks up a row's terms with a thread each)
+    const int64_t least = std::max<int64_t>(32, std::min<int64_t>(K, MFR_MAX_STAGED_K));
+    const int64_t share = (chunks + 255) / 256;
+    if (rows * share <= sms * 16 && (share == 1 || (may_split && share <= 65535))) {
+        const int64_t threads = share == 1 && rows <= sms ? 256 : std::max((chunks + share - 1) / share, least);
+        return {dim3(static_cast<unsigned>(rows), static_cast<unsigned>(share)), static_cast<unsigned>((threads + 31) / 32 * 32)};
+    }
+    auto used = [&](int64_t threads) {
+        return static_cast<double>(chunks) / static_cast<double>((chunks + threads - 1) / threads * threads);
+    };
+    const double best = std::max({used(96), used(128), used(160)});
+    int64_t threads = 160;
+    for (int64_t t : {128, 96}) {
+        if (t >= least && used(t) >= best - 0.06) {
+            threads = t;
+        }
+    }
+    const int64_t places = sms * (3072 / threads);
+    if (used(256) >= best || rows < places / 2) {
+        return {dim3(few), 256};
+    }
+    return {dim3(static_cast<unsigned>(std::min<int64_t>(rows, places))), static_cast<unsigned>(threads)};
+}
+
+}  // namespace w8a8
+
 extern "C" int w8a8_combine(const void* rows, const float* probs, const int64_t* expanded_pos, void* out, int64_t T,
                             int64_t topk, int64_t H, int dtype, void* stream)
 {
@@ -1301,8 +1357,7 @@ extern "C" int w8a8_combine(const void* rows, const float* probs, const int64_t*
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool vec = (H % 8 == 0) && w8a8::is_aligned(rows, 16) && w8a8::is_aligned(out, 16);
-    const int64_t cap = static_cast<int64_t>(w8a8::sm_count()) * 8;
-    const unsigned grid = static_cast<unsigned>(T < cap ? T : cap);
+    const w8a8::MfrShape shape = w8a8::mfr_shape(T, H / 8, topk, vec, true);
     // The scales-only, row-arranged case of the finalize kernel with 64-bit positions (no upper bound on them).
     if (topk > w8a8::MFR_MAX_STAGED_K) {
         return W8A8_ERR_LIMIT;
@@ -1312,9 +1367,12 @@ extern "C" int w8a8_combine(const void* rows, const float* probs, const int64_t*
                            : w8a8::mfr_kernel<W8A8_DT_BF16, false, false, int64_t>)
                     : (vec ? w8a8::mfr_kernel<W8A8_DT_F16, true, false, int64_t>
                            : w8a8::mfr_kernel<W8A8_DT_F16, false, false, int64_t>);
-    const cudaError_t e = w8a8::launch_chained(kern, grid, 256, 0, st, rows, expanded_pos, nullptr, nullptr, nullptr,
-                                               probs,
-                                               nullptr, out, T, H, static_cast<int>(topk), 0, INT64_MAX, 0, W8A8_DT_F32);
+    if (shape.grid.y > 1) {
+        kern = (dtype == W8A8_DT_BF16) ? w8a8::mfr_kernel<W8A8_DT_BF16, true, false, int64_t, true>
+                                       : w8a8::mfr_kernel<W8A8_DT_F16, true, false, int64_t, true>;
+    }
+    const cudaError_t e = w8a8::launch_chained(kern, shape.grid, shape.threads, 0, st, rows, expanded_pos, nullptr, nullptr,
+                                               nullptr, probs, nullptr, out, T, H, static_cast<int>(topk), 0, INT64_MAX, 0, W8A8_DT_F32);
     return w8a8::launch_status(e);
 }
 
@@ -1412,15 +1470,16 @@ static int launch_mfr(const void* rows, const int32_t* esdr, const void* skip1, 
                       const void* scales, const int32_t* expert, void* out, int64_t R, int64_t H, int64_t K, int64_t E,
                       int64_t num_dst, int col_mode, int scale_dt, bool vec, cudaStream_t st)
 {
-    const int64_t cap = static_cast<int64_t>(w8a8::sm_count()) * 8;
-    const unsigned grid = static_cast<unsigned>(R < cap ? R : cap);
     const bool has_bias = (bias != nullptr) && (expert != nullptr);
+    const w8a8::MfrShape shape = w8a8::mfr_shape(R, DT == W8A8_DT_F32 ? H / 4 : H / 8, K, vec, !has_bias);
     auto kern = vec ? (has_bias ? w8a8::mfr_kernel<DT, true, true, int32_t> : w8a8::mfr_kernel<DT, true, false, int32_t>)
                     : (has_bias ? w8a8::mfr_kernel<DT, false, true, int32_t>
                                 : w8a8::mfr_kernel<DT, false, false, int32_t>);
-    const cudaError_t e = w8a8::launch_chained(kern, grid, 256, 0, st, rows, esdr, skip1, skip2, bias, scales, expert,
-                                               out, R,
-                                               H, static_cast<int>(K), E, num_dst, col_mode, scale_dt);
+    if (shape.grid.y > 1) {
+        kern = w8a8::mfr_kernel<DT, true, false, int32_t, true>;
+    }
+    const cudaError_t e = w8a8::launch_chained(kern, shape.grid, shape.threads, 0, st, rows, esdr, skip1, skip2, bias, scales,
+                                               expert, out, R, H, static_cast<int>(K), E, num_dst, col_mode, scale_dt);
     return w8a8::launch_status(e);
 }
 
