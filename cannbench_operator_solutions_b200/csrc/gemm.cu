@@ -902,6 +902,32 @@ using namespace w8a8;
 // ===========================================================================
 // quant_matmul
 // ===========================================================================
+// The epilogues read per-channel vectors in 16-byte pieces from their first element on (see load_vec), each batch's bias
+// from its own; a single value and the rows' factors are read as what they are.
+static bool qmm_vectors_aligned(const void* scale, const float* offset, const float* pertoken, const void* bias,
+                                int64_t flags, int64_t batch, int64_t bias_batch_stride)
+{
+    const size_t scale_size = (flags & W8A8_QM_SCALE_BF16) ? 2 : 4;
+    if (!is_aligned(scale, (flags & W8A8_QM_SCALE_PERCHAN) ? 16 : scale_size)) {
+        return false;
+    }
+    if ((flags & W8A8_QM_HAS_OFFSET) && !is_aligned(offset, (flags & W8A8_QM_OFFSET_PERCHAN) ? 16 : 4)) {
+        return false;
+    }
+    if ((flags & W8A8_QM_HAS_PT) && !is_aligned(pertoken, 4)) {
+        return false;
+    }
+    const int64_t bias_kind = (flags & W8A8_QM_BIAS_MASK) >> W8A8_QM_BIAS_SHIFT;
+    if (bias_kind == W8A8_QM_BIAS_NONE) {
+        return true;
+    }
+    const int64_t bias_size = (bias_kind == W8A8_QM_BIAS_F16 || bias_kind == W8A8_QM_BIAS_BF16) ? 2 : 4;
+    if (!(flags & W8A8_QM_BIAS_PERCHAN)) {
+        return is_aligned(bias, static_cast<size_t>(bias_size));
+    }
+    return is_aligned(bias, 16) && (batch == 1 || (bias_batch_stride * bias_size) % 16 == 0);
+}
+
 static int quant_matmul_impl(const int8_t* x1, const int8_t* x2, const void* scale, const float* offset,
                              const float* pertoken, const void* bias, void* out, int64_t batch, int64_t M, int64_t N,
                              int64_t K, int64_t flags, int out_dtype, int x2_layout, int64_t bias_batch_stride,
@@ -932,6 +958,9 @@ static int quant_matmul_impl(const int8_t* x1, const int8_t* x2, const void* sca
         return W8A8_ERR_UNSUPPORTED;
     }
     if (!is_aligned(x1, 16) || !is_aligned(x2, 16) || !is_aligned(out, 16)) {
+        return W8A8_ERR_ALIGN;
+    }
+    if (!raw_i32 && !qmm_vectors_aligned(scale, offset, pertoken, bias, flags, batch, bias_batch_stride)) {
         return W8A8_ERR_ALIGN;
     }
     if (batch * M >= (int64_t(1) << 31) || N >= (int64_t(1) << 31) || K >= (int64_t(1) << 31)) {
@@ -1048,7 +1077,8 @@ extern "C" int w8a8_grouped_matmul_swiglu_quant(const int8_t* x, const int8_t* w
     if ((K % 16) != 0 || (N % 32) != 0) {
         return W8A8_ERR_UNSUPPORTED;
     }
-    if (!is_aligned(x, 16) || !is_aligned(w, 16) || !is_aligned(w_scale, 16) || !is_aligned(y, 4)) {
+    if (!is_aligned(x, 16) || !is_aligned(w, 16) || !is_aligned(w_scale, 16) || !is_aligned(x_scale, 4) || !is_aligned(y, 4) ||
+        !is_aligned(y_scale, 4)) {
         return W8A8_ERR_ALIGN;
     }
     if (M >= (int64_t(1) << 31) - 256 || N >= (int64_t(1) << 31) || K >= (int64_t(1) << 31)) {
@@ -1183,6 +1213,10 @@ static int grouped_matmul_impl(const void* x, const void* w, const void* bias, v
         return W8A8_ERR_UNSUPPORTED;
     }
     if (!is_aligned(x, 16) || !is_aligned(w, 16) || (y != nullptr && !is_aligned(y, 16))) {
+        return W8A8_ERR_ALIGN;
+    }
+    // the epilogue reads both vectors in 16-byte pieces; scales belong to int8 operands only
+    if (!is_aligned(bias, 16) || (kind == KIND_I8 && (!is_aligned(w_scale, 16) || !is_aligned(x_scale, 4)))) {
         return W8A8_ERR_ALIGN;
     }
     if (M >= (int64_t(1) << 31) - 256 || N >= (int64_t(1) << 31) || K >= (int64_t(1) << 31)) {

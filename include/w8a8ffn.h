@@ -24,7 +24,10 @@
  *   - dtype codes: W8A8_DT_F16 / W8A8_DT_BF16 / W8A8_DT_F32 / W8A8_DT_I8 / W8A8_DT_I32.
  *   - Row-major, densely packed tensors.  Rows that are 16-byte aligned
  *     take the vectorised kernels; anything else takes a slower generic path
- *     with identical results.
+ *     with identical results.  The matmuls have no such path: their operands,
+ *     results and per-channel vectors (scale, offset, bias, w_scale) must be
+ *     16-byte aligned (W8A8_ERR_ALIGN otherwise), a single value or a row
+ *     factor like its type.
  */
 #ifndef W8A8FFN_H
 #define W8A8FFN_H
