@@ -565,6 +565,9 @@ int add_rms_norm_dynamic_quant_beside(const void* x1, const void* x2, const void
 int dispatch_rows_local(const void* src, const float* src_scale, const int64_t* expanded_pos, void* dst, float* dst_scale,
                         int64_t T, int64_t topk, int64_t row_bytes, void* stream);
 
+// whether w8a8_ep_tables takes this many ranks and experts
+bool ep_tables_hold(int64_t P, int64_t E);
+
 inline bool is_aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 
 int sm_count();  // cached multiprocessor count of the current device

@@ -1532,6 +1532,8 @@ extern "C" int w8a8_moe_finalize_routing(const void* rows, const int32_t* src_to
     }
 }
 
+bool w8a8::ep_tables_hold(int64_t P, int64_t E) { return P <= EP_MAX_RANKS && E <= 1024 && P * E <= EP_MAX_CELLS; }
+
 extern "C" int w8a8_ep_tables(const int64_t* counts, int64_t P, int64_t E, int64_t rank, const uint64_t* peer_base,
                               uint64_t off_x, uint64_t off_s, uint64_t off_back, int64_t row_bytes,
                               int64_t back_row_bytes, int64_t cap_rows, uint64_t* row_dst, uint64_t* scale_dst,
@@ -1542,7 +1544,7 @@ extern "C" int w8a8_ep_tables(const int64_t* counts, int64_t P, int64_t E, int64
         cap_rows < 0) {
         return W8A8_ERR_INVALID;
     }
-    if (P > w8a8::EP_MAX_RANKS || E > 1024 || P * E > w8a8::EP_MAX_CELLS) {
+    if (!w8a8::ep_tables_hold(P, E)) {
         return W8A8_ERR_LIMIT;
     }
     if (counts == nullptr || peer_base == nullptr || row_dst == nullptr || scale_dst == nullptr ||

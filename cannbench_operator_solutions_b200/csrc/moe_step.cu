@@ -315,6 +315,9 @@ extern "C" int w8a8_moe_ffn_step(const W8A8MoeFfnStep* s, const void* x, const v
     if (T * topk > s->home_rows) {
         return W8A8_ERR_LIMIT;  // the return buffer holds home_rows rows
     }
+    if (!ep_tables_hold(P, E)) {
+        return W8A8_ERR_LIMIT;  // in every form of the step, whether it needs the tables or not
+    }
     const StepBuffers b = carve_step(s->workspace, T, topk, hidden, inter, E, P, cap);
     if (s->workspace == nullptr || s->workspace_bytes < b.total) {
         return W8A8_ERR_WORKSPACE;

@@ -468,7 +468,7 @@ int w8a8_gmsq_host_pipe_destroy(W8A8HostPipe* pipe);
  */
 typedef struct W8A8MoeFfnStep {
     int32_t world, rank;
-    int32_t num_experts; /* global; a multiple of world */
+    int32_t num_experts; /* global; a multiple of world; within w8a8_ep_tables' limits */
     int32_t topk;
     int32_t dtype;       /* W8A8_DT_F16 / W8A8_DT_BF16: x, residual, gamma, outputs */
     int32_t reserved;
