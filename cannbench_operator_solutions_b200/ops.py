@@ -11,6 +11,8 @@ native code (``csrc/plugin/py_calls.cpp``).
 """
 from __future__ import annotations
 
+import os
+import warnings
 from array import array
 from typing import List, Optional, Sequence, Tuple, Union
 
@@ -21,8 +23,12 @@ from . import _lib as L
 try:
     # the same functions in native code for calls in their plain form; None comes back from any other call
     from . import _calls
-except ImportError:  # not built yet, as while building
+except ImportError as error:
+    # not built yet, as while building - or built and of no use (another torch, no libw8a8ffn.so): not an error, since a
+    # build starts by importing this package
     _calls = None
+    if os.path.exists(os.path.join(L.PKG_DIR, "_calls.so")):
+        warnings.warn(f"_calls.so does not load, operator calls take about 8 us longer: {error}", RuntimeWarning)
 
 
 def _check(cond: bool, msg: str) -> None:
