@@ -75,3 +75,44 @@ def test_registers_of_the_unvectorised_combine(tmp_path):
                        r".*?Used (\d+) registers", log, flags=re.S)
     assert len(forms) == 4  # fp16 and bf16, 32- and 64-bit positions
     assert [f for f in forms if int(f[1]) > 0 or int(f[2]) > 80] == []
+
+
+def _bodies():
+    for path in FILES:
+        code = _code(path)
+        for m in re.finditer(r"__global__", code):
+            start = code.index("\n{", m.end())
+            yield re.search(r"(\w+_kernel)\s*\(", code[m.end():start]).group(1), code[start:code.index("\n}", start)]
+
+
+def test_kernels_beside_the_one_before_them_wait_at_their_end():
+    """Whoever waits for such a kernel has then waited for both; its reads are behind a fence, not behind a wait."""
+    code = _code(os.path.join(CSRC, "beside.cuh"))
+    steps = re.findall(r"griddepcontrol\.\w+|fence\.\w+\.\w+", code)
+    assert steps == ["griddepcontrol.launch_dependents", "fence.acq_rel.gpu", "griddepcontrol.wait"]
+    kernels = {name: body for name, body in _bodies() if "beside_previous()" in body}
+    assert sorted(kernels) == ["ardq_rows_kernel", "gemm_tc_kernel"]
+    for body in kernels.values():
+        assert body.count("beside_previous()") == body.count("previous_complete()") == 1
+        assert body.index("beside_previous()") < body.index("previous_complete()")
+
+
+def test_what_runs_before_a_kernel_beside_it_lets_it_in_after_its_own_wait():
+    """A kernel beside the one before it does not wait at its start: all that came before the two must be complete when it is
+    let in.  The route plan's last kernel in both of its forms, and the first of a grouped matmul's two launches."""
+    bodies = dict(_bodies())
+    assert "after_previous<false>()" in bodies["rp_rank_kernel"] and "after_previous()" not in bodies["rp_rank_kernel"]
+    plan = _code(os.path.join(CSRC, "ep.cu")).split("int w8a8_route_plan(")[1].split("\n}")[0]
+    forms = plan.split("RP_MAX_EXPERTS)")[1].split("return")[0].split("} else {")
+    assert [re.findall(r"(rp_\w+_kernel)", form)[-1] for form in forms] == ["rp_rank_kernel", "rp_rank_kernel"]
+    step = _code(os.path.join(CSRC, "moe_step.cu"))
+    assert re.findall(r"rc = (\w+)\(", step.split("int one_rank_step(")[1])[:3] == [
+        "w8a8_route_plan", "add_rms_norm_dynamic_quant_beside", "dispatch_rows_local"]
+    assert step.count("_beside(") == 1  # nobody else asks for it
+    # the matmul: FIRST waits, then lets the next in; SECOND is only ever launched behind FIRST
+    assert re.search(r"order == ORDER_FIRST_OF_TWO\) \{\s*after_previous<false>\(\);\s*\} else if \(p\.order == ORDER_SECOND_OF_TWO\)"
+                     r" \{\s*beside_previous\(\);", bodies["gemm_tc_kernel"])
+    run = _code(os.path.join(CSRC, "gemm.cu")).split("static int run_grouped(")[1].split("\n}")[0]
+    assert re.findall(r"ORDER_\w+", run) == ["ORDER_FIRST_OF_TWO", "ORDER_PLAIN", "ORDER_ALONE", "ORDER_SECOND_OF_TWO",
+                                             "ORDER_ALONE"]
+    assert run.count("overlap ? ORDER_") == 2
