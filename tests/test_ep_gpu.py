@@ -82,7 +82,9 @@ def test_single_gpu_chain_matches_oracle_chain(ops, oracle):
 
 def test_single_gpu_chain_peer_transport_equals_collective_transport(ops):
     """The fused transport (dispatch kernel and down-projection epilogue store rows at their final positions)
-    gives the same bits as pack / all-to-all / regroup; with one rank the 'peer' buffers are this GPU's own."""
+    gives the same bits as pack / all-to-all / regroup; with one rank the 'peer' buffers are this GPU's own.  (The C++
+    step of one rank with room for all pairs needs no tables and no addresses: test_moe_step_forms_gpu.py compares its
+    forms.)"""
     from test_ep_cpu import _problem
 
     from cannbench_operator_solutions_b200.ep import ExpertShard, MoeFfnChain
@@ -129,9 +131,9 @@ def test_single_gpu_chain_peer_transport_equals_collective_transport(ops):
 
 
 def test_native_step_captures_into_a_cuda_graph(ops):
-    """The C++ step enqueues everything on the caller's stream and on a second stream forked from and joined to it by
-    events, reads nothing back and allocates nothing: a stream capture follows both streams, and replaying the graph
-    after the inputs have been overwritten in place gives the result of an eager step on the new inputs."""
+    """The C++ step reads nothing back and allocates nothing, so a stream capture holds all of it (here one chain of kernels
+    on the caller's stream; test_moe_step_forms_gpu.py has the form with a second stream): replaying the graph after the
+    inputs have been overwritten in place gives the result of an eager step on the new inputs."""
     from test_ep_cpu import _problem
 
     from cannbench_operator_solutions_b200.ep import ExpertShard, MoeFfnChain
@@ -171,8 +173,8 @@ def test_native_step_captures_into_a_cuda_graph(ops):
 
 
 def test_chain_with_requantisation_inside_the_matmul_kernels(ops):
-    """The optional in-kernel requantisation of grouped_matmul_swiglu_quant on the chain's capacity-sized buffers (a
-    device group list that ends below the row capacity): same bits as the default two-kernel form."""
+    """The optional in-kernel requantisation of grouped_matmul_swiglu_quant in the chain, with a device group list: same bits
+    as the default two-kernel form."""
     from test_ep_cpu import _problem
 
     from cannbench_operator_solutions_b200 import _lib as L

@@ -1,5 +1,5 @@
 """Requantisation of SwiGLU activations with a row held by one CTA: row lengths around a warp's and a CTA's worth, one too long
-to be held, rows that hold infinities and NaN, against the definition."""
+to be held, one and several rows per CTA, rows that hold infinities and NaN, against the definition."""
 import array
 
 import pytest
@@ -10,11 +10,13 @@ from cannbench_operator_solutions_b200 import _lib as L
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("h", [16, 496, 512, 528, 2048, 2064, 16384, 16400])
-@pytest.mark.parametrize("rows", [1, 2500])
+LENGTHS = [16, 496, 512, 528, 2048, 2064, 16384, 16400]
+# more rows than CTAs (at most 32 per SM of one warp, 12 of four, one of 32): each takes several in turn
+SEVERAL_PER_CTA = [(64, 12000), (512, 9000), (2048, 5000), (2064, 4000), (16384, 1000), (16400, 500)]
+
+
+@pytest.mark.parametrize("h,rows", [(h, 1) for h in LENGTHS] + [(h, 2500 if h <= 528 else 37) for h in LENGTHS] + SEVERAL_PER_CTA)
 def test_matches_the_definition(h, rows):
-    if rows * h > 3_000_000:
-        rows = 37
     lib, st = L.load(), torch.cuda.current_stream().cuda_stream
     g = torch.Generator(device="cuda").manual_seed(h + rows)
     k, n = 16, 2 * h
@@ -37,7 +39,9 @@ def test_matches_the_definition(h, rows):
     first = need - tail - (rows * h * 4 + 255) // 256 * 256
     act = ws[first : first + rows * h * 4].view(torch.float32).view(rows, h)
     assert (act == 0).all()
-    act.copy_(torch.randn((rows, h), generator=g, device="cuda") * torch.logspace(-3, 3, rows, device="cuda").unsqueeze(1))
+    # in no order: a row whose maximum came from another row of its CTA could not pass
+    size_of_row = torch.logspace(-3, 3, rows, device="cuda")[torch.randperm(rows, generator=g, device="cuda")]
+    act.copy_(torch.randn((rows, h), generator=g, device="cuda") * size_of_row.unsqueeze(1))
     if rows > 1:
         act[0, 3], act[1, h - 1], act[2] = float("nan"), float("inf"), 0.0
     assert run(L.F_STAGE_REQUANT) == L.OK
