@@ -343,13 +343,10 @@ struct GroupEndsByValue {
     int32_t ends[PLAN_MAX_BY_VALUE];
 };
 
-constexpr int PLAN_BOTH = 3;  // host side only: PLAN_WHOLE at 256 rows and PLAN_LEFTOVER at 128 rows in one launch
-
 __device__ __forceinline__ void plan_groups_body(int64_t zero, const int64_t* dev_list,
                                                  const GroupEndsByValue& by_value, int use_by_value, int64_t E,
                                                  int64_t M, GroupedHeader* header, TileEntry* tiles,
-                                                 int64_t max_tiles, int tile_m, int mode, int32_t* shared_error,
-                                                 int allow_prefix)
+                                                 int64_t max_tiles, int tile_m, int mode, int allow_prefix)
 {
     extern __shared__ int32_t s_first[];  // first tile index of each group, E + 1 entries
     __shared__ int32_t s_warp_sum[8];
@@ -412,9 +409,6 @@ __device__ __forceinline__ void plan_groups_body(int64_t zero, const int64_t* de
         header->num_m_tiles = bad ? 0 : total;
         header->error = bad;
         header->rows_total = bad ? 0 : static_cast<int32_t>(end_of(E - 1));
-        if (bad && shared_error != nullptr) {
-            *shared_error = 1;  // the error word the caller reads lives in the first header
-        }
     }
     __syncthreads();
     if (bad) {
@@ -440,12 +434,11 @@ __device__ __forceinline__ void plan_groups_body(int64_t zero, const int64_t* de
 __global__ void __launch_bounds__(256) plan_groups_kernel(const int64_t* dev_list,
                                                           const GroupEndsByValue by_value, int use_by_value,
                                                           int64_t E, int64_t M, GroupedHeader* header,
-                                                          TileEntry* tiles, int64_t max_tiles, int tile_m, int mode,
-                                                          int32_t* shared_error, int allow_prefix)
+                                                          TileEntry* tiles, int64_t max_tiles, int tile_m,
+                                                          int allow_prefix)
 {
     const int64_t zero = after_previous();
-    plan_groups_body(zero, dev_list, by_value, use_by_value, E, M, header, tiles, max_tiles, tile_m, mode, shared_error,
-                     allow_prefix);
+    plan_groups_body(zero, dev_list, by_value, use_by_value, E, M, header, tiles, max_tiles, tile_m, PLAN_ALL, allow_prefix);
 }
 
 __global__ void __launch_bounds__(256) zero_words_kernel(uint4* __restrict__ words, int64_t count)
@@ -473,11 +466,11 @@ __global__ void __launch_bounds__(256) plan_groups_both_kernel(const int64_t* de
 {
     const int64_t zero = after_previous();
     if (blockIdx.x == 0) {
-        plan_groups_body(zero, dev_list, by_value, use_by_value, E, M, header, tiles, max_tiles, 256, PLAN_WHOLE, nullptr,
+        plan_groups_body(zero, dev_list, by_value, use_by_value, E, M, header, tiles, max_tiles, 256, PLAN_WHOLE,
                          allow_prefix);
     } else if (blockIdx.x == 1) {
         plan_groups_body(zero, dev_list, by_value, use_by_value, E, M, tail_header, tail_tiles, tail_max_tiles, 128,
-                         PLAN_LEFTOVER, nullptr, allow_prefix);
+                         PLAN_LEFTOVER, allow_prefix);
     } else {
         const int64_t stride = static_cast<int64_t>(gridDim.x - 2) * blockDim.x;
         for (int64_t i = static_cast<int64_t>(blockIdx.x - 2) * blockDim.x + threadIdx.x; i < clear16; i += stride) {
@@ -707,15 +700,11 @@ static int check_host_group_list(const int64_t* group_list, int list_on_device, 
     return (prev == M) ? W8A8_OK : W8A8_ERR_GROUP_LIST;
 }
 
-// returns W8A8_OK or an error; launches the planner on `st`
-static int plan_groups(const int64_t* group_list, int list_on_device, int64_t E, int64_t M,
-                       const GroupedWorkspace& g, int tile_m, cudaStream_t st, int mode = PLAN_ALL,
-                       void* clear = nullptr, size_t clear_bytes = 0)
+// returns W8A8_OK or an error; launches the planner on `st`: of one table with tiles of tile_m rows, or of `both` tables of
+// the two-launch form, which zeroes `clear` too
+static int plan_groups(const int64_t* group_list, int list_on_device, int64_t E, int64_t M, const GroupedWorkspace& g,
+                       cudaStream_t st, int tile_m, bool both = false, void* clear = nullptr, size_t clear_bytes = 0)
 {
-    GroupedHeader* header = (mode == PLAN_LEFTOVER) ? g.tail_header : g.header;
-    TileEntry* tiles = (mode == PLAN_LEFTOVER) ? g.tail_tiles : g.tiles;
-    const int64_t max_tiles = (mode == PLAN_LEFTOVER) ? g.tail_max_tiles : g.max_tiles;
-    int32_t* shared_error = (mode == PLAN_LEFTOVER) ? &g.header->error : nullptr;
     GroupEndsByValue bv;
     int use_bv = 0;
     const int64_t* dev_list = group_list;
@@ -746,15 +735,15 @@ static int plan_groups(const int64_t* group_list, int list_on_device, int64_t E,
         return W8A8_ERR_UNSUPPORTED;
     }
     cudaError_t e;
-    if (mode == PLAN_BOTH) {
+    if (both) {
         const int64_t clear16 = static_cast<int64_t>(clear_bytes / 16);
         const unsigned grid = 2 + (clear16 > 0 ? PLAN_CLEAR_CTAS : 0);
         e = launch_chained(plan_groups_both_kernel, grid, 256, smem, st, dev_list, bv, use_bv, E, M, g.header, g.tiles,
                            g.max_tiles, g.tail_header, g.tail_tiles, g.tail_max_tiles, list_on_device == 2 ? 1 : 0,
                            static_cast<uint4*>(clear), clear16);
     } else {
-        e = launch_chained(plan_groups_kernel, 1, 256, smem, st, dev_list, bv, use_bv, E, M, header, tiles, max_tiles,
-                           tile_m, mode, shared_error, list_on_device == 2 ? 1 : 0);
+        e = launch_chained(plan_groups_kernel, 1, 256, smem, st, dev_list, bv, use_bv, E, M, g.header, g.tiles, g.max_tiles,
+                           tile_m, list_on_device == 2 ? 1 : 0);
     }
     return launch_status(e);
 }
@@ -824,8 +813,8 @@ static int run_grouped(const int64_t* group_list, int list_on_device, int64_t E,
         }
     }
     if (E > GROUPS_IN_CTA) {
-        const int rc = hybrid ? plan_groups(group_list, list_on_device, E, M, g, 256, st, PLAN_BOTH, clear, clear_bytes)
-                              : plan_groups(group_list, list_on_device, E, M, g, 128 * shape, st);
+        const int rc = hybrid ? plan_groups(group_list, list_on_device, E, M, g, st, 256, true, clear, clear_bytes)
+                              : plan_groups(group_list, list_on_device, E, M, g, st, 128 * shape);
         if (rc != W8A8_OK) {
             return rc;
         }
@@ -1424,9 +1413,10 @@ extern "C" int w8a8_grouped_matmul_swiglu_quant_static(const int8_t* x, const in
     if (rc != W8A8_OK) {
         return rc;
     }
-    // From here on this is the ordinary operator with the built-in bytes as its workspace.  That path rewrites
-    // the header and tile table and zeroes the row maxima on the stream before it uses them, so whatever the
-    // previous call left behind is never read.
+    // From here on this is the ordinary operator with the built-in bytes as its workspace.  Whatever the call before left
+    // there is never read: the first matmul launch rewrites the header (the planner does, and the tile tables with it, for
+    // more than GROUPS_IN_CTA groups) once that call is complete, the matmuls write every activation that the
+    // requantisation reads, and row maxima and counters, where they are used, are zeroed first.
     return w8a8_grouped_matmul_swiglu_quant(x, w, w_scale, x_scale, y, y_scale, M, K, N, E, group_list, list_on_device,
                                             w_layout, flags, scratch, static_cast<size_t>(W8A8_STATIC_SCRATCH_BYTES),
                                             stream);

@@ -4,8 +4,8 @@
 // kernel takes.  Each function here does the same for the form in which such calls come - dense CUDA tensors of the
 // accepted types on the current device, shapes in order, no tensor subclass or mode that wants to see the call - with the
 // same outputs through the same C-ABI call.  Anything else returns None, and ops.py goes on with its own code, which
-// copies, switches devices or raises as ever.  So the rules are not repeated here: a call that this file takes is one that
-// would have passed all of them.
+// copies, switches devices or raises as ever.  So no message is repeated here, but the rules are: a call that this file
+// takes must be one that passes all of ops.py's checks, and a check that is added there is added here.
 #include <ATen/ATen.h>
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/cuda/CUDAContext.h>
