@@ -1300,12 +1300,14 @@ struct MfrShape {
 // 160), or, where 256 are not enough and `may_split`, on several (one sum of eight rows of 6256 16-bit elements 6.6 ->
 // 2.7 us, 64 of eight of 4096 4.25 -> 2.97, 653 of four of 1072 4.55 -> 3.47, in a row of calls).  Others run on 96,
 // 128 or 160 threads - the fewest that leave no more than 6 % more of their passes over a row empty than the best of
-// the three - and 3072 threads per SM in all: 256 left most of a last pass empty (a row of 2176 elements is 272 chunks)
-// and let all of them wait for a row's look-up at once (16000 sums of four of 2176 122.7 -> 91.7 us, 23000 of two of
-// 1184 90.4 -> 68.4, 3761 of eight of 4432 64.8 -> 56.1, 8192 of eight of 7168 193 -> 189).  256 threads and 8 CTAs per
-// SM, as it was for all rows, stay where their passes are as full (50000 rows of 6144 regrouped, then summed by eights:
-// 232 us, 237 on 96), where the rows are too few to fill half of the smaller CTAs' places (470 sums of eight of 4432
-// after their regrouping 22.7 us, 31 on 96), and for rows that are read an element at a time.  The split is a form of
+// the three: 256 left most of a last pass empty (a row of 2176 elements is 272 chunks) and let all of them wait for a
+// row's look-up at once (16000 sums of four of 2176 122.7 -> 91.7 us, 23000 of two of 1184 90.4 -> 68.4, 3761 of eight of
+// 4432 64.8 -> 56.1, 8192 of eight of 7168 193 -> 189).  Their grid ends at 3072 threads per SM, more than twice what its
+// registers hold at once: CTAs that start as others end even out what rows cost (16000 of four of 2176 62 us, 64 with 2048
+// and 83 with 1280 threads, what is resident; 60000 of two of 1024 98, 99, 136).  256 threads and 8 CTAs per SM, as it was
+// for all rows, stay where their passes are as full (50000 rows of 6144 regrouped, then summed by eights: 232 us, 237 on
+// 96), where there are fewer rows than half of that grid (470 sums of eight of 4432 after their regrouping 22.7 us, 31 on
+// 96), and for rows that are read an element at a time.  The split is a form of
 // its own: in every kernel it cost 8 % (59463 rows of 2176 regrouped, summed by fours: 119 us, 129).
 static MfrShape mfr_shape(int64_t rows, int64_t chunks, int64_t K, bool vec, bool may_split)
 {
@@ -1331,11 +1333,11 @@ static MfrShape mfr_shape(int64_t rows, int64_t chunks, int64_t K, bool vec, boo
             threads = t;
         }
     }
-    const int64_t places = sms * (3072 / threads);
-    if (used(256) >= best || rows < places / 2) {
+    const int64_t most = sms * (3072 / threads);
+    if (used(256) >= best || rows < most / 2) {
         return {dim3(few), 256};
     }
-    return {dim3(static_cast<unsigned>(std::min<int64_t>(rows, places))), static_cast<unsigned>(threads)};
+    return {dim3(static_cast<unsigned>(std::min<int64_t>(rows, most))), static_cast<unsigned>(threads)};
 }
 
 }  // namespace w8a8
