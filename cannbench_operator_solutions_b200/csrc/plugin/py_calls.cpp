@@ -424,6 +424,11 @@ PyObject* moe_finalize_routing(PyObject*, PyObject* const* a, Py_ssize_t)
         Py_RETURN_NONE;
     }
     const int64_t num_rows = index->numel() / k;
+    const auto too_few = [](const Tensor* t, int64_t elements) { return t != nullptr && t->numel() < elements; };
+    if (too_few(skip1, num_rows * h) || too_few(skip2, num_rows * h) || too_few(scales, index->numel()) ||
+        (has_bias && too_few(expert, index->numel()))) {
+        Py_RETURN_NONE;
+    }
     Tensor result;
     int status;
     {

@@ -446,13 +446,17 @@ def moe_finalize_routing(expanded_permuted_rows: torch.Tensor, expanded_src_to_d
     _check(k > 0, "moe_finalize_routing: K must be positive.")
     _check(nk % k == 0, "moe_finalize_routing: expanded_src_to_dst_row length must be K*NUM_ROWS.")
     num_rows = nk // k
+    # what the kernel reads of each, whatever its shape
+    has_bias = bias is not None and expert_for_source_row is not None
+    for name, t, elements in (("skip1", skip1, num_rows * h), ("skip2", skip2, num_rows * h), ("scales", scales, nk),
+                              ("expert_for_source_row", expert_for_source_row if has_bias else None, nk)):
+        _check(t is None or t.numel() >= elements, f"moe_finalize_routing: {name} has too few elements.")
     _need_cuda(epr, expanded_src_to_dst_row, skip1, skip2, bias, scales, expert_for_source_row)
     out = torch.empty((num_rows, h), dtype=epr.dtype, device=epr.device)
     if num_rows <= 0 or h <= 0:
         return out
     eprc = epr.contiguous()
     esdr = expanded_src_to_dst_row.contiguous()
-    has_bias = bias is not None and expert_for_source_row is not None
     if has_bias:
         _check(bias.size(1) == h, "moe_finalize_routing: bias head dim must equal H.")
     for name, t in (("skip1", skip1), ("skip2", skip2), ("bias", bias if has_bias else None)):
